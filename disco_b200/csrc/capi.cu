@@ -7,6 +7,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -14,6 +15,7 @@
 
 #include "common.cuh"
 #include "field.cuh"
+#include "tree.cuh"
 
 namespace disco {
 int choose_split(int64_t n, int nimg, int resident_ctas);
@@ -37,6 +39,12 @@ struct disco_plan {
     int32_t near_cap = 0;
     std::vector<double> loop_evals;          // per input loop: segments or loopons
     disco_plan_stats stats;
+    // the sum by cells: its shape for the last atom count, and whether this
+    // plan holds the device's scratch pool (both set by execute)
+    std::mutex tree_mutex;
+    int64_t tree_n = -1;
+    disco::TreeShape tree;
+    bool tree_pool = false;
 };
 
 namespace {
@@ -95,7 +103,32 @@ void free_plan(disco_plan* p)
     if (p->d_status) cudaFree(p->d_status);
     if (p->d_near) cudaFree(p->d_near);
     if (p->d_near_count) cudaFree(p->d_near_count);
+    if (p->tree_pool) disco::tree_pool_release(p->device);
     delete p;
+}
+
+// The shape of the sum by cells for n atoms; use = false: sum directly.  A
+// caller's own image split names the direct kernel, a stream under capture
+// keeps to it (its launches allocate nothing), and so does a sum over far
+// shells alone (image_min > 0): that is the term-by-term sum the learned form
+// is measured and tested against, in error and in time.
+disco::TreeShape plan_tree(disco_plan* p, int64_t n, cudaStream_t s)
+{
+    disco::TreeShape none;
+    if (!p->tables[0].aux_tree || p->opt.image_split != 0 || p->opt.image_min > 0) return none;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &cap) != cudaSuccess) { cudaGetLastError(); return none; }
+    if (cap != cudaStreamCaptureStatusNone) return none;
+    std::lock_guard<std::mutex> lock(p->tree_mutex);
+    if (p->tree_n != n) {
+        p->tree = disco::tree_shape(p->tables[0], n, p->box, p->opt.images);
+        p->tree_n = n;
+    }
+    if (p->tree.use && !p->tree_pool) {
+        disco::tree_pool_retain(p->device);
+        p->tree_pool = true;
+    }
+    return p->tree;
 }
 
 double now_s()
@@ -203,6 +236,7 @@ int disco_b200_plan_create(const disco_loop* loops, int32_t nloops, const double
                  ? disco::build_table_fp32(loops, nloops, kind, o.nu, p->tables[k], err, cap)
                  : disco::build_table(loops, nloops, kind, o.precision, o.nu, p->tables[k], err, cap);
         if (st) { free_plan(p); return fail(st, err); }
+        if (k == 0) disco::append_tree_pieces(p->tables[k]);
         const disco::HostTable& T = p->tables[k];
         for (int l = 0; l < nloops; ++l) p->loop_evals[l] += T.loop_evals[l];
         p->stats.n_segments += T.n_segments;
@@ -279,6 +313,15 @@ int disco_b200_plan_execute(disco_plan* p, const disco_atoms* a, void* stream)
         }
         std::string err;
         const int kind = k == 0 ? disco::kLineKind : disco::kLooponKind;
+        if (k == 0) {
+            const disco::TreeShape shape = plan_tree(p, a->n, s);
+            if (shape.use) {
+                bool ran = false;
+                const int st = disco::launch_tree(fa, T, shape, p->box, p->sm_count, s, &ran, err);
+                if (st) return fail(st, err);
+                if (ran) continue;
+            }
+        }
         const int st = T.fp32
             ? disco::launch_field_fp32(fa, kind, p->sm_count, p->opt.image_split, s, err)
             : disco::launch_field(fa, kind, false, p->sm_count, p->opt.threads_per_block,

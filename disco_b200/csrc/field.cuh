@@ -158,6 +158,11 @@ struct HostTable {
     uint64_t aux_pieces = 0, aux_segs = 0;
     // line tables: byte offset of the raw vertex triplets (0 when absent)
     uint64_t aux_raw = 0;
+    // line tables of a plan: byte offset of the tree pieces (tree.cuh; 0 when
+    // absent), and their radii and segment counts for the choice of cells
+    uint64_t aux_tree = 0;
+    std::vector<double> tree_rho;
+    std::vector<int32_t> tree_terms;
 };
 
 // Appends a line table's raw vertex triplets after its chunks (sets aux_raw).

@@ -199,14 +199,17 @@ static __device__ __noinline__ double fan_solid_angle_ref(const double* __restri
 // since on the plane the running product's sign is a rounding residue of
 // other operations than the reference's.  Outside the band the product's
 // argument is at least about pi hband / rho away from the branch cut, far
-// above its rounding.
+// above its rounding.  kFar: P is further from the apex than rho (a node of a
+// cell that sums the piece from afar), where |Omega| stays well below 2 pi and
+// no side has to be chosen.
+template <bool kFar = false>
 __device__ __forceinline__ void line_piece_fp64(const LinePiece& pc, const LineSeg* seg,
                                                 double Px, double Py, double Pz, double cJK,
                                                 double& ux, double& uy, double& uz, bool& plane)
 {
     // unit vector from P to the fan apex
     const double rx = pc.cx - Px, ry = pc.cy - Py, rz = pc.cz - Pz;
-    const bool on_plane = fabs(pc.nx * rx + pc.ny * ry + pc.nz * rz) <= pc.hband;
+    const bool on_plane = !kFar && fabs(pc.nx * rx + pc.ny * ry + pc.nz * rz) <= pc.hband;
     const double l1sq = rx * rx + ry * ry + rz * rz;
     const double il1 = rsqrt_nr(l1sq);
     const double ex = rx * il1, ey = ry * il1, ez = rz * il1;

@@ -1,0 +1,1346 @@
+// The sum over loops and images by cells (line method).
+//
+// Away from a loop its displacement is smooth, and nearly all of the sum's
+// (piece, image) pairs are far from any given atom.  So the atoms' bounding
+// box is cut into cells, level by level; a pair that is far from a cell (but
+// was not far from the cell around it on the level before) is evaluated, by
+// the same closed form in FP64, at the q^3 Chebyshev points of that cell
+// instead of at every atom in it.  The values are interpolated from each level
+// to the next, last to small cells whose Chebyshev coefficients every atom
+// evaluates once.  What is far from no cell around the atom is summed at the
+// atom itself, exactly as the plain kernels do it.
+//
+// "Far" is per axis: |cell centre - piece centre - image shift| >
+// theta(q) h + rho along some axis, with h the cell's half width (the largest
+// over the axes) and rho the radius of the ball around the piece's apex that
+// holds its vertices.  The near images of a piece are then a box of indices,
+// (2I + 1)^3 cut by three intervals, and a cell's table holds one packed box
+// per piece.  The boxes are nested by intersection (cell in cell), so every
+// (atom, piece, image) enters exactly once, on whatever level.
+//
+// theta(q): interpolation at q Chebyshev points converges like the Bernstein
+// ellipse's parameter to the power -q, and theta is where the measured worst
+// error over loops of 25 and 40 A radius, directions and cells of 12 to 30 A
+// half width falls below 4e-15 A for |b| = 2.5 A (plus 3 to 10 %), under the
+// rounding of the direct sum (1e-14 A).
+//
+// FP64 line tables only: the FP32 compensated form's own rounding (1e-6 A) is
+// part of what it returns, and its far terms summed in FP64 would change it.
+//
+// Measured against the plain kernel on one B200 (ms a call): FCC 100^3 cells
+// (4.0 M atoms), 16 loops, +-2 images 986 -> 15.3; BCC 61 x 47 x 33 (184 k
+// atoms), 9 loops, +-3 86.9 -> 9.5; BCC 40^3 (128 k), 4 loops of 64 segments,
+// +-1 4.94 -> 3.34.  A sum too small to gain (2 000 atoms, 2 loops: 0.02 ms of
+// terms) stays with the plain kernel: tree_shape compares operation counts of
+// both, launches included.
+//
+// Every result is a fixed sequence of operations per atom (its cell's nodes,
+// then its near pairs in piece order), so it does not depend on the order of
+// the atoms or of the blocks.
+#include <algorithm>
+#include <cmath>
+#include <cstring>
+#include <mutex>
+#include <string>
+#include <vector>
+
+#include "common.cuh"
+#include "field.cuh"
+#include "field_device.cuh"
+#include "tree.cuh"
+
+namespace disco {
+
+namespace {
+
+// ---- orders ----------------------------------------------------------------------------
+
+constexpr int kOrders = 9;
+constexpr int kOrderQ[kOrders] = { 9, 10, 11, 12, 13, 15, 17, 19, 21 };
+constexpr double kOrderTheta[kOrders] = { 18.0, 13.2, 10.2, 8.2, 6.9, 5.1, 4.15, 3.55, 3.1 };
+constexpr int kMaxFinalQ = 13;                 // the atoms' cells hold three components in shared memory
+constexpr int kWarps = 4;                      // warps per CTA of the tile kernels
+constexpr int kMaxCells = 1 << 18;
+constexpr double kClip = 2.0;                  // atoms within +-2 box lengths are sorted into cells
+
+__host__ __device__ constexpr int padded(int q) { return (q + 1) & ~1; }
+
+// ---- device arguments ------------------------------------------------------------------
+
+struct LevelArgs {
+    int32_t m[3];
+    int32_t q, q3, split;
+    int32_t r[3];             // cells per axis of this level in a cell of the level before
+    int32_t tiles;            // warp tiles per cell
+    int64_t tile0;            // first warp tile of the level
+    int64_t cell0;            // first cell of the level (tables, occupancy)
+    double theta;
+    double* val;              // [cell][3][q3]
+};
+
+struct TreeArgs {
+    FieldArgs f;
+    const TreePiece* pieces;
+    int32_t np;
+    int32_t levels;
+    LevelArgs lv[TreeShape::kMaxLevels];
+    int32_t mf[3], qf;        // final cells
+    int32_t rf[3];            // final cells per axis in a cell of the last level
+    int32_t cells_s, cells_f; // cells of the last level, final cells
+    int32_t near_split;
+    int32_t images;
+    int64_t level_cells;      // cells over all levels
+    unsigned long long* box;  // 6: ordered bits of min x, y, z and max x, y, z
+    uint64_t* near;           // [level cell][piece]: packed box of near images
+    uint8_t* occ;             // [level cell]: holds atoms
+    uint32_t* key[2];         // [atom], [slot]: final cell, the sort's two buffers
+    int32_t* idx[2];          // the atoms that go with them
+    uint32_t* digits;         // [256][sort tile]
+    uint32_t* digit_total;    // [256]
+    int32_t sort_tiles;
+    uint32_t* start;          // [final cell + 2]: first sorted slot
+    uint32_t* near_tile;      // [last-level cell + 2]: first warp tile of the near pass
+    const int32_t* perm;      // sorted slot -> atom
+    double* mat;              // interpolation matrices, transition by transition
+    int32_t mat_off[TreeShape::kMaxLevels + 1][3];
+};
+
+// Order-preserving bits of a double.
+__device__ __forceinline__ unsigned long long ord_bits(double v)
+{
+    const unsigned long long b = (unsigned long long)__double_as_longlong(v);
+    return (b >> 63) ? ~b : (b | 0x8000000000000000ull);
+}
+__device__ __forceinline__ double ord_value(unsigned long long k)
+{
+    return __longlong_as_double((long long)((k >> 63) ? (k & 0x7FFFFFFFFFFFFFFFull) : ~k));
+}
+
+// An atom that is sorted into a cell (a NaN or a far outlier is not: it takes
+// every pair itself).
+__device__ __forceinline__ bool sorted_in(const FieldArgs& f, double x, double y, double z)
+{
+    return fabs(x) <= kClip * f.Lx && fabs(y) <= kClip * f.Ly && fabs(z) <= kClip * f.Lz;
+}
+
+struct Geo {
+    double lo[3], ext[3];
+};
+
+// The cells' grid: the bounding box of the sorted atoms, no axis thinner than
+// a thousandth of the longest.
+__device__ __forceinline__ Geo load_geo(const TreeArgs& a)
+{
+    Geo g;
+    double hi[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        g.lo[d] = ord_value(a.box[d]);
+        hi[d] = ord_value(a.box[3 + d]);
+    }
+    if (!(g.lo[0] <= hi[0])) {                       // no sorted atom
+#pragma unroll
+        for (int d = 0; d < 3; ++d) { g.lo[d] = 0.0; g.ext[d] = 1.0; }
+        return g;
+    }
+    double big = 0.0;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) big = fmax(big, hi[d] - g.lo[d]);
+    const double least = fmax(1e-3 * big, 1e-6);
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        const double e = hi[d] - g.lo[d];
+        if (e < least) g.lo[d] -= 0.5 * (least - e);
+        g.ext[d] = fmax(e, least);
+    }
+    return g;
+}
+
+// Final-cell coordinates of a sorted atom.
+__device__ __forceinline__ void final_coord(const TreeArgs& a, const Geo& g, double x, double y, double z, int (&c)[3])
+{
+    const double p[3] = { x, y, z };
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        const int i = (int)((p[d] - g.lo[d]) * ((double)a.mf[d] / g.ext[d]));
+        c[d] = min(max(i, 0), a.mf[d] - 1);
+    }
+}
+
+// Index of a final cell: the cell of the last level first, so that each of
+// those owns a contiguous run of final cells (and of sorted slots).
+__device__ __forceinline__ int last_index(const TreeArgs& a, const int (&c)[3])
+{
+    const LevelArgs& L = a.lv[a.levels - 1];
+    return ((c[0] / a.rf[0]) * L.m[1] + c[1] / a.rf[1]) * L.m[2] + c[2] / a.rf[2];
+}
+__device__ __forceinline__ int final_index(const TreeArgs& a, const int (&c)[3])
+{
+    const int sub = ((c[0] % a.rf[0]) * a.rf[1] + c[1] % a.rf[1]) * a.rf[2] + c[2] % a.rf[2];
+    return last_index(a, c) * (a.rf[0] * a.rf[1] * a.rf[2]) + sub;
+}
+__device__ __forceinline__ int cell_of(const TreeArgs& a, const Geo& g, double x, double y, double z)
+{
+    if (!sorted_in(a.f, x, y, z)) return a.cells_f;
+    int c[3];
+    final_coord(a, g, x, y, z, c);
+    return final_index(a, c);
+}
+
+// ---- sorting ----------------------------------------------------------------------------
+
+__global__ void __launch_bounds__(256) tree_box_kernel(const TreeArgs a)
+{
+    unsigned long long k[6] = { ~0ull, ~0ull, ~0ull, 0ull, 0ull, 0ull };
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < a.f.n; i += (int64_t)gridDim.x * blockDim.x) {
+        const double p[3] = { a.f.x[i], a.f.y[i], a.f.z[i] };
+        if (!sorted_in(a.f, p[0], p[1], p[2])) continue;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            const unsigned long long b = ord_bits(p[d]);
+            k[d] = min(k[d], b);
+            k[3 + d] = max(k[3 + d], b);
+        }
+    }
+#pragma unroll
+    for (int d = 0; d < 6; ++d)
+        for (int o = 16; o > 0; o >>= 1) {
+            const unsigned long long t = __shfl_xor_sync(0xffffffffu, k[d], o);
+            k[d] = d < 3 ? min(k[d], t) : max(k[d], t);
+        }
+    __shared__ unsigned long long part[8][6];
+    if ((threadIdx.x & 31) == 0)
+        for (int d = 0; d < 6; ++d) part[threadIdx.x >> 5][d] = k[d];
+    __syncthreads();
+    if (threadIdx.x < 6) {
+        const int d = threadIdx.x;
+        unsigned long long v = part[0][d];
+        for (int w = 1; w < 8; ++w) v = d < 3 ? min(v, part[w][d]) : max(v, part[w][d]);
+        if (d < 3) atomicMin(&a.box[d], v); else atomicMax(&a.box[d], v);
+    }
+}
+
+__global__ void tree_init_kernel(const TreeArgs a)
+{
+    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
+    if (t < 6) a.box[t] = t < 3 ? ~0ull : 0ull;
+    for (int64_t i = t; i < a.level_cells; i += step) a.occ[i] = 0;
+}
+
+// Stable radix sort of the atoms by final cell, 8 bits a pass: which atoms
+// share a warp decides the series that a piece takes there, so the order
+// within a cell is fixed (ascending atoms) to keep results reproducible.
+// Tiles of 2048 atoms; warp w of a tile owns 256 consecutive ones.
+constexpr int kSortThreads = 256, kSortItems = 8, kSortTile = kSortThreads * kSortItems;
+
+template <bool kFirst>
+__global__ void __launch_bounds__(kSortThreads) tree_digits_kernel(const TreeArgs a, const uint32_t* key_in, int shift)
+{
+    __shared__ uint32_t hist[256];
+    hist[threadIdx.x] = 0;
+    __syncthreads();
+    Geo g;
+    if (kFirst) g = load_geo(a);
+    const int64_t base = (int64_t)blockIdx.x * kSortTile;
+    for (int r = 0; r < kSortItems; ++r) {
+        const int64_t i = base + r * kSortThreads + threadIdx.x;
+        if (i >= a.f.n) break;
+        uint32_t key;
+        if (kFirst) {
+            key = (uint32_t)cell_of(a, g, a.f.x[i], a.f.y[i], a.f.z[i]);
+            a.key[0][i] = key;
+        } else {
+            key = key_in[i];
+        }
+        atomicAdd(&hist[(key >> shift) & 255u], 1u);
+    }
+    __syncthreads();
+    a.digits[(int64_t)threadIdx.x * a.sort_tiles + blockIdx.x] = hist[threadIdx.x];
+}
+
+// One CTA per digit: exclusive sums over its tiles, the total behind them.
+__global__ void __launch_bounds__(256) tree_digit_scan_kernel(const TreeArgs a);
+
+template <bool kFirst>
+__global__ void __launch_bounds__(kSortThreads) tree_reorder_kernel(const TreeArgs a, const uint32_t* key_in,
+                                                                    const int32_t* idx_in, uint32_t* key_out,
+                                                                    int32_t* idx_out, int shift);
+
+// Exclusive scan over one CTA of v per thread; *total = the sum.
+__device__ __forceinline__ uint32_t block_scan(uint32_t v, uint32_t* total)
+{
+    __shared__ uint32_t warp_sum[32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    uint32_t inc = v;
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t t = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += t;
+    }
+    if (lane == 31) warp_sum[w] = inc;
+    __syncthreads();
+    if (w == 0) {
+        uint32_t s = lane < (int)(blockDim.x >> 5) ? warp_sum[lane] : 0;
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t t = __shfl_up_sync(0xffffffffu, s, o);
+            if (lane >= o) s += t;
+        }
+        warp_sum[lane] = s;
+    }
+    __syncthreads();
+    const uint32_t base = w ? warp_sum[w - 1] : 0;
+    *total = warp_sum[(blockDim.x >> 5) - 1];
+    __syncthreads();
+    return base + inc - v;
+}
+
+__global__ void __launch_bounds__(256) tree_digit_scan_kernel(const TreeArgs a)
+{
+    uint32_t* row = a.digits + (int64_t)blockIdx.x * a.sort_tiles;
+    uint32_t carry = 0;
+    for (int t0 = 0; t0 < a.sort_tiles; t0 += 256) {
+        const int t = t0 + threadIdx.x;
+        const uint32_t v = t < a.sort_tiles ? row[t] : 0u;
+        uint32_t tot;
+        const uint32_t ex = block_scan(v, &tot);
+        if (t < a.sort_tiles) row[t] = carry + ex;
+        carry += tot;
+    }
+    if (threadIdx.x == 0) a.digit_total[blockIdx.x] = carry;
+}
+
+template <bool kFirst>
+__global__ void __launch_bounds__(kSortThreads) tree_reorder_kernel(const TreeArgs a, const uint32_t* key_in,
+                                                                    const int32_t* idx_in, uint32_t* key_out,
+                                                                    int32_t* idx_out, int shift)
+{
+    __shared__ uint32_t at[kSortThreads / 32][256];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    for (int e = threadIdx.x; e < 256 * (kSortThreads / 32); e += kSortThreads) at[e >> 8][e & 255] = 0;
+    uint32_t tot;
+    const uint32_t digit_base = block_scan(a.digit_total[threadIdx.x], &tot);   // its barriers cover the clearing
+    const int64_t base = (int64_t)blockIdx.x * kSortTile + w * (32 * kSortItems);
+    uint32_t key[kSortItems], rank[kSortItems];
+#pragma unroll
+    for (int r = 0; r < kSortItems; ++r) {
+        const int64_t i = base + r * 32 + lane;
+        const bool valid = i < a.f.n;
+        key[r] = valid ? key_in[i] : 0u;
+        const uint32_t d = valid ? (key[r] >> shift) & 255u : 256u + lane;
+        const unsigned peers = __match_any_sync(0xffffffffu, d);
+        uint32_t before = 0;
+        if (valid) before = at[w][d];
+        __syncwarp();
+        if (valid && lane == __ffs(peers) - 1) at[w][d] = before + (uint32_t)__popc(peers);
+        __syncwarp();
+        rank[r] = before + (uint32_t)__popc(peers & ((1u << lane) - 1u));
+    }
+    __syncthreads();
+    uint32_t sum = digit_base + a.digits[(int64_t)threadIdx.x * a.sort_tiles + blockIdx.x];
+#pragma unroll
+    for (int k = 0; k < kSortThreads / 32; ++k) {
+        const uint32_t c = at[k][threadIdx.x];
+        at[k][threadIdx.x] = sum;
+        sum += c;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < kSortItems; ++r) {
+        const int64_t i = base + r * 32 + lane;
+        if (i >= a.f.n) break;
+        const uint32_t slot = at[w][(key[r] >> shift) & 255u] + rank[r];
+        key_out[slot] = key[r];
+        idx_out[slot] = kFirst ? (int32_t)i : idx_in[i];
+    }
+}
+
+// First sorted slot of every final cell (and of the atoms outside the grid,
+// one more cell at the end).
+__global__ void __launch_bounds__(256) tree_starts_kernel(const TreeArgs a, const uint32_t* key)
+{
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i <= a.f.n; i += (int64_t)gridDim.x * blockDim.x) {
+        const int lo = i == 0 ? -1 : (int)key[i - 1], hi = i == a.f.n ? a.cells_f + 1 : (int)key[i];
+        for (int c = lo + 1; c <= hi; ++c) a.start[c] = (uint32_t)i;
+    }
+}
+
+// Warp tiles of the near pass, by the last level's cells (plus the outside
+// cell), and which cells of each level hold atoms; one CTA.
+__global__ void __launch_bounds__(1024) tree_scan_kernel(const TreeArgs a)
+{
+    const int nf = a.cells_f + 1;
+    const int rr = a.rf[0] * a.rf[1] * a.rf[2];
+    const int ns = a.cells_s + 1, per = (ns + 1023) / 1024;
+    const int s0 = min(ns, (int)threadIdx.x * per), s1 = min(ns, s0 + per);
+    const uint32_t per_tile = 32u / (uint32_t)a.near_split;
+    const LevelArgs& E = a.lv[a.levels - 1];
+    auto atoms_of = [&](int s) { return a.start[s < a.cells_s ? (s + 1) * rr : nf] - a.start[s * rr]; };
+    uint32_t mine = 0, tot;
+    for (int s = s0; s < s1; ++s) {
+        const uint32_t k = atoms_of(s);
+        mine += (k + per_tile - 1) / per_tile;
+        if (k == 0 || s == a.cells_s) continue;
+        const int c[3] = { s / (E.m[1] * E.m[2]), s / E.m[2] % E.m[1], s % E.m[2] };
+        for (int l = 0; l < a.levels; ++l) {
+            const LevelArgs& L = a.lv[l];
+            const int lc = ((c[0] / (E.m[0] / L.m[0])) * L.m[1] + c[1] / (E.m[1] / L.m[1])) * L.m[2] +
+                           c[2] / (E.m[2] / L.m[2]);
+            a.occ[L.cell0 + lc] = 1;
+        }
+    }
+    uint32_t at = block_scan(mine, &tot);
+    if (threadIdx.x == 0) a.near_tile[ns] = tot;
+    for (int s = s0; s < s1; ++s) {
+        a.near_tile[s] = at;
+        at += (atoms_of(s) + per_tile - 1) / per_tile;
+    }
+}
+
+// ---- near boxes --------------------------------------------------------------------------
+
+// Packed box of image indices: lo and hi per axis, offset by 16, one byte
+// each; an empty box is 0.
+__host__ __device__ __forceinline__ uint64_t full_box(int images)
+{
+    uint64_t w = 0;
+    for (int d = 0; d < 3; ++d) {
+        w |= (uint64_t)(uint8_t)(16 - images) << (16 * d);
+        w |= (uint64_t)(uint8_t)(16 + images) << (16 * d + 8);
+    }
+    return w;
+}
+struct ImgBox {
+    int lo[3], n[3];
+    __device__ __forceinline__ explicit ImgBox(uint64_t w)
+    {
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            lo[d] = (int)((w >> (16 * d)) & 0xFF) - 16;
+            n[d] = (int)((w >> (16 * d + 8)) & 0xFF) - 16 - lo[d] + 1;
+        }
+    }
+    __device__ __forceinline__ int count() const { return n[0] * n[1] * n[2]; }
+    __device__ __forceinline__ void at(int idx, int& i, int& j, int& k) const
+    {
+        const int yz = n[1] * n[2];
+        const int qi = idx / yz, r = idx - qi * yz;
+        const int qj = r / n[2];
+        i = lo[0] + qi;
+        j = lo[1] + qj;
+        k = lo[2] + (r - qj * n[2]);
+    }
+};
+
+// The images of a box U outside a box O inside it (O may be empty), counted and
+// numbered: the planes of U before and after O along x, then along y within
+// O's x range, then along z.
+struct ImgShell {
+    ImgBox U, O;
+    int a0, a1, b0, b1, c0, total;      // ends of the x-, x+, y-, y+ and z- parts
+    bool whole;
+    __device__ __forceinline__ ImgShell(uint64_t u, uint64_t o) : U(u), O(o == 0 ? u : o), whole(o == 0)
+    {
+        const int yz = U.n[1] * U.n[2];
+        if (whole) { a0 = a1 = b0 = b1 = c0 = total = U.count(); return; }
+        a0 = (O.lo[0] - U.lo[0]) * yz;
+        a1 = a0 + (U.lo[0] + U.n[0] - O.lo[0] - O.n[0]) * yz;
+        b0 = a1 + O.n[0] * (O.lo[1] - U.lo[1]) * U.n[2];
+        b1 = b0 + O.n[0] * (U.lo[1] + U.n[1] - O.lo[1] - O.n[1]) * U.n[2];
+        c0 = b1 + O.n[0] * O.n[1] * (O.lo[2] - U.lo[2]);
+        total = c0 + O.n[0] * O.n[1] * (U.lo[2] + U.n[2] - O.lo[2] - O.n[2]);
+    }
+    __device__ __forceinline__ void at(int idx, int& i, int& j, int& k) const
+    {
+        int x = U.lo[0], y = U.lo[1], z = U.lo[2], ny = U.n[1], nz = U.n[2];
+        if (idx >= a0) {
+            if (idx < a1) { idx -= a0; x = O.lo[0] + O.n[0]; }
+            else {
+                x = O.lo[0];
+                if (idx < b0) { idx -= a1; ny = O.lo[1] - U.lo[1]; }
+                else if (idx < b1) { idx -= b0; y = O.lo[1] + O.n[1]; ny = U.lo[1] + U.n[1] - y; }
+                else {
+                    y = O.lo[1];
+                    ny = O.n[1];
+                    if (idx < c0) { idx -= b1; nz = O.lo[2] - U.lo[2]; }
+                    else { idx -= c0; z = O.lo[2] + O.n[2]; nz = U.lo[2] + U.n[2] - z; }
+                }
+            }
+        }
+        const int yz = ny * nz, q = idx / yz, r = idx - q * yz, p = r / nz;
+        i = x + q;
+        j = y + p;
+        k = z + (r - p * nz);
+    }
+};
+
+// One thread per (level cell, piece): the intersection of the near boxes of
+// the cell and of the cells around it on the levels before.
+__global__ void __launch_bounds__(256) tree_near_kernel(const TreeArgs a)
+{
+    const Geo g = load_geo(a);
+    const double L[3] = { a.f.Lx, a.f.Ly, a.f.Lz };
+    const int64_t total = a.level_cells * a.np;
+    for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t lc = t / a.np;
+        const int p = (int)(t - lc * a.np);
+        int k = a.levels - 1;
+        while (a.lv[k].cell0 > lc) --k;
+        const int c = (int)(lc - a.lv[k].cell0);
+        const TreePiece& tp = a.pieces[p];
+        const double s[3] = { tp.x, tp.y, tp.z };
+        const int ci[3] = { c / (a.lv[k].m[1] * a.lv[k].m[2]), c / a.lv[k].m[2] % a.lv[k].m[1], c % a.lv[k].m[2] };
+        int lo[3], hi[3];
+        for (int d = 0; d < 3; ++d) { lo[d] = -a.images; hi[d] = a.images; }
+        for (int j = 0; j <= k; ++j) {
+            const LevelArgs& v = a.lv[j];
+            double h = 0.0;
+            for (int d = 0; d < 3; ++d) h = fmax(h, 0.5 * g.ext[d] / v.m[d]);
+            const double R = v.theta * h + tp.rho;
+            for (int d = 0; d < 3; ++d) {
+                const int cj = ci[d] / (a.lv[k].m[d] / v.m[d]);
+                const double cc = g.lo[d] + (cj + 0.5) * (g.ext[d] / v.m[d]) - s[d];
+                // |cc - i L| <= R; clamped before the conversion to int
+                lo[d] = max(lo[d], (int)fmin(fmax(ceil((cc - R) / L[d]), -64.0), 64.0));
+                hi[d] = min(hi[d], (int)fmin(fmax(floor((cc + R) / L[d]), -64.0), 64.0));
+            }
+        }
+        uint64_t w = 0;
+        if (lo[0] <= hi[0] && lo[1] <= hi[1] && lo[2] <= hi[2])
+            for (int d = 0; d < 3; ++d) {
+                w |= (uint64_t)(uint8_t)(16 + lo[d]) << (16 * d);
+                w |= (uint64_t)(uint8_t)(16 + hi[d]) << (16 * d + 8);
+            }
+        a.near[t] = w;
+    }
+}
+
+// ---- node sums ---------------------------------------------------------------------------
+
+// One warp: 32 / split nodes of one cell; its far pairs are those in the near
+// boxes of the level before and not in its own.  FP64 bound like the plain
+// line kernel (records are read through L1 as warp-uniform 16-byte loads).
+__global__ void __launch_bounds__(32 * kWarps, 4) tree_node_kernel(const TreeArgs a)
+{
+    const int lane = threadIdx.x & 31;
+    const int64_t w = (int64_t)blockIdx.x * kWarps + (threadIdx.x >> 5);
+    int k = a.levels - 1;
+    while (k > 0 && a.lv[k].tile0 > w) --k;
+    const LevelArgs& v = a.lv[k];
+    const int64_t local = w - v.tile0;
+    const int64_t cells = (int64_t)v.m[0] * v.m[1] * v.m[2];
+    if (local >= cells * v.tiles) return;
+    const int cell = (int)(local / v.tiles), tile = (int)(local % v.tiles);
+    if (!a.occ[v.cell0 + cell]) return;
+    const Geo g = load_geo(a);
+    const int split = v.split;
+    const int node = tile * (32 / split) + lane / split, part = lane % split;
+    const bool valid = node < v.q3;
+    const int nd = valid ? node : v.q3 - 1;
+    const int ci[3] = { cell / (v.m[1] * v.m[2]), cell / v.m[2] % v.m[1], cell % v.m[2] };
+    const int ni[3] = { nd / (v.q * v.q), nd / v.q % v.q, nd % v.q };
+    double P[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        const double e = g.ext[d] / v.m[d];
+        P[d] = g.lo[d] + (ci[d] + 0.5) * e + 0.5 * e * cospi((2 * ni[d] + 1) / (2.0 * v.q));
+    }
+    const uint64_t* own = a.near + (v.cell0 + cell) * (int64_t)a.np;
+    const uint64_t* up = nullptr;
+    if (k > 0) {
+        const LevelArgs& u = a.lv[k - 1];
+        const int uc = ((ci[0] / v.r[0]) * u.m[1] + ci[1] / v.r[1]) * u.m[2] + ci[2] / v.r[2];
+        up = a.near + (u.cell0 + uc) * (int64_t)a.np;
+    }
+    const uint64_t all = full_box(a.images);
+    const double cJK = a.f.cJ / a.f.cK;
+    double ux = 0.0, uy = 0.0, uz = 0.0;
+    bool plane = false;
+    for (int base = 0; base < a.np; base += 32) {
+        uint64_t wu = 0, wo = 0;
+        if (base + lane < a.np) {
+            wu = up ? up[base + lane] : all;
+            wo = own[base + lane];
+        }
+        unsigned todo = __ballot_sync(0xffffffffu, wu != 0 && wu != wo);
+        while (todo) {
+            const int b = __ffs(todo) - 1;
+            todo &= todo - 1;
+            const uint64_t bu = __shfl_sync(0xffffffffu, wu, b), bo = __shfl_sync(0xffffffffu, wo, b);
+            const TreePiece& tp = a.pieces[base + b];
+            const LinePiece& pc = *reinterpret_cast<const LinePiece*>(a.f.table + tp.piece);
+            const LineSeg* seg = reinterpret_cast<const LineSeg*>(a.f.table + tp.rec);
+            const ImgShell far(bu, bo);
+            for (int idx = part; idx < far.total; idx += split) {
+                int i, j, l;
+                far.at(idx, i, j, l);
+                line_piece_fp64<true>(pc, seg, P[0] - a.f.Lx * i, P[1] - a.f.Ly * j, P[2] - a.f.Lz * l, cJK, ux, uy,
+                                      uz, plane);
+            }
+        }
+    }
+    for (int o = split / 2; o > 0; o >>= 1) {
+        ux += __shfl_xor_sync(0xffffffffu, ux, o);
+        uy += __shfl_xor_sync(0xffffffffu, uy, o);
+        uz += __shfl_xor_sync(0xffffffffu, uz, o);
+    }
+    if (valid && part == 0) {
+        double* out = v.val + (int64_t)cell * 3 * v.q3 + node;
+        out[0] = ux;
+        out[v.q3] = uy;
+        out[2 * v.q3] = uz;
+    }
+}
+
+// ---- interpolation -----------------------------------------------------------------------
+
+// Matrices of transition t (level t-1 -> t, or last level -> final cells for
+// t = levels): for axis d and sub-position s of r, M[s][i][j] takes the
+// parent's value at its node i to the child's node j (final: to the child's
+// Chebyshev coefficient j).  Interpolation at q Chebyshev points is
+// f(x) = sum_i f_i (1/q) (1 + 2 sum_k T_k(x_i) T_k(x)).
+constexpr int kMaxQ = 21;
+
+// cq[t] = cos(pi t / (2 q)), t < 4 q
+__device__ __forceinline__ double interp_weight(const double* cq, int q, int i, double x)
+{
+    double t0 = 1.0, t1 = x, s = 0.5;
+    int ph = 0;
+    for (int k = 1; k < q; ++k) {
+        ph += 2 * i + 1;
+        if (ph >= 4 * q) ph -= 4 * q;
+        s = fma(cq[ph], t1, s);
+        const double t2 = fma(2.0 * x, t1, -t0);
+        t0 = t1;
+        t1 = t2;
+    }
+    return 2.0 * s / q;
+}
+
+__global__ void __launch_bounds__(128) tree_matrix_kernel(const TreeArgs a)
+{
+    __shared__ double cp[4 * kMaxQ], cc[4 * kMaxQ];
+    const int t = blockIdx.x + 1, d = blockIdx.y;      // transitions 1..levels
+    const bool last = t == a.levels;
+    const int qp = a.lv[t - 1].q, qc = last ? a.qf : a.lv[t].q, r = last ? a.rf[d] : a.lv[t].r[d];
+    for (int e = threadIdx.x; e < 4 * qp; e += blockDim.x) cp[e] = cospi(e / (2.0 * qp));
+    for (int e = threadIdx.x; e < 4 * qc; e += blockDim.x) cc[e] = cospi(e / (2.0 * qc));
+    __syncthreads();
+    double* M = a.mat + a.mat_off[t][d];
+    for (int e = blockIdx.z * blockDim.x + threadIdx.x; e < r * qp * qc; e += gridDim.z * blockDim.x) {
+        const int s = e / (qp * qc), i = e / qc % qp, j = e % qc;
+        const double x0 = (2.0 * s + 1.0) / r - 1.0;
+        double v = 0.0;
+        if (!last) {
+            v = interp_weight(cp, qp, i, x0 + cc[2 * j + 1] / r);
+        } else {
+            for (int n = 0; n < qc; ++n)
+                v = fma(interp_weight(cp, qp, i, x0 + cc[2 * n + 1] / r), cc[(j * (2 * n + 1)) % (4 * qc)], v);
+            v *= (j ? 2.0 : 1.0) / qc;
+        }
+        M[e] = v;
+    }
+}
+
+// One axis of the tensor interpolation: in[a][i][b] -> out[a][j][b] for
+// na x nb columns, each thread one column with the QC sums in registers.
+template <int QC>
+__device__ __forceinline__ void contract(const double* in, const double* M, double* out, int na, int qp, int nb)
+{
+    for (int c = threadIdx.x; c < na * nb; c += blockDim.x) {
+        const int ia = c / nb, ib = c - ia * nb;
+        const double* src = in + ia * qp * nb + ib;
+        double acc[QC];
+#pragma unroll
+        for (int j = 0; j < QC; ++j) acc[j] = 0.0;
+#pragma unroll 2
+        for (int i = 0; i < qp; ++i) {
+            const double f = src[i * nb];
+#pragma unroll
+            for (int j = 0; j < QC; ++j) acc[j] = fma(M[i * QC + j], f, acc[j]);
+        }
+        double* dst = out + ia * QC * nb + ib;
+#pragma unroll
+        for (int j = 0; j < QC; ++j) dst[j * nb] = acc[j];
+    }
+}
+
+// Level t - 1 -> t: one CTA adds one component of one cell's values, read
+// from the cell around it (in L2: its children read it together).
+template <int QC>
+__global__ void __launch_bounds__(256) tree_down_kernel(const TreeArgs a, int t)
+{
+    extern __shared__ double sm[];
+    const LevelArgs& up = a.lv[t - 1];
+    const LevelArgs& v = a.lv[t];
+    const int qp = up.q, comp = blockIdx.y, cell = blockIdx.x;
+    if (!a.occ[v.cell0 + cell]) return;
+    const int ci[3] = { cell / (v.m[1] * v.m[2]), cell / v.m[2] % v.m[1], cell % v.m[2] };
+    const int pc = ((ci[0] / v.r[0]) * up.m[1] + ci[1] / v.r[1]) * up.m[2] + ci[2] / v.r[2];
+    double* b0 = sm;                                   // [QC][qp][qp], then [QC][QC][QC]
+    double* b1 = b0 + max(QC * qp * qp, QC * QC * QC); // [QC][QC][qp]
+    double* M = b1 + QC * QC * qp;
+    for (int d = 0; d < 3; ++d) {
+        const double* m = a.mat + a.mat_off[t][d] + (ci[d] % v.r[d]) * qp * QC;
+        for (int e = threadIdx.x; e < qp * QC; e += blockDim.x) M[d * qp * QC + e] = m[e];
+    }
+    __syncthreads();
+    contract<QC>(up.val + ((int64_t)pc * 3 + comp) * up.q3, M, b0, 1, qp, qp * qp);
+    __syncthreads();
+    contract<QC>(b0, M + qp * QC, b1, QC, qp, qp);
+    __syncthreads();
+    contract<QC>(b1, M + 2 * qp * QC, b0, QC * QC, qp, 1);
+    __syncthreads();
+    double* out = v.val + ((int64_t)cell * 3 + comp) * (QC * QC * QC);
+    for (int e = threadIdx.x; e < QC * QC * QC; e += blockDim.x) out[e] += b0[e];
+}
+
+// One axis of the tensor interpolation with the matrix rows padded to QP and
+// read as pairs: in[c][i] at stride `in_step` -> QC sums in registers.
+template <int QC>
+__device__ __forceinline__ void column(const double* src, int step, const double* M, int qp, double (&acc)[padded(QC)])
+{
+    constexpr int QP = padded(QC);
+#pragma unroll
+    for (int j = 0; j < QP; ++j) acc[j] = 0.0;
+#pragma unroll 6
+    for (int i = 0; i < qp; ++i) {
+        const double f = src[i * step];
+        const double2* m = reinterpret_cast<const double2*>(M + i * QP);
+#pragma unroll
+        for (int j = 0; j < QP / 2; ++j) {
+            const double2 w = m[j];
+            acc[2 * j] = fma(w.x, f, acc[2 * j]);
+            if (2 * j + 1 < QC) acc[2 * j + 1] = fma(w.y, f, acc[2 * j + 1]);
+        }
+    }
+}
+
+// Last level -> atoms: one CTA per (cell of the last level, x and y
+// sub-position, component) interpolates along x and y once for the rf[2] final
+// cells of that column; for each of them it makes the Chebyshev coefficients
+// in shared memory (the transform is folded into the matrices) and evaluates
+// them at the cell's atoms, 64 atoms (two per lane) and a share of the x orders
+// per warp; u += the sum.  Bound by FP64 multiply-adds: QC qp^3 + QC^2 qp^2 per
+// column, QC^3 qp per cell, QC^3 per atom; a pair of coefficients loaded from
+// shared memory feeds four of them.  One component per CTA keeps the shared
+// memory at 40 to 70 KB (three CTAs per SM; one with all three components).
+template <int QC>
+__global__ void __launch_bounds__(256, 3) tree_leaf_kernel(const TreeArgs a)
+{
+    extern __shared__ double sm[];
+    constexpr int QP = padded(QC), kWarpsPerCta = 8;
+    const int t = a.levels;
+    const LevelArgs& up = a.lv[t - 1];
+    const int qp = up.q, comp = blockIdx.y;
+    const int rxy = a.rf[0] * a.rf[1], rz = a.rf[2];
+    const int s = blockIdx.x / rxy, sub = blockIdx.x % rxy;
+    const int bx = sub / a.rf[1], by = sub % a.rf[1];
+    const int cell0 = (s * rxy + sub) * rz;             // the column's first final cell
+    if (a.start[cell0] == a.start[cell0 + rz]) return;
+    double* coef = sm;                                  // [QC][QC][QP]
+    double* b1 = coef + QC * QC * QP;                   // [QC][QC][qp]
+    double* b0 = b1 + padded(QC * QC * qp);             // [QC][qp][qp]; later the atoms' partial sums
+    double* M = b0 + padded(max(QC * qp * qp, 8 * 64)); // x, y and the rz matrices of z, [qp][QP] each
+    for (int k = 0; k < 2 + rz; ++k) {
+        const int d = min(k, 2), b = k == 0 ? bx : k == 1 ? by : k - 2;
+        const double* m = a.mat + a.mat_off[t][d] + b * qp * QC;
+        for (int e = threadIdx.x; e < qp * QP; e += 256)
+            M[k * qp * QP + e] = e % QP < QC ? m[(e / QP) * QC + e % QP] : 0.0;
+    }
+    __syncthreads();
+    {
+        double acc[QP];
+        const double* val = up.val + ((int64_t)s * 3 + comp) * up.q3;
+        for (int c = threadIdx.x; c < qp * qp; c += 256) {
+            column<QC>(val + c, qp * qp, M, qp, acc);
+#pragma unroll
+            for (int j = 0; j < QC; ++j) b0[j * qp * qp + c] = acc[j];
+        }
+        __syncthreads();
+        for (int c = threadIdx.x; c < QC * qp; c += 256) {
+            const int ia = c / qp, ib = c - ia * qp;
+            column<QC>(b0 + ia * qp * qp + ib, qp, M + qp * QP, qp, acc);
+#pragma unroll
+            for (int j = 0; j < QC; ++j) b1[(ia * QC + j) * qp + ib] = acc[j];
+        }
+        __syncthreads();
+    }
+    const Geo g = load_geo(a);
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int cx = (s / (up.m[1] * up.m[2])) * a.rf[0] + bx, cy = (s / up.m[2] % up.m[1]) * a.rf[1] + by;
+    double* uo = comp == 0 ? a.f.ux : comp == 1 ? a.f.uy : a.f.uz;
+    double* red = b0;                                   // [warp][2][32]
+    for (int bz = 0; bz < rz; ++bz) {
+        const uint32_t s0 = a.start[cell0 + bz];
+        const int cnt = (int)(a.start[cell0 + bz + 1] - s0);
+        if (cnt == 0) continue;
+        for (int c = threadIdx.x; c < QC * QC; c += 256) {
+            double acc[QP];
+            column<QC>(b1 + c * qp, 1, M + (2 + bz) * qp * QP, qp, acc);
+            double2* dst = reinterpret_cast<double2*>(coef + c * QP);
+#pragma unroll
+            for (int j = 0; j < QP / 2; ++j) dst[j] = make_double2(acc[2 * j], acc[2 * j + 1]);
+        }
+        __syncthreads();
+        const int ci[3] = { cx, cy, (s % up.m[2]) * rz + bz };
+        // groups of G warps per 64 atoms, each warp QC / G of the x orders
+        const int G = cnt <= 64 ? 8 : cnt <= 128 ? 4 : cnt <= 256 ? 2 : 1;
+        const int part = w % G, i0 = QC * part / G, i1 = QC * (part + 1) / G;
+        const int step = 64 * (kWarpsPerCta / G);
+        for (int base = 0; base < cnt; base += step) {
+            const int first = base + 64 * (w / G);
+            int32_t atom[2];
+            double X[2], Y[2], Tz[2][QC];
+            double u[2] = {};
+            if (first < cnt) {
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    atom[h] = a.perm[s0 + min(first + lane + 32 * h, cnt - 1)];
+                    const double p[3] = { a.f.x[atom[h]], a.f.y[atom[h]], a.f.z[atom[h]] };
+                    double tt[3];
+#pragma unroll
+                    for (int d = 0; d < 3; ++d) {
+                        const double e = g.ext[d] / a.mf[d];
+                        tt[d] = fmin(fmax((p[d] - (g.lo[d] + (ci[d] + 0.5) * e)) * (2.0 / e), -1.0), 1.0);
+                    }
+                    X[h] = tt[0];
+                    Y[h] = tt[1];
+                    Tz[h][0] = 1.0;
+                    Tz[h][1] = tt[2];
+#pragma unroll
+                    for (int i = 2; i < QC; ++i) Tz[h][i] = fma(2.0 * tt[2], Tz[h][i - 1], -Tz[h][i - 2]);
+                }
+                double ax0 = 1.0, bx0 = X[0], ax1 = 1.0, bx1 = X[1];        // T_i, T_{i+1}
+                for (int i = 0; i < i1; ++i) {
+                    if (i >= i0) {
+                        double ay0 = 1.0, by0 = Y[0], ay1 = 1.0, by1 = Y[1];
+                        double sy0 = 0.0, sy1 = 0.0;
+#pragma unroll 2
+                        for (int j = 0; j < QC; ++j) {
+                            const double2* C = reinterpret_cast<const double2*>(coef + (i * QC + j) * QP);
+                            double v0 = 0.0, v1 = 0.0;
+#pragma unroll
+                            for (int k = 0; k < QP / 2; ++k) {
+                                const double2 c = C[k];
+                                v0 = fma(c.x, Tz[0][2 * k], v0);
+                                v1 = fma(c.x, Tz[1][2 * k], v1);
+                                if (2 * k + 1 < QC) {
+                                    v0 = fma(c.y, Tz[0][2 * k + 1], v0);
+                                    v1 = fma(c.y, Tz[1][2 * k + 1], v1);
+                                }
+                            }
+                            sy0 = fma(ay0, v0, sy0);
+                            sy1 = fma(ay1, v1, sy1);
+                            const double n0 = fma(2.0 * Y[0], by0, -ay0), n1 = fma(2.0 * Y[1], by1, -ay1);
+                            ay0 = by0; by0 = n0;
+                            ay1 = by1; by1 = n1;
+                        }
+                        u[0] = fma(ax0, sy0, u[0]);
+                        u[1] = fma(ax1, sy1, u[1]);
+                    }
+                    const double n0 = fma(2.0 * X[0], bx0, -ax0), n1 = fma(2.0 * X[1], bx1, -ax1);
+                    ax0 = bx0; bx0 = n0;
+                    ax1 = bx1; bx1 = n1;
+                }
+            }
+            if (G > 1) {
+                // the shares of the x orders, added in order by the group's first warp
+                red[(w * 2) * 32 + lane] = u[0];
+                red[(w * 2 + 1) * 32 + lane] = u[1];
+                __syncthreads();
+                if (part == 0)
+                    for (int k = 1; k < G; ++k) {
+                        u[0] += red[((w + k) * 2) * 32 + lane];
+                        u[1] += red[((w + k) * 2 + 1) * 32 + lane];
+                    }
+            }
+            if (part == 0) {
+                if (first + lane < cnt) uo[atom[0]] += u[0];
+                if (first + lane + 32 < cnt) uo[atom[1]] += u[1];
+            }
+            if (G > 1) __syncthreads();
+        }
+        __syncthreads();                                // the coefficients are free again
+    }
+}
+
+// The cell of a tile, by bisection of the tiles' prefix sums.
+__device__ __forceinline__ int cell_of_tile(const uint32_t* first, int cells, uint32_t tile)
+{
+    int lo = 0, hi = cells;                    // first[lo] <= tile < first[hi]
+    while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (first[mid] <= tile) lo = mid; else hi = mid;
+    }
+    return lo;
+}
+
+// ---- near pairs --------------------------------------------------------------------------
+
+// The pieces with near images of one cell, 32 at a time; F(piece, box) for each.
+template <class F>
+__device__ __forceinline__ void for_near(const TreeArgs& a, int scell, F f)
+{
+    const int lane = threadIdx.x & 31;
+    const uint64_t all = full_box(a.images);
+    const uint64_t* own = scell < a.cells_s ? a.near + (a.lv[a.levels - 1].cell0 + scell) * (int64_t)a.np : nullptr;
+    for (int base = 0; base < a.np; base += 32) {
+        uint64_t w = 0;
+        if (base + lane < a.np) w = own ? own[base + lane] : all;
+        unsigned todo = __ballot_sync(0xffffffffu, w != 0);
+        while (todo) {
+            const int b = __ffs(todo) - 1;
+            todo &= todo - 1;
+            f(a.pieces[base + b], ImgBox(__shfl_sync(0xffffffffu, w, b)));
+        }
+    }
+}
+
+// One warp: 32 / near_split atoms of one cell of the last level (or atoms
+// outside the grid, which take every image), lanes of an atom splitting the
+// images of each piece.
+__global__ void __launch_bounds__(32 * kWarps, 4) tree_near_sum_kernel(const TreeArgs a)
+{
+    const int lane = threadIdx.x & 31;
+    const uint32_t w = blockIdx.x * kWarps + (threadIdx.x >> 5);
+    if (w >= a.near_tile[a.cells_s + 1]) return;
+    const int cell = cell_of_tile(a.near_tile, a.cells_s + 1, w);
+    const int split = a.near_split, part = lane % split;
+    const int rr = a.rf[0] * a.rf[1] * a.rf[2];
+    const uint32_t s1 = a.start[cell < a.cells_s ? (cell + 1) * rr : a.cells_f + 1];
+    const uint32_t slot = a.start[cell * rr] + (w - a.near_tile[cell]) * (32 / split) + lane / split;
+    const bool valid = slot < s1;
+    const int64_t atom = a.perm[valid ? slot : s1 - 1];
+    const double px = a.f.x[atom], py = a.f.y[atom], pz = a.f.z[atom];
+    const double cJK = a.f.cJ / a.f.cK;
+    double ux = 0.0, uy = 0.0, uz = 0.0;
+    bool plane = false;
+    for_near(a, cell, [&](const TreePiece& tp, const ImgBox& B) {
+        const LinePiece& pc = *reinterpret_cast<const LinePiece*>(a.f.table + tp.piece);
+        const LineSeg* seg = reinterpret_cast<const LineSeg*>(a.f.table + tp.rec);
+        const int cnt = B.count();
+        for (int idx = part; idx < cnt; idx += split) {
+            int i, j, k;
+            B.at(idx, i, j, k);
+            line_piece_fp64(pc, seg, px - a.f.Lx * i, py - a.f.Ly * j, pz - a.f.Lz * k, cJK, ux, uy, uz, plane);
+        }
+    });
+    if (__any_sync(0xffffffffu, plane)) {         // atoms in a loop's plane band: the reference's solid angle
+        for_near(a, cell, [&](const TreePiece& tp, const ImgBox& B) {
+            const LinePiece& pc = *reinterpret_cast<const LinePiece*>(a.f.table + tp.piece);
+            const int cnt = B.count();
+            for (int idx = part; idx < cnt; idx += split) {
+                int i, j, k;
+                B.at(idx, i, j, k);
+                if (plane)
+                    line_piece_plane(pc, a.f.raw, px - a.f.Lx * i, py - a.f.Ly * j, pz - a.f.Lz * k, ux, uy, uz);
+            }
+        });
+    }
+    for (int o = split / 2; o > 0; o >>= 1) {
+        ux += __shfl_xor_sync(0xffffffffu, ux, o);
+        uy += __shfl_xor_sync(0xffffffffu, uy, o);
+        uz += __shfl_xor_sync(0xffffffffu, uz, o);
+    }
+    if (valid && part == 0) {
+        a.f.ux[atom] += ux;
+        a.f.uy[atom] += uy;
+        a.f.uz[atom] += uz;
+    }
+}
+
+// ---- host: choice of the cells -----------------------------------------------------------
+
+int order_for(double theta)
+{
+    for (int i = 0; i < kOrders; ++i)
+        if (kOrderTheta[i] <= theta) return i;
+    return -1;
+}
+
+// Expected near (piece, image) pairs of a cell, in segments: pieces are taken
+// as spread evenly over the box.
+double near_terms(const HostTable& T, const double box[3], int images, double reach)
+{
+    const double W = 2.0 * images + 1.0;
+    double sum = 0.0;
+    for (size_t p = 0; p < T.tree_rho.size(); ++p) {
+        double v = T.tree_terms[p];
+        for (int d = 0; d < 3; ++d) v *= std::min(W, 2.0 * (reach + T.tree_rho[p]) / box[d]);
+        sum += v;
+    }
+    return sum;
+}
+
+} // namespace
+
+void append_tree_pieces(HostTable& T)
+{
+    if (T.kind != kLineKind || T.fp32 || T.chunks.empty()) return;
+    std::vector<TreePiece> out;
+    T.tree_rho.clear();
+    T.tree_terms.clear();
+    for (const Chunk& c : T.chunks) {
+        const unsigned char* base = T.bytes.data() + c.offset;
+        for (int i = 0; i < c.npieces; ++i) {
+            LinePiece p;
+            std::memcpy(&p, base + i * sizeof(p), sizeof(p));
+            TreePiece t;
+            std::memset(&t, 0, sizeof(t));
+            t.piece = (uint32_t)(c.offset + i * sizeof(p));
+            t.rec = (uint32_t)(c.offset + c.npieces * sizeof(p) + p.rec * sizeof(LineSeg));
+            t.x = p.cx; t.y = p.cy; t.z = p.cz;
+            t.rho = p.rho;
+            t.terms = p.nseg;
+            // a ball the far rule cannot use, or offsets past 32 bits: no cells
+            if (!std::isfinite(t.rho + std::fabs(t.x) + std::fabs(t.y) + std::fabs(t.z)) ||
+                T.bytes.size() > 0xFFFFFFFFull) {
+                T.tree_rho.clear();
+                T.tree_terms.clear();
+                return;
+            }
+            T.tree_rho.push_back(t.rho);
+            T.tree_terms.push_back(t.terms);
+            out.push_back(t);
+        }
+    }
+    while (T.bytes.size() % 16) T.bytes.push_back(0);
+    T.aux_tree = T.bytes.size();
+    const unsigned char* s = reinterpret_cast<const unsigned char*>(out.data());
+    T.bytes.insert(T.bytes.end(), s, s + out.size() * sizeof(TreePiece));
+}
+
+TreeShape tree_shape(const HostTable& T, int64_t n, const double box[3], int images)
+{
+    TreeShape S;
+    const int np = (int)T.tree_rho.size();
+    if (!T.aux_tree || np == 0 || n > 0x7FFFFFFF - 64) return S;
+    // FP64 operations of a term, and a microsecond of the GPU in them (18.6e12
+    // per second at the 75 % that the line kernels reach)
+    const double e64 = 78.0, us = 1.4e7;
+    const double W = (double)(2 * images + 1), nimg = W * W * W;
+    double terms = 0.0;
+    for (int32_t t : T.tree_terms) terms += t;
+    const double all = terms * nimg;
+    S.direct = (double)n * all * e64 + 5.0 * us;
+    // the boxes' aspect: axes get m0 2^k cells
+    const double lmin = std::min(box[0], std::min(box[1], box[2]));
+    int m0[3];
+    for (int d = 0; d < 3; ++d) m0[d] = (int)std::min(8.0, std::max(1.0, std::round(box[d] / lmin)));
+    struct State { double cost, near, h; double cells; int a, o, prev; };
+    std::vector<State> st;
+    constexpr int kDepth = 6;
+    for (int a = 0; a < kDepth; ++a) {
+        double h = 0.0, cells = 1.0;
+        for (int d = 0; d < 3; ++d) {
+            const int m = m0[d] << a;
+            h = std::max(h, 0.5 * box[d] / m);
+            cells *= m;
+        }
+        if (cells > 32768.0 || cells * np > 1.6e7) break;
+        for (int o = 0; o < kOrders; ++o) {
+            const double q = kOrderQ[o], q3 = q * q * q;
+            if (cells * q3 > 1.5 * (double)n + 1e5) continue;
+            State s = { 0.0, near_terms(T, box, images, kOrderTheta[o] * h), h, cells, a, o, -1 };
+            if (s.near > 0.97 * all) continue;
+            double best = 1e300;
+            for (int p = -1; p < (int)st.size(); ++p) {
+                const double before = p < 0 ? all : st[p].near;
+                if (p >= 0 && (st[p].near < s.near * 1.02 || st[p].a > a || (st[p].a == a && st[p].o >= o))) continue;
+                double c = (p < 0 ? 0.0 : st[p].cost) + (before - s.near) * cells * q3 * e64 * 1.1 + 3.0 * us +
+                           cells * q3 * np * 0.5;
+                if (p >= 0) {
+                    const double qp = kOrderQ[st[p].o];
+                    c += 3.0 * cells * (q * qp * qp * qp + q * q * qp * qp + q3 * qp) * 2.0 + 4.0 * us;
+                }
+                if (c < best) { best = c; s.prev = p; }
+            }
+            if (best >= 1e299) continue;
+            int depth = 1;
+            for (int p = s.prev; p >= 0; p = st[p].prev) ++depth;
+            if (depth >= TreeShape::kMaxLevels) continue;
+            s.cost = best;
+            st.push_back(s);
+        }
+    }
+    double best = S.direct;
+    int pick = -1, pick_r = 1, pick_q = 0;
+    for (int p = 0; p < (int)st.size(); ++p) {
+        const double theta = kOrderTheta[st[p].o];
+        for (int r = 1; r <= 8; r *= 2) {
+            const double cells = st[p].cells * r * r * r;
+            if (cells > kMaxCells) break;
+            const int o = order_for((theta - 1.0) * r + 1.0);
+            const double q = kOrderQ[o], q3 = q * q * q, qp = kOrderQ[st[p].o];
+            if (kOrderQ[o] > kMaxFinalQ) continue;
+            const double atoms = std::max(1.0, (double)n / cells);
+            const double fill = (std::floor(atoms / 64.0) + 1.0) * 64.0 / atoms;
+            const double c = st[p].cost + (double)n * st[p].near * e64 * 1.1 + (double)n * np * 0.5 +
+                             3.0 * cells * ((q * qp * qp * qp + q * q * qp * qp) / r + q3 * qp) * 2.5 +
+                             (double)n * 3.0 * q3 * 2.0 * std::min(fill, 64.0) + 60.0 * us + (double)n * 60.0;
+            if (c < best) { best = c; pick = p; pick_r = r; pick_q = o; }
+        }
+    }
+    S.cost = best;
+    if (pick < 0) return S;
+    std::vector<int> chain;
+    for (int p = pick; p >= 0; p = st[p].prev) chain.push_back(p);
+    std::reverse(chain.begin(), chain.end());
+    S.use = true;
+    S.levels = (int)chain.size();
+    double before = all;
+    for (int k = 0; k < S.levels; ++k) {
+        const State& s = st[chain[k]];
+        for (int d = 0; d < 3; ++d) S.m[k][d] = m0[d] << s.a;
+        S.q[k] = kOrderQ[s.o];
+        S.theta[k] = kOrderTheta[s.o];
+        // lanes per node: enough images per piece for each lane, more lanes
+        // where the level has few nodes
+        const double per = (before - s.near) / terms;
+        int split = 1;
+        while (split < 32 && per >= 6.0 * split) split *= 2;
+        S.split[k] = split;
+        before = s.near;
+    }
+    for (int d = 0; d < 3; ++d) S.mf[d] = S.m[S.levels - 1][d] * pick_r;
+    S.qf = kOrderQ[pick_q];
+    // lanes per atom: as many as the near images feed, while the atoms alone do
+    // not fill the GPU several times
+    const double per_atom = st[pick].near / terms;
+    while (S.near_split < 32 && per_atom >= 4.0 * S.near_split && n * S.near_split < 600000) S.near_split *= 2;
+    return S;
+}
+
+// ---- host: scratch and launches ----------------------------------------------------------
+
+namespace {
+
+// One pool per device: at most 256 MB stay reserved while a plan that has
+// used it lives, nothing after the last one.
+constexpr int kMaxDevices = 64;
+constexpr uint64_t kPoolKeep = 256ull << 20;
+std::mutex g_pool_mutex;
+cudaMemPool_t g_pool[kMaxDevices] = {};
+int g_pool_users[kMaxDevices] = {};
+
+cudaMemPool_t tree_pool(int device)
+{
+    if (device < 0 || device >= kMaxDevices) return nullptr;
+    std::lock_guard<std::mutex> lock(g_pool_mutex);
+    return g_pool[device];
+}
+
+template <int QC>
+cudaError_t down(const TreeArgs& a, int t, int cells, cudaStream_t s)
+{
+    const int qp = a.lv[t - 1].q;
+    const size_t smem = ((size_t)std::max(QC * qp * qp, QC * QC * QC) + (size_t)QC * QC * qp + 3 * (size_t)qp * QC) *
+                        sizeof(double);
+    const cudaError_t e = cudaFuncSetAttribute(tree_down_kernel<QC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)smem);
+    if (e != cudaSuccess) return e;
+    tree_down_kernel<QC><<<dim3((unsigned)cells, 3), 256, smem, s>>>(a, t);
+    return cudaGetLastError();
+}
+
+template <int QC>
+cudaError_t leaf(const TreeArgs& a, cudaStream_t s)
+{
+    const int qp = a.lv[a.levels - 1].q;
+    constexpr int QP = padded(QC);
+    const size_t smem = ((size_t)QC * QC * QP + padded(QC * QC * qp) + padded(std::max(QC * qp * qp, 8 * 64)) +
+                         (size_t)(2 + a.rf[2]) * qp * QP) * sizeof(double);
+    const cudaError_t e = cudaFuncSetAttribute(tree_leaf_kernel<QC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)smem);
+    if (e != cudaSuccess) return e;
+    tree_leaf_kernel<QC><<<dim3((unsigned)(a.cells_f / a.rf[2]), 3), 256, smem, s>>>(a);
+    return cudaGetLastError();
+}
+
+cudaError_t down_any(const TreeArgs& a, int t, int cells, cudaStream_t s)
+{
+    switch (a.lv[t].q) {
+    case 9:  return down<9>(a, t, cells, s);
+    case 10: return down<10>(a, t, cells, s);
+    case 11: return down<11>(a, t, cells, s);
+    case 12: return down<12>(a, t, cells, s);
+    case 13: return down<13>(a, t, cells, s);
+    case 15: return down<15>(a, t, cells, s);
+    case 17: return down<17>(a, t, cells, s);
+    case 19: return down<19>(a, t, cells, s);
+    default: return down<21>(a, t, cells, s);
+    }
+}
+
+cudaError_t leaf_any(const TreeArgs& a, cudaStream_t s)
+{
+    switch (a.qf) {
+    case 9:  return leaf<9>(a, s);
+    case 10: return leaf<10>(a, s);
+    case 11: return leaf<11>(a, s);
+    case 12: return leaf<12>(a, s);
+    default: return leaf<13>(a, s);
+    }
+}
+
+} // namespace
+
+void tree_pool_retain(int device)
+{
+    if (device < 0 || device >= kMaxDevices) return;
+    std::lock_guard<std::mutex> lock(g_pool_mutex);
+    ++g_pool_users[device];
+    if (g_pool[device]) return;
+    cudaMemPoolProps props;
+    std::memset(&props, 0, sizeof(props));
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = device;
+    cudaMemPool_t p = nullptr;
+    uint64_t keep = kPoolKeep;
+    if (cudaMemPoolCreate(&p, &props) != cudaSuccess) { cudaGetLastError(); return; }
+    if (cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) cudaGetLastError();
+    g_pool[device] = p;
+}
+
+void tree_pool_release(int device)
+{
+    if (device < 0 || device >= kMaxDevices) return;
+    std::lock_guard<std::mutex> lock(g_pool_mutex);
+    if (--g_pool_users[device] > 0 || !g_pool[device]) return;
+    if (cudaMemPoolTrimTo(g_pool[device], 0) != cudaSuccess) cudaGetLastError();
+}
+
+int launch_tree(const FieldArgs& f, const HostTable& T, const TreeShape& S, const double box[3], int sm_count,
+                cudaStream_t s, bool* ran, std::string& err)
+{
+    *ran = false;
+    (void)box;
+    TreeArgs a;
+    std::memset(&a, 0, sizeof(a));
+    a.f = f;
+    a.pieces = reinterpret_cast<const TreePiece*>(f.table + T.aux_tree);
+    a.np = (int32_t)T.tree_rho.size();
+    a.levels = S.levels;
+    a.images = f.images;
+    a.near_split = S.near_split;
+    a.qf = S.qf;
+    // scratch layout
+    size_t at = 0;
+    auto take = [&](size_t bytes) { const size_t o = at; at += (bytes + 255) & ~size_t(255); return o; };
+    const size_t o_box = take(6 * sizeof(unsigned long long));
+    int64_t lcells = 0, tiles = 0;
+    size_t o_val[TreeShape::kMaxLevels], mats = 0;
+    int lvcells[TreeShape::kMaxLevels];
+    for (int k = 0; k < S.levels; ++k) {
+        LevelArgs& v = a.lv[k];
+        int64_t cells = 1;
+        for (int d = 0; d < 3; ++d) {
+            v.m[d] = S.m[k][d];
+            v.r[d] = k ? S.m[k][d] / S.m[k - 1][d] : 1;
+            cells *= v.m[d];
+        }
+        v.q = S.q[k];
+        v.q3 = v.q * v.q * v.q;
+        v.split = S.split[k];
+        v.theta = S.theta[k];
+        v.tiles = (v.q3 * v.split + 31) / 32;
+        v.tile0 = tiles;
+        v.cell0 = lcells;
+        tiles += cells * v.tiles;
+        lcells += cells;
+        lvcells[k] = (int)cells;
+        o_val[k] = take((size_t)cells * 3 * v.q3 * sizeof(double));
+    }
+    a.level_cells = lcells;
+    int64_t cf = 1;
+    for (int d = 0; d < 3; ++d) {
+        a.mf[d] = S.mf[d];
+        a.rf[d] = S.mf[d] / S.m[S.levels - 1][d];
+        cf *= a.mf[d];
+    }
+    a.cells_s = lvcells[S.levels - 1];
+    a.cells_f = (int32_t)cf;
+    for (int t = 1; t <= S.levels; ++t) {
+        const bool last = t == S.levels;
+        const int qp = a.lv[t - 1].q, qc = last ? a.qf : a.lv[t].q;
+        for (int d = 0; d < 3; ++d) {
+            a.mat_off[t][d] = (int32_t)mats;
+            mats += (size_t)(last ? a.rf[d] : a.lv[t].r[d]) * qp * qc;
+        }
+    }
+    const size_t o_near = take((size_t)lcells * a.np * sizeof(uint64_t));
+    const size_t o_occ = take((size_t)lcells);
+    const size_t o_start = take((size_t)(cf + 2) * sizeof(uint32_t));
+    const size_t o_ntile = take((size_t)(a.cells_s + 2) * sizeof(uint32_t));
+    a.sort_tiles = (int32_t)((f.n + kSortTile - 1) / kSortTile);
+    const size_t o_sort = take((size_t)f.n * 4 * sizeof(uint32_t));
+    const size_t o_digits = take(((size_t)a.sort_tiles * 256 + 256) * sizeof(uint32_t));
+    const size_t o_mat = take(mats * sizeof(double));
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) { cudaGetLastError(); return DISCO_OK; }
+    cudaMemPool_t pool = tree_pool(dev);
+    if (!pool) return DISCO_OK;
+    unsigned char* ws = nullptr;
+    if (cudaMallocFromPoolAsync(reinterpret_cast<void**>(&ws), at, pool, s) != cudaSuccess) {
+        cudaGetLastError();
+        return DISCO_OK;
+    }
+    *ran = true;
+    a.box = reinterpret_cast<unsigned long long*>(ws + o_box);
+    for (int k = 0; k < S.levels; ++k) a.lv[k].val = reinterpret_cast<double*>(ws + o_val[k]);
+    a.near = reinterpret_cast<uint64_t*>(ws + o_near);
+    a.occ = ws + o_occ;
+    a.start = reinterpret_cast<uint32_t*>(ws + o_start);
+    a.near_tile = reinterpret_cast<uint32_t*>(ws + o_ntile);
+    for (int b = 0; b < 2; ++b) {
+        a.key[b] = reinterpret_cast<uint32_t*>(ws + o_sort) + (size_t)b * f.n;
+        a.idx[b] = reinterpret_cast<int32_t*>(ws + o_sort) + (size_t)(2 + b) * f.n;
+    }
+    a.digits = reinterpret_cast<uint32_t*>(ws + o_digits);
+    a.digit_total = a.digits + (size_t)a.sort_tiles * 256;
+    a.mat = reinterpret_cast<double*>(ws + o_mat);
+
+    auto queue = [&]() -> cudaError_t {
+        const int64_t sweep = std::min<int64_t>((f.n + 255) / 256, (int64_t)sm_count * 8);
+        cudaError_t e;
+        tree_init_kernel<<<(unsigned)std::min<int64_t>((lcells + 255) / 256, sm_count * 4), 256, 0, s>>>(a);
+        tree_box_kernel<<<(unsigned)sweep, 256, 0, s>>>(a);
+        const unsigned nt = (unsigned)a.sort_tiles;
+        int in = 0;
+        for (int shift = 0; shift == 0 || (cf >> shift) > 0; shift += 8) {
+            if (shift == 0) {
+                tree_digits_kernel<true><<<nt, kSortThreads, 0, s>>>(a, nullptr, shift);
+                tree_digit_scan_kernel<<<256, 256, 0, s>>>(a);
+                tree_reorder_kernel<true><<<nt, kSortThreads, 0, s>>>(a, a.key[0], nullptr, a.key[1], a.idx[1], shift);
+            } else {
+                tree_digits_kernel<false><<<nt, kSortThreads, 0, s>>>(a, a.key[in], shift);
+                tree_digit_scan_kernel<<<256, 256, 0, s>>>(a);
+                tree_reorder_kernel<false><<<nt, kSortThreads, 0, s>>>(a, a.key[in], a.idx[in], a.key[in ^ 1],
+                                                                       a.idx[in ^ 1], shift);
+            }
+            in ^= 1;
+        }
+        a.perm = a.idx[in];
+        tree_starts_kernel<<<(unsigned)((f.n + 256) / 256), 256, 0, s>>>(a, a.key[in]);
+        tree_scan_kernel<<<1, 1024, 0, s>>>(a);
+        tree_near_kernel<<<(unsigned)std::min<int64_t>((lcells * a.np + 255) / 256, (int64_t)sm_count * 16), 256, 0, s>>>(a);
+        tree_matrix_kernel<<<dim3((unsigned)S.levels, 3, 8), 128, 0, s>>>(a);
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        tree_node_kernel<<<(unsigned)((tiles + kWarps - 1) / kWarps), 32 * kWarps, 0, s>>>(a);
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        for (int t = 1; t < S.levels; ++t)
+            if ((e = down_any(a, t, lvcells[t], s)) != cudaSuccess) return e;
+        if ((e = leaf_any(a, s)) != cudaSuccess) return e;
+        const int64_t ntiles = f.n * S.near_split / 32 + a.cells_s + 2;
+        const unsigned ngrid = (unsigned)((ntiles + kWarps - 1) / kWarps);
+        tree_near_sum_kernel<<<ngrid, 32 * kWarps, 0, s>>>(a);
+        return cudaGetLastError();
+    };
+    const cudaError_t e = queue();
+    const cudaError_t ef = cudaFreeAsync(ws, s);
+    if (e != cudaSuccess) { err = cudaGetErrorString(e); return DISCO_ECUDA; }
+    if (ef != cudaSuccess) { err = cudaGetErrorString(ef); return DISCO_ECUDA; }
+    return DISCO_OK;
+}
+
+} // namespace disco

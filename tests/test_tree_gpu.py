@@ -1,0 +1,136 @@
+"""The sum by cells (tree.cu) against the plain sum over every image, which an
+explicit image split selects, and against the oracle.
+
+Tolerance: the cells' interpolation stays below 4e-15 A per loop at
+|b| = 2.5 A where theta(q) was set, at most about three levels add at an atom,
+and the plain sum itself is within 1e-14 A of the oracle on these sizes: 2e-14
+A per loop, plus 2e-14 A."""
+import numpy as np
+import pytest
+
+import oracle as O
+from disco_b200 import _capi as C
+from disco_b200 import backend as B
+from disco_b200 import workloads as W
+
+pytestmark = pytest.mark.gpu
+
+
+def _sum(torch, w, pos, split, precision=C.DISCO_FP64):
+    p = B.Plan(w.loops, w.box, precision=precision, images=w.images, nu=w.nu, image_split=split,
+               max_atoms=pos.shape[1])
+    u = torch.zeros_like(pos)
+    p.execute(pos, u)
+    p.sync(torch.cuda.current_stream().cuda_stream)
+    p.close()
+    return u
+
+
+def _positions(torch, w):
+    return torch.tensor(np.stack([w.x, w.y, w.z]), dtype=torch.float64, device="cuda")
+
+
+def _uneven():
+    """A 3 : 2 : 1 box, odd atom count."""
+    w = W.batch(nsamples=1, edge=(60, 60), nloops=(6, 6), radius=(6.0, 20.0), images=(2, 2), seed=11)[0]
+    keep = (np.abs(w.y) < w.box[1] / 3) & (np.abs(w.z) < w.box[2] / 6)
+    keep[::977] = False
+    s = w.subset(np.flatnonzero(keep))
+    s.box = (w.box[0], w.box[1] * 2 / 3, w.box[2] / 3)
+    return s
+
+
+CASES = {
+    "fcc": lambda: W.fcc_random(cells=36, n_circles=4, n_hex=2, n_rect=2),
+    "uneven": _uneven,
+    "large cells": lambda: W.fcc_random(cells=70, images=3, n_circles=2, n_hex=1, n_rect=1),
+}
+
+
+@pytest.mark.parametrize("name", list(CASES))
+@pytest.mark.parametrize("form", ["plain", "shifted", "shuffled"])
+def test_cells_match_plain_sum(name, form):
+    torch = pytest.importorskip("torch")
+    w = CASES[name]()
+    pos = _positions(torch, w)
+    if form == "shifted":
+        pos += torch.tensor([[0.5 * w.box[0]], [0.25 * w.box[1]], [-0.4 * w.box[2]]], device="cuda")
+    elif form == "shuffled":
+        g = torch.Generator(device="cuda")
+        g.manual_seed(1)
+        pos = pos[:, torch.randperm(pos.shape[1], generator=g, device="cuda")].contiguous()
+    tol = 2e-14 * len(w.loops) + 2e-14
+    a = _sum(torch, w, pos, 1)
+    b = _sum(torch, w, pos, 0)
+    c = _sum(torch, w, pos, 0)
+    assert float((a - b).abs().max()) <= tol
+    assert torch.equal(b, c)                       # same atoms, same bits
+    if form == "plain":
+        idx = np.random.default_rng(0).permutation(w.n)[:1500]
+        s = w.subset(idx)
+        ref = np.stack(O.displace(s.x, s.y, s.z, s.loops, s.box, images=s.images, nu=s.nu))
+        assert np.abs(b.cpu().numpy()[:, idx] - ref).max() <= tol
+
+
+def test_atoms_outside_the_cells():
+    """Outliers, a NaN and an infinity take every image themselves and leave
+    the other atoms alone; atoms that fill a corner of the box only."""
+    torch = pytest.importorskip("torch")
+    w = W.fcc_random(cells=36, n_circles=4, n_hex=2, n_rect=2)
+    pos = _positions(torch, w)
+    pos[:, 7] = torch.tensor([5.0, -3.1, 0.2], device="cuda") * w.box[0]
+    pos[0, 100] = float("nan")
+    pos[2, 4001] = float("inf")
+    pos[:, 9000:] = pos[:, 9000:] * 0.45 + 0.1 * w.box[0]
+    a, b = _sum(torch, w, pos, 1), _sum(torch, w, pos, 0)
+    odd = torch.zeros(pos.shape[1], dtype=torch.bool, device="cuda")
+    odd[100] = odd[4001] = True
+    assert torch.isfinite(b[:, ~odd]).all()
+    assert float((a - b)[:, ~odd].abs().max()) <= 2e-14 * len(w.loops) + 2e-14
+    assert torch.equal(torch.isnan(a[:, 100]), torch.isnan(b[:, 100]))
+
+
+def test_accumulates_and_captures():
+    """execute adds into u; a captured stream keeps to the plain kernels."""
+    torch = pytest.importorskip("torch")
+    w = W.fcc_random(cells=36, n_circles=4, n_hex=2, n_rect=2)
+    pos = _positions(torch, w)
+    one = _sum(torch, w, pos, 0)
+    plan = B.Plan(w.loops, w.box, images=w.images, nu=w.nu, max_atoms=w.n)
+    u = torch.ones_like(pos)
+    plan.execute(pos, u)
+    torch.cuda.synchronize()
+    tol = 2e-14 * len(w.loops) + 2e-14
+    assert float((u - 1.0 - one).abs().max()) <= 1e-15 + tol
+    v = torch.zeros_like(pos)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        plan.execute(pos, v)
+    for _ in range(2):
+        v.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert float((v - one).abs().max()) <= tol
+    del graph
+    plan.close()
+
+
+def test_two_streams_at_once():
+    """Calls in flight on two streams have their own scratch."""
+    torch = pytest.importorskip("torch")
+    w = W.fcc_random(cells=36, n_circles=4, n_hex=2, n_rect=2)
+    pos = _positions(torch, w)
+    one = _sum(torch, w, pos, 0)
+    plan = B.Plan(w.loops, w.box, images=w.images, nu=w.nu, max_atoms=w.n)
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    us = [torch.zeros_like(pos) for _ in streams]
+    torch.cuda.synchronize()
+    for _ in range(3):
+        for s, u in zip(streams, us):
+            with torch.cuda.stream(s):
+                u.zero_()
+                plan.execute(pos, u, s)
+    torch.cuda.synchronize()
+    for u in us:
+        assert torch.equal(u, one)
+    plan.close()
