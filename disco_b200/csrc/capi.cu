@@ -42,8 +42,8 @@ struct disco_plan {
     // the sum by cells: its shape for the last atom count, and whether this
     // plan holds the device's scratch pool (both set by execute)
     std::mutex tree_mutex;
-    int64_t tree_n = -1;
-    disco::TreeShape tree;
+    int64_t tree_n[2] = { -1, -1 };
+    disco::TreeShape tree[2];
     bool tree_pool = false;
 };
 
@@ -112,23 +112,23 @@ void free_plan(disco_plan* p)
 // keeps to it (its launches allocate nothing), and so does a sum over far
 // shells alone (image_min > 0): that is the term-by-term sum the learned form
 // is measured and tested against, in error and in time.
-disco::TreeShape plan_tree(disco_plan* p, int64_t n, cudaStream_t s)
+disco::TreeShape plan_tree(disco_plan* p, int k, int64_t n, cudaStream_t s)
 {
     disco::TreeShape none;
-    if (!p->tables[0].aux_tree || p->opt.image_split != 0 || p->opt.image_min > 0) return none;
+    if (!p->tables[k].aux_tree || p->opt.image_split != 0 || p->opt.image_min > 0) return none;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(s, &cap) != cudaSuccess) { cudaGetLastError(); return none; }
     if (cap != cudaStreamCaptureStatusNone) return none;
     std::lock_guard<std::mutex> lock(p->tree_mutex);
-    if (p->tree_n != n) {
-        p->tree = disco::tree_shape(p->tables[0], n, p->box, p->opt.images);
-        p->tree_n = n;
+    if (p->tree_n[k] != n) {
+        p->tree[k] = disco::tree_shape(p->tables[k], n, p->box, p->opt.images);
+        p->tree_n[k] = n;
     }
-    if (p->tree.use && !p->tree_pool) {
+    if (p->tree[k].use && !p->tree_pool) {
         disco::tree_pool_retain(p->device);
         p->tree_pool = true;
     }
-    return p->tree;
+    return p->tree[k];
 }
 
 double now_s()
@@ -234,9 +234,9 @@ int disco_b200_plan_create(const disco_loop* loops, int32_t nloops, const double
         const uint32_t cap = o.stage_kb > 0 ? (uint32_t)o.stage_kb * 1024u : 0u;
         st = o.precision == DISCO_FP32C
                  ? disco::build_table_fp32(loops, nloops, kind, o.nu, p->tables[k], err, cap)
-                 : disco::build_table(loops, nloops, kind, o.precision, o.nu, p->tables[k], err, cap);
+                 : disco::build_table(loops, nloops, kind, o.precision, o.nu, p->tables[k], err, cap, true);
         if (st) { free_plan(p); return fail(st, err); }
-        if (k == 0) disco::append_tree_pieces(p->tables[k]);
+        disco::append_tree_pieces(p->tables[k]);
         const disco::HostTable& T = p->tables[k];
         for (int l = 0; l < nloops; ++l) p->loop_evals[l] += T.loop_evals[l];
         p->stats.n_segments += T.n_segments;
@@ -313,14 +313,12 @@ int disco_b200_plan_execute(disco_plan* p, const disco_atoms* a, void* stream)
         }
         std::string err;
         const int kind = k == 0 ? disco::kLineKind : disco::kLooponKind;
-        if (k == 0) {
-            const disco::TreeShape shape = plan_tree(p, a->n, s);
-            if (shape.use) {
-                bool ran = false;
-                const int st = disco::launch_tree(fa, T, shape, p->box, p->sm_count, s, &ran, err);
-                if (st) return fail(st, err);
-                if (ran) continue;
-            }
+        const disco::TreeShape shape = plan_tree(p, k, a->n, s);
+        if (shape.use) {
+            bool ran = false;
+            const int st = disco::launch_tree(fa, T, shape, p->sm_count, s, &ran, err);
+            if (st) return fail(st, err);
+            if (ran) continue;
         }
         const int st = T.fp32
             ? disco::launch_field_fp32(fa, kind, p->sm_count, p->opt.image_split, s, err)

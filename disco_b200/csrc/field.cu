@@ -41,8 +41,116 @@ void append_raw(HostTable& T, const std::vector<double>& raw)
     T.bytes.insert(T.bytes.end(), s, s + raw.size() * sizeof(double));
 }
 
+namespace {
+
+// Quadtree order of one loop's loopons: squares of the loop's plane halved
+// until a leaf holds about 200, numbered along the Z curve, so that every
+// square's loopons are consecutive.  order[k] = the loopon at place k;
+// nodes: the squares that hold any, parents first (parent, leaf0, leaves and
+// terms relative to this loop; `rec` holds a leaf's first place).  False where
+// the loopons do not lie in one plane normal to n (or are not finite): no tree.
+bool quadtree(const disco_loop& lp, std::vector<int32_t>& order, std::vector<TreePiece>& nodes)
+{
+    const int np = lp.n_loopons;
+    const disco_loop_phys& ph = lp.phys;
+    double n[3] = { ph.nx, ph.ny, ph.nz };
+    const double nn = std::sqrt(n[0] * n[0] + n[1] * n[1] + n[2] * n[2]);
+    if (!(nn > 0.5) || !std::isfinite(nn)) return false;
+    for (double& v : n) v /= nn;
+    int ax = 0;
+    for (int d = 1; d < 3; ++d)
+        if (std::fabs(n[d]) < std::fabs(n[ax])) ax = d;
+    double e1[3] = { -n[ax] * n[0], -n[ax] * n[1], -n[ax] * n[2] };      // axis ax, made normal to n
+    e1[ax] += 1.0;
+    const double l1 = std::sqrt(e1[0] * e1[0] + e1[1] * e1[1] + e1[2] * e1[2]);
+    for (double& v : e1) v /= l1;
+    const double e2[3] = { n[1] * e1[2] - n[2] * e1[1], n[2] * e1[0] - n[0] * e1[2], n[0] * e1[1] - n[1] * e1[0] };
+    const double o[3] = { lp.x[0], lp.y[0], lp.z[0] };
+    std::vector<double> a((size_t)np), b((size_t)np);
+    double lo[2] = { 0, 0 }, hi[2] = { 0, 0 }, off = 0.0, big = 0.0;
+    for (int k = 0; k < np; ++k) {
+        const double r[3] = { lp.x[k] - o[0], lp.y[k] - o[1], lp.z[k] - o[2] };
+        a[k] = e1[0] * r[0] + e1[1] * r[1] + e1[2] * r[2];
+        b[k] = e2[0] * r[0] + e2[1] * r[1] + e2[2] * r[2];
+        off = std::max(off, std::fabs(n[0] * r[0] + n[1] * r[1] + n[2] * r[2]));
+        big = std::max(big, std::fabs(lp.x[k]) + std::fabs(lp.y[k]) + std::fabs(lp.z[k]));
+        lo[0] = std::min(lo[0], a[k]); hi[0] = std::max(hi[0], a[k]);
+        lo[1] = std::min(lo[1], b[k]); hi[1] = std::max(hi[1], b[k]);
+    }
+    // rounding of the positions' own sums, nothing more
+    if (!std::isfinite(big) || !(off <= 1e-14 * (big + 10.0))) return false;
+    const double half = 0.5 * std::max(hi[0] - lo[0], hi[1] - lo[1]) * (1.0 + 1e-12) + 1e-9;
+    const double mid[2] = { 0.5 * (lo[0] + hi[0]), 0.5 * (lo[1] + hi[1]) };
+    int depth = 0;
+    while (depth < 8 && (double)np / std::ldexp(1.0, 2 * depth) > 256.0) ++depth;
+    const int side = 1 << depth;
+    std::vector<int32_t> code((size_t)np), first((size_t)side * side + 1, 0);
+    for (int k = 0; k < np; ++k) {
+        const int i = std::min(side - 1, std::max(0, (int)((a[k] - mid[0] + half) / (2.0 * half) * side)));
+        const int j = std::min(side - 1, std::max(0, (int)((b[k] - mid[1] + half) / (2.0 * half) * side)));
+        int c = 0;
+        for (int t = 0; t < depth; ++t) c |= ((i >> t & 1) << (2 * t + 1)) | ((j >> t & 1) << (2 * t));
+        code[k] = c;
+        ++first[c + 1];
+    }
+    for (int c = 0; c < side * side; ++c) {
+        if (first[c + 1] > kMaxLooponPiece) return false;
+        first[c + 1] += first[c];
+    }
+    order.resize((size_t)np);
+    std::vector<int32_t> at(first.begin(), first.end() - 1);
+    for (int k = 0; k < np; ++k) order[at[code[k]]++] = k;
+    // squares that hold loopons, from the whole loop down
+    std::vector<int32_t> above(1, -1), mine;
+    for (int t = 0; t <= depth; ++t) {
+        const int cells = 1 << (2 * t), span = 1 << (2 * (depth - t));
+        mine.assign((size_t)cells, -1);
+        for (int c = 0; c < cells; ++c) {
+            const int k0 = first[c * span], k1 = first[(c + 1) * span];
+            if (k0 == k1) continue;
+            double l[2] = { 1e300, 1e300 }, h[2] = { -1e300, -1e300 };
+            for (int k = k0; k < k1; ++k) {
+                l[0] = std::min(l[0], a[order[k]]); h[0] = std::max(h[0], a[order[k]]);
+                l[1] = std::min(l[1], b[order[k]]); h[1] = std::max(h[1], b[order[k]]);
+            }
+            TreePiece q;
+            std::memset(&q, 0, sizeof(q));
+            const double ca = 0.5 * (l[0] + h[0]), cb = 0.5 * (l[1] + h[1]);
+            q.x = o[0] + ca * e1[0] + cb * e2[0];
+            q.y = o[1] + ca * e1[1] + cb * e2[1];
+            q.z = o[2] + ca * e1[2] + cb * e2[2];
+            q.a1 = 0.5 * (h[0] - l[0]);
+            q.a2 = 0.5 * (h[1] - l[1]);
+            q.rho = std::sqrt(q.a1 * q.a1 + q.a2 * q.a2) * (1.0 + 1e-12) + 1e-9;
+            for (int d = 0; d < 3; ++d) { q.e1[d] = e1[d]; q.e2[d] = e2[d]; }
+            q.size = half / (1 << t);
+            q.terms = k1 - k0;
+            q.rec = (uint32_t)k0;
+            q.parent = t ? above[c >> 2] : -1;
+            q.leaf0 = -1;
+            mine[c] = (int32_t)nodes.size();
+            nodes.push_back(q);
+        }
+        above.swap(mine);
+    }
+    // leaves are the last depth, in order: count them up the tree
+    const int total = (int)nodes.size();
+    for (int k = total - 1; k >= 0; --k) {
+        TreePiece& q = nodes[k];
+        if (q.leaves == 0) { q.leaf0 = k; q.leaves = 1; }
+        if (q.parent >= 0) {
+            TreePiece& up = nodes[q.parent];
+            up.leaf0 = q.leaf0;                 // children come last to first
+            up.leaves += q.leaves;
+        }
+    }
+    return true;
+}
+
+} // namespace
+
 int build_table(const disco_loop* loops, int nloops, int kind, int precision, double nu,
-                HostTable& T, std::string& err, uint32_t stage_cap)
+                HostTable& T, std::string& err, uint32_t stage_cap, bool tree)
 {
     T = HostTable();
     T.kind = kind;
@@ -77,6 +185,10 @@ int build_table(const disco_loop* loops, int nloops, int kind, int precision, do
         if (!T.chunks.empty()) append_raw(T, raw);
     } else {
         PieceList<LooponPiece, LooponRec> L;
+        // tree pieces; a leaf's `piece` and `rec` hold its table piece and its
+        // place in it until the chunks have their offsets
+        std::vector<TreePiece> nodes, mine;
+        std::vector<int32_t> order;
         for (int l = 0; l < nloops; ++l) {
             const disco_loop& lp = loops[l];
             if (lp.line) continue;
@@ -89,8 +201,22 @@ int build_table(const disco_loop* loops, int nloops, int kind, int precision, do
             double cx = 0.0, cy = 0.0, cz = 0.0;
             for (int k = 0; k < np; ++k) { cx += lp.x[k]; cy += lp.y[k]; cz += lp.z[k]; }
             cx /= np; cy /= np; cz /= np;
-            for (int k0 = 0; k0 < np; k0 += kMaxLooponPiece) {
-                const int k1e = std::min(np, k0 + kMaxLooponPiece);
+            mine.clear();
+            order.clear();
+            if (tree && !quadtree(lp, order, mine)) { tree = false; order.clear(); mine.clear(); }
+            // a piece ends at kMaxLooponPiece loopons, with a tree before the
+            // leaf that would pass them
+            size_t leaf = 0;
+            while (leaf < mine.size() && mine[leaf].leaf0 != (int32_t)leaf) ++leaf;
+            const int32_t base = (int32_t)nodes.size();
+            int k0 = 0;
+            while (k0 < np) {
+                int k1e = std::min(np, k0 + kMaxLooponPiece);
+                for (; leaf < mine.size() && (int)mine[leaf].rec + mine[leaf].terms <= k1e; ++leaf) {
+                    mine[leaf].piece = (uint32_t)L.pieces.size();
+                    mine[leaf].rec -= (uint32_t)k0;
+                }
+                if (leaf < mine.size()) k1e = (int)mine[leaf].rec;
                 LooponPiece p;
                 std::memset(&p, 0, sizeof(p));
                 p.cx = cx; p.cy = cy; p.cz = cz;
@@ -103,18 +229,45 @@ int build_table(const disco_loop* loops, int nloops, int kind, int precision, do
                 p.n = k1e - k0;
                 std::vector<LooponRec> recs;
                 for (int k = k0; k < k1e; ++k) {
+                    const int i = order.empty() ? k : order[k];
                     LooponRec r;
-                    r.x = lp.x[k] - cx; r.y = lp.y[k] - cy; r.z = lp.z[k] - cz;
+                    r.x = lp.x[i] - cx; r.y = lp.y[i] - cy; r.z = lp.z[i] - cz;
                     r.ml = ph.mx * r.x + ph.my * r.y + ph.mz * r.z;
                     r.nl = ph.nx * r.x + ph.ny * r.y + ph.nz * r.z;
-                    r.pad = 0.0;
+                    r.w = 1.0;
                     recs.push_back(r);
                 }
                 L.pieces.push_back(p);
                 L.recs.push_back(std::move(recs));
+                k0 = k1e;
+            }
+            for (TreePiece q : mine) {
+                if (q.parent >= 0) q.parent += base;
+                q.leaf0 += base;
+                nodes.push_back(q);
             }
         }
         pack_chunks(L, T, stage_cap);
+        if (tree) {
+            std::vector<uint32_t> at_piece, at_rec;
+            for (const Chunk& c : T.chunks) {
+                uint64_t rec = c.offset + (uint64_t)c.npieces * sizeof(LooponPiece);
+                for (int i = 0; i < c.npieces; ++i) {
+                    at_piece.push_back((uint32_t)(c.offset + i * sizeof(LooponPiece)));
+                    at_rec.push_back((uint32_t)rec);
+                    rec += (uint64_t)L.pieces[at_piece.size() - 1].n * sizeof(LooponRec);
+                }
+            }
+            for (size_t k = 0; k < nodes.size(); ++k) {
+                TreePiece& q = nodes[k];
+                if (q.leaf0 != (int32_t)k) continue;
+                const uint32_t i = q.piece;
+                q.piece = at_piece[i];
+                q.rec = at_rec[i] + q.rec * (uint32_t)sizeof(LooponRec);
+            }
+            for (TreePiece& q : nodes) q.piece = nodes[q.leaf0].piece;      // m, n and b are the loop's
+            T.tree = std::move(nodes);
+        }
     }
     return DISCO_OK;
 }

@@ -59,7 +59,7 @@ struct alignas(16) LooponPiece {
 struct alignas(16) LooponRec {
     double x, y, z;       // loopon - reference point
     double ml, nl;        // m . (loopon - c), n . (loopon - c)
-    double pad;
+    double w;             // weight: 1 for a loopon (tree.cu's equivalent loopons have others)
 };
 static_assert(sizeof(LooponPiece) == 112 && sizeof(LooponRec) == 48, "loopon table layout");
 
@@ -102,6 +102,21 @@ struct alignas(16) LooponRecF {
     float nl, pad0, pad1, pad2;   // 32 B
 };
 static_assert(sizeof(LooponPieceF) == 80 && sizeof(LooponRecF) == 32, "fp32 loopon table layout");
+
+// A source of the sum by cells (tree.cuh): a line piece, or a square patch of a
+// loop's loopons at some depth of its quadtree.  The ball (x, y, z, rho) holds
+// it; records are byte offsets into the table.
+struct alignas(16) TreePiece {
+    double x, y, z, rho;
+    double a1, a2;               // loopons: half extents along e1 and e2 about x, y, z
+    double e1[3], e2[3];
+    double size;                 // loopons: half edge of the patch's square; 0 for a line piece
+    uint32_t piece, rec;         // LinePiece or LooponPiece; first LineSeg or LooponRec (a leaf's)
+    int32_t terms;               // segments or loopons
+    int32_t parent;              // the patch that holds this one, or -1
+    int32_t leaf0, leaves;       // loopons: the finest patches it holds (consecutive)
+};
+static_assert(sizeof(TreePiece) == 128, "tree piece layout");
 
 struct Chunk {
     uint64_t offset;      // byte offset of the chunk in the table
@@ -158,11 +173,10 @@ struct HostTable {
     uint64_t aux_pieces = 0, aux_segs = 0;
     // line tables: byte offset of the raw vertex triplets (0 when absent)
     uint64_t aux_raw = 0;
-    // line tables of a plan: byte offset of the tree pieces (tree.cuh; 0 when
-    // absent), and their radii and segment counts for the choice of cells
+    // FP64 tables of a plan: byte offset of the tree pieces (tree.cuh; 0 when
+    // absent) and a copy of them for the choice of cells
     uint64_t aux_tree = 0;
-    std::vector<double> tree_rho;
-    std::vector<int32_t> tree_terms;
+    std::vector<TreePiece> tree;
 };
 
 // Appends a line table's raw vertex triplets after its chunks (sets aux_raw).
@@ -172,8 +186,10 @@ void append_raw(HostTable& T, const std::vector<double>& raw);
 // kLooponKind: the others); returns DISCO_OK or an error code.
 // stage_cap: 0 = automatic chunking, > 0 = streamed chunks of at most stage_cap
 // bytes (which must hold the largest piece: 20.6 KB line, 46.2 KB loopon).
+// tree: loopons in quadtree order with their tree pieces (the caller appends
+// them: append_tree_pieces).
 int build_table(const disco_loop* loops, int nloops, int kind, int precision, double nu,
-                HostTable& out, std::string& err, uint32_t stage_cap = 0);
+                HostTable& out, std::string& err, uint32_t stage_cap = 0, bool tree = false);
 int build_table_fp32(const disco_loop* loops, int nloops, int kind, double nu, HostTable& out,
                      std::string& err, uint32_t stage_cap = 0);
 

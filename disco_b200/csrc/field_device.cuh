@@ -253,17 +253,18 @@ __device__ __forceinline__ void line_piece_plane(const LinePiece& pc, const doub
 // is fac fb (alpha n + beta m + gamma rho) with alpha = c2 ir mr,
 // beta = c2 ir nr, gamma = ir (3 mr nr ir^2 - c2 b_n); fb factors out of the
 // sum over the piece's loopons.  1/rho from the kernels' own rsqrt.
-__device__ __forceinline__ void loopon_piece_fp64(const LooponPiece& pc, const LooponRec* __restrict__ rec,
+// kWeighted: each record's term times its weight.  Records first, first + step, ...
+template <bool kWeighted = false>
+__device__ __forceinline__ void loopon_terms_fp64(const LooponPiece& pc, const LooponRec* __restrict__ rec, int n,
                                                   double Px, double Py, double Pz, double c2,
-                                                  double& ux, double& uy, double& uz)
+                                                  double& ux, double& uy, double& uz, int first = 0, int step = 1)
 {
     const double mP = pc.mx * Px + pc.my * Py + pc.mz * Pz;
     const double nP = pc.nx * Px + pc.ny * Py + pc.nz * Pz;
     const double c2bn = c2 * pc.b_n;
     double dx = 0.0, dy = 0.0, dz = 0.0;
-    const int n = pc.n;
 #pragma unroll 2
-    for (int k = 0; k < n; ++k) {
+    for (int k = first; k < n; k += step) {
         const LooponRec l = rec[k];
         const double rx = Px - l.x, ry = Py - l.y, rz = Pz - l.z;
         const double r2 = rx * rx + ry * ry + rz * rz;
@@ -274,7 +275,7 @@ __device__ __forceinline__ void loopon_piece_fp64(const LooponPiece& pc, const L
         const double cir = c2 * ir;
         const double al = cir * mr, be = cir * nr;
         const double ga = ir * fma(3.0 * mr * nr, ir2, -c2bn);
-        const double fac = keep ? ir2 : 0.0;
+        const double fac = keep ? (kWeighted ? ir2 * l.w : ir2) : 0.0;
         dx = fma(fac, fma(al, pc.nx, fma(be, pc.mx, ga * rx)), dx);
         dy = fma(fac, fma(al, pc.ny, fma(be, pc.my, ga * ry)), dy);
         dz = fma(fac, fma(al, pc.nz, fma(be, pc.mz, ga * rz)), dz);
@@ -282,6 +283,13 @@ __device__ __forceinline__ void loopon_piece_fp64(const LooponPiece& pc, const L
     ux = fma(pc.fbx, dx, ux);
     uy = fma(pc.fby, dy, uy);
     uz = fma(pc.fbz, dz, uz);
+}
+
+__device__ __forceinline__ void loopon_piece_fp64(const LooponPiece& pc, const LooponRec* __restrict__ rec,
+                                                  double Px, double Py, double Pz, double c2,
+                                                  double& ux, double& uy, double& uz)
+{
+    loopon_terms_fp64(pc, rec, pc.n, Px, Py, Pz, c2, ux, uy, uz);
 }
 
 // ---- the two FP64 policies ----------------------------------------------------------------

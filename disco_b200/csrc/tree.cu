@@ -1,7 +1,7 @@
-// The sum over loops and images by cells (line method).
+// The sum over loops and images by cells.
 //
 // Away from a loop its displacement is smooth, and nearly all of the sum's
-// (piece, image) pairs are far from any given atom.  So the atoms' bounding
+// (source, image) pairs are far from any given atom.  So the atoms' bounding
 // box is cut into cells, level by level; a pair that is far from a cell (but
 // was not far from the cell around it on the level before) is evaluated, by
 // the same closed form in FP64, at the q^3 Chebyshev points of that cell
@@ -10,13 +10,21 @@
 // evaluates once.  What is far from no cell around the atom is summed at the
 // atom itself, exactly as the plain kernels do it.
 //
-// "Far" is per axis: |cell centre - piece centre - image shift| >
+// A source is a line piece, or a square of a loop's loopons (quadtree): the
+// field is as smooth in the loopon's place, so from afar a square acts as
+// q x q equivalent loopons.  The squares shrink with the cells, and at the
+// atoms themselves the squares that are far enough from a final cell for
+// their equivalents are taken first, the rest loopon by loopon.
+//
+// "Far" is per axis: |cell centre - source centre - image shift| >
 // theta(q) h + rho along some axis, with h the cell's half width (the largest
-// over the axes) and rho the radius of the ball around the piece's apex that
-// holds its vertices.  The near images of a piece are then a box of indices,
-// (2I + 1)^3 cut by three intervals, and a cell's table holds one packed box
-// per piece.  The boxes are nested by intersection (cell in cell), so every
-// (atom, piece, image) enters exactly once, on whatever level.
+// over the axes) and rho the radius of the ball that holds the source (a line
+// piece's apex and vertices, a square's loopons); for equivalent loopons also
+// > h + theta(q) A, A the square's half extent.  The near images of a source
+// are then a box of indices, (2I + 1)^3 cut by three intervals, and a cell's
+// table holds one packed box per source.  The boxes are nested by intersection
+// (cell in cell, square in square), so every (atom, term, image) enters exactly
+// once, on whatever level.
 //
 // theta(q): interpolation at q Chebyshev points converges like the Bernstein
 // ellipse's parameter to the power -q, and theta is where the measured worst
@@ -24,13 +32,14 @@
 // half width falls below 4e-15 A for |b| = 2.5 A (plus 3 to 10 %), under the
 // rounding of the direct sum (1e-14 A).
 //
-// FP64 line tables only: the FP32 compensated form's own rounding (1e-6 A) is
+// FP64 tables only: the FP32 compensated form's own rounding (1e-6 A) is
 // part of what it returns, and its far terms summed in FP64 would change it.
 //
 // Measured against the plain kernel on one B200 (ms a call): FCC 100^3 cells
 // (4.0 M atoms), 16 loops, +-2 images 986 -> 15.3; BCC 61 x 47 x 33 (184 k
 // atoms), 9 loops, +-3 86.9 -> 9.5; BCC 40^3 (128 k), 4 loops of 64 segments,
-// +-1 4.94 -> 3.34.  A sum too small to gain (2 000 atoms, 2 loops: 0.02 ms of
+// +-1 4.94 -> 3.33; loopons: BCC 40^3 (127 k), 8 prismatic loops of R 20 to 50
+// (39 k loopons), +-1 255 -> 57.  A sum too small to gain (2 000 atoms, 2 loops: 0.02 ms of
 // terms) stays with the plain kernel: tree_shape compares operation counts of
 // both, launches included.
 //
@@ -74,24 +83,33 @@ struct LevelArgs {
     int32_t tiles;            // warp tiles per cell
     int64_t tile0;            // first warp tile of the level
     int64_t cell0;            // first cell of the level (tables, occupancy)
-    double theta;
+    double theta, cut;
+    int32_t np;               // sources of the level
+    int64_t near0;            // first entry in the table of near boxes: [cell][source]
+    int64_t list0;            // first entry in the lists of sources
     double* val;              // [cell][3][q3]
+    LooponRec* eq;            // [source][q q]: equivalent loopons
 };
 
 struct TreeArgs {
     FieldArgs f;
     const TreePiece* pieces;
-    int32_t np;
-    int32_t levels;
+    int32_t nodes;            // tree pieces
+    int32_t* list;            // [level][source]: tree piece
+    int32_t* up;              // [level][source]: the source on the level before that holds it
+    int32_t* pos;             // [level][tree piece]: its place in the level's list
+    int32_t levels, total;    // levels of cells; with the levels summed at the atoms
     LevelArgs lv[TreeShape::kMaxLevels];
     int32_t mf[3], qf;        // final cells
     int32_t rf[3];            // final cells per axis in a cell of the last level
     int32_t cells_s, cells_f; // cells of the last level, final cells
+    int32_t cells_n, near_rr; // cells of the near pass, final cells in each of them
     int32_t near_split;
     int32_t images;
     int64_t level_cells;      // cells over all levels
     unsigned long long* box;  // 6: ordered bits of min x, y, z and max x, y, z
-    uint64_t* near;           // [level cell][piece]: packed box of near images
+    uint64_t* near;           // [level cell][source]: packed box of near images
+    int64_t near_size;
     uint8_t* occ;             // [level cell]: holds atoms
     uint32_t* key[2];         // [atom], [slot]: final cell, the sort's two buffers
     int32_t* idx[2];          // the atoms that go with them
@@ -99,7 +117,7 @@ struct TreeArgs {
     uint32_t* digit_total;    // [256]
     int32_t sort_tiles;
     uint32_t* start;          // [final cell + 2]: first sorted slot
-    uint32_t* near_tile;      // [last-level cell + 2]: first warp tile of the near pass
+    uint32_t* near_tile;      // [near cell + 2]: first warp tile of the near pass
     const int32_t* perm;      // sorted slot -> atom
     double* mat;              // interpolation matrices, transition by transition
     int32_t mat_off[TreeShape::kMaxLevels + 1][3];
@@ -178,6 +196,14 @@ __device__ __forceinline__ int final_index(const TreeArgs& a, const int (&c)[3])
 {
     const int sub = ((c[0] % a.rf[0]) * a.rf[1] + c[1] % a.rf[1]) * a.rf[2] + c[2] % a.rf[2];
     return last_index(a, c) * (a.rf[0] * a.rf[1] * a.rf[2]) + sub;
+}
+__device__ __forceinline__ void final_cell(const TreeArgs& a, int index, int (&c)[3])
+{
+    const LevelArgs& L = a.lv[a.levels - 1];
+    const int rr = a.rf[0] * a.rf[1] * a.rf[2], s = index / rr, sub = index % rr;
+    c[0] = (s / (L.m[1] * L.m[2])) * a.rf[0] + sub / (a.rf[1] * a.rf[2]);
+    c[1] = (s / L.m[2] % L.m[1]) * a.rf[1] + sub / a.rf[2] % a.rf[1];
+    c[2] = (s % L.m[2]) * a.rf[2] + sub % a.rf[2];
 }
 __device__ __forceinline__ int cell_of(const TreeArgs& a, const Geo& g, double x, double y, double z)
 {
@@ -363,22 +389,14 @@ __global__ void __launch_bounds__(256) tree_starts_kernel(const TreeArgs a, cons
     }
 }
 
-// Warp tiles of the near pass, by the last level's cells (plus the outside
-// cell), and which cells of each level hold atoms; one CTA.
+// Warp tiles of the near pass, by its cells (plus the outside cell), and which
+// cells of each level hold atoms; one CTA.
 __global__ void __launch_bounds__(1024) tree_scan_kernel(const TreeArgs a)
 {
-    const int nf = a.cells_f + 1;
     const int rr = a.rf[0] * a.rf[1] * a.rf[2];
-    const int ns = a.cells_s + 1, per = (ns + 1023) / 1024;
-    const int s0 = min(ns, (int)threadIdx.x * per), s1 = min(ns, s0 + per);
-    const uint32_t per_tile = 32u / (uint32_t)a.near_split;
     const LevelArgs& E = a.lv[a.levels - 1];
-    auto atoms_of = [&](int s) { return a.start[s < a.cells_s ? (s + 1) * rr : nf] - a.start[s * rr]; };
-    uint32_t mine = 0, tot;
-    for (int s = s0; s < s1; ++s) {
-        const uint32_t k = atoms_of(s);
-        mine += (k + per_tile - 1) / per_tile;
-        if (k == 0 || s == a.cells_s) continue;
+    for (int s = threadIdx.x; s < a.cells_s; s += 1024) {
+        if (a.start[(s + 1) * rr] == a.start[s * rr]) continue;
         const int c[3] = { s / (E.m[1] * E.m[2]), s / E.m[2] % E.m[1], s % E.m[2] };
         for (int l = 0; l < a.levels; ++l) {
             const LevelArgs& L = a.lv[l];
@@ -387,11 +405,20 @@ __global__ void __launch_bounds__(1024) tree_scan_kernel(const TreeArgs a)
             a.occ[L.cell0 + lc] = 1;
         }
     }
+    const int ns = a.cells_n + 1, per = (ns + 1023) / 1024;
+    const int s0 = min(ns, (int)threadIdx.x * per), s1 = min(ns, s0 + per);
+    const uint32_t per_tile = 32u / (uint32_t)a.near_split;
+    auto tiles_of = [&](int s) {
+        const uint32_t k = a.start[s < a.cells_n ? (s + 1) * a.near_rr : a.cells_f + 1] - a.start[s * a.near_rr];
+        return (k + per_tile - 1) / per_tile;
+    };
+    uint32_t mine = 0, tot;
+    for (int s = s0; s < s1; ++s) mine += tiles_of(s);
     uint32_t at = block_scan(mine, &tot);
     if (threadIdx.x == 0) a.near_tile[ns] = tot;
     for (int s = s0; s < s1; ++s) {
         a.near_tile[s] = at;
-        at += (atoms_of(s) + per_tile - 1) / per_tile;
+        at += tiles_of(s);
     }
 }
 
@@ -472,29 +499,88 @@ struct ImgShell {
     }
 };
 
-// One thread per (level cell, piece): the intersection of the near boxes of
-// the cell and of the cells around it on the levels before.
+// A tree piece is a source of a level whose cut its square fits and the one
+// above it does not.
+__device__ __forceinline__ bool in_cut(const TreeArgs& a, const TreePiece& t, int self, double cut)
+{
+    const bool fits = t.size <= cut || t.leaf0 == self;
+    return fits && (t.parent < 0 || a.pieces[t.parent].size > cut);
+}
+
+// One CTA per level: its sources in order.
+__global__ void __launch_bounds__(1024) tree_list_kernel(const TreeArgs a)
+{
+    const LevelArgs& v = a.lv[blockIdx.x];
+    uint32_t at = 0;
+    for (int n0 = 0; n0 < a.nodes; n0 += 1024) {
+        const int n = n0 + threadIdx.x;
+        const bool in = n < a.nodes && in_cut(a, a.pieces[n], n, v.cut);
+        uint32_t tot;
+        const uint32_t k = at + block_scan(in ? 1u : 0u, &tot);
+        if (in && k < (uint32_t)v.np) {
+            a.list[v.list0 + k] = n;
+            a.pos[(int64_t)blockIdx.x * a.nodes + n] = (int32_t)k;
+        }
+        at += tot;
+    }
+}
+
+// The tree piece that holds n (or n itself) among the sources of a level with
+// a coarser (or the same) cut.
+__device__ __forceinline__ int holder(const TreeArgs& a, int n, double cut)
+{
+    for (;;) {
+        const int up = a.pieces[n].parent;
+        if (up < 0 || a.pieces[up].size > cut) return n;
+        n = up;
+    }
+}
+
+// Whether a source is summed through its q x q equivalent loopons: a square
+// that holds others, or a leaf with more loopons than that.
+__device__ __forceinline__ bool uses_eq(const LevelArgs& v, const TreePiece& t, int self)
+{
+    return v.eq != nullptr && (t.leaf0 != self || t.terms > v.q * v.q);
+}
+
+// One thread per (level cell, source): the intersection of the near boxes of
+// the cell and of the cells around it on the levels before, each for the
+// source there that holds this one.  Equivalent loopons hold from
+// theta(q) half extents of the square on, so where they are used the cell has
+// to be that far as well; a level summed at the atoms asks for nothing else.
 __global__ void __launch_bounds__(256) tree_near_kernel(const TreeArgs a)
 {
     const Geo g = load_geo(a);
     const double L[3] = { a.f.Lx, a.f.Ly, a.f.Lz };
-    const int64_t total = a.level_cells * a.np;
-    for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t lc = t / a.np;
-        const int p = (int)(t - lc * a.np);
-        int k = a.levels - 1;
-        while (a.lv[k].cell0 > lc) --k;
-        const int c = (int)(lc - a.lv[k].cell0);
-        const TreePiece& tp = a.pieces[p];
-        const double s[3] = { tp.x, tp.y, tp.z };
-        const int ci[3] = { c / (a.lv[k].m[1] * a.lv[k].m[2]), c / a.lv[k].m[2] % a.lv[k].m[1], c % a.lv[k].m[2] };
+    for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < a.near_size;
+         t += (int64_t)gridDim.x * blockDim.x) {
+        int k = a.total - 1;
+        while (a.lv[k].near0 > t) --k;
+        const int64_t local = t - a.lv[k].near0;
+        const int c = (int)(local / a.lv[k].np), e = (int)(local % a.lv[k].np);
+        int ci[3];
+        if (k < a.levels) {
+            ci[0] = c / (a.lv[k].m[1] * a.lv[k].m[2]);
+            ci[1] = c / a.lv[k].m[2] % a.lv[k].m[1];
+            ci[2] = c % a.lv[k].m[2];
+        } else {
+            final_cell(a, c, ci);
+        }
         int lo[3], hi[3];
         for (int d = 0; d < 3; ++d) { lo[d] = -a.images; hi[d] = a.images; }
-        for (int j = 0; j <= k; ++j) {
+        int n = a.list[a.lv[k].list0 + e];
+        for (int j = k; j >= 0; --j) {
             const LevelArgs& v = a.lv[j];
+            n = holder(a, n, v.cut);
+            if (j == k - 1 && c == 0) a.up[a.lv[k].list0 + e] = a.pos[(int64_t)j * a.nodes + n];
+            const TreePiece& tp = a.pieces[n];
             double h = 0.0;
             for (int d = 0; d < 3; ++d) h = fmax(h, 0.5 * g.ext[d] / v.m[d]);
-            const double R = v.theta * h + tp.rho;
+            const bool eq = uses_eq(v, tp, n);
+            if (j >= a.levels && !eq) continue;           // summed at the atoms one by one
+            double R = j < a.levels ? v.theta * h + tp.rho : 0.0;
+            if (eq) R = fmax(R, h + v.theta * fmax(tp.a1, tp.a2));
+            const double s[3] = { tp.x, tp.y, tp.z };
             for (int d = 0; d < 3; ++d) {
                 const int cj = ci[d] / (a.lv[k].m[d] / v.m[d]);
                 const double cc = g.lo[d] + (cj + 0.5) * (g.ext[d] / v.m[d]) - s[d];
@@ -513,11 +599,89 @@ __global__ void __launch_bounds__(256) tree_near_kernel(const TreeArgs a)
     }
 }
 
+// Equivalent loopons of a square: the field is smooth in the loopon's place
+// too, so from afar the square's loopons act as q x q loopons at the Chebyshev
+// points of its extent, weighted by the sums of the interpolation weights of
+// all its loopons: with the moments M_ab = sum T_a(x) T_b(y) over the loopons,
+// w_ij = sum_ab c_a T_a(x_i) c_b T_b(x_j) M_ab, c_0 = 1/q, c_a = 2/q.  One CTA
+// per source, a moment per thread; the loopons come in batches of 64.
+constexpr int kMaxQ = 21;
+constexpr int kEqThreads = 448;                    // 21 x 21 and whole warps
+__global__ void __launch_bounds__(kEqThreads) tree_equivalent_kernel(const TreeArgs a)
+{
+    const LevelArgs& v = a.lv[blockIdx.y];
+    if (v.eq == nullptr || blockIdx.x >= (unsigned)v.np) return;
+    const int self = a.list[v.list0 + blockIdx.x];
+    const TreePiece& tp = a.pieces[self];
+    if (!uses_eq(v, tp, self)) return;
+    constexpr int kBatch = 64;
+    __shared__ double cq[4 * kMaxQ], T1[kBatch][kMaxQ], T2[kBatch][kMaxQ];
+    const int q = v.q, t = threadIdx.x, ma = t / q, mb = t % q;
+    for (int e = t; e < 4 * q; e += kEqThreads) cq[e] = cospi(e / (2.0 * q));
+    const LooponPiece& pc = *reinterpret_cast<const LooponPiece*>(a.f.table + tp.piece);
+    const double ox = tp.x - pc.cx, oy = tp.y - pc.cy, oz = tp.z - pc.cz;
+    const double i1 = tp.a1 > 0.0 ? 1.0 / tp.a1 : 0.0, i2 = tp.a2 > 0.0 ? 1.0 / tp.a2 : 0.0;
+    double acc = 0.0;
+    for (int leaf = tp.leaf0; leaf < tp.leaf0 + tp.leaves; ++leaf) {
+        const LooponRec* rec = reinterpret_cast<const LooponRec*>(a.f.table + a.pieces[leaf].rec);
+        const int terms = a.pieces[leaf].terms;
+        for (int k0 = 0; k0 < terms; k0 += kBatch) {
+            const int nb = min(kBatch, terms - k0);
+            __syncthreads();
+            if (t < 2 * nb) {
+                const bool y = t >= nb;
+                const int k = y ? t - nb : t;
+                const LooponRec& r = rec[k0 + k];
+                const double* d = y ? tp.e2 : tp.e1;
+                double x = (d[0] * (r.x - ox) + d[1] * (r.y - oy) + d[2] * (r.z - oz)) * (y ? i2 : i1);
+                x = fmin(fmax(x, -1.0), 1.0);
+                double* T = y ? T2[k] : T1[k];
+                double t0 = 1.0, t1 = x;
+                for (int i = 0; i < q; ++i) {
+                    T[i] = t0;
+                    const double t2 = fma(2.0 * x, t1, -t0);
+                    t0 = t1;
+                    t1 = t2;
+                }
+            }
+            __syncthreads();
+            if (ma < q)
+                for (int k = 0; k < nb; ++k) acc = fma(T1[k][ma], T2[k][mb], acc);
+        }
+    }
+    __syncthreads();
+    // c_a T_a(x_i), the moments over b, then over a
+    double (*M)[kMaxQ] = T1, (*R)[kMaxQ] = T2;
+    if (ma < q) M[ma][mb] = acc;
+    __syncthreads();
+    const int wi = ma, wj = mb;
+    if (ma < q) {
+        double s = 0.0;
+        for (int b = 0; b < q; ++b) s = fma((b ? 2.0 : 1.0) / q * cq[(b * (2 * wj + 1)) % (4 * q)], M[ma][b], s);
+        R[ma][wj] = s;
+    }
+    __syncthreads();
+    if (wi < q) {
+        double s = 0.0;
+        for (int k = 0; k < q; ++k) s = fma((k ? 2.0 : 1.0) / q * cq[(k * (2 * wi + 1)) % (4 * q)], R[k][wj], s);
+        const double t1 = tp.a1 * cq[2 * wi + 1], t2 = tp.a2 * cq[2 * wj + 1];
+        LooponRec r;
+        r.x = ox + t1 * tp.e1[0] + t2 * tp.e2[0];
+        r.y = oy + t1 * tp.e1[1] + t2 * tp.e2[1];
+        r.z = oz + t1 * tp.e1[2] + t2 * tp.e2[2];
+        r.ml = pc.mx * r.x + pc.my * r.y + pc.mz * r.z;
+        r.nl = pc.nx * r.x + pc.ny * r.y + pc.nz * r.z;
+        r.w = s;
+        v.eq[(int64_t)blockIdx.x * q * q + t] = r;
+    }
+}
+
 // ---- node sums ---------------------------------------------------------------------------
 
 // One warp: 32 / split nodes of one cell; its far pairs are those in the near
 // boxes of the level before and not in its own.  FP64 bound like the plain
 // line kernel (records are read through L1 as warp-uniform 16-byte loads).
+template <int kKind>
 __global__ void __launch_bounds__(32 * kWarps, 4) tree_node_kernel(const TreeArgs a)
 {
     const int lane = threadIdx.x & 31;
@@ -543,21 +707,21 @@ __global__ void __launch_bounds__(32 * kWarps, 4) tree_node_kernel(const TreeArg
         const double e = g.ext[d] / v.m[d];
         P[d] = g.lo[d] + (ci[d] + 0.5) * e + 0.5 * e * cospi((2 * ni[d] + 1) / (2.0 * v.q));
     }
-    const uint64_t* own = a.near + (v.cell0 + cell) * (int64_t)a.np;
+    const uint64_t* own = a.near + v.near0 + (int64_t)cell * v.np;
     const uint64_t* up = nullptr;
     if (k > 0) {
         const LevelArgs& u = a.lv[k - 1];
         const int uc = ((ci[0] / v.r[0]) * u.m[1] + ci[1] / v.r[1]) * u.m[2] + ci[2] / v.r[2];
-        up = a.near + (u.cell0 + uc) * (int64_t)a.np;
+        up = a.near + u.near0 + (int64_t)uc * u.np;
     }
     const uint64_t all = full_box(a.images);
     const double cJK = a.f.cJ / a.f.cK;
     double ux = 0.0, uy = 0.0, uz = 0.0;
     bool plane = false;
-    for (int base = 0; base < a.np; base += 32) {
+    for (int base = 0; base < v.np; base += 32) {
         uint64_t wu = 0, wo = 0;
-        if (base + lane < a.np) {
-            wu = up ? up[base + lane] : all;
+        if (base + lane < v.np) {
+            wu = up ? up[a.up[v.list0 + base + lane]] : all;
             wo = own[base + lane];
         }
         unsigned todo = __ballot_sync(0xffffffffu, wu != 0 && wu != wo);
@@ -565,15 +729,31 @@ __global__ void __launch_bounds__(32 * kWarps, 4) tree_node_kernel(const TreeArg
             const int b = __ffs(todo) - 1;
             todo &= todo - 1;
             const uint64_t bu = __shfl_sync(0xffffffffu, wu, b), bo = __shfl_sync(0xffffffffu, wo, b);
-            const TreePiece& tp = a.pieces[base + b];
-            const LinePiece& pc = *reinterpret_cast<const LinePiece*>(a.f.table + tp.piece);
-            const LineSeg* seg = reinterpret_cast<const LineSeg*>(a.f.table + tp.rec);
+            const int self = a.list[v.list0 + base + b];
+            const TreePiece& tp = a.pieces[self];
             const ImgShell far(bu, bo);
-            for (int idx = part; idx < far.total; idx += split) {
-                int i, j, l;
-                far.at(idx, i, j, l);
-                line_piece_fp64<true>(pc, seg, P[0] - a.f.Lx * i, P[1] - a.f.Ly * j, P[2] - a.f.Lz * l, cJK, ux, uy,
-                                      uz, plane);
+            if constexpr (kKind == kLineKind) {
+                const LinePiece& pc = *reinterpret_cast<const LinePiece*>(a.f.table + tp.piece);
+                const LineSeg* seg = reinterpret_cast<const LineSeg*>(a.f.table + tp.rec);
+                for (int idx = part; idx < far.total; idx += split) {
+                    int i, j, l;
+                    far.at(idx, i, j, l);
+                    line_piece_fp64<true>(pc, seg, P[0] - a.f.Lx * i, P[1] - a.f.Ly * j, P[2] - a.f.Lz * l, cJK, ux,
+                                          uy, uz, plane);
+                }
+            } else {
+                const LooponPiece& pc = *reinterpret_cast<const LooponPiece*>(a.f.table + tp.piece);
+                const bool eq = uses_eq(v, tp, self);
+                const LooponRec* rec = eq ? v.eq + (int64_t)(base + b) * v.q * v.q
+                                          : reinterpret_cast<const LooponRec*>(a.f.table + tp.rec);
+                const int n = eq ? v.q * v.q : tp.terms;
+                const double qx = P[0] - pc.cx, qy = P[1] - pc.cy, qz = P[2] - pc.cz;
+                for (int idx = 0; idx < far.total; ++idx) {
+                    int i, j, l;
+                    far.at(idx, i, j, l);
+                    loopon_terms_fp64<true>(pc, rec, n, qx - a.f.Lx * i, qy - a.f.Ly * j, qz - a.f.Lz * l, a.f.c2, ux,
+                                            uy, uz, part, split);
+                }
             }
         }
     }
@@ -597,8 +777,6 @@ __global__ void __launch_bounds__(32 * kWarps, 4) tree_node_kernel(const TreeArg
 // parent's value at its node i to the child's node j (final: to the child's
 // Chebyshev coefficient j).  Interpolation at q Chebyshev points is
 // f(x) = sum_i f_i (1/q) (1 + 2 sum_k T_k(x_i) T_k(x)).
-constexpr int kMaxQ = 21;
-
 // cq[t] = cos(pi t / (2 q)), t < 4 q
 __device__ __forceinline__ double interp_weight(const double* cq, int q, int i, double x)
 {
@@ -876,63 +1054,121 @@ __device__ __forceinline__ int cell_of_tile(const uint32_t* first, int cells, ui
 
 // ---- near pairs --------------------------------------------------------------------------
 
-// The pieces with near images of one cell, 32 at a time; F(piece, box) for each.
+// The sources of the last level with near images of one near cell, 32 at a time;
+// F(tree piece, box) for each.
 template <class F>
-__device__ __forceinline__ void for_near(const TreeArgs& a, int scell, F f)
+__device__ __forceinline__ void for_near(const TreeArgs& a, int cell, F f)
 {
     const int lane = threadIdx.x & 31;
     const uint64_t all = full_box(a.images);
-    const uint64_t* own = scell < a.cells_s ? a.near + (a.lv[a.levels - 1].cell0 + scell) * (int64_t)a.np : nullptr;
-    for (int base = 0; base < a.np; base += 32) {
+    const LevelArgs& v = a.lv[a.total - 1];
+    // boxes by final cell on the levels summed at the atoms, by the last level's
+    // cell where there are none
+    const int row = a.total > a.levels ? cell : cell / (a.cells_n / a.cells_s);
+    const uint64_t* own = cell < a.cells_n ? a.near + v.near0 + (int64_t)row * v.np : nullptr;
+    for (int base = 0; base < v.np; base += 32) {
         uint64_t w = 0;
-        if (base + lane < a.np) w = own ? own[base + lane] : all;
+        if (base + lane < v.np) w = own ? own[base + lane] : all;
         unsigned todo = __ballot_sync(0xffffffffu, w != 0);
         while (todo) {
             const int b = __ffs(todo) - 1;
             todo &= todo - 1;
-            f(a.pieces[base + b], ImgBox(__shfl_sync(0xffffffffu, w, b)));
+            f(a.pieces[a.list[v.list0 + base + b]], ImgBox(__shfl_sync(0xffffffffu, w, b)));
         }
     }
 }
 
-// One warp: 32 / near_split atoms of one cell of the last level (or atoms
-// outside the grid, which take every image), lanes of an atom splitting the
-// images of each piece.
+// One warp: 32 / near_split atoms of one near cell (or atoms outside the grid,
+// which take every image), lanes of an atom splitting the images of each
+// piece (line) or the loopons of each source.
+template <int kKind>
 __global__ void __launch_bounds__(32 * kWarps, 4) tree_near_sum_kernel(const TreeArgs a)
 {
     const int lane = threadIdx.x & 31;
     const uint32_t w = blockIdx.x * kWarps + (threadIdx.x >> 5);
-    if (w >= a.near_tile[a.cells_s + 1]) return;
-    const int cell = cell_of_tile(a.near_tile, a.cells_s + 1, w);
+    if (w >= a.near_tile[a.cells_n + 1]) return;
+    const int cell = cell_of_tile(a.near_tile, a.cells_n + 1, w);
     const int split = a.near_split, part = lane % split;
-    const int rr = a.rf[0] * a.rf[1] * a.rf[2];
-    const uint32_t s1 = a.start[cell < a.cells_s ? (cell + 1) * rr : a.cells_f + 1];
-    const uint32_t slot = a.start[cell * rr] + (w - a.near_tile[cell]) * (32 / split) + lane / split;
+    const uint32_t s1 = a.start[cell < a.cells_n ? (cell + 1) * a.near_rr : a.cells_f + 1];
+    const uint32_t slot = a.start[cell * a.near_rr] + (w - a.near_tile[cell]) * (32 / split) + lane / split;
     const bool valid = slot < s1;
     const int64_t atom = a.perm[valid ? slot : s1 - 1];
     const double px = a.f.x[atom], py = a.f.y[atom], pz = a.f.z[atom];
-    const double cJK = a.f.cJ / a.f.cK;
     double ux = 0.0, uy = 0.0, uz = 0.0;
-    bool plane = false;
-    for_near(a, cell, [&](const TreePiece& tp, const ImgBox& B) {
-        const LinePiece& pc = *reinterpret_cast<const LinePiece*>(a.f.table + tp.piece);
-        const LineSeg* seg = reinterpret_cast<const LineSeg*>(a.f.table + tp.rec);
-        const int cnt = B.count();
-        for (int idx = part; idx < cnt; idx += split) {
-            int i, j, k;
-            B.at(idx, i, j, k);
-            line_piece_fp64(pc, seg, px - a.f.Lx * i, py - a.f.Ly * j, pz - a.f.Lz * k, cJK, ux, uy, uz, plane);
-        }
-    });
-    if (__any_sync(0xffffffffu, plane)) {         // atoms in a loop's plane band: the reference's solid angle
+    if constexpr (kKind == kLineKind) {
+        const double cJK = a.f.cJ / a.f.cK;
+        bool plane = false;
         for_near(a, cell, [&](const TreePiece& tp, const ImgBox& B) {
             const LinePiece& pc = *reinterpret_cast<const LinePiece*>(a.f.table + tp.piece);
+            const LineSeg* seg = reinterpret_cast<const LineSeg*>(a.f.table + tp.rec);
             const int cnt = B.count();
             for (int idx = part; idx < cnt; idx += split) {
                 int i, j, k;
                 B.at(idx, i, j, k);
-                if (plane)
-                    line_piece_plane(pc, a.f.raw, px - a.f.Lx * i, py - a.f.Ly * j, pz - a.f.Lz * k, ux, uy, uz);
+                line_piece_fp64(pc, seg, px - a.f.Lx * i, py - a.f.Ly * j, pz - a.f.Lz * k, cJK, ux, uy, uz, plane);
+            }
+        });
+        if (__any_sync(0xffffffffu, plane)) {         // atoms in a loop's plane band: the reference's solid angle
+            for_near(a, cell, [&](const TreePiece& tp, const ImgBox& B) {
+                const LinePiece& pc = *reinterpret_cast<const LinePiece*>(a.f.table + tp.piece);
+                const int cnt = B.count();
+                for (int idx = part; idx < cnt; idx += split) {
+                    int i, j, k;
+                    B.at(idx, i, j, k);
+                    if (plane)
+                        line_piece_plane(pc, a.f.raw, px - a.f.Lx * i, py - a.f.Ly * j, pz - a.f.Lz * k, ux, uy, uz);
+                }
+            });
+        }
+    } else {
+        // squares far enough from the cell for their equivalent loopons
+        for (int l = a.levels; l < a.total && cell < a.cells_n; ++l) {
+            const LevelArgs &v = a.lv[l], &u = a.lv[l - 1];
+            const uint64_t* own = a.near + v.near0 + (int64_t)cell * v.np;
+            const uint64_t* up = a.near + u.near0 + (int64_t)(l > a.levels ? cell : cell / (a.cells_n / a.cells_s)) * u.np;
+            const int q2 = v.q * v.q;
+            for (int base = 0; base < v.np; base += 32) {
+                uint64_t wu = 0, wo = 0;
+                if (base + lane < v.np) {
+                    wu = up[a.up[v.list0 + base + lane]];
+                    wo = own[base + lane];
+                }
+                unsigned todo = __ballot_sync(0xffffffffu, wu != 0 && wu != wo);
+                while (todo) {
+                    const int b = __ffs(todo) - 1;
+                    todo &= todo - 1;
+                    const ImgShell far(__shfl_sync(0xffffffffu, wu, b), __shfl_sync(0xffffffffu, wo, b));
+                    const int self = a.list[v.list0 + base + b];
+                    const TreePiece& tp = a.pieces[self];
+                    const bool eq = uses_eq(v, tp, self);
+                    const LooponRec* rec = eq ? v.eq + (int64_t)(base + b) * q2
+                                              : reinterpret_cast<const LooponRec*>(a.f.table + tp.rec);
+                    const int n = eq ? q2 : tp.terms;
+                    const LooponPiece& pc = *reinterpret_cast<const LooponPiece*>(a.f.table + tp.piece);
+                    const double qx = px - pc.cx, qy = py - pc.cy, qz = pz - pc.cz;
+                    for (int idx = 0; idx < far.total; ++idx) {
+                        int i, j, k;
+                        far.at(idx, i, j, k);
+                        loopon_terms_fp64<true>(pc, rec, n, qx - a.f.Lx * i, qy - a.f.Ly * j, qz - a.f.Lz * k,
+                                                a.f.c2, ux, uy, uz, part, split);
+                    }
+                }
+            }
+        }
+        // what is left: the squares' loopons one by one
+        for_near(a, cell, [&](const TreePiece& tp, const ImgBox& B) {
+            const LooponPiece& pc = *reinterpret_cast<const LooponPiece*>(a.f.table + tp.piece);
+            const double qx = px - pc.cx, qy = py - pc.cy, qz = pz - pc.cz;
+            const int cnt = B.count();
+            for (int leaf = tp.leaf0; leaf < tp.leaf0 + tp.leaves; ++leaf) {
+                const LooponRec* rec = reinterpret_cast<const LooponRec*>(a.f.table + a.pieces[leaf].rec);
+                const int n = a.pieces[leaf].terms;
+                for (int idx = 0; idx < cnt; ++idx) {
+                    int i, j, k;
+                    B.at(idx, i, j, k);
+                    loopon_terms_fp64(pc, rec, n, qx - a.f.Lx * i, qy - a.f.Ly * j, qz - a.f.Lz * k, a.f.c2, ux, uy,
+                                      uz, part, split);
+                }
             }
         });
     }
@@ -957,76 +1193,103 @@ int order_for(double theta)
     return -1;
 }
 
-// Expected near (piece, image) pairs of a cell, in segments: pieces are taken
-// as spread evenly over the box.
-double near_terms(const HostTable& T, const double box[3], int images, double reach)
+// One loop (line: one piece) by the depths of its quadtree: half edge, radius
+// and count of its squares there, and its terms.
+struct Depth { double size, rho; int squares; };
+struct Root { double terms; std::vector<Depth> depth; };
+
+std::vector<Root> roots_of(const HostTable& T)
 {
-    const double W = 2.0 * images + 1.0;
-    double sum = 0.0;
-    for (size_t p = 0; p < T.tree_rho.size(); ++p) {
-        double v = T.tree_terms[p];
-        for (int d = 0; d < 3; ++d) v *= std::min(W, 2.0 * (reach + T.tree_rho[p]) / box[d]);
-        sum += v;
+    std::vector<Root> out;
+    std::vector<int> root(T.tree.size()), level(T.tree.size());
+    for (size_t k = 0; k < T.tree.size(); ++k) {
+        const TreePiece& t = T.tree[k];
+        if (t.parent < 0) {
+            root[k] = (int)out.size();
+            level[k] = 0;
+            out.push_back({ (double)t.terms, {} });
+        } else {
+            root[k] = root[t.parent];
+            level[k] = level[t.parent] + 1;
+        }
+        std::vector<Depth>& d = out[root[k]].depth;
+        if ((int)d.size() <= level[k]) d.push_back({ t.size, 0.0, 0 });
+        Depth& e = d[level[k]];
+        e.rho = std::max(e.rho, t.rho);
+        e.squares++;
     }
-    return sum;
+    return out;
+}
+
+// The depth a cut takes a loop at.
+const Depth& depth_at(const Root& r, double cut)
+{
+    size_t k = 0;
+    while (k + 1 < r.depth.size() && r.depth[k].size > cut) ++k;
+    return r.depth[k];
 }
 
 } // namespace
 
 void append_tree_pieces(HostTable& T)
 {
-    if (T.kind != kLineKind || T.fp32 || T.chunks.empty()) return;
-    std::vector<TreePiece> out;
-    T.tree_rho.clear();
-    T.tree_terms.clear();
-    for (const Chunk& c : T.chunks) {
-        const unsigned char* base = T.bytes.data() + c.offset;
-        for (int i = 0; i < c.npieces; ++i) {
-            LinePiece p;
-            std::memcpy(&p, base + i * sizeof(p), sizeof(p));
-            TreePiece t;
-            std::memset(&t, 0, sizeof(t));
-            t.piece = (uint32_t)(c.offset + i * sizeof(p));
-            t.rec = (uint32_t)(c.offset + c.npieces * sizeof(p) + p.rec * sizeof(LineSeg));
-            t.x = p.cx; t.y = p.cy; t.z = p.cz;
-            t.rho = p.rho;
-            t.terms = p.nseg;
-            // a ball the far rule cannot use, or offsets past 32 bits: no cells
-            if (!std::isfinite(t.rho + std::fabs(t.x) + std::fabs(t.y) + std::fabs(t.z)) ||
-                T.bytes.size() > 0xFFFFFFFFull) {
-                T.tree_rho.clear();
-                T.tree_terms.clear();
-                return;
+    if (T.fp32 || T.chunks.empty()) { T.tree.clear(); return; }
+    if (T.kind == kLineKind) {
+        T.tree.clear();
+        for (const Chunk& c : T.chunks) {
+            const unsigned char* base = T.bytes.data() + c.offset;
+            for (int i = 0; i < c.npieces; ++i) {
+                LinePiece p;
+                std::memcpy(&p, base + i * sizeof(p), sizeof(p));
+                TreePiece t;
+                std::memset(&t, 0, sizeof(t));
+                t.piece = (uint32_t)(c.offset + i * sizeof(p));
+                t.rec = (uint32_t)(c.offset + c.npieces * sizeof(p) + p.rec * sizeof(LineSeg));
+                t.x = p.cx; t.y = p.cy; t.z = p.cz;
+                t.rho = p.rho;
+                t.terms = p.nseg;
+                t.parent = -1;
+                t.leaf0 = (int32_t)T.tree.size();
+                t.leaves = 1;
+                T.tree.push_back(t);
             }
-            T.tree_rho.push_back(t.rho);
-            T.tree_terms.push_back(t.terms);
-            out.push_back(t);
         }
     }
+    // a ball the far rule cannot use, or offsets past 32 bits: no cells
+    bool ok = !T.tree.empty() && T.bytes.size() <= 0xFFFFFFFFull;
+    for (const TreePiece& t : T.tree)
+        ok = ok && std::isfinite(t.rho + std::fabs(t.x) + std::fabs(t.y) + std::fabs(t.z));
+    if (!ok) { T.tree.clear(); return; }
     while (T.bytes.size() % 16) T.bytes.push_back(0);
     T.aux_tree = T.bytes.size();
-    const unsigned char* s = reinterpret_cast<const unsigned char*>(out.data());
-    T.bytes.insert(T.bytes.end(), s, s + out.size() * sizeof(TreePiece));
+    const unsigned char* s = reinterpret_cast<const unsigned char*>(T.tree.data());
+    T.bytes.insert(T.bytes.end(), s, s + T.tree.size() * sizeof(TreePiece));
 }
 
 TreeShape tree_shape(const HostTable& T, int64_t n, const double box[3], int images)
 {
     TreeShape S;
-    const int np = (int)T.tree_rho.size();
-    if (!T.aux_tree || np == 0 || n > 0x7FFFFFFF - 64) return S;
+    if (!T.aux_tree || T.tree.empty() || n > 0x7FFFFFFF - 64) return S;
+    const bool line = T.kind == kLineKind;
     // FP64 operations of a term, and a microsecond of the GPU in them (18.6e12
-    // per second at the 75 % that the line kernels reach)
-    const double e64 = 78.0, us = 1.4e7;
+    // per second at the 75 % that the field kernels reach)
+    const double e64 = line ? 78.0 : 34.0, us = 1.4e7;
     const double W = (double)(2 * images + 1), nimg = W * W * W;
+    const std::vector<Root> roots = roots_of(T);
     double terms = 0.0;
-    for (int32_t t : T.tree_terms) terms += t;
+    for (const Root& r : roots) terms += r.terms;
     const double all = terms * nimg;
     S.direct = (double)n * all * e64 + 5.0 * us;
     // the boxes' aspect: axes get m0 2^k cells
     const double lmin = std::min(box[0], std::min(box[1], box[2]));
     int m0[3];
     for (int d = 0; d < 3; ++d) m0[d] = (int)std::min(8.0, std::max(1.0, std::round(box[d] / lmin)));
-    struct State { double cost, near, h; double cells; int a, o, prev; };
+    struct State {
+        double cost, near, h, cells, cut;
+        int a, o, prev, np;
+        bool eq;
+        std::vector<double> v;       // near images of a source, per loop
+    };
     std::vector<State> st;
     constexpr int kDepth = 6;
     for (int a = 0; a < kDepth; ++a) {
@@ -1036,18 +1299,41 @@ TreeShape tree_shape(const HostTable& T, int64_t n, const double box[3], int ima
             h = std::max(h, 0.5 * box[d] / m);
             cells *= m;
         }
-        if (cells > 32768.0 || cells * np > 1.6e7) break;
-        for (int o = 0; o < kOrders; ++o) {
-            const double q = kOrderQ[o], q3 = q * q * q;
+        if (cells > 32768.0) break;
+        for (int ob = 0; ob < kOrders * (line ? 1 : 2); ++ob) {
+            const int o = ob % kOrders;
+            const double q = kOrderQ[o], q3 = q * q * q, theta = kOrderTheta[o];
             if (cells * q3 > 1.5 * (double)n + 1e5) continue;
-            State s = { 0.0, near_terms(T, box, images, kOrderTheta[o] * h), h, cells, a, o, -1 };
-            if (s.near > 0.97 * all) continue;
+            State s;
+            s.h = h; s.cells = cells; s.a = a; s.o = o; s.prev = -1; s.np = 0; s.eq = false;
+            s.cut = ob < kOrders ? h : 0.5 * h;      // squares as large as the cells, or half
+            s.near = 0.0;
+            std::vector<double> far(roots.size());       // far terms per image pair of the loop
+            for (size_t l = 0; l < roots.size(); ++l) {
+                const Depth& d = depth_at(roots[l], s.cut);
+                const bool leaf = &d == &roots[l].depth.back();
+                const double raw = roots[l].terms / d.squares;
+                const bool eq = !line && (!leaf || raw > q * q);
+                double R = theta * h + d.rho;
+                if (eq) R = std::max(R, h + theta * d.size);
+                double v = 1.0;
+                for (int k = 0; k < 3; ++k) v *= std::min(W, 2.0 * R / box[k]);
+                s.v.push_back(v);
+                s.near += v * roots[l].terms;
+                far[l] = d.squares * (eq ? q * q : raw);
+                s.eq = s.eq || eq;
+                s.np += d.squares;
+            }
+            if (s.near > 0.97 * all || cells * s.np > 1.6e7) continue;
             double best = 1e300;
             for (int p = -1; p < (int)st.size(); ++p) {
-                const double before = p < 0 ? all : st[p].near;
-                if (p >= 0 && (st[p].near < s.near * 1.02 || st[p].a > a || (st[p].a == a && st[p].o >= o))) continue;
-                double c = (p < 0 ? 0.0 : st[p].cost) + (before - s.near) * cells * q3 * e64 * 1.1 + 3.0 * us +
-                           cells * q3 * np * 0.5;
+                if (p >= 0 && (st[p].near < s.near * 1.02 || st[p].cut < s.cut || (st[p].a == a && st[p].o >= o)))
+                    continue;
+                double pairs = 0.0;
+                for (size_t l = 0; l < roots.size(); ++l)
+                    pairs += std::max(0.0, (p < 0 ? nimg : st[p].v[l]) - s.v[l]) * far[l];
+                double c = (p < 0 ? 0.0 : st[p].cost) + pairs * cells * q3 * e64 * 1.1 + 3.0 * us +
+                           cells * q3 * s.np * 0.5 + (line ? 0.0 : terms * q * q * 2.0 + 10.0 * us);
                 if (p >= 0) {
                     const double qp = kOrderQ[st[p].o];
                     c += 3.0 * cells * (q * qp * qp * qp + q * q * qp * qp + q3 * qp) * 2.0 + 4.0 * us;
@@ -1059,25 +1345,91 @@ TreeShape tree_shape(const HostTable& T, int64_t n, const double box[3], int ima
             for (int p = s.prev; p >= 0; p = st[p].prev) ++depth;
             if (depth >= TreeShape::kMaxLevels) continue;
             s.cost = best;
-            st.push_back(s);
+            st.push_back(std::move(s));
         }
     }
+    // what is left at the atoms of a last level: its near terms one by one, or
+    // (loopons) first the squares that are far enough from the cell for their
+    // equivalent loopons, by falling size and rising order
+    struct Step { double cost, cut; int o, prev, np; bool eq; std::vector<double> v; };
+    auto near_steps = [&](const State& p, double h, double cells, std::vector<Step>& steps, int& end) {
+        auto rest = [&](const std::vector<double>& v) {
+            double t = 0.0;
+            for (size_t l = 0; l < roots.size(); ++l) t += v[l] * roots[l].terms;
+            return (double)n * t * e64 * 1.1;
+        };
+        double least = rest(p.v);
+        end = -1;
+        if (line) return least;
+        double smallest = 1e300;
+        for (const Root& r : roots) smallest = std::min(smallest, r.depth.back().size);
+        for (double cut = p.cut; cut > 0.5 * smallest; cut *= 0.5)
+            for (int o = 0; o < kOrders; ++o) {
+                const double q2 = (double)kOrderQ[o] * kOrderQ[o];
+                Step s;
+                s.cut = cut; s.o = o; s.prev = -1; s.np = 0; s.eq = false;
+                s.cost = 1e300;
+                std::vector<double> own(roots.size()), far(roots.size());
+                for (size_t l = 0; l < roots.size(); ++l) {
+                    const Depth& d = depth_at(roots[l], cut);
+                    const bool leaf = &d == &roots[l].depth.back();
+                    const bool eq = !leaf || roots[l].terms / d.squares > q2;
+                    own[l] = 1e300;
+                    far[l] = d.squares * q2;
+                    s.np += d.squares;
+                    if (!eq) continue;
+                    s.eq = true;
+                    own[l] = 1.0;
+                    for (int k = 0; k < 3; ++k) own[l] *= std::min(W, 2.0 * (h + kOrderTheta[o] * d.size) / box[k]);
+                }
+                if (!s.eq || cells * s.np > 1.6e7) continue;
+                for (int b = -1; b < (int)steps.size(); ++b) {
+                    if (b >= 0 && steps[b].cut <= cut && steps[b].o >= o) continue;
+                    const std::vector<double>& before = b < 0 ? p.v : steps[b].v;
+                    double pairs = 0.0;
+                    for (size_t l = 0; l < roots.size(); ++l) pairs += std::max(0.0, before[l] - own[l]) * far[l];
+                    const double c = (b < 0 ? 0.0 : steps[b].cost) + (double)n * pairs * e64 * 1.13 +
+                                     (double)n * s.np * 0.5 + terms * q2 * 2.0 + 15.0 * us;
+                    if (c < s.cost) { s.cost = c; s.prev = b; }
+                }
+                int depth = 1;
+                for (int b = s.prev; b >= 0; b = steps[b].prev) ++depth;
+                if (depth > 6) continue;
+                s.v = s.prev < 0 ? p.v : steps[s.prev].v;
+                for (size_t l = 0; l < roots.size(); ++l) s.v[l] = std::min(s.v[l], own[l]);
+                steps.push_back(std::move(s));
+                const double c = steps.back().cost + rest(steps.back().v);
+                if (c < least) { least = c; end = (int)steps.size() - 1; }
+            }
+        return least;
+    };
     double best = S.direct;
-    int pick = -1, pick_r = 1, pick_q = 0;
+    int pick = -1, pick_r = 1, pick_q = 0, pick_end = -1;
+    std::vector<Step> pick_steps;
     for (int p = 0; p < (int)st.size(); ++p) {
         const double theta = kOrderTheta[st[p].o];
+        if (st[p].cost >= best) continue;
+        int levels = 1, end = -1;
+        for (int b = st[p].prev; b >= 0; b = st[b].prev) ++levels;
+        if (levels + 6 > TreeShape::kMaxLevels) continue;
         for (int r = 1; r <= 8; r *= 2) {
             const double cells = st[p].cells * r * r * r;
-            if (cells > kMaxCells) break;
+            if (cells > (line ? kMaxCells : 32768)) break;
             const int o = order_for((theta - 1.0) * r + 1.0);
             const double q = kOrderQ[o], q3 = q * q * q, qp = kOrderQ[st[p].o];
             if (kOrderQ[o] > kMaxFinalQ) continue;
             const double atoms = std::max(1.0, (double)n / cells);
             const double fill = (std::floor(atoms / 64.0) + 1.0) * 64.0 / atoms;
-            const double c = st[p].cost + (double)n * st[p].near * e64 * 1.1 + (double)n * np * 0.5 +
+            std::vector<Step> steps;
+            double near = near_steps(st[p], st[p].h / r, cells, steps, end);
+            if (!line) near *= (std::floor(atoms / 16.0) + 1.0) * 16.0 / atoms;     // partly filled warps
+            const double c = st[p].cost + near + (double)n * st[p].np * 0.5 +
                              3.0 * cells * ((q * qp * qp * qp + q * q * qp * qp) / r + q3 * qp) * 2.5 +
                              (double)n * 3.0 * q3 * 2.0 * std::min(fill, 64.0) + 60.0 * us + (double)n * 60.0;
-            if (c < best) { best = c; pick = p; pick_r = r; pick_q = o; }
+            if (c < best) {
+                best = c; pick = p; pick_r = r; pick_q = o; pick_end = end;
+                pick_steps = steps;
+            }
         }
     }
     S.cost = best;
@@ -1087,26 +1439,44 @@ TreeShape tree_shape(const HostTable& T, int64_t n, const double box[3], int ima
     std::reverse(chain.begin(), chain.end());
     S.use = true;
     S.levels = (int)chain.size();
-    double before = all;
     for (int k = 0; k < S.levels; ++k) {
         const State& s = st[chain[k]];
         for (int d = 0; d < 3; ++d) S.m[k][d] = m0[d] << s.a;
         S.q[k] = kOrderQ[s.o];
         S.theta[k] = kOrderTheta[s.o];
-        // lanes per node: enough images per piece for each lane, more lanes
-        // where the level has few nodes
-        const double per = (before - s.near) / terms;
+        S.cut[k] = s.cut;
+        S.np[k] = s.np;
+        S.eq[k] = s.eq;
+        // lanes per node: enough images per source for each lane
+        double per = 0.0;
+        for (size_t l = 0; l < roots.size(); ++l)
+            per += ((k ? st[chain[k - 1]].v[l] : nimg) - s.v[l]) / (double)roots.size();
         int split = 1;
-        while (split < 32 && per >= 6.0 * split) split *= 2;
+        if (line) while (split < 32 && per >= 6.0 * split) split *= 2;
+        else while (split < 8 && s.cells * S.q[k] * S.q[k] * S.q[k] * split < 300000.0) split *= 2;
         S.split[k] = split;
-        before = s.near;
+    }
+    S.total = S.levels;
+    std::vector<int> tail;
+    for (int b = pick_end; b >= 0; b = pick_steps[b].prev) tail.push_back(b);
+    for (auto it = tail.rbegin(); it != tail.rend(); ++it, ++S.total) {
+        const Step& s = pick_steps[*it];
+        for (int d = 0; d < 3; ++d) S.m[S.total][d] = S.m[S.levels - 1][d] * pick_r;
+        S.q[S.total] = kOrderQ[s.o];
+        S.theta[S.total] = kOrderTheta[s.o];
+        S.cut[S.total] = s.cut;
+        S.np[S.total] = s.np;
+        S.eq[S.total] = s.eq;
+        S.split[S.total] = 1;
     }
     for (int d = 0; d < 3; ++d) S.mf[d] = S.m[S.levels - 1][d] * pick_r;
     S.qf = kOrderQ[pick_q];
-    // lanes per atom: as many as the near images feed, while the atoms alone do
-    // not fill the GPU several times
+    S.fine = !line;
+    // lanes per atom: as many as the near images (or the loopons) feed, while the
+    // atoms alone do not fill the GPU several times
     const double per_atom = st[pick].near / terms;
-    while (S.near_split < 32 && per_atom >= 4.0 * S.near_split && n * S.near_split < 600000) S.near_split *= 2;
+    if (line) while (S.near_split < 32 && per_atom >= 4.0 * S.near_split && n * S.near_split < 600000) S.near_split *= 2;
+    else while (S.near_split < 8 && n * S.near_split < 600000) S.near_split *= 2;
     return S;
 }
 
@@ -1210,17 +1580,17 @@ void tree_pool_release(int device)
     if (cudaMemPoolTrimTo(g_pool[device], 0) != cudaSuccess) cudaGetLastError();
 }
 
-int launch_tree(const FieldArgs& f, const HostTable& T, const TreeShape& S, const double box[3], int sm_count,
+int launch_tree(const FieldArgs& f, const HostTable& T, const TreeShape& S, int sm_count,
                 cudaStream_t s, bool* ran, std::string& err)
 {
     *ran = false;
-    (void)box;
     TreeArgs a;
     std::memset(&a, 0, sizeof(a));
     a.f = f;
     a.pieces = reinterpret_cast<const TreePiece*>(f.table + T.aux_tree);
-    a.np = (int32_t)T.tree_rho.size();
+    a.nodes = (int32_t)T.tree.size();
     a.levels = S.levels;
+    a.total = S.total;
     a.images = f.images;
     a.near_split = S.near_split;
     a.qf = S.qf;
@@ -1229,10 +1599,12 @@ int launch_tree(const FieldArgs& f, const HostTable& T, const TreeShape& S, cons
     auto take = [&](size_t bytes) { const size_t o = at; at += (bytes + 255) & ~size_t(255); return o; };
     const size_t o_box = take(6 * sizeof(unsigned long long));
     int64_t lcells = 0, tiles = 0;
-    size_t o_val[TreeShape::kMaxLevels], mats = 0;
+    size_t o_val[TreeShape::kMaxLevels], o_eq[TreeShape::kMaxLevels], mats = 0;
+    int64_t sources = 0;
     int lvcells[TreeShape::kMaxLevels];
-    for (int k = 0; k < S.levels; ++k) {
+    for (int k = 0; k < S.total; ++k) {
         LevelArgs& v = a.lv[k];
+        const bool nodes = k < S.levels;
         int64_t cells = 1;
         for (int d = 0; d < 3; ++d) {
             v.m[d] = S.m[k][d];
@@ -1243,6 +1615,14 @@ int launch_tree(const FieldArgs& f, const HostTable& T, const TreeShape& S, cons
         v.q3 = v.q * v.q * v.q;
         v.split = S.split[k];
         v.theta = S.theta[k];
+        v.cut = S.cut[k];
+        v.np = S.np[k];
+        v.near0 = a.near_size;
+        v.list0 = sources;
+        a.near_size += cells * v.np;
+        sources += v.np;
+        o_eq[k] = !S.eq[k] ? 0 : take((size_t)v.np * v.q * v.q * sizeof(LooponRec));
+        if (!nodes) continue;
         v.tiles = (v.q3 * v.split + 31) / 32;
         v.tile0 = tiles;
         v.cell0 = lcells;
@@ -1260,6 +1640,8 @@ int launch_tree(const FieldArgs& f, const HostTable& T, const TreeShape& S, cons
     }
     a.cells_s = lvcells[S.levels - 1];
     a.cells_f = (int32_t)cf;
+    a.near_rr = S.fine ? 1 : a.rf[0] * a.rf[1] * a.rf[2];
+    a.cells_n = a.cells_f / a.near_rr;
     for (int t = 1; t <= S.levels; ++t) {
         const bool last = t == S.levels;
         const int qp = a.lv[t - 1].q, qc = last ? a.qf : a.lv[t].q;
@@ -1268,10 +1650,12 @@ int launch_tree(const FieldArgs& f, const HostTable& T, const TreeShape& S, cons
             mats += (size_t)(last ? a.rf[d] : a.lv[t].r[d]) * qp * qc;
         }
     }
-    const size_t o_near = take((size_t)lcells * a.np * sizeof(uint64_t));
+    const size_t o_near = take((size_t)a.near_size * sizeof(uint64_t));
+    const size_t o_list = take((size_t)sources * 2 * sizeof(int32_t));
+    const size_t o_pos = take((size_t)S.total * a.nodes * sizeof(int32_t));
     const size_t o_occ = take((size_t)lcells);
     const size_t o_start = take((size_t)(cf + 2) * sizeof(uint32_t));
-    const size_t o_ntile = take((size_t)(a.cells_s + 2) * sizeof(uint32_t));
+    const size_t o_ntile = take((size_t)(a.cells_n + 2) * sizeof(uint32_t));
     a.sort_tiles = (int32_t)((f.n + kSortTile - 1) / kSortTile);
     const size_t o_sort = take((size_t)f.n * 4 * sizeof(uint32_t));
     const size_t o_digits = take(((size_t)a.sort_tiles * 256 + 256) * sizeof(uint32_t));
@@ -1287,7 +1671,15 @@ int launch_tree(const FieldArgs& f, const HostTable& T, const TreeShape& S, cons
     }
     *ran = true;
     a.box = reinterpret_cast<unsigned long long*>(ws + o_box);
-    for (int k = 0; k < S.levels; ++k) a.lv[k].val = reinterpret_cast<double*>(ws + o_val[k]);
+    int most = 0;
+    for (int k = 0; k < S.total; ++k) {
+        if (k < S.levels) a.lv[k].val = reinterpret_cast<double*>(ws + o_val[k]);
+        if (o_eq[k]) a.lv[k].eq = reinterpret_cast<LooponRec*>(ws + o_eq[k]);
+        most = std::max(most, S.np[k]);
+    }
+    a.list = reinterpret_cast<int32_t*>(ws + o_list);
+    a.up = a.list + sources;
+    a.pos = reinterpret_cast<int32_t*>(ws + o_pos);
     a.near = reinterpret_cast<uint64_t*>(ws + o_near);
     a.occ = ws + o_occ;
     a.start = reinterpret_cast<uint32_t*>(ws + o_start);
@@ -1300,6 +1692,7 @@ int launch_tree(const FieldArgs& f, const HostTable& T, const TreeShape& S, cons
     a.digit_total = a.digits + (size_t)a.sort_tiles * 256;
     a.mat = reinterpret_cast<double*>(ws + o_mat);
 
+    const bool line = T.kind == kLineKind;
     auto queue = [&]() -> cudaError_t {
         const int64_t sweep = std::min<int64_t>((f.n + 255) / 256, (int64_t)sm_count * 8);
         cudaError_t e;
@@ -1323,17 +1716,22 @@ int launch_tree(const FieldArgs& f, const HostTable& T, const TreeShape& S, cons
         a.perm = a.idx[in];
         tree_starts_kernel<<<(unsigned)((f.n + 256) / 256), 256, 0, s>>>(a, a.key[in]);
         tree_scan_kernel<<<1, 1024, 0, s>>>(a);
-        tree_near_kernel<<<(unsigned)std::min<int64_t>((lcells * a.np + 255) / 256, (int64_t)sm_count * 16), 256, 0, s>>>(a);
+        tree_list_kernel<<<(unsigned)S.total, 1024, 0, s>>>(a);
+        tree_near_kernel<<<(unsigned)std::min<int64_t>((a.near_size + 255) / 256, (int64_t)sm_count * 16), 256, 0, s>>>(a);
+        if (!line) tree_equivalent_kernel<<<dim3((unsigned)most, (unsigned)S.total), kEqThreads, 0, s>>>(a);
         tree_matrix_kernel<<<dim3((unsigned)S.levels, 3, 8), 128, 0, s>>>(a);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
-        tree_node_kernel<<<(unsigned)((tiles + kWarps - 1) / kWarps), 32 * kWarps, 0, s>>>(a);
+        const unsigned nodes = (unsigned)((tiles + kWarps - 1) / kWarps);
+        if (line) tree_node_kernel<kLineKind><<<nodes, 32 * kWarps, 0, s>>>(a);
+        else tree_node_kernel<kLooponKind><<<nodes, 32 * kWarps, 0, s>>>(a);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
         for (int t = 1; t < S.levels; ++t)
             if ((e = down_any(a, t, lvcells[t], s)) != cudaSuccess) return e;
         if ((e = leaf_any(a, s)) != cudaSuccess) return e;
-        const int64_t ntiles = f.n * S.near_split / 32 + a.cells_s + 2;
+        const int64_t ntiles = f.n * S.near_split / 32 + a.cells_n + 2;
         const unsigned ngrid = (unsigned)((ntiles + kWarps - 1) / kWarps);
-        tree_near_sum_kernel<<<ngrid, 32 * kWarps, 0, s>>>(a);
+        if (line) tree_near_sum_kernel<kLineKind><<<ngrid, 32 * kWarps, 0, s>>>(a);
+        else tree_near_sum_kernel<kLooponKind><<<ngrid, 32 * kWarps, 0, s>>>(a);
         return cudaGetLastError();
     };
     const cudaError_t e = queue();

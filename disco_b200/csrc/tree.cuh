@@ -12,30 +12,25 @@
 
 namespace disco {
 
-// One piece of the table as the cell sum sees it: a ball that holds the
-// piece's whole source (apex and vertices), and its records as byte offsets
-// into the table.
-struct alignas(16) TreePiece {
-    double x, y, z, rho;
-    uint32_t piece, rec;         // LinePiece and its first LineSeg
-    int32_t terms;               // segments
-    int32_t pad;
-};
-static_assert(sizeof(TreePiece) == 48, "tree piece layout");
-
-// Appends the tree pieces of an FP64 line table after its bytes (sets aux_tree).
+// Appends an FP64 table's tree pieces after its bytes (sets aux_tree); a line
+// table's are made here, one per piece.
 void append_tree_pieces(HostTable& T);
 
 // The sum's shape for one atom count: chosen once per plan and count.
 struct TreeShape {
-    static constexpr int kMaxLevels = 18;
+    static constexpr int kMaxLevels = 24;
     bool use = false;
-    int levels = 0;
+    int levels = 0;              // levels of cells with nodes
+    int total = 0;               // and after them the levels of squares summed at the atoms
     int m[kMaxLevels][3] = {};   // cells per axis
-    int q[kMaxLevels] = {};      // nodes per axis of a cell
+    int q[kMaxLevels] = {};      // nodes per axis of a cell, equivalent loopons per axis of a square
     double theta[kMaxLevels] = {};
+    double cut[kMaxLevels] = {}; // loopons: half edge of the largest square used as one source
+    int np[kMaxLevels] = {};     // sources: tree pieces of that cut
+    bool eq[kMaxLevels] = {};    // loopons: some of them summed through equivalent loopons
     int split[kMaxLevels] = {};  // lanes that share a node's images
     int mf[3] = {}, qf = 0;      // the cells the atoms are sorted into
+    bool fine = false;           // the near pass goes by the final cells (else by the last level's)
     int near_split = 1;          // lanes that share an atom's near images
     double cost = 0.0, direct = 0.0;
 };
@@ -46,7 +41,7 @@ TreeShape tree_shape(const HostTable& T, int64_t n, const double box[3], int ima
 
 // Queues the sum on `stream`.  *ran is false (and nothing was queued) when the
 // scratch memory could not be had: the caller then sums directly.
-int launch_tree(const FieldArgs& a, const HostTable& T, const TreeShape& S, const double box[3], int sm_count,
+int launch_tree(const FieldArgs& a, const HostTable& T, const TreeShape& S, int sm_count,
                 cudaStream_t stream, bool* ran, std::string& err);
 
 // Scratch pool of the cell sum: one per device, shared by the plans that have

@@ -1,10 +1,12 @@
 """The sum by cells (tree.cu) against the plain sum over every image, which an
 explicit image split selects, and against the oracle.
 
-Tolerance: the cells' interpolation stays below 4e-15 A per loop at
+Tolerance (line): the cells' interpolation stays below 4e-15 A per loop at
 |b| = 2.5 A where theta(q) was set, at most about three levels add at an atom,
 and the plain sum itself is within 1e-14 A of the oracle on these sizes: 2e-14
-A per loop, plus 2e-14 A."""
+A per loop, plus 2e-14 A.  Loopons: the plain sum over 1e4 to 1e6 terms is
+within about 1e-13 A of the reference's, and the squares' interpolation is of
+the line's size per loop: 2e-14 A per loop, plus 2e-13 A."""
 import numpy as np
 import pytest
 
@@ -40,9 +42,22 @@ def _uneven():
     return s
 
 
+def _prismatic(cells, n, rmin, rmax, images=1):
+    w = W.bcc_prismatic(cells=cells, n_inter=n, n_vac=n, rmin=rmin, rmax=rmax)
+    w.images = images
+    return w
+
+
+def _tolerance(w):
+    return 2e-14 * len(w.loops) + (2e-14 if w.method == "line" else 2e-13)
+
+
 CASES = {
     "fcc": lambda: W.fcc_random(cells=36, n_circles=4, n_hex=2, n_rect=2),
     "uneven": _uneven,
+    "loopons": lambda: _prismatic(40, 2, 15.0, 40.0),
+    "loopons, two shells": lambda: _prismatic(30, 2, 12.0, 30.0, 2),
+    "small loopon loops": lambda: _prismatic(24, 4, 6.0, 12.0, 2),
     "large cells": lambda: W.fcc_random(cells=70, images=3, n_circles=2, n_hex=1, n_rect=1),
 }
 
@@ -59,7 +74,7 @@ def test_cells_match_plain_sum(name, form):
         g = torch.Generator(device="cuda")
         g.manual_seed(1)
         pos = pos[:, torch.randperm(pos.shape[1], generator=g, device="cuda")].contiguous()
-    tol = 2e-14 * len(w.loops) + 2e-14
+    tol = _tolerance(w)
     a = _sum(torch, w, pos, 1)
     b = _sum(torch, w, pos, 0)
     c = _sum(torch, w, pos, 0)
@@ -72,11 +87,12 @@ def test_cells_match_plain_sum(name, form):
         assert np.abs(b.cpu().numpy()[:, idx] - ref).max() <= tol
 
 
-def test_atoms_outside_the_cells():
+@pytest.mark.parametrize("name", ["fcc", "loopons"])
+def test_atoms_outside_the_cells(name):
     """Outliers, a NaN and an infinity take every image themselves and leave
     the other atoms alone; atoms that fill a corner of the box only."""
     torch = pytest.importorskip("torch")
-    w = W.fcc_random(cells=36, n_circles=4, n_hex=2, n_rect=2)
+    w = CASES[name]()
     pos = _positions(torch, w)
     pos[:, 7] = torch.tensor([5.0, -3.1, 0.2], device="cuda") * w.box[0]
     pos[0, 100] = float("nan")
@@ -86,7 +102,7 @@ def test_atoms_outside_the_cells():
     odd = torch.zeros(pos.shape[1], dtype=torch.bool, device="cuda")
     odd[100] = odd[4001] = True
     assert torch.isfinite(b[:, ~odd]).all()
-    assert float((a - b)[:, ~odd].abs().max()) <= 2e-14 * len(w.loops) + 2e-14
+    assert float((a - b)[:, ~odd].abs().max()) <= _tolerance(w)
     assert torch.equal(torch.isnan(a[:, 100]), torch.isnan(b[:, 100]))
 
 
@@ -134,3 +150,13 @@ def test_two_streams_at_once():
     for u in us:
         assert torch.equal(u, one)
     plan.close()
+
+
+def test_loopons_off_one_plane():
+    """Loopons that do not lie in one plane have no squares: the plain sum."""
+    torch = pytest.importorskip("torch")
+    w = _prismatic(30, 2, 12.0, 30.0)
+    w.loops[1].z = w.loops[1].z + 0.3 * np.sin(w.loops[1].x)
+    pos = _positions(torch, w)
+    a, b = _sum(torch, w, pos, 1), _sum(torch, w, pos, 0)
+    assert float((a - b).abs().max()) <= _tolerance(w)
