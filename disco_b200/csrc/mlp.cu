@@ -1,17 +1,29 @@
 // The learned far-image surrogate's network: 14 -> 128 -> 128 -> 128 -> 3,
 // SiLU, BF16 weights and activations on the tensor cores, FP32 accumulation,
-// FP32 master weights and Adam.  Every matrix product, forward and backward,
-// runs through one hand-written tcgen05 GEMM kernel:
+// FP32 master weights and Adam.
 //
-//     C[M x N] = A[M x K] * B[N x K]^T        (BF16 x BF16 -> FP32 in TMEM)
+// net_kernel does a whole forward pass, or forward and backward, for 128 rows
+// at a time in one CTA of 256 threads (row r is tensor-memory lane r; warps w
+// and w + 4 read the same lanes and split the columns).  Weights, activations
+// and their transposes sit in shared memory as BF16 K-major tiles (tcgen05.cuh;
+// 224 KB in all), the three layers' FP32 pre-activations stay in tensor memory
+// until the backward pass has used them, and their columns then take the weight
+// gradients:
 //
-// A and B are read from global memory (FP32 or BF16, stored as given or
-// transposed) and written into shared memory in the no-swizzle K-major
-// layout of tcgen05.cuh, converting to BF16 on the way; one elected thread
-// issues the MMAs (K = 16 each) and commits them to an mbarrier; four warps
-// read the accumulator back with tcgen05.ld (warp w owns rows 32w..32w+31)
-// and apply a fused epilogue.  Transposed operands (dW = dpre^T h,
-// dh = dpre W) are transposed by the loader, so every descriptor is K-major.
+//     columns    0..127   pre-activation 1, then dW1
+//              128..255   pre-activation 2, then dW2
+//              256..383   pre-activation 3, then dW3
+//              384..511   output, dW4, then dh3, dh2, dh1
+//
+// dh = dpre W needs W transposed, dW = dpre^T h both operands: the epilogues
+// write each tile in both orders (a transposed tile of h makes room for the
+// transposed dpre of the layer above), and W3, W2 are staged again transposed
+// over themselves.  Each CTA keeps its own partial gradient in global memory;
+// sum_kernel adds the partials in order, so a gradient is the same in every run.
+// The latency of one tile's chain of layers bounds a step (4096 rows are 32
+// tiles; the kernel issues on 15 % of the cycles, waiting for L2 and for
+// barriers): 0.40 ms with one launch per product and reduction (18 launches),
+// 0.052 ms with this kernel (45 to 50 us alone), the sum (10 us) and Adam (4).
 //
 // Inputs are padded to 16 features and outputs to 16 (the MMA's N >= 16 for
 // M = 128); the padding columns of W1 and rows of W4 are zero and stay zero
@@ -32,42 +44,41 @@
 namespace disco {
 namespace mlp {
 
-enum { kF32 = 0, kBF16 = 1 };
-enum { EPI_STORE = 0, EPI_SILU = 1, EPI_DSILU = 2, EPI_ATOMIC = 3, EPI_ATOMIC_T = 4 };
+constexpr int kNetThreads = 256;
+constexpr int kRows = 128;                        // rows per tile
+constexpr uint32_t kTile = kRows * kHid * 2;      // a 128 x 128 BF16 tile
+constexpr uint32_t kThin = kRows * kIn * 2;       // a 128 x 16 (or 16 x 128) one
+constexpr uint32_t oSW1 = 0;                      // [128 x 16]
+constexpr uint32_t oSW2 = oSW1 + kThin;           // [128 x 128], in the backward pass transposed
+constexpr uint32_t oSW3 = oSW2 + kTile;
+constexpr uint32_t oSW4 = oSW3 + kTile;           // [16 x 128]
+constexpr uint32_t oSW4T = oSW4 + kThin;          // [128 x 16]
+constexpr uint32_t oSX = oSW4T + kThin;           // [rows x 16]
+constexpr uint32_t oSXT = oSX + kThin;            // [16 x rows]
+constexpr uint32_t oSH = oSXT + kThin;            // activations, then dpre: [rows x 128]
+constexpr uint32_t oST = oSH + kTile;             // three tiles [128 x rows]: h1, h2, h3 transposed, then dpre
+constexpr uint32_t oSDy = oST + 3 * kTile;        // [rows x 16]
+constexpr uint32_t oSDyT = oSDy + kThin;          // [16 x rows]
+constexpr uint32_t oSBias = oSDyT + kThin;        // b1, b2, b3, b4 (FP32)
+constexpr uint32_t oSLoss = oSBias + (3 * kHid + kOut) * 4;     // the warps' losses
+constexpr uint32_t oSBar = oSLoss + 32;
+constexpr uint32_t kNetSmem = oSBar + 32;
+static_assert(kNetSmem <= 227 * 1024, "one CTA's shared memory");
+constexpr int kPart = kParams + 4;                // a partial gradient and its loss
 
-struct Operand {
-    const void* ptr;
-    int32_t dtype;        // kF32 or kBF16
-    int32_t transposed;   // 0: element (r, k) at r*ld + k; 1: at k*ld + r
-    int64_t ld;
-};
-
-struct GemmArgs {
-    Operand A, B;
-    int32_t M, N, K;
-    int32_t k_per_split;  // split-K: blockIdx.z takes K range [z*k_per_split, ...)
-    int32_t epi;
-    float* C;             // FP32 output (pre-activation, dpre, raw result or gradient)
-    int64_t ldc;
-    __nv_bfloat16* H;     // BF16 output (activation or dpre)
-    int64_t ldh;
-    const float* bias;    // per output column (EPI_STORE / EPI_SILU)
-    const float* pre;     // EPI_DSILU: pre-activations
-    int64_t ldp;
-    int32_t n_valid;      // EPI_ATOMIC*: columns >= n_valid are not accumulated
-    int32_t m_valid;      // EPI_ATOMIC*: rows >= m_valid are not accumulated
+struct NetArgs {
+    const float* P;
+    const float* X;           // [n x 16]
+    const float* T;           // [n x 3], null: forward only
+    float* Y;                 // [n x 16], forward only
+    float* part;              // [CTA][kPart]
+    float* dpre;              // [3][n x 128]
+    float* dy;                // [n x 4]
+    int64_t n;
+    int32_t tiles;
+    int32_t x16, y16;         // X, Y 16-byte aligned
     int* status;
 };
-
-constexpr int kThreads = 128;
-constexpr int kTileM = 128, kTileK = 128;
-
-__device__ __forceinline__ float load_elem(const Operand& o, int64_t r, int64_t k)
-{
-    const int64_t idx = o.transposed ? k * o.ld + r : r * o.ld + k;
-    return o.dtype == kF32 ? static_cast<const float*>(o.ptr)[idx]
-                           : __bfloat162float(static_cast<const __nv_bfloat16*>(o.ptr)[idx]);
-}
 
 __device__ __forceinline__ uint32_t bf16x2(float lo, float hi)
 {
@@ -75,226 +86,381 @@ __device__ __forceinline__ uint32_t bf16x2(float lo, float hi)
     return *reinterpret_cast<const uint32_t*>(&v);
 }
 
-// 8 consecutive elements (along the row in memory) at p as 8 floats
-__device__ __forceinline__ void load8(const Operand& o, int64_t idx, float* v)
+// W [rows x cols] (FP32, row-major) as a BF16 K-major tile; transposed: the
+// tile of W^T (cols x rows).
+__device__ __forceinline__ void stage_weights(unsigned char* tile, const float* W, int rows, int cols)
 {
-    if (o.dtype == kF32) {
-        const float4* q = reinterpret_cast<const float4*>(static_cast<const float*>(o.ptr) + idx);
+#pragma unroll 4
+    for (int e = threadIdx.x; e < rows * (cols / 8); e += kNetThreads) {
+        const int r = e % rows, k8 = (e / rows) * 8;
+        const float4* q = reinterpret_cast<const float4*>(W + r * cols + k8);
         const float4 a = q[0], b = q[1];
-        v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
-    } else {
-        const uint4 u = *reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(o.ptr) + idx);
-        const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&u);
+        *reinterpret_cast<uint4*>(tile + tc::kmajor_offset(r, k8, rows)) =
+            make_uint4(bf16x2(a.x, a.y), bf16x2(a.z, a.w), bf16x2(b.x, b.y), bf16x2(b.z, b.w));
+    }
+}
+__device__ __forceinline__ void stage_transposed(unsigned char* tile, const float* W, int rows, int cols)
+{
+    for (int e = threadIdx.x; e < (rows / 8) * (cols / 8); e += kNetThreads) {
+        const int r8 = (e % (cols / 8)) * 8, k8 = (e / (cols / 8)) * 8;      // tile row = W's column
+        float v[8][8];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const float2 f = __bfloat1622float2(h[i]);
-            v[2 * i] = f.x;
-            v[2 * i + 1] = f.y;
+        for (int k = 0; k < 8; ++k) {
+            const float4* q = reinterpret_cast<const float4*>(W + (k8 + k) * cols + r8);
+            const float4 a = q[0], b = q[1];
+            v[k][0] = a.x; v[k][1] = a.y; v[k][2] = a.z; v[k][3] = a.w;
+            v[k][4] = b.x; v[k][5] = b.y; v[k][6] = b.z; v[k][7] = b.w;
         }
-    }
-}
-
-// Whole tile in range and 16-byte aligned along memory rows: 8-element vector
-// loads, and 16-byte shared stores of 8 K-consecutive values (transposed
-// operands: 8 x 8 blocks transposed in registers).  Rows vary fastest across
-// threads, so the stores of a warp fill whole 128-byte core matrices.
-__device__ __forceinline__ bool tile_fast(const Operand& o, int rows, int64_t r0, int64_t rmax, int64_t k0, int kc,
-                                          int64_t kmax)
-{
-    const int esz = o.dtype == kF32 ? 4 : 2;
-    const bool in = r0 + rows <= rmax && k0 + kc <= kmax && (kc % 8) == 0;
-    const bool al = ((reinterpret_cast<uintptr_t>(o.ptr) & 15) == 0) && ((o.ld * esz) % 16 == 0) &&
-                    (((o.transposed ? r0 : k0) * esz) % 16 == 0);
-    return in && al;
-}
-
-__device__ __forceinline__ void load_tile_fast(const Operand& o, unsigned char* base, int rows, int64_t r0,
-                                               int64_t k0, int kc)
-{
-    if (!o.transposed) {
-        const int total = rows * (kc / 8);
-        for (int e = threadIdx.x; e < total; e += kThreads) {
-            const int r = e % rows, k8 = (e / rows) * 8;
-            float v[8];
-            load8(o, (r0 + r) * o.ld + k0 + k8, v);
-            *reinterpret_cast<uint4*>(base + tc::kmajor_offset(r, k8, rows)) =
-                make_uint4(bf16x2(v[0], v[1]), bf16x2(v[2], v[3]), bf16x2(v[4], v[5]), bf16x2(v[6], v[7]));
-        }
-    } else {
-        const int total = (rows / 8) * (kc / 8);
-        for (int e = threadIdx.x; e < total; e += kThreads) {
-            const int r8 = (e % (rows / 8)) * 8, k8 = (e / (rows / 8)) * 8;
-            float v[8][8];                   // v[k][r]
 #pragma unroll
-            for (int kk = 0; kk < 8; ++kk) load8(o, (k0 + k8 + kk) * o.ld + r0 + r8, v[kk]);
-#pragma unroll
-            for (int rr = 0; rr < 8; ++rr)
-                *reinterpret_cast<uint4*>(base + tc::kmajor_offset(r8 + rr, k8, rows)) =
-                    make_uint4(bf16x2(v[0][rr], v[1][rr]), bf16x2(v[2][rr], v[3][rr]), bf16x2(v[4][rr], v[5][rr]),
-                               bf16x2(v[6][rr], v[7][rr]));
-        }
+        for (int r = 0; r < 8; ++r)
+            *reinterpret_cast<uint4*>(tile + tc::kmajor_offset(r8 + r, k8, cols)) =
+                make_uint4(bf16x2(v[0][r], v[1][r]), bf16x2(v[2][r], v[3][r]), bf16x2(v[4][r], v[5][r]),
+                           bf16x2(v[6][r], v[7][r]));
     }
 }
 
-// rows x kc tile of an operand into shared memory (K-major, BF16), zero-padded
-__device__ __forceinline__ void load_tile(const Operand& o, __nv_bfloat16* smem, int rows, int64_t r0, int64_t rmax,
-                                          int64_t k0, int kc, int64_t kmax)
+// One product D (+)= A B^T over K = 16 nk, issued by the calling thread.
+__device__ __forceinline__ void product(uint32_t tmem, uint32_t a, int arows, uint32_t b, int brows, int nk, int N)
 {
-    unsigned char* base = reinterpret_cast<unsigned char*>(smem);
-    if (tile_fast(o, rows, r0, rmax, k0, kc, kmax)) {
-        load_tile_fast(o, base, rows, r0, k0, kc);
-        return;
-    }
-    const int total = rows * kc;
-    if (!o.transposed) {
-        for (int e = threadIdx.x; e < total; e += kThreads) {
-            const int r = e / kc, k = e % kc;
-            const float v = (r0 + r < rmax && k0 + k < kmax) ? load_elem(o, r0 + r, k0 + k) : 0.0f;
-            *reinterpret_cast<__nv_bfloat16*>(base + tc::kmajor_offset(r, k, rows)) = __float2bfloat16_rn(v);
-        }
-    } else {
-        for (int e = threadIdx.x; e < total; e += kThreads) {
-            const int k = e / rows, r = e % rows;
-            const float v = (r0 + r < rmax && k0 + k < kmax) ? load_elem(o, r0 + r, k0 + k) : 0.0f;
-            *reinterpret_cast<__nv_bfloat16*>(base + tc::kmajor_offset(r, k, rows)) = __float2bfloat16_rn(v);
-        }
-    }
+    const uint32_t alb = (uint32_t)(arows / 8) * 128, blb = (uint32_t)(brows / 8) * 128;
+    const uint32_t id = tc::idesc_bf16(kRows, N);
+    for (int j = 0; j < nk; ++j)
+        tc::mma_bf16(tmem, tc::smem_desc(a + j * 2 * alb, alb, 128), tc::smem_desc(b + j * 2 * blb, blb, 128), id, j > 0);
 }
 
-
-template <int NT>
-__global__ void __launch_bounds__(kThreads) gemm_kernel(const GemmArgs g)
+// Publishes every thread's tile writes and finished tensor-memory loads, has
+// one thread issue the products and waits for them (bounded); false, agreed by
+// the whole CTA, on a timeout.
+template <class Issue>
+__device__ __forceinline__ bool products(uint64_t* bar, uint32_t& phase, Issue issue)
 {
-    extern __shared__ __align__(128) unsigned char gemm_smem[];
-    __nv_bfloat16* sA = reinterpret_cast<__nv_bfloat16*>(gemm_smem);
-    __nv_bfloat16* sB = sA + kTileM * kTileK;
-    __shared__ __align__(8) uint64_t bar;
-    __shared__ uint32_t tmem_slot;
-    constexpr uint32_t kCols = NT < 32 ? 32 : NT;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int64_t m0 = (int64_t)blockIdx.x * kTileM;
-    const int64_t n0 = (int64_t)blockIdx.y * NT;
-    const int64_t kbeg = (int64_t)blockIdx.z * g.k_per_split;
-    const int64_t kend = ((int64_t)g.K < kbeg + g.k_per_split) ? (int64_t)g.K : kbeg + g.k_per_split;
-    if (warp == 0) tc::alloc(&tmem_slot, kCols);
+    fence_proxy_async_smem();
+    tc::fence_before_sync();
+    __syncthreads();
     if (threadIdx.x == 0) {
-        mbar_init(&bar, 1);
+        tc::fence_after_sync();
+        issue();
+        tc::commit(bar);
+    }
+    const bool mine = mbar_wait_bounded(bar, phase);
+    phase ^= 1;
+    const bool bad = __syncthreads_or(!mine);
+    tc::fence_after_sync();
+    return !bad;
+}
+
+// 32 consecutive columns of one row into a transposed tile [columns x rows].
+__device__ __forceinline__ void put_transposed(unsigned char* tile, const float (&h)[32], int row, int c0)
+{
+#pragma unroll
+    for (int i = 0; i < 32; ++i)
+        *reinterpret_cast<__nv_bfloat16*>(tile + tc::kmajor_offset(c0 + i, row, kHid)) = __float2bfloat16_rn(h[i]);
+}
+__device__ __forceinline__ void put_row(unsigned char* tile, const float (&h)[32], int row, int c0)
+{
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+        *reinterpret_cast<uint4*>(tile + tc::kmajor_offset(row, c0 + 8 * q, kRows)) =
+            make_uint4(bf16x2(h[8 * q], h[8 * q + 1]), bf16x2(h[8 * q + 2], h[8 * q + 3]),
+                       bf16x2(h[8 * q + 4], h[8 * q + 5]), bf16x2(h[8 * q + 6], h[8 * q + 7]));
+}
+
+template <bool kTrain>
+__global__ void __launch_bounds__(kNetThreads, 1) net_kernel(const NetArgs a)
+{
+    extern __shared__ __align__(128) unsigned char sm[];
+    uint64_t* bar = reinterpret_cast<uint64_t*>(sm + oSBar);
+    uint32_t* slot = reinterpret_cast<uint32_t*>(sm + oSBar + 16);
+    float* bias = reinterpret_cast<float*>(sm + oSBias);
+    float* losses = reinterpret_cast<float*>(sm + oSLoss);
+    const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+    const int row = t & 127, half = t >> 7;
+    if (warp == 0) tc::alloc(slot, 512);
+    if (t == 0) {
+        mbar_init(bar, 1);
         fence_mbar_init();
     }
+    stage_weights(sm + oSW1, a.P + oW1, kHid, kIn);
+    stage_weights(sm + oSW4, a.P + oW4, kOut, kHid);
+    if (kTrain) stage_transposed(sm + oSW4T, a.P + oW4, kOut, kHid);
+    if (!kTrain) {
+        stage_weights(sm + oSW2, a.P + oW2, kHid, kHid);
+        stage_weights(sm + oSW3, a.P + oW3, kHid, kHid);
+    }
+    for (int e = t; e < 3 * kHid + kOut; e += kNetThreads)
+        bias[e] = a.P[e < kHid ? ob1 + e : e < 2 * kHid ? ob2 + e - kHid : e < 3 * kHid ? ob3 + e - 2 * kHid
+                                                                                     : ob4 + e - 3 * kHid];
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
-    const uint32_t tmem = tmem_slot;
-    const uint32_t idesc = tc::idesc_bf16(kTileM, NT);
-    const uint32_t lboA = (kTileM / 8) * 128, lboB = (NT / 8) * 128;
+    const uint32_t tmem = *slot;
+    const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;             // this warp's tensor-memory lanes
+    const uint32_t s0 = smem_addr(sm);
+    const int c0 = half * (kHid / 2);
     uint32_t phase = 0;
     bool ok = true;
-    for (int64_t kk = kbeg; kk < kend; kk += kTileK) {
-        const int64_t rem = ((kend - kk + 15) / 16) * 16;
-        const int kc = (int)(rem < kTileK ? rem : kTileK);
-        load_tile(g.A, sA, kTileM, m0, g.M, kk, kc, kend);
-        load_tile(g.B, sB, NT, n0, g.N, kk, kc, kend);
-        fence_proxy_async_smem();
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            tc::fence_after_sync();
-            const uint32_t a0 = smem_addr(sA), b0 = smem_addr(sB);
-            for (int j = 0; j < kc / 16; ++j) {
-                const uint64_t ad = tc::smem_desc(a0 + j * 2 * lboA, lboA, 128);
-                const uint64_t bd = tc::smem_desc(b0 + j * 2 * lboB, lboB, 128);
-                tc::mma_bf16(tmem, ad, bd, idesc, kk > kbeg || j > 0);
-            }
-            tc::commit(&bar);
-        }
-        const bool mine = mbar_wait_bounded(&bar, phase);
-        phase ^= 1;
-        if (__syncthreads_or(!mine)) { ok = false; break; }     // every thread agrees
-        tc::fence_after_sync();
-    }
-    if (ok) {
-        const int64_t row = m0 + warp * 32 + lane;
-        const bool rvalid = row < g.M && kend > kbeg;
-        for (int c = 0; c < NT; c += 16) {
-            float v[16];
-            tc::ld16(tmem + ((uint32_t)(warp * 32) << 16) + c, v);
-            if (!rvalid) continue;
+    float loss = 0.0f;
+    float* const part = kTrain ? a.part + (int64_t)blockIdx.x * kPart : nullptr;
+
+    // a hidden layer's activations from its pre-activation in columns `col`
+    auto activate = [&](uint32_t col, const float* b, unsigned char* T) {
+#pragma unroll 1
+        for (int c = c0; c < c0 + kHid / 2; c += 32) {
+            float v[32];
+            tc::ld32(tmem + lanes + col + c, v);
 #pragma unroll
-            for (int i = 0; i < 16; ++i) {
-                const int64_t col = n0 + c + i;
-                if (col >= g.N) continue;
-                float x = v[i];
-                switch (g.epi) {
-                case EPI_STORE:
-                    if (g.bias) x += g.bias[col];
-                    g.C[row * g.ldc + col] = x;
-                    break;
-                case EPI_SILU: {
-                    if (g.bias) x += g.bias[col];
-                    g.C[row * g.ldc + col] = x;
-                    g.H[row * g.ldh + col] = __float2bfloat16_rn(silu_half(0.5f * x));
-                    break;
-                }
-                case EPI_DSILU: {
-                    const float p = g.pre[row * g.ldp + col];
-                    const float d = x * dsilu(p);
-                    g.C[row * g.ldc + col] = d;
-                    g.H[row * g.ldh + col] = __float2bfloat16_rn(d);
-                    break;
-                }
-                case EPI_ATOMIC:
-                    if (row < g.m_valid && col < g.n_valid) atomicAdd(&g.C[row * g.ldc + col], x);
-                    break;
-                default:   // EPI_ATOMIC_T: C^T += D
-                    if (row < g.m_valid && col < g.n_valid) atomicAdd(&g.C[col * g.ldc + row], x);
-                    break;
+            for (int i = 0; i < 32; ++i) v[i] = silu_half(0.5f * (v[i] + b[c + i]));
+            put_row(sm + oSH, v, row, c);
+            if (kTrain) put_transposed(T, v, row, c);
+        }
+    };
+    for (int tile = blockIdx.x; ok && tile < a.tiles; tile += gridDim.x) {
+        const int64_t r = (int64_t)tile * kRows + row;
+        const bool valid = r < a.n;
+        const bool first = tile == (int)blockIdx.x;
+        if (kTrain) {
+            stage_weights(sm + oSW2, a.P + oW2, kHid, kHid);
+            stage_weights(sm + oSW3, a.P + oW3, kHid, kHid);
+        }
+        {
+            float x[kIn];
+#pragma unroll
+            for (int k = 0; k < kIn; ++k) x[k] = 0.0f;
+            if (valid) {
+                const float* src = a.X + r * kIn;
+                if (a.x16) {
+#pragma unroll
+                    for (int q = 0; q < kIn / 4; ++q) {
+                        const float4 f = reinterpret_cast<const float4*>(src)[q];
+                        x[4 * q] = f.x; x[4 * q + 1] = f.y; x[4 * q + 2] = f.z; x[4 * q + 3] = f.w;
+                    }
+                } else {
+#pragma unroll
+                    for (int k = 0; k < kIn; ++k) x[k] = src[k];
                 }
             }
+            if (half == 0) {
+#pragma unroll
+                for (int q = 0; q < 2; ++q)
+                    *reinterpret_cast<uint4*>(sm + oSX + tc::kmajor_offset(row, 8 * q, kRows)) =
+                        make_uint4(bf16x2(x[8 * q], x[8 * q + 1]), bf16x2(x[8 * q + 2], x[8 * q + 3]),
+                                   bf16x2(x[8 * q + 4], x[8 * q + 5]), bf16x2(x[8 * q + 6], x[8 * q + 7]));
+            } else if (kTrain) {
+#pragma unroll
+                for (int k = 0; k < kIn; ++k)
+                    *reinterpret_cast<__nv_bfloat16*>(sm + oSXT + tc::kmajor_offset(k, row, kIn)) = __float2bfloat16_rn(x[k]);
+            }
         }
-    } else if (threadIdx.x == 0) {
-        report(g.status, DISCO_ETIMEOUT);
-        mbar_wait_bounded(&bar, phase ^ 1);
+        // forward
+        ok = products(bar, phase, [&] { product(tmem, s0 + oSX, kRows, s0 + oSW1, kHid, kIn / 16, kHid); });
+        if (!ok) break;
+        activate(0, bias, sm + oST);
+        ok = products(bar, phase, [&] { product(tmem + 128, s0 + oSH, kRows, s0 + oSW2, kHid, kHid / 16, kHid); });
+        if (!ok) break;
+        activate(128, bias + kHid, sm + oST + kTile);
+        ok = products(bar, phase, [&] { product(tmem + 256, s0 + oSH, kRows, s0 + oSW3, kHid, kHid / 16, kHid); });
+        if (!ok) break;
+        activate(256, bias + 2 * kHid, sm + oST + 2 * kTile);
+        ok = products(bar, phase, [&] { product(tmem + 384, s0 + oSH, kRows, s0 + oSW4, kOut, kHid / 16, kOut); });
+        if (!ok) break;
+        if (!kTrain) {
+            if (half == 0) {
+                float y[16];
+                tc::ld16(tmem + lanes + 384, y);
+                if (valid) {
+                    float* o = a.Y + r * kOut;
+#pragma unroll
+                    for (int k = 0; k < kOut; ++k) y[k] += bias[3 * kHid + k];
+                    if (a.y16) {
+#pragma unroll
+                        for (int q = 0; q < kOut / 4; ++q)
+                            reinterpret_cast<float4*>(o)[q] = make_float4(y[4 * q], y[4 * q + 1], y[4 * q + 2], y[4 * q + 3]);
+                    } else {
+#pragma unroll
+                        for (int k = 0; k < kOut; ++k) o[k] = y[k];
+                    }
+                }
+            }
+            continue;
+        }
+        // dy = 2 (y - t) / n on the real outputs, 0 on padding and past the last row
+        if (half == 0) {
+            float y[16], g[kOutReal];
+            tc::ld16(tmem + lanes + 384, y);
+#pragma unroll
+            for (int k = 0; k < kOutReal; ++k) {
+                g[k] = 0.0f;
+                if (valid) {
+                    const float d = (y[k] + bias[3 * kHid + k]) - a.T[r * kOutReal + k];
+                    loss += d * d;
+                    g[k] = 2.0f * d / (float)a.n;
+                }
+            }
+            *reinterpret_cast<uint4*>(sm + oSDy + tc::kmajor_offset(row, 0, kRows)) =
+                make_uint4(bf16x2(g[0], g[1]), bf16x2(g[2], 0.0f), 0u, 0u);
+            *reinterpret_cast<uint4*>(sm + oSDy + tc::kmajor_offset(row, 8, kRows)) = make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+            for (int k = 0; k < kOut; ++k)
+                *reinterpret_cast<__nv_bfloat16*>(sm + oSDyT + tc::kmajor_offset(k, row, kOut)) =
+                    __float2bfloat16_rn(k < kOutReal ? g[k] : 0.0f);
+            if (valid) reinterpret_cast<float4*>(a.dy)[r] = make_float4(g[0], g[1], g[2], 0.0f);
+        }
+        // the weights of dh2 and dh1 over those the forward pass is done with
+        stage_transposed(sm + oSW3, a.P + oW3, kHid, kHid);
+        stage_transposed(sm + oSW2, a.P + oW2, kHid, kHid);
+        auto put = [&](float* dst, float v) { *dst = first ? v : *dst + v; };
+        auto put4 = [&](float* dst, float x, float y, float z, float w) {
+            float4* d = reinterpret_cast<float4*>(dst);
+            float4 o = make_float4(x, y, z, w);
+            if (!first) {
+                const float4 p = *d;
+                o.x = p.x + x; o.y = p.y + y; o.z = p.z + z; o.w = p.w + w;
+            }
+            *d = o;
+        };
+        // 64 columns of this thread's row of a 128 x 128 weight gradient
+        auto put_gradient = [&](uint32_t col, int off) {
+#pragma unroll 1
+            for (int c = c0; c < c0 + kHid / 2; c += 32) {
+                float v[32];
+                tc::ld32(tmem + lanes + col + c, v);
+#pragma unroll
+                for (int q = 0; q < 8; ++q)
+                    put4(part + off + row * kHid + c + 4 * q, v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+            }
+        };
+        // dpre = dh dSiLU(pre) of one layer: its tiles, and its FP32 rows for db
+        auto dpre = [&](uint32_t col, const float* b, unsigned char* T, int layer, bool rows) {
+#pragma unroll 1
+            for (int c = c0; c < c0 + kHid / 2; c += 32) {
+                float p[32], v[32];
+                tc::ld32(tmem + lanes + col + c, p);
+                tc::ld32(tmem + lanes + 384 + c, v);
+#pragma unroll
+                for (int i = 0; i < 32; ++i) v[i] *= dsilu(p[i] + b[c + i]);
+                if (rows) put_row(sm + oSH, v, row, c);
+                put_transposed(T, v, row, c);
+                if (valid) {
+                    float4* o = reinterpret_cast<float4*>(a.dpre + ((int64_t)layer * a.n + r) * kHid + c);
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) o[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+                }
+            }
+        };
+        // dW4 = (h3^T dy)^T
+        ok = products(bar, phase, [&] {
+            product(tmem + 384, s0 + oST + 2 * kTile, kHid, s0 + oSDyT, kOut, kRows / 16, kOut);
+        });
+        if (!ok) break;
+        if (half == 0) {
+            float v[16];
+            tc::ld16(tmem + lanes + 384, v);
+#pragma unroll
+            for (int k = 0; k < kOut; ++k) put(part + oW4 + k * kHid + row, k < kOutReal ? v[k] : 0.0f);
+        }
+        // dh3 = dy W4
+        ok = products(bar, phase, [&] { product(tmem + 384, s0 + oSDy, kRows, s0 + oSW4T, kHid, kOut / 16, kHid); });
+        if (!ok) break;
+        dpre(256, bias + 2 * kHid, sm + oST + 2 * kTile, 2, true);
+        // dh2 = dpre3 W3, dW3 = dpre3^T h2
+        ok = products(bar, phase, [&] {
+            product(tmem + 384, s0 + oSH, kRows, s0 + oSW3, kHid, kHid / 16, kHid);
+            product(tmem + 256, s0 + oST + 2 * kTile, kHid, s0 + oST + kTile, kHid, kRows / 16, kHid);
+        });
+        if (!ok) break;
+        dpre(128, bias + kHid, sm + oST + kTile, 1, true);
+        put_gradient(256, oW3);
+        // dh1 = dpre2 W2, dW2 = dpre2^T h1
+        ok = products(bar, phase, [&] {
+            product(tmem + 384, s0 + oSH, kRows, s0 + oSW2, kHid, kHid / 16, kHid);
+            product(tmem + 128, s0 + oST + kTile, kHid, s0 + oST, kHid, kRows / 16, kHid);
+        });
+        if (!ok) break;
+        dpre(0, bias, sm + oST, 0, false);
+        put_gradient(128, oW2);
+        // dW1 = dpre1^T x
+        ok = products(bar, phase, [&] { product(tmem, s0 + oST, kHid, s0 + oSXT, kIn, kRows / 16, kIn); });
+        if (!ok) break;
+        if (half == 0) {
+            float v[16];
+            tc::ld16(tmem + lanes, v);
+            v[14] = v[15] = 0.0f;
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                put4(part + oW1 + row * kIn + 4 * q, v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+        }
+    }
+    if (!ok && t == 0) {
+        report(a.status, DISCO_ETIMEOUT);
+        mbar_wait_bounded(bar, phase ^ 1);
+    }
+    if (kTrain) {
+        for (int o = 16; o > 0; o >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, o);
+        if (lane == 0) losses[warp] = loss;
+        __syncthreads();
+        if (t == 0) part[kParams] = ((losses[0] + losses[1]) + losses[2]) + losses[3];
     }
     tc::fence_before_sync();
     __syncthreads();
-    if (warp == 0) tc::dealloc(tmem, kCols);
+    if (warp == 0) tc::dealloc(tmem, 512);
 }
 
-// dy = 2 (y - t) / n on the real outputs (0 on padding); loss += sum (y - t)^2 / n
-__global__ void mse_grad_kernel(const float* y, const float* t, int64_t n, float* dy, float* loss)
+// grads += the gradients of one call, loss = its mean squared error.  Blocks
+// below kWeightBlocks add the CTAs' partial weight gradients and losses (FP64, in
+// CTA order); the others the biases' column sums, eight columns of one
+// layer's dpre (or the output's dy) each: row k, k + 256, ... per thread, then
+// the threads.
+constexpr int kWeightBlocks = (kParams + 1 + 255) / 256;
+constexpr int kBiasBlocks = 3 * (kHid / 8) + 1;
+__global__ void __launch_bounds__(256) sum_kernel(const float* part, const float* dpre, const float* dy, int ctas,
+                                                  int64_t n, float* grads, float* loss)
 {
-    float acc = 0.0f;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n * kOut;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t r = i / kOut;
-        const int c = (int)(i % kOut);
-        float g = 0.0f;
-        if (c < kOutReal) {
-            const float d = y[i] - t[r * kOutReal + c];
-            acc += d * d;
-            g = 2.0f * d / (float)n;
+    const int t = threadIdx.x;
+    if (blockIdx.x < kWeightBlocks) {
+        const int i = blockIdx.x * 256 + t;
+        const bool bias = (i >= ob1 && i < oW2) || (i >= ob2 && i < oW3) || (i >= ob3 && i < oW4) ||
+                          (i >= ob4 && i < kParams);
+        if (i > kParams || bias) return;
+        double s = 0.0;
+#pragma unroll 8
+        for (int c = 0; c < ctas; ++c) s += (double)part[(int64_t)c * kPart + i];
+        if (i < kParams) grads[i] += (float)s;
+        else *loss = (float)(s / (double)n);
+        return;
+    }
+    const int b = blockIdx.x - kWeightBlocks, layer = b / (kHid / 8), c0 = (b % (kHid / 8)) * 8;
+    float v[8] = {};
+    if (layer < 3) {
+#pragma unroll 4
+        for (int64_t r = t; r < n; r += 256) {
+            const float4* q = reinterpret_cast<const float4*>(dpre + ((int64_t)layer * n + r) * kHid + c0);
+            const float4 x = q[0], y = q[1];
+            v[0] += x.x; v[1] += x.y; v[2] += x.z; v[3] += x.w;
+            v[4] += y.x; v[5] += y.y; v[6] += y.z; v[7] += y.w;
         }
-        dy[i] = g;
+    } else {
+#pragma unroll 4
+        for (int64_t r = t; r < n; r += 256) {
+            const float4 x = reinterpret_cast<const float4*>(dy)[r];
+            v[0] += x.x; v[1] += x.y; v[2] += x.z;
+        }
     }
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if ((threadIdx.x & 31) == 0) atomicAdd(loss, acc / (float)n);
-}
-
-// grad[col] += sum over rows of x[row * ld + col] (cols < n_valid)
-__global__ void colsum_kernel(const float* x, int64_t rows, int cols, int64_t ld, int n_valid, float* grad)
-{
-    const int col = blockIdx.x;
-    float acc = 0.0f;
-    for (int64_t r = threadIdx.x; r < rows; r += blockDim.x) acc += x[r * ld + col];
-    __shared__ float part[32];
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = acc;
+    __shared__ float part8[8][8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+        for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
+    if ((t & 31) == 0)
+#pragma unroll
+        for (int k = 0; k < 8; ++k) part8[k][t >> 5] = v[k];
     __syncthreads();
-    if (threadIdx.x < 32) {
-        float s = threadIdx.x < (blockDim.x >> 5) ? part[threadIdx.x] : 0.0f;
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (threadIdx.x == 0 && col < n_valid) grad[col] += s;
+    if (t < 8) {
+        const float* s = part8[t];
+        const float sum = ((s[0] + s[4]) + (s[2] + s[6])) + ((s[1] + s[5]) + (s[3] + s[7]));
+        if (layer == 0) grads[ob1 + c0 + t] += sum;
+        else if (layer == 1) grads[ob2 + c0 + t] += sum;
+        else if (layer == 2) grads[ob3 + c0 + t] += sum;
+        else if (t < kOutReal) grads[ob4 + t] += sum;
     }
-    (void)cols;
 }
 
 __global__ void adam_kernel(float* p, float* g, float* m, float* v, int n, float lr, float b1, float b2,
@@ -334,120 +500,58 @@ int mcuda(cudaError_t e, const char* what)
     return e == cudaErrorMemoryAllocation ? DISCO_ENOMEM : DISCO_ECUDA;
 }
 
-Operand op(const void* p, int dtype, int transposed, int64_t ld) { return Operand{ p, dtype, transposed, ld }; }
-
-// One GEMM launch; split > 1 splits K over blockIdx.z (EPI_ATOMIC* only).
-int gemm(const Operand& A, const Operand& B, int M, int N, int K, int epi, float* C, int64_t ldc,
-         __nv_bfloat16* H, int64_t ldh, const float* bias, const float* pre, int64_t ldp, int split,
-         int n_valid, int m_valid, int* status, cudaStream_t s)
-{
-    GemmArgs g;
-    std::memset(&g, 0, sizeof(g));
-    g.A = A; g.B = B; g.M = M; g.N = N; g.K = K;
-    g.k_per_split = split > 1 ? (int)(((K + split - 1) / split + kTileK - 1) / kTileK * kTileK) : K;
-    g.epi = epi; g.C = C; g.ldc = ldc; g.H = H; g.ldh = ldh; g.bias = bias; g.pre = pre; g.ldp = ldp;
-    g.n_valid = n_valid; g.m_valid = m_valid; g.status = status;
-    const int zs = (int)((K + g.k_per_split - 1) / g.k_per_split);
-    if (N == 16) {
-        const size_t smem = (size_t)(kTileM + 16) * kTileK * sizeof(__nv_bfloat16);
-        cudaFuncSetAttribute(gemm_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        dim3 grid((M + kTileM - 1) / kTileM, 1, zs);
-        gemm_kernel<16><<<grid, kThreads, smem, s>>>(g);
-    } else if (N % 128 == 0) {
-        const size_t smem = (size_t)(kTileM + 128) * kTileK * sizeof(__nv_bfloat16);
-        cudaFuncSetAttribute(gemm_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        dim3 grid((M + kTileM - 1) / kTileM, N / 128, zs);
-        gemm_kernel<128><<<grid, kThreads, smem, s>>>(g);
-    } else {
-        return mfail(DISCO_EINVAL, "GEMM N must be 16 or a multiple of 128");
-    }
-    const cudaError_t e = cudaGetLastError();
-    return e == cudaSuccess ? DISCO_OK : mcuda(e, "gemm launch");
-}
-
 void free_mlp(disco_mlp* p)
 {
     if (!p) return;
-    float* fs[] = { p->params, p->grads, p->m, p->v, p->loss, p->pre1, p->pre2, p->pre3, p->y, p->dy, p->dpre };
+    float* fs[] = { p->params, p->grads, p->m, p->v, p->loss, p->part };
     for (float* f : fs) if (f) cudaFree(f);
-    __nv_bfloat16* hs[] = { p->h1, p->h2, p->h3, p->dpre_h };
-    for (auto* h : hs) if (h) cudaFree(h);
     if (p->status) cudaFree(p->status);
     if (p->packed) cudaFree(p->packed);
     delete p;
 }
 
-int ensure_workspace(disco_mlp* p, int64_t n)
+// Queues the network over n rows of X: forward into Y (T null), or forward and
+// backward into the gradients and the loss.
+int run_net(disco_mlp* p, const float* X, const float* T, int64_t n, float* Y, cudaStream_t s)
 {
-    if (n <= p->cap) return DISCO_OK;
-    float** fs[] = { &p->pre1, &p->pre2, &p->pre3, &p->dpre };
-    for (float** f : fs) { if (*f) cudaFree(*f); *f = nullptr; }
-    if (p->y) cudaFree(p->y);
-    if (p->dy) cudaFree(p->dy);
-    __nv_bfloat16** hs[] = { &p->h1, &p->h2, &p->h3, &p->dpre_h };
-    for (auto** h : hs) { if (*h) cudaFree(*h); *h = nullptr; }
-    p->y = p->dy = nullptr;
-    cudaError_t e = cudaSuccess;
-    for (float** f : fs) if (e == cudaSuccess) e = cudaMalloc(f, (size_t)n * kHid * sizeof(float));
-    if (e == cudaSuccess) e = cudaMalloc(&p->y, (size_t)n * kOut * sizeof(float));
-    if (e == cudaSuccess) e = cudaMalloc(&p->dy, (size_t)n * kOut * sizeof(float));
-    for (auto** h : hs) if (e == cudaSuccess) e = cudaMalloc(h, (size_t)n * kHid * sizeof(__nv_bfloat16));
-    if (e != cudaSuccess) { p->cap = 0; return mcuda(e, "MLP workspace"); }
-    p->cap = n;
-    return DISCO_OK;
-}
-
-// Forward over n rows of X [n x 16] (FP32): fills pre1..3, h1..3 and y [n x 16].
-int forward(disco_mlp* p, const float* X, int64_t n, cudaStream_t s)
-{
-    const float* P = p->params;
-    int st = gemm(op(X, kF32, 0, kIn), op(P + oW1, kF32, 0, kIn), (int)n, kHid, kIn, EPI_SILU,
-                  p->pre1, kHid, p->h1, kHid, P + ob1, nullptr, 0, 1, 0, 0, p->status, s);
-    if (!st) st = gemm(op(p->h1, kBF16, 0, kHid), op(P + oW2, kF32, 0, kHid), (int)n, kHid, kHid, EPI_SILU,
-                       p->pre2, kHid, p->h2, kHid, P + ob2, nullptr, 0, 1, 0, 0, p->status, s);
-    if (!st) st = gemm(op(p->h2, kBF16, 0, kHid), op(P + oW3, kF32, 0, kHid), (int)n, kHid, kHid, EPI_SILU,
-                       p->pre3, kHid, p->h3, kHid, P + ob3, nullptr, 0, 1, 0, 0, p->status, s);
-    if (!st) st = gemm(op(p->h3, kBF16, 0, kHid), op(P + oW4, kF32, 0, kHid), (int)n, kOut, kHid, EPI_STORE,
-                       p->y, kOut, nullptr, 0, P + ob4, nullptr, 0, 1, 0, 0, p->status, s);
-    return st;
-}
-
-// Backward of the MSE loss after forward(): accumulates into p->grads.
-int backward(disco_mlp* p, const float* X, const float* T, int64_t n, cudaStream_t s)
-{
-    const float* P = p->params;
-    float* G = p->grads;
-    const int nb = (int)std::min<int64_t>(1024, (n * kOut + 255) / 256);
-    mse_grad_kernel<<<nb, 256, 0, s>>>(p->y, T, n, p->dy, p->loss);
-    const int split = (int)std::max<int64_t>(1, std::min<int64_t>(64, n / kTileK));
-    const int N = (int)n;
-    // layer 4: dW4^T = h3^T dy, db4, dh3 = dy W4 -> dpre3
-    int st = gemm(op(p->h3, kBF16, 1, kHid), op(p->dy, kF32, 1, kOut), kHid, kOut, N, EPI_ATOMIC_T,
-                  G + oW4, kHid, nullptr, 0, nullptr, nullptr, 0, split, kOutReal, kHid, p->status, s);
-    if (!st) { colsum_kernel<<<kOut, 256, 0, s>>>(p->dy, n, kOut, kOut, kOutReal, G + ob4); }
-    if (!st) st = gemm(op(p->dy, kF32, 0, kOut), op(P + oW4, kF32, 1, kHid), N, kHid, kOut, EPI_DSILU,
-                       p->dpre, kHid, p->dpre_h, kHid, nullptr, p->pre3, kHid, 1, 0, 0, p->status, s);
-    // layer 3
-    if (!st) st = gemm(op(p->dpre_h, kBF16, 1, kHid), op(p->h2, kBF16, 1, kHid), kHid, kHid, N, EPI_ATOMIC,
-                       G + oW3, kHid, nullptr, 0, nullptr, nullptr, 0, split, kHid, kHid, p->status, s);
-    if (!st) { colsum_kernel<<<kHid, 256, 0, s>>>(p->dpre, n, kHid, kHid, kHid, G + ob3); }
-    if (!st) st = gemm(op(p->dpre_h, kBF16, 0, kHid), op(P + oW3, kF32, 1, kHid), N, kHid, kHid, EPI_DSILU,
-                       p->dpre, kHid, p->h3, kHid, nullptr, p->pre2, kHid, 1, 0, 0, p->status, s);
-    // (h3 is free now and holds dpre2 in BF16)
-    if (!st) st = gemm(op(p->h3, kBF16, 1, kHid), op(p->h1, kBF16, 1, kHid), kHid, kHid, N, EPI_ATOMIC,
-                       G + oW2, kHid, nullptr, 0, nullptr, nullptr, 0, split, kHid, kHid, p->status, s);
-    if (!st) { colsum_kernel<<<kHid, 256, 0, s>>>(p->dpre, n, kHid, kHid, kHid, G + ob2); }
-    if (!st) st = gemm(op(p->h3, kBF16, 0, kHid), op(P + oW2, kF32, 1, kHid), N, kHid, kHid, EPI_DSILU,
-                       p->dpre, kHid, p->dpre_h, kHid, nullptr, p->pre1, kHid, 1, 0, 0, p->status, s);
-    // layer 1: dW1 = dpre1^T X (input padding columns masked), db1
-    if (!st) st = gemm(op(p->dpre_h, kBF16, 1, kHid), op(X, kF32, 1, kIn), kHid, kIn, N, EPI_ATOMIC,
-                       G + oW1, kIn, nullptr, 0, nullptr, nullptr, 0, split, kInReal, kHid, p->status, s);
-    if (!st) { colsum_kernel<<<kHid, 256, 0, s>>>(p->dpre, n, kHid, kHid, kHid, G + ob1); }
-    if (!st) {
-        const cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) st = mcuda(e, "MLP backward");
+    if (n > (int64_t)0x7FFFFFFF * kRows) return mfail(DISCO_ELIMIT, "too many rows");
+    if (!p->sms) {
+        int dev = 0;
+        cudaError_t e = cudaGetDevice(&dev);
+        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&p->sms, cudaDevAttrMultiProcessorCount, dev);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(net_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kNetSmem);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(net_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kNetSmem);
+        if (e != cudaSuccess) { p->sms = 0; return mcuda(e, "network setup"); }
     }
-    return st;
+    NetArgs a;
+    std::memset(&a, 0, sizeof(a));
+    a.P = p->params;
+    a.X = X; a.T = T; a.Y = Y;
+    a.n = n;
+    a.tiles = (int32_t)((n + kRows - 1) / kRows);
+    a.x16 = (reinterpret_cast<uintptr_t>(X) & 15) == 0;
+    a.y16 = (reinterpret_cast<uintptr_t>(Y) & 15) == 0;
+    a.status = p->status;
+    const int grid = std::min(a.tiles, p->sms);
+    if (T && n > p->cap) {
+        // partial gradients, and dpre and dy of n rows
+        if (p->part) cudaFree(p->part);
+        const size_t floats = (size_t)p->sms * kPart + (size_t)n * (3 * kHid + 4);
+        const cudaError_t e = cudaMalloc(&p->part, floats * sizeof(float));
+        if (e != cudaSuccess) { p->part = nullptr; p->cap = 0; return mcuda(e, "MLP workspace"); }
+        p->cap = n;
+    }
+    a.part = p->part;
+    a.dpre = p->part ? p->part + (size_t)p->sms * kPart : nullptr;
+    a.dy = a.dpre ? a.dpre + (size_t)n * 3 * kHid : nullptr;
+    if (T) {
+        net_kernel<true><<<grid, kNetThreads, kNetSmem, s>>>(a);
+        sum_kernel<<<kWeightBlocks + kBiasBlocks, 256, 0, s>>>(a.part, a.dpre, a.dy, grid, n, p->grads, p->loss);
+    } else {
+        net_kernel<false><<<grid, kNetThreads, kNetSmem, s>>>(a);
+    }
+    const cudaError_t e = cudaGetLastError();
+    return e == cudaSuccess ? DISCO_OK : mcuda(e, "network launch");
 }
 
 } // namespace
@@ -531,13 +635,7 @@ int disco_b200_mlp_forward(disco_mlp* p, const float* X, int64_t n, float* Y, vo
 {
     if (!p || n < 0 || (n > 0 && (!X || !Y))) return mfail(DISCO_EINVAL, "bad argument");
     if (n == 0) return DISCO_OK;
-    int st = ensure_workspace(p, n);
-    if (st) return st;
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
-    st = forward(p, X, n, s);
-    if (st) return st;
-    const cudaError_t e = cudaMemcpyAsync(Y, p->y, (size_t)n * kOut * sizeof(float), cudaMemcpyDeviceToDevice, s);
-    return e == cudaSuccess ? DISCO_OK : mcuda(e, "forward output");
+    return run_net(p, X, nullptr, n, Y, static_cast<cudaStream_t>(stream));
 }
 
 // Forward + backward of the MSE loss over n rows; gradients accumulate in the
@@ -545,14 +643,10 @@ int disco_b200_mlp_forward(disco_mlp* p, const float* X, int64_t n, float* Y, vo
 int disco_b200_mlp_grad(disco_mlp* p, const float* X, const float* T, int64_t n, float* loss, void* stream)
 {
     if (!p || n <= 0 || !X || !T) return mfail(DISCO_EINVAL, "bad argument");
-    int st = ensure_workspace(p, n);
-    if (st) return st;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    cudaError_t e = cudaMemsetAsync(p->loss, 0, sizeof(float), s);
-    if (e != cudaSuccess) return mcuda(e, "loss reset");
-    st = forward(p, X, n, s);
-    if (!st) st = backward(p, X, T, n, s);
+    const int st = run_net(p, X, T, n, nullptr, s);
     if (st) return st;
+    cudaError_t e;
     if (loss) {
         e = cudaMemcpyAsync(loss, p->loss, sizeof(float), cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);

@@ -43,9 +43,9 @@ struct disco_mlp {
     float* m = nullptr;
     float* v = nullptr;
     float* loss = nullptr;     // device scalar
-    int64_t cap = 0;           // rows of the workspace below
-    float *pre1 = nullptr, *pre2 = nullptr, *pre3 = nullptr, *y = nullptr, *dy = nullptr, *dpre = nullptr;
-    __nv_bfloat16 *h1 = nullptr, *h2 = nullptr, *h3 = nullptr, *dpre_h = nullptr;
+    float* part = nullptr;     // one call's partial gradients, dpre and dy
+    int64_t cap = 0;           // rows that `part` holds
+    int sms = 0;
     int64_t step = 0;
     int* status = nullptr;
     unsigned char* packed = nullptr;   // inference image of the weights (far.cu)

@@ -66,3 +66,28 @@ def test_training_reduces_loss():
         first = loss if first is None else first
     m.status()
     assert loss < 0.1 * first
+
+
+@pytest.mark.parametrize("n", [1, 127, 129, 5000, 148 * 128 + 1])
+def test_row_counts_and_unaligned_rows(n):
+    """One row, the edges of a tile and more tiles than CTAs, rows that are only
+    4-byte aligned; a repeated call adds the same bits to the gradients."""
+    torch = pytest.importorskip("torch")
+    m = MLP(seed=5)
+    X, T = _data(n, seed=n)
+    flat = torch.zeros(n * 16 + 1, dtype=torch.float32, device="cuda")
+    Xd = flat[1:].view(n, 16)
+    Xd.copy_(torch.from_numpy(X))
+    Td = torch.from_numpy(T).cuda()
+    loss = m.grad(Xd, Td)
+    m.status()
+    g = m.grads()
+    ref_loss, ref = R.grads(m.params(), X, T)
+    assert abs(loss - ref_loss) <= 1e-3 * ref_loss
+    for name, (o, s) in R.OFF.items():
+        a, b = g[o:o + s].astype(np.float64), ref[o:o + s]
+        nb = np.linalg.norm(b)
+        assert np.linalg.norm(a - b) <= 2e-2 * nb if nb else np.abs(a).max() == 0.0, name
+    m.grad(Xd, Td)
+    assert np.array_equal(m.grads(), g + g)
+    assert torch.equal(m.forward(Xd), m.forward(torch.from_numpy(X).cuda()))
