@@ -103,7 +103,7 @@ void free_plan(disco_plan* p)
     if (p->d_status) cudaFree(p->d_status);
     if (p->d_near) cudaFree(p->d_near);
     if (p->d_near_count) cudaFree(p->d_near_count);
-    if (p->tree_pool) disco::tree_pool_release(p->device);
+    if (p->tree_pool) disco::scratch_release(p->device);
     delete p;
 }
 
@@ -125,7 +125,7 @@ disco::TreeShape plan_tree(disco_plan* p, int k, int64_t n, cudaStream_t s)
         p->tree_n[k] = n;
     }
     if (p->tree[k].use && !p->tree_pool) {
-        disco::tree_pool_retain(p->device);
+        disco::scratch_retain(p->device);
         p->tree_pool = true;
     }
     return p->tree[k];
@@ -138,6 +138,57 @@ double now_s()
 }
 
 } // namespace
+
+namespace {
+
+constexpr int kMaxDevices = 64;
+constexpr uint64_t kScratchKeep = 4ull << 20, kScratchKeepPlans = 256ull << 20;
+std::mutex g_scratch_mutex;
+cudaMemPool_t g_scratch[kMaxDevices] = {};
+int g_scratch_plans[kMaxDevices] = {};
+
+void scratch_keep(int device, uint64_t bytes)
+{
+    if (!g_scratch[device]) return;
+    if (cudaMemPoolSetAttribute(g_scratch[device], cudaMemPoolAttrReleaseThreshold, &bytes) != cudaSuccess)
+        cudaGetLastError();
+}
+
+} // namespace
+
+cudaMemPool_t disco::scratch_pool(int device)
+{
+    if (device < 0 || device >= kMaxDevices) return nullptr;
+    std::lock_guard<std::mutex> lock(g_scratch_mutex);
+    if (!g_scratch[device]) {
+        cudaMemPoolProps props;
+        std::memset(&props, 0, sizeof(props));
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = device;
+        cudaMemPool_t p = nullptr;
+        if (cudaMemPoolCreate(&p, &props) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+        g_scratch[device] = p;
+        scratch_keep(device, g_scratch_plans[device] > 0 ? kScratchKeepPlans : kScratchKeep);
+    }
+    return g_scratch[device];
+}
+
+void disco::scratch_retain(int device)
+{
+    if (device < 0 || device >= kMaxDevices) return;
+    std::lock_guard<std::mutex> lock(g_scratch_mutex);
+    if (++g_scratch_plans[device] == 1) scratch_keep(device, kScratchKeepPlans);
+}
+
+void disco::scratch_release(int device)
+{
+    if (device < 0 || device >= kMaxDevices) return;
+    std::lock_guard<std::mutex> lock(g_scratch_mutex);
+    if (--g_scratch_plans[device] > 0 || !g_scratch[device]) return;
+    scratch_keep(device, kScratchKeep);
+    if (cudaMemPoolTrimTo(g_scratch[device], kScratchKeep) != cudaSuccess) cudaGetLastError();
+}
 
 void disco::set_last_error(const std::string& msg) { store_error(msg.c_str()); }
 void disco::set_last_error(const char* msg) { store_error(msg); }

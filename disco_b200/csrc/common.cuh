@@ -15,6 +15,14 @@ namespace disco {
 void set_last_error(const std::string& msg);
 void set_last_error(const char* msg);
 
+// Stream-ordered scratch memory, one pool per device (null where none could be
+// made).  4 MB stay reserved in it, and up to 256 MB while a plan that has used
+// it lives (retain / release): the default pool gives its memory back at every
+// synchronisation, and a call after one then pays for mapping it again (0.4 ms).
+cudaMemPool_t scratch_pool(int device);
+void scratch_retain(int device);
+void scratch_release(int device);
+
 // A bounded wait gives up after this many nanoseconds of %globaltimer.  A stage
 // copy of a few hundred KB completes in microseconds; the bound only exists so
 // that no wait can spin forever.

@@ -49,7 +49,6 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
-#include <mutex>
 #include <string>
 #include <vector>
 
@@ -1484,21 +1483,6 @@ TreeShape tree_shape(const HostTable& T, int64_t n, const double box[3], int ima
 
 namespace {
 
-// One pool per device: at most 256 MB stay reserved while a plan that has
-// used it lives, nothing after the last one.
-constexpr int kMaxDevices = 64;
-constexpr uint64_t kPoolKeep = 256ull << 20;
-std::mutex g_pool_mutex;
-cudaMemPool_t g_pool[kMaxDevices] = {};
-int g_pool_users[kMaxDevices] = {};
-
-cudaMemPool_t tree_pool(int device)
-{
-    if (device < 0 || device >= kMaxDevices) return nullptr;
-    std::lock_guard<std::mutex> lock(g_pool_mutex);
-    return g_pool[device];
-}
-
 template <int QC>
 cudaError_t down(const TreeArgs& a, int t, int cells, cudaStream_t s)
 {
@@ -1553,32 +1537,6 @@ cudaError_t leaf_any(const TreeArgs& a, cudaStream_t s)
 }
 
 } // namespace
-
-void tree_pool_retain(int device)
-{
-    if (device < 0 || device >= kMaxDevices) return;
-    std::lock_guard<std::mutex> lock(g_pool_mutex);
-    ++g_pool_users[device];
-    if (g_pool[device]) return;
-    cudaMemPoolProps props;
-    std::memset(&props, 0, sizeof(props));
-    props.allocType = cudaMemAllocationTypePinned;
-    props.location.type = cudaMemLocationTypeDevice;
-    props.location.id = device;
-    cudaMemPool_t p = nullptr;
-    uint64_t keep = kPoolKeep;
-    if (cudaMemPoolCreate(&p, &props) != cudaSuccess) { cudaGetLastError(); return; }
-    if (cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) cudaGetLastError();
-    g_pool[device] = p;
-}
-
-void tree_pool_release(int device)
-{
-    if (device < 0 || device >= kMaxDevices) return;
-    std::lock_guard<std::mutex> lock(g_pool_mutex);
-    if (--g_pool_users[device] > 0 || !g_pool[device]) return;
-    if (cudaMemPoolTrimTo(g_pool[device], 0) != cudaSuccess) cudaGetLastError();
-}
 
 int launch_tree(const FieldArgs& f, const HostTable& T, const TreeShape& S, int sm_count,
                 cudaStream_t s, bool* ran, std::string& err)
@@ -1662,7 +1620,7 @@ int launch_tree(const FieldArgs& f, const HostTable& T, const TreeShape& S, int 
     const size_t o_mat = take(mats * sizeof(double));
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) { cudaGetLastError(); return DISCO_OK; }
-    cudaMemPool_t pool = tree_pool(dev);
+    cudaMemPool_t pool = scratch_pool(dev);
     if (!pool) return DISCO_OK;
     unsigned char* ws = nullptr;
     if (cudaMallocFromPoolAsync(reinterpret_cast<void**>(&ws), at, pool, s) != cudaSuccess) {

@@ -44,9 +44,4 @@ TreeShape tree_shape(const HostTable& T, int64_t n, const double box[3], int ima
 int launch_tree(const FieldArgs& a, const HostTable& T, const TreeShape& S, int sm_count,
                 cudaStream_t stream, bool* ran, std::string& err);
 
-// Scratch pool of the cell sum: one per device, shared by the plans that have
-// used it and given back when the last of them goes.
-void tree_pool_retain(int device);
-void tree_pool_release(int device);
-
 } // namespace disco

@@ -94,3 +94,36 @@ def test_finalize_then_format_matches_the_reference_epilogue_and_writer():
         assert np.array_equal(f[d], ref[d])
     text = _format(0, "W", fin[:3].contiguous())
     assert text == O.format_atoms(0, "W", ref[0], ref[1], ref[2])
+
+
+def test_lengths_at_powers_of_ten_and_any_output_address():
+    """Values a few units in the last place around every 10^k - 5e-9 (where a
+    digit is gained by rounding) and 10^k, both signs, the longest element name,
+    and a text that starts at every address modulo 16."""
+    v = []
+    for k in range(0, 12):
+        for c in (10.0 ** k, 10.0 ** k - 5e-9):
+            x = c
+            for _ in range(4):
+                x = np.nextafter(x, 0.0)
+            for _ in range(9):
+                v += [x, -x]
+                x = np.nextafter(x, np.inf)
+    v = np.array(v[: len(v) // 3 * 3]).reshape(3, -1)
+    pos = torch.tensor(v, dtype=torch.float64, device="cuda")
+    element = "E" * 64
+    want = O.format_atoms(0, element, v[0], v[1], v[2])
+    assert _format(0, element, pos) == want
+    lib = C.cuda_lib()
+    n = v.shape[1]
+    buf = torch.full((len(want) + 64,), 7, dtype=torch.uint8, device="cuda")
+    got = ctypes.c_int64()
+    s = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    for off in range(16):
+        buf.fill_(7)
+        C.check(lib.disco_b200_format_atoms(0, element.encode(), pos[0].data_ptr(), pos[1].data_ptr(),
+                                            pos[2].data_ptr(), n, buf.data_ptr() + off, len(want), ctypes.byref(got),
+                                            s), lib)
+        b = bytes(buf.cpu().numpy())
+        assert b[off:off + len(want)] == want
+        assert set(b[:off]) <= {7} and set(b[off + len(want):]) == {7}
