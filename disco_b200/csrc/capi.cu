@@ -11,6 +11,7 @@
 #include <string>
 #include <vector>
 
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include "common.cuh"
@@ -31,10 +32,16 @@ struct disco_plan {
     int nimg = 1;
     int nloops = 0;
     disco::HostTable tables[2];              // line, loopon
+    // one block of device memory: the image (status word, tables, chunk lists)
+    // and behind it the FP32 line form's list of atoms with near-cut pairs
+    std::vector<unsigned char> image;        // host copy until the upload
+    size_t table_at[2] = { 0, 0 }, chunks_at[2] = { 0, 0 }, near_at = 0, bytes = 0;
+    unsigned char* block = nullptr;          // owned where `own`
+    bool own = false;
     unsigned char* d_table[2] = { nullptr, nullptr };
     disco::Chunk* d_chunks[2] = { nullptr, nullptr };
     int* d_status = nullptr;
-    int32_t* d_near = nullptr;               // FP32 line form: atoms with near-cut pairs
+    int32_t* d_near = nullptr;
     unsigned int* d_near_count = nullptr;
     int32_t near_cap = 0;
     std::vector<double> loop_evals;          // per input loop: segments or loopons
@@ -96,13 +103,7 @@ int check_options(const disco_options& o)
 void free_plan(disco_plan* p)
 {
     if (!p) return;
-    for (int k = 0; k < 2; ++k) {
-        if (p->d_table[k]) cudaFree(p->d_table[k]);
-        if (p->d_chunks[k]) cudaFree(p->d_chunks[k]);
-    }
-    if (p->d_status) cudaFree(p->d_status);
-    if (p->d_near) cudaFree(p->d_near);
-    if (p->d_near_count) cudaFree(p->d_near_count);
+    if (p->own && p->block) cudaFree(p->block);
     if (p->tree_pool) disco::scratch_release(p->device);
     delete p;
 }
@@ -142,10 +143,21 @@ double now_s()
 namespace {
 
 constexpr int kMaxDevices = 64;
-constexpr uint64_t kScratchKeep = 4ull << 20, kScratchKeepPlans = 256ull << 20;
+constexpr uint64_t kScratchKeep = 32ull << 20, kScratchKeepPlans = 256ull << 20;
 std::mutex g_scratch_mutex;
 cudaMemPool_t g_scratch[kMaxDevices] = {};
+unsigned long long g_scratch_ctx[kMaxDevices] = {};     // the context each pool was made in
 int g_scratch_plans[kMaxDevices] = {};
+
+// Idle non-blocking streams of host calls, at most four: making and destroying
+// one costs 0.12 ms, more than such a call's copies.
+struct IdleStream { cudaStream_t stream; int device; unsigned long long ctx; };
+constexpr size_t kIdleStreams = 4;
+std::mutex g_idle_mutex;
+std::vector<IdleStream> g_idle;
+
+using CtxGetCurrentFn = CUresult (*)(CUcontext*);
+using CtxGetIdFn = CUresult (*)(CUcontext, unsigned long long*);
 
 void scratch_keep(int device, uint64_t bytes)
 {
@@ -154,13 +166,65 @@ void scratch_keep(int device, uint64_t bytes)
         cudaGetLastError();
 }
 
+cudaError_t take_stream(int device, IdleStream& out)
+{
+    out = { nullptr, device, disco::current_context_id() };
+    {
+        std::lock_guard<std::mutex> lock(g_idle_mutex);
+        for (size_t k = 0; k < g_idle.size(); ++k)
+            if (g_idle[k].device == device && g_idle[k].ctx == out.ctx && out.ctx != 0) {
+                out.stream = g_idle[k].stream;
+                g_idle.erase(g_idle.begin() + k);
+                return cudaSuccess;
+            }
+    }
+    return cudaStreamCreateWithFlags(&out.stream, cudaStreamNonBlocking);
+}
+
+void give_stream(const IdleStream& s, bool healthy)
+{
+    if (!s.stream) return;
+    if (healthy && s.ctx != 0) {
+        std::lock_guard<std::mutex> lock(g_idle_mutex);
+        // streams of a context that is gone are gone with it
+        for (size_t k = g_idle.size(); k-- > 0;)
+            if (g_idle[k].device == s.device && g_idle[k].ctx != s.ctx) g_idle.erase(g_idle.begin() + k);
+        if (g_idle.size() < kIdleStreams) { g_idle.push_back(s); return; }
+    }
+    cudaStreamDestroy(s.stream);
+}
+
 } // namespace
+
+// The driver's cuCtxGetId, reached through the runtime without linking libcuda.
+unsigned long long disco::current_context_id()
+{
+    static CtxGetCurrentFn get_current = nullptr;
+    static CtxGetIdFn get_id = nullptr;
+    static std::once_flag once;
+    std::call_once(once, [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPointByVersion("cuCtxGetCurrent", &f, 12000, cudaEnableDefault, &q) == cudaSuccess &&
+            q == cudaDriverEntryPointSuccess)
+            get_current = reinterpret_cast<CtxGetCurrentFn>(f);
+        f = nullptr;
+        if (cudaGetDriverEntryPointByVersion("cuCtxGetId", &f, 12000, cudaEnableDefault, &q) == cudaSuccess &&
+            q == cudaDriverEntryPointSuccess)
+            get_id = reinterpret_cast<CtxGetIdFn>(f);
+    });
+    CUcontext c = nullptr;
+    unsigned long long id = 0;
+    if (get_current && get_id && get_current(&c) == CUDA_SUCCESS && c && get_id(c, &id) == CUDA_SUCCESS) return id;
+    return 0;
+}
 
 cudaMemPool_t disco::scratch_pool(int device)
 {
     if (device < 0 || device >= kMaxDevices) return nullptr;
+    const unsigned long long ctx = current_context_id();
     std::lock_guard<std::mutex> lock(g_scratch_mutex);
-    if (!g_scratch[device]) {
+    if (!g_scratch[device] || ctx == 0 || ctx != g_scratch_ctx[device]) {
         cudaMemPoolProps props;
         std::memset(&props, 0, sizeof(props));
         props.allocType = cudaMemAllocationTypePinned;
@@ -169,6 +233,7 @@ cudaMemPool_t disco::scratch_pool(int device)
         cudaMemPool_t p = nullptr;
         if (cudaMemPoolCreate(&p, &props) != cudaSuccess) { cudaGetLastError(); return nullptr; }
         g_scratch[device] = p;
+        g_scratch_ctx[device] = ctx;
         scratch_keep(device, g_scratch_plans[device] > 0 ? kScratchKeepPlans : kScratchKeep);
     }
     return g_scratch[device];
@@ -178,14 +243,15 @@ void disco::scratch_retain(int device)
 {
     if (device < 0 || device >= kMaxDevices) return;
     std::lock_guard<std::mutex> lock(g_scratch_mutex);
-    if (++g_scratch_plans[device] == 1) scratch_keep(device, kScratchKeepPlans);
+    if (++g_scratch_plans[device] == 1 && current_context_id() == g_scratch_ctx[device])
+        scratch_keep(device, kScratchKeepPlans);
 }
 
 void disco::scratch_release(int device)
 {
     if (device < 0 || device >= kMaxDevices) return;
     std::lock_guard<std::mutex> lock(g_scratch_mutex);
-    if (--g_scratch_plans[device] > 0 || !g_scratch[device]) return;
+    if (--g_scratch_plans[device] > 0 || !g_scratch[device] || current_context_id() != g_scratch_ctx[device]) return;
     scratch_keep(device, kScratchKeep);
     if (cudaMemPoolTrimTo(g_scratch[device], kScratchKeep) != cudaSuccess) cudaGetLastError();
 }
@@ -247,8 +313,13 @@ void disco_b200_options_default(disco_options* o)
     o->chunk_pairs = -1.0;        // GpuOptions default (Code/backend.hpp:55)
 }
 
-int disco_b200_plan_create(const disco_loop* loops, int32_t nloops, const double box[3],
-                           const disco_options* opt, int64_t max_atoms, disco_plan** out)
+} // extern "C"
+
+namespace {
+
+// A plan without its device memory: checks, tables, and the block's layout.
+int plan_build(const disco_loop* loops, int32_t nloops, const double box[3], const disco_options* opt,
+               int64_t max_atoms, disco_plan** out)
 {
     if (!out) return fail(DISCO_EINVAL, "null plan pointer");
     *out = nullptr;
@@ -292,31 +363,74 @@ int disco_b200_plan_create(const disco_loop* loops, int32_t nloops, const double
         for (int l = 0; l < nloops; ++l) p->loop_evals[l] += T.loop_evals[l];
         p->stats.n_segments += T.n_segments;
         p->stats.n_loopons += T.n_loopons;
-        if (T.chunks.empty()) continue;
-        e = cudaMalloc(&p->d_table[k], T.bytes.size());
-        if (e == cudaSuccess) e = cudaMemcpy(p->d_table[k], T.bytes.data(), T.bytes.size(), cudaMemcpyHostToDevice);
-        if (e == cudaSuccess) e = cudaMalloc(&p->d_chunks[k], T.chunks.size() * sizeof(disco::Chunk));
-        if (e == cudaSuccess)
-            e = cudaMemcpy(p->d_chunks[k], T.chunks.data(), T.chunks.size() * sizeof(disco::Chunk),
-                           cudaMemcpyHostToDevice);
-        if (e != cudaSuccess) { free_plan(p); return cuda_fail(e, "loop table upload"); }
     }
     {
         const int inner = o.image_min > 0 ? 2 * o.image_min - 1 : 0;
         p->stats.n_images = p->nimg - inner * inner * inner;
     }
     p->stats.evals_per_atom = (double)(p->stats.n_segments + p->stats.n_loopons) * p->stats.n_images;
-    e = cudaMalloc(&p->d_status, sizeof(int));
-    if (e == cudaSuccess) e = cudaMemset(p->d_status, 0, sizeof(int));
-    if (e != cudaSuccess) { free_plan(p); return cuda_fail(e, "status word"); }
+    size_t at = 256;                                     // the status word
+    auto take = [&](size_t bytes) { const size_t o = at; at += (bytes + 255) & ~size_t(255); return o; };
+    for (int k = 0; k < 2; ++k) {
+        if (p->tables[k].chunks.empty()) continue;
+        p->table_at[k] = take(p->tables[k].bytes.size());
+        p->chunks_at[k] = take(p->tables[k].chunks.size() * sizeof(disco::Chunk));
+    }
+    p->image.assign(at, 0);
+    for (int k = 0; k < 2; ++k) {
+        disco::HostTable& T = p->tables[k];
+        if (T.chunks.empty()) continue;
+        std::memcpy(p->image.data() + p->table_at[k], T.bytes.data(), T.bytes.size());
+        std::memcpy(p->image.data() + p->chunks_at[k], T.chunks.data(), T.chunks.size() * sizeof(disco::Chunk));
+        std::vector<unsigned char>().swap(T.bytes);
+    }
     if (o.precision == DISCO_FP32C && !p->tables[0].chunks.empty()) {
         // the list of atoms with near-cut pairs: up to 2^21 (a longer list
         // overflows and the FP64 pass visits every atom)
         p->near_cap = (int32_t)std::min<int64_t>(std::max<int64_t>(max_atoms, 1 << 16), 1 << 21);
-        e = cudaMalloc(&p->d_near, (size_t)p->near_cap * sizeof(int32_t));
-        if (e == cudaSuccess) e = cudaMalloc(&p->d_near_count, sizeof(unsigned int));
-        if (e != cudaSuccess) { free_plan(p); return cuda_fail(e, "near-cut list"); }
+        p->near_at = take(256 + (size_t)p->near_cap * sizeof(int32_t));
     }
+    p->bytes = at;
+    *out = p;
+    return DISCO_OK;
+}
+
+// Gives a plan its block (p->bytes, 256-byte aligned; the image still has to be
+// copied to its start).
+void plan_place(disco_plan* p, unsigned char* block)
+{
+    p->block = block;
+    p->d_status = reinterpret_cast<int*>(block);
+    for (int k = 0; k < 2; ++k) {
+        if (p->tables[k].chunks.empty()) continue;
+        p->d_table[k] = block + p->table_at[k];
+        p->d_chunks[k] = reinterpret_cast<disco::Chunk*>(block + p->chunks_at[k]);
+    }
+    if (p->near_at) {
+        p->d_near_count = reinterpret_cast<unsigned int*>(block + p->near_at);
+        p->d_near = reinterpret_cast<int32_t*>(block + p->near_at + 256);
+    }
+}
+
+} // namespace
+
+extern "C" {
+
+int disco_b200_plan_create(const disco_loop* loops, int32_t nloops, const double box[3],
+                           const disco_options* opt, int64_t max_atoms, disco_plan** out)
+{
+    int st = plan_build(loops, nloops, box, opt, max_atoms, out);
+    if (st) return st;
+    disco_plan* p = *out;
+    *out = nullptr;
+    unsigned char* block = nullptr;
+    cudaError_t e = cudaMalloc(&block, p->bytes);
+    if (e != cudaSuccess) { free_plan(p); return cuda_fail(e, "plan memory"); }
+    plan_place(p, block);
+    p->own = true;
+    e = cudaMemcpy(block, p->image.data(), p->image.size(), cudaMemcpyHostToDevice);
+    if (e != cudaSuccess) { free_plan(p); return cuda_fail(e, "loop table upload"); }
+    std::vector<unsigned char>().swap(p->image);
     *out = p;
     return DISCO_OK;
 }
@@ -422,34 +536,64 @@ int disco_b200_displace(const disco_atoms* atoms, const disco_loop* loops, int32
 
     const double t0 = now_s();
     disco_plan* plan = nullptr;
-    int st = disco_b200_plan_create(loops, nloops, box, &o, n, &plan);
+    int st = plan_build(loops, nloops, box, &o, n, &plan);
     if (st) return st;
     if (o.verbose) {
         std::printf("Precision: %s\n", o.precision == DISCO_FP32C
                     ? "single (fp32 pair term, compensated sums)" : "double");
     }
-    double* d = nullptr;
-    cudaStream_t s = nullptr;
+    // one block of device memory: x, y, z, ux, uy, uz, then the plan's (its
+    // status word first), from the scratch pool or, without one, cudaMalloc
+    const size_t bytes = (size_t)n * sizeof(double), atoms_at = (6 * bytes + 255) & ~size_t(255);
+    unsigned char* block = nullptr;
+    bool pooled = false, healthy = false;
+    IdleStream is = { nullptr, 0, 0 };
     cudaEvent_t ev[2] = { nullptr, nullptr };
     auto cleanup = [&]() {
-        if (d) cudaFree(d);
-        if (s) cudaStreamDestroy(s);
-        for (auto& x : ev) if (x) cudaEventDestroy(x);
         disco_b200_plan_destroy(plan);
+        if (block && pooled) cudaFreeAsync(block, is.stream);
+        else if (block) cudaFree(block);
+        give_stream(is, healthy);
+        for (auto& x : ev) if (x) cudaEventDestroy(x);
     };
-    const size_t bytes = (size_t)n * sizeof(double);
-    cudaError_t e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
+    cudaError_t e = cudaFree(nullptr);                    // the primary context, before its identifier is read
+    if (e == cudaSuccess) e = take_stream(plan->device, is);
+    cudaStream_t s = is.stream;
     if (e == cudaSuccess) e = cudaEventCreate(&ev[0]);
     if (e == cudaSuccess) e = cudaEventCreate(&ev[1]);
-    if (e == cudaSuccess && n > 0) e = cudaMalloc(&d, 6 * bytes);
+    if (e == cudaSuccess) {
+        cudaMemPool_t pool = disco::scratch_pool(plan->device);
+        pooled = pool && cudaMallocFromPoolAsync(reinterpret_cast<void**>(&block), atoms_at + plan->bytes, pool, s) ==
+                             cudaSuccess;
+        if (!pooled) {
+            cudaGetLastError();
+            block = nullptr;
+            e = cudaMalloc(&block, atoms_at + plan->bytes);
+        }
+    }
+    if (e != cudaSuccess) { cleanup(); return cuda_fail(e, "atom allocation"); }
+    plan_place(plan, block + atoms_at);
+    // small calls: one copy each way through a packed host buffer
+    std::vector<unsigned char> pack;
+    const bool small = atoms_at + plan->image.size() <= (size_t)128 << 10;
     const double* src[6] = { atoms->x, atoms->y, atoms->z, atoms->ux, atoms->uy, atoms->uz };
-    for (int k = 0; k < 6 && e == cudaSuccess && n > 0; ++k)
-        e = cudaMemcpyAsync(d + (size_t)k * n, src[k], bytes, cudaMemcpyHostToDevice, s);
+    if (small) {
+        pack.resize(atoms_at + plan->image.size());
+        for (int k = 0; k < 6 && n > 0; ++k) std::memcpy(pack.data() + k * bytes, src[k], bytes);
+        std::memcpy(pack.data() + atoms_at, plan->image.data(), plan->image.size());
+        e = cudaMemcpyAsync(block, pack.data(), pack.size(), cudaMemcpyHostToDevice, s);
+    } else {
+        for (int k = 0; k < 6 && e == cudaSuccess && n > 0; ++k)
+            e = cudaMemcpyAsync(block + k * bytes, src[k], bytes, cudaMemcpyHostToDevice, s);
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(block + atoms_at, plan->image.data(), plan->image.size(), cudaMemcpyHostToDevice, s);
+    }
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) { cleanup(); return cuda_fail(e, "atom upload"); }
     const double t1 = now_s();
 
     if (o.verbose) std::printf("Running GPU kernels...\n");
+    double* d = reinterpret_cast<double*>(block);
     disco_atoms da;
     da.x = d; da.y = d + n; da.z = d + 2 * n;
     da.ux = d + 3 * n; da.uy = d + 4 * n; da.uz = d + 5 * n;
@@ -457,21 +601,39 @@ int disco_b200_displace(const disco_atoms* atoms, const disco_loop* loops, int32
     e = cudaEventRecord(ev[0], s);
     if (e != cudaSuccess) { cleanup(); return cuda_fail(e, "event"); }
     st = disco_b200_plan_execute(plan, &da, s);
-    if (st) { cleanup(); return st; }
+    if (st) { std::string m = g_last_error; cleanup(); return fail(st, m); }
     e = cudaEventRecord(ev[1], s);
-    if (e != cudaSuccess) { cleanup(); return cuda_fail(e, "event"); }
-    st = disco_b200_plan_sync(plan, s);
-    if (st) { std::string m = g_last_error; cleanup(); return fail(st, m); }  // keep the kernel's message
+    if (e == cudaSuccess) e = cudaEventSynchronize(ev[1]);
+    if (e != cudaSuccess) { cleanup(); return cuda_fail(e, "displacement kernels"); }
     float ms = 0.f;
     cudaEventElapsedTime(&ms, ev[0], ev[1]);
     const double t2 = now_s();
     if (o.verbose) std::printf("\nGPU kernel time: %g ms\n\n", (double)ms);
 
+    // the status word first (small calls: behind uz in the same copy)
+    int status = 0;
+    if (small) {
+        e = cudaMemcpyAsync(pack.data(), block + 3 * bytes, atoms_at - 3 * bytes + sizeof(int), cudaMemcpyDeviceToHost, s);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+        if (e == cudaSuccess) std::memcpy(&status, pack.data() + atoms_at - 3 * bytes, sizeof(int));
+    } else {
+        e = cudaMemcpyAsync(&status, plan->d_status, sizeof(int), cudaMemcpyDeviceToHost, s);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    }
+    if (e == cudaSuccess && status) {
+        cleanup();
+        return fail(status, "a kernel reported: " + std::string(disco_b200_strerror(status)));
+    }
     double* dst[3] = { atoms->ux, atoms->uy, atoms->uz };
-    for (int k = 0; k < 3 && e == cudaSuccess && n > 0; ++k)
-        e = cudaMemcpyAsync(dst[k], d + (size_t)(3 + k) * n, bytes, cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (small) {
+        for (int k = 0; k < 3 && e == cudaSuccess && n > 0; ++k) std::memcpy(dst[k], pack.data() + k * bytes, bytes);
+    } else {
+        for (int k = 0; k < 3 && e == cudaSuccess && n > 0; ++k)
+            e = cudaMemcpyAsync(dst[k], block + (3 + k) * bytes, bytes, cudaMemcpyDeviceToHost, s);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    }
     if (e != cudaSuccess) { cleanup(); return cuda_fail(e, "displacement download"); }
+    healthy = true;
     std::vector<double> evals = plan->loop_evals;
     cleanup();
     const double t3 = now_s();

@@ -1664,34 +1664,6 @@ unsigned char* g_noalloc_addr[kMaxDevices] = {};
 unsigned long long g_noalloc_ctx[kMaxDevices] = {};
 bool g_noalloc_dirty[kMaxDevices] = {};     // the control words may not be zero
 
-using CtxGetCurrentFn = CUresult (*)(CUcontext*);
-using CtxGetIdFn = CUresult (*)(CUcontext, unsigned long long*);
-
-// Unique identifier of the calling thread's current context (the driver's
-// cuCtxGetId, reached through the runtime without linking libcuda), 0 when
-// it cannot be read.
-unsigned long long current_context_id()
-{
-    static CtxGetCurrentFn get_current = nullptr;
-    static CtxGetIdFn get_id = nullptr;
-    static std::once_flag once;
-    std::call_once(once, [] {
-        void* f = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPointByVersion("cuCtxGetCurrent", &f, 12000, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            get_current = reinterpret_cast<CtxGetCurrentFn>(f);
-        f = nullptr;
-        if (cudaGetDriverEntryPointByVersion("cuCtxGetId", &f, 12000, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            get_id = reinterpret_cast<CtxGetIdFn>(f);
-    });
-    CUcontext c = nullptr;
-    unsigned long long id = 0;
-    if (get_current && get_id && get_current(&c) == CUDA_SUCCESS && c && get_id(c, &id) == CUDA_SUCCESS) return id;
-    return 0;
-}
-
 // Device address of g_noalloc_scratch on the current device.  In host code the
 // array's name is a host-side stand-in, not a device address: the address is
 // looked up with that device current and cached with the identifier of the
@@ -1706,7 +1678,7 @@ int noalloc_scratch(unsigned char** out, unsigned long long* ctx_out, int* dev_o
     // make the primary context current before its identifier is read
     e = cudaFree(nullptr);
     if (e != cudaSuccess) return cfail(e, "device context");
-    const unsigned long long ctx = current_context_id();
+    const unsigned long long ctx = disco::current_context_id();
     std::lock_guard<std::mutex> lock(g_noalloc_mutex);
     if (!g_noalloc_addr[dev] || ctx == 0 || ctx != g_noalloc_ctx[dev]) {
         void* p = nullptr;
