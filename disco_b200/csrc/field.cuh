@@ -97,11 +97,14 @@ struct alignas(16) LooponPieceF {
     int32_t n, rec;
     int32_t pad0, pad1;     // 80 B
 };
+// Every value twice: the kernel works on two images of an atom at a time
+// (packed FP32 instructions), and a pair loaded from the record feeds both.
 struct alignas(16) LooponRecF {
-    float x, y, z, ml;      // loopon - c, m . (loopon - c)
-    float nl, pad0, pad1, pad2;   // 32 B
+    float2 x, y, z;          // -(loopon - c), each value twice
+    float2 ml, nl;           // -m . (loopon - c), -n . (loopon - c)
+    float2 pad;              // 48 B
 };
-static_assert(sizeof(LooponPieceF) == 80 && sizeof(LooponRecF) == 32, "fp32 loopon table layout");
+static_assert(sizeof(LooponPieceF) == 80 && sizeof(LooponRecF) == 48, "fp32 loopon table layout");
 
 // A source of the sum by cells (tree.cuh): a line piece, or a square patch of a
 // loop's loopons at some depth of its quadtree.  The ball (x, y, z, rho) holds

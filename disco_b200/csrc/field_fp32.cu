@@ -144,9 +144,10 @@ int build_table_fp32(const disco_loop* loops, int nloops, int kind, double nu, H
                     const double x = lp.x[k] - cx, y = lp.y[k] - cy, z = lp.z[k] - cz;
                     LooponRecF r;
                     std::memset(&r, 0, sizeof(r));
-                    r.x = (float)x; r.y = (float)y; r.z = (float)z;
-                    r.ml = (float)(ph.mx * x + ph.my * y + ph.mz * z);
-                    r.nl = (float)(ph.nx * x + ph.ny * y + ph.nz * z);
+                    auto two = [](double v) { return make_float2((float)v, (float)v); };
+                    r.x = two(-x); r.y = two(-y); r.z = two(-z);
+                    r.ml = two(-(ph.mx * x + ph.my * y + ph.mz * z));
+                    r.nl = two(-(ph.nx * x + ph.ny * y + ph.nz * z));
                     recs.push_back(r);
                 }
                 L.pieces.push_back(p);

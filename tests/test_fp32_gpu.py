@@ -86,3 +86,25 @@ def test_near_list_and_its_overflow():
     assert np.abs(overflow - f64).max() <= 1e-12
     default = run(precision=C.DISCO_FP32C, max_atoms=w.n)
     assert np.abs(default - f64).max() <= 2e-5
+
+
+@pytest.mark.parametrize("images", [0, 1, 2])
+@pytest.mark.parametrize("split", [1, 2, 8, 32])
+def test_loopons_over_odd_and_even_image_counts_per_lane(images, split):
+    """Images are taken two at a time: one image in all, a lane without a
+    second one, lanes without any.  The loopon form's error against FP64 is
+    below 5e-6 A (the reference's own bound for its FP32 loopons) whatever the
+    split."""
+    torch = pytest.importorskip("torch")
+    from disco_b200 import backend as B
+    w = W.bcc_prismatic(cells=12, n_inter=2, n_vac=1, rmin=5.0, rmax=9.0)
+    pos = torch.tensor(np.stack([w.x, w.y, w.z]), dtype=torch.float64, device="cuda")
+    out = []
+    for prec in (C.DISCO_FP32C, C.DISCO_FP64):
+        p = B.Plan(w.loops, w.box, precision=prec, images=images, nu=w.nu, image_split=split)
+        u = torch.zeros_like(pos)
+        p.execute(pos, u)
+        p.sync(torch.cuda.current_stream().cuda_stream)
+        p.close()
+        out.append(u)
+    assert float((out[0] - out[1]).abs().max()) <= 5e-6
