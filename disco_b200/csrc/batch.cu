@@ -225,6 +225,10 @@ __global__ void __launch_bounds__(kBatchThreads, 2) batch_near_list_kernel(const
 
 struct disco_batch_plan {
     int device = 0, sm_count = 0;
+    // device memory: cudaMalloc, or for a plan inside the library from the
+    // scratch pool in the order of `stream`
+    cudaMemPool_t pool = nullptr;
+    cudaStream_t stream = nullptr;
     disco_options opt;
     int nsamples = 0;
     int split = 1;
@@ -262,20 +266,37 @@ int bcuda(cudaError_t e, const char* what)
     return e == cudaErrorMemoryAllocation ? DISCO_ENOMEM : DISCO_ECUDA;
 }
 
+template <class T>
+cudaError_t batch_alloc(disco_batch_plan* p, T** out, size_t bytes)
+{
+    return p->pool ? cudaMallocFromPoolAsync(reinterpret_cast<void**>(out), bytes, p->pool, p->stream)
+                   : cudaMalloc(reinterpret_cast<void**>(out), bytes);
+}
+
+cudaError_t batch_upload(disco_batch_plan* p, void* dst, const void* src, size_t bytes)
+{
+    return p->pool ? cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, p->stream)
+                   : cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice);
+}
+
 void free_batch(disco_batch_plan* p)
 {
     if (!p) return;
     if (p->exec) cudaGraphExecDestroy(p->exec);
     if (p->graph) cudaGraphDestroy(p->graph);
+    auto release = [&](void* d) {
+        if (d && p->pool) cudaFreeAsync(d, p->stream);
+        else if (d) cudaFree(d);
+    };
     for (int k = 0; k < 2; ++k) {
-        if (p->d_table[k]) cudaFree(p->d_table[k]);
-        if (p->d_samples[k]) cudaFree(p->d_samples[k]);
-        if (p->d_units[k]) cudaFree(p->d_units[k]);
-        if (p->d_cta_first[k]) cudaFree(p->d_cta_first[k]);
+        release(p->d_table[k]);
+        release(p->d_samples[k]);
+        release(p->d_units[k]);
+        release(p->d_cta_first[k]);
     }
-    if (p->d_status) cudaFree(p->d_status);
-    if (p->d_near) cudaFree(p->d_near);
-    if (p->d_near_count) cudaFree(p->d_near_count);
+    release(p->d_status);
+    release(p->d_near);
+    release(p->d_near_count);
     delete p;
 }
 
@@ -382,10 +403,10 @@ int launch_all(disco_batch_plan* p, cudaStream_t s)
 
 } // namespace
 
-extern "C" {
+namespace {
 
-int disco_b200_batch_plan_create(const disco_sample* samples, int32_t nsamples, const disco_options* opt,
-                                 disco_batch_plan** out)
+int batch_create(const disco_sample* samples, int32_t nsamples, const disco_options* opt, cudaMemPool_t pool,
+                 cudaStream_t stream, disco_batch_plan** out)
 {
     using namespace disco;
     if (!out) return bfail(DISCO_EINVAL, "null plan pointer");
@@ -416,6 +437,8 @@ int disco_b200_batch_plan_create(const disco_sample* samples, int32_t nsamples, 
     }
     if (!disco_b200_available()) return bfail(DISCO_ENODEV, "no CUDA device");
     disco_batch_plan* p = new disco_batch_plan();
+    p->pool = pool;
+    p->stream = stream;
     p->opt = o;
     p->nsamples = nsamples;
     p->split = split;
@@ -424,8 +447,8 @@ int disco_b200_batch_plan_create(const disco_sample* samples, int32_t nsamples, 
     std::memset(&p->stats, 0, sizeof(p->stats));
     cudaError_t e = cudaGetDevice(&p->device);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&p->sm_count, cudaDevAttrMultiProcessorCount, p->device);
-    if (e == cudaSuccess) e = cudaMalloc(&p->d_status, sizeof(int));
-    if (e == cudaSuccess) e = cudaMemset(p->d_status, 0, sizeof(int));
+    if (e == cudaSuccess) e = batch_alloc(p, &p->d_status, sizeof(int));
+    if (e == cudaSuccess) e = cudaMemsetAsync(p->d_status, 0, sizeof(int), stream);
     if (e != cudaSuccess) { free_batch(p); return bcuda(e, "device setup"); }
     const int atoms_per_tile = kBatchThreads / split;
     uint32_t max_stage = 16;
@@ -482,12 +505,12 @@ int disco_b200_batch_plan_create(const disco_sample* samples, int32_t nsamples, 
             all_chunks.insert(all_chunks.end(), chunks[s].begin(), chunks[s].end());
         }
         Chunk* d_chunks = nullptr;
-        e = cudaMalloc(&p->d_table[k], bytes.size() + all_chunks.size() * sizeof(Chunk) + 256);
-        if (e == cudaSuccess) e = cudaMemcpy(p->d_table[k], bytes.data(), bytes.size(), cudaMemcpyHostToDevice);
+        e = batch_alloc(p, &p->d_table[k], bytes.size() + all_chunks.size() * sizeof(Chunk) + 256);
+        if (e == cudaSuccess) e = batch_upload(p, p->d_table[k], bytes.data(), bytes.size());
         const size_t chunks_at = (bytes.size() + 255) & ~size_t(255);
         d_chunks = reinterpret_cast<Chunk*>(p->d_table[k] + chunks_at);
         if (e == cudaSuccess && !all_chunks.empty())
-            e = cudaMemcpy(d_chunks, all_chunks.data(), all_chunks.size() * sizeof(Chunk), cudaMemcpyHostToDevice);
+            e = batch_upload(p, d_chunks, all_chunks.data(), all_chunks.size() * sizeof(Chunk));
         if (e != cudaSuccess) { free_batch(p); return bcuda(e, "batch table upload"); }
         for (int s = 0; s < nsamples; ++s) {
             if (chunks[s].empty()) continue;
@@ -551,15 +574,15 @@ int disco_b200_batch_plan_create(const disco_sample* samples, int32_t nsamples, 
         }
         first[grid] = (int32_t)units.size();
         if (units.size() > 2147483647u) { free_batch(p); return bfail(DISCO_ELIMIT, "too many work units"); }
-        e = cudaMalloc(&p->d_samples[k], std::max<size_t>(1, sdev.size()) * sizeof(SampleDev));
+        e = batch_alloc(p, &p->d_samples[k], std::max<size_t>(1, sdev.size()) * sizeof(SampleDev));
         if (e == cudaSuccess && nsamples > 0)
-            e = cudaMemcpy(p->d_samples[k], sdev.data(), sdev.size() * sizeof(SampleDev), cudaMemcpyHostToDevice);
-        if (e == cudaSuccess) e = cudaMalloc(&p->d_units[k], std::max<size_t>(1, units.size()) * sizeof(UnitDev));
+            e = batch_upload(p, p->d_samples[k], sdev.data(), sdev.size() * sizeof(SampleDev));
+        if (e == cudaSuccess) e = batch_alloc(p, &p->d_units[k], std::max<size_t>(1, units.size()) * sizeof(UnitDev));
         if (e == cudaSuccess && !units.empty())
-            e = cudaMemcpy(p->d_units[k], units.data(), units.size() * sizeof(UnitDev), cudaMemcpyHostToDevice);
-        if (e == cudaSuccess) e = cudaMalloc(&p->d_cta_first[k], first.size() * sizeof(int32_t));
+            e = batch_upload(p, p->d_units[k], units.data(), units.size() * sizeof(UnitDev));
+        if (e == cudaSuccess) e = batch_alloc(p, &p->d_cta_first[k], first.size() * sizeof(int32_t));
         if (e == cudaSuccess)
-            e = cudaMemcpy(p->d_cta_first[k], first.data(), first.size() * sizeof(int32_t), cudaMemcpyHostToDevice);
+            e = batch_upload(p, p->d_cta_first[k], first.data(), first.size() * sizeof(int32_t));
         if (e != cudaSuccess) { free_batch(p); return bcuda(e, "batch queue upload"); }
         p->grid[k] = items.empty() ? 0 : grid;
         if (k == 0) p->stats.n_line_loops = 1; else p->stats.n_loopon_loops = 1;
@@ -571,8 +594,8 @@ int disco_b200_batch_plan_create(const disco_sample* samples, int32_t nsamples, 
         int per_sm = 0;
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batch_near_list_kernel<8>, kBatchThreads, 0);
         p->near_grid = std::max(1, p->sm_count * std::max(per_sm, 1));
-        if (e == cudaSuccess) e = cudaMalloc(&p->d_near, (size_t)p->near_cap * sizeof(int2));
-        if (e == cudaSuccess) e = cudaMalloc(&p->d_near_count, sizeof(unsigned int));
+        if (e == cudaSuccess) e = batch_alloc(p, &p->d_near, (size_t)p->near_cap * sizeof(int2));
+        if (e == cudaSuccess) e = batch_alloc(p, &p->d_near_count, sizeof(unsigned int));
         if (e != cudaSuccess) { free_batch(p); return bcuda(e, "near-cut list"); }
     }
     p->stage_bytes = (max_stage + 15) & ~15u;
@@ -580,6 +603,29 @@ int disco_b200_batch_plan_create(const disco_sample* samples, int32_t nsamples, 
     p->stats.evals_per_atom = evals;        // for a batch: total evaluations of one execute
     *out = p;
     return DISCO_OK;
+}
+
+} // namespace
+
+// For one call inside the library: device memory from the scratch pool in the
+// order of `s` (cudaMalloc without one); the caller has waited for the plan's
+// last kernel before it destroys it.
+int disco::batch_plan_create_on(const disco_sample* samples, int32_t nsamples, const disco_options* opt,
+                                cudaStream_t s, disco_batch_plan** out)
+{
+    int dev = 0;
+    cudaMemPool_t pool = cudaGetDevice(&dev) == cudaSuccess ? scratch_pool(dev) : nullptr;
+    if (pool && batch_create(samples, nsamples, opt, pool, s, out) == DISCO_OK) return DISCO_OK;
+    cudaGetLastError();
+    return batch_create(samples, nsamples, opt, nullptr, nullptr, out);
+}
+
+extern "C" {
+
+int disco_b200_batch_plan_create(const disco_sample* samples, int32_t nsamples, const disco_options* opt,
+                                 disco_batch_plan** out)
+{
+    return batch_create(samples, nsamples, opt, nullptr, nullptr, out);
 }
 
 int disco_b200_batch_plan_execute(disco_batch_plan* p, void* stream)

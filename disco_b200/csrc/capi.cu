@@ -36,8 +36,9 @@ struct disco_plan {
     // and behind it the FP32 line form's list of atoms with near-cut pairs
     std::vector<unsigned char> image;        // host copy until the upload
     size_t table_at[2] = { 0, 0 }, chunks_at[2] = { 0, 0 }, near_at = 0, bytes = 0;
-    unsigned char* block = nullptr;          // owned where `own`
-    bool own = false;
+    unsigned char* block = nullptr;          // owned where `own`: cudaMalloc'd, or from the
+    bool own = false, pooled = false;        // scratch pool in the order of `stream`
+    cudaStream_t stream = nullptr;
     unsigned char* d_table[2] = { nullptr, nullptr };
     disco::Chunk* d_chunks[2] = { nullptr, nullptr };
     int* d_status = nullptr;
@@ -103,7 +104,8 @@ int check_options(const disco_options& o)
 void free_plan(disco_plan* p)
 {
     if (!p) return;
-    if (p->own && p->block) cudaFree(p->block);
+    if (p->own && p->block && p->pooled) cudaFreeAsync(p->block, p->stream);
+    else if (p->own && p->block) cudaFree(p->block);
     if (p->tree_pool) disco::scratch_release(p->device);
     delete p;
 }
@@ -237,6 +239,15 @@ cudaMemPool_t disco::scratch_pool(int device)
         scratch_keep(device, g_scratch_plans[device] > 0 ? kScratchKeepPlans : kScratchKeep);
     }
     return g_scratch[device];
+}
+
+cudaError_t disco::scratch_alloc(void** p, size_t bytes, cudaStream_t s)
+{
+    int dev = 0;
+    cudaMemPool_t pool = cudaGetDevice(&dev) == cudaSuccess ? scratch_pool(dev) : nullptr;
+    if (pool && cudaMallocFromPoolAsync(p, bytes, pool, s) == cudaSuccess) return cudaSuccess;
+    cudaGetLastError();
+    return cudaMallocAsync(p, bytes, s);
 }
 
 void disco::scratch_retain(int device)
@@ -413,6 +424,35 @@ void plan_place(disco_plan* p, unsigned char* block)
 }
 
 } // namespace
+
+// A plan for one call inside the library: its block comes from the scratch pool
+// in the order of `s` (cudaMalloc without one), and the caller has waited for
+// its last kernel before it destroys the plan.
+int disco::plan_create_on(const disco_loop* loops, int32_t nloops, const double box[3], const disco_options* opt,
+                          int64_t max_atoms, cudaStream_t s, disco_plan** out)
+{
+    int st = plan_build(loops, nloops, box, opt, max_atoms, out);
+    if (st) return st;
+    disco_plan* p = *out;
+    *out = nullptr;
+    unsigned char* block = nullptr;
+    cudaMemPool_t pool = scratch_pool(p->device);
+    p->pooled = pool && cudaMallocFromPoolAsync(reinterpret_cast<void**>(&block), p->bytes, pool, s) == cudaSuccess;
+    cudaError_t e = cudaSuccess;
+    if (!p->pooled) {
+        cudaGetLastError();
+        block = nullptr;
+        e = cudaMalloc(&block, p->bytes);
+    }
+    if (e != cudaSuccess) { free_plan(p); return cuda_fail(e, "plan memory"); }
+    plan_place(p, block);
+    p->own = true;
+    p->stream = s;
+    e = cudaMemcpyAsync(block, p->image.data(), p->image.size(), cudaMemcpyHostToDevice, s);
+    if (e != cudaSuccess) { free_plan(p); return cuda_fail(e, "loop table upload"); }
+    *out = p;
+    return DISCO_OK;
+}
 
 extern "C" {
 

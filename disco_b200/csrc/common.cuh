@@ -27,6 +27,12 @@ unsigned long long current_context_id();
 cudaMemPool_t scratch_pool(int device);
 void scratch_retain(int device);
 void scratch_release(int device);
+int plan_create_on(const disco_loop* loops, int32_t nloops, const double box[3], const disco_options* opt,
+                   int64_t max_atoms, cudaStream_t s, disco_plan** out);
+int batch_plan_create_on(const disco_sample* samples, int32_t nsamples, const disco_options* opt, cudaStream_t s,
+                         disco_batch_plan** out);
+// Stream-ordered scratch of a call: from the pool, or the device's default one.
+cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t s);
 
 // A bounded wait gives up after this many nanoseconds of %globaltimer.  A stage
 // copy of a few hundred KB completes in microseconds; the bound only exists so

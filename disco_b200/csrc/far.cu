@@ -458,7 +458,7 @@ int apply_impl(disco_mlp* m, const disco_far_norm* norm, const disco_atoms* a, c
     // per-call descriptor upload (a pageable copy returns once the source is consumed)
     const size_t bl = fl.size() * sizeof(FarLoop), bs = idx.size() * sizeof(int32_t);
     void* dbuf = nullptr;
-    FAR_TRY(cudaMallocAsync(&dbuf, bl + bs, s), "far loop descriptors");
+    FAR_TRY(disco::scratch_alloc(&dbuf, bl + bs, s), "far loop descriptors");
     cudaError_t e = cudaMemcpyAsync(dbuf, fl.data(), bl, cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(static_cast<char*>(dbuf) + bl, idx.data(), bs, cudaMemcpyHostToDevice, s);
@@ -510,15 +510,19 @@ uint64_t splitmix(uint64_t& st)
     return z ^ (z >> 31);
 }
 
-// Device buffers of one learned call, released on every exit path.
+// Device buffers of one learned call, released on every exit path, in the
+// order of its stream (cudaMalloc and cudaFree map and unmap memory, 0.3 ms
+// each, and wait for the device).
 struct Bufs {
+    cudaStream_t s;
     std::vector<void*> ptrs;
-    ~Bufs() { for (void* p : ptrs) cudaFree(p); }
+    explicit Bufs(cudaStream_t stream) : s(stream) {}
+    ~Bufs() { for (void* p : ptrs) cudaFreeAsync(p, s); }
     template <class T>
     cudaError_t get(T** out, size_t count)
     {
         void* p = nullptr;
-        const cudaError_t e = cudaMalloc(&p, std::max<size_t>(count, 1) * sizeof(T));
+        const cudaError_t e = disco::scratch_alloc(&p, std::max<size_t>(count, 1) * sizeof(T), s);
         if (e == cudaSuccess) ptrs.push_back(p);
         *out = static_cast<T*>(p);
         return e;
@@ -544,7 +548,7 @@ int disco_b200_far_features(const disco_atoms* a, const disco_loop* loops, int32
     if (a->n == 0 || nloops == 0) return DISCO_OK;
     if (!a->x || !a->y || !a->z || !X) return ffail(DISCO_EINVAL, "far_features: null array");
     void* dl = nullptr;
-    FAR_TRY(cudaMallocAsync(&dl, fl.size() * sizeof(FarLoop), s), "far loop descriptors");
+    FAR_TRY(disco::scratch_alloc(&dl, fl.size() * sizeof(FarLoop), s), "far loop descriptors");
     cudaError_t e = cudaMemcpyAsync(dl, fl.data(), fl.size() * sizeof(FarLoop), cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess) {
         const int64_t rows = a->n * nloops;
@@ -586,7 +590,10 @@ int disco_b200_learned_displace(disco_mlp* m, const disco_far_norm* norm, const 
     // kernels of one exact sum of line loops: FP32C adds the near-cut FP64 pass
     auto sum_launches = [](int precision) { return precision == DISCO_FP32C ? 2 : 1; };
     int launches = 0;
-    Bufs B;
+    int dev = 0, sms = 0;
+    FAR_TRY(cudaGetDevice(&dev), "device query");
+    FAR_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "device query");
+    Bufs B(s);
     Ev ec, en, ef, eb;
 
     // 1. exact far shells and the network, per loop, on the subsample
@@ -644,8 +651,15 @@ int disco_b200_learned_displace(disco_mlp* m, const disco_far_norm* norm, const 
         disco_b200_options_default(&bo);
         bo.precision = opt->check_precision;
         bo.nu = opt->nu;
+        // 1 % of the atoms are few tiles of 256: split each atom's images over
+        // lanes until there are four rounds of work for the two resident CTAs of
+        // every SM (1 080 checked atoms, 9 loops, 702 images: the whole check 4.3 ms
+        // with one lane, 2.1 ms with eight)
+        bo.image_split = 1;
+        while (bo.image_split < 8 && (int64_t)nloops * ((nc * bo.image_split + 255) / 256) < 8 * (int64_t)sms)
+            bo.image_split *= 2;
         disco_batch_plan* bp = nullptr;
-        int st2 = disco_b200_batch_plan_create(smp.data(), nloops, &bo, &bp);
+        int st2 = disco::batch_plan_create_on(smp.data(), nloops, &bo, s, &bp);
         if (st2) return st2;
         st2 = disco_b200_batch_plan_execute(bp, s);
         if (!st2) st2 = disco_b200_batch_plan_sync(bp, s);
@@ -703,7 +717,7 @@ int disco_b200_learned_displace(disco_mlp* m, const disco_far_norm* norm, const 
         no.nu = opt->nu;
         no.images = norm->image_min - 1;
         disco_plan* p = nullptr;
-        int st2 = disco_b200_plan_create(loops, nloops, box, &no, n, &p);
+        int st2 = disco::plan_create_on(loops, nloops, box, &no, n, s, &p);
         if (st2) return st2;
         st2 = disco_b200_plan_execute(p, a, s);
         if (!st2) st2 = disco_b200_plan_sync(p, s);
@@ -736,7 +750,7 @@ int disco_b200_learned_displace(disco_mlp* m, const disco_far_norm* norm, const 
         fo.images = norm->images;
         fo.image_min = norm->image_min;
         disco_plan* p = nullptr;
-        int st2 = disco_b200_plan_create(sub.data(), (int32_t)sub.size(), box, &fo, n, &p);
+        int st2 = disco::plan_create_on(sub.data(), (int32_t)sub.size(), box, &fo, n, s, &p);
         if (st2) return st2;
         st2 = disco_b200_plan_execute(p, a, s);
         if (!st2) st2 = disco_b200_plan_sync(p, s);

@@ -334,13 +334,8 @@ extern "C" int disco_b200_format_atoms(int32_t format, const char* element, cons
     a.x = x; a.y = y; a.z = z; a.n = n;
     a.len = lengths();
     a.ntiles = ntiles;
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return wfail(DISCO_ECUDA, std::string("format_atoms: ") + cudaGetErrorString(e));
     void* scratch = nullptr;
-    const size_t bytes_needed = (size_t)(ntiles + 2) * sizeof(int64_t);
-    cudaMemPool_t pool = disco::scratch_pool(dev);
-    e = pool ? cudaMallocFromPoolAsync(&scratch, bytes_needed, pool, s) : cudaMallocAsync(&scratch, bytes_needed, s);
+    cudaError_t e = disco::scratch_alloc(&scratch, (size_t)(ntiles + 2) * sizeof(int64_t), s);
     if (e != cudaSuccess) return wfail(DISCO_ENOMEM, std::string("format_atoms: ") + cudaGetErrorString(e));
     a.tile_len = static_cast<int64_t*>(scratch);
     a.bad = reinterpret_cast<unsigned int*>(a.tile_len + ntiles + 1);
