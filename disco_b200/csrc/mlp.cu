@@ -18,12 +18,14 @@
 // dh = dpre W needs W transposed, dW = dpre^T h both operands: the epilogues
 // write each tile in both orders (a transposed tile of h makes room for the
 // transposed dpre of the layer above), and W3, W2 are staged again transposed
-// over themselves.  Each CTA keeps its own partial gradient in global memory;
+// over themselves (bulk copies of BF16 tiles that Adam writes with the weights).
+// Each CTA keeps its own partial gradient in global memory;
 // sum_kernel adds the partials in order, so a gradient is the same in every run.
 // The latency of one tile's chain of layers bounds a step (4096 rows are 32
 // tiles; the kernel issues on 15 % of the cycles, waiting for L2 and for
 // barriers): 0.40 ms with one launch per product and reduction (18 launches),
-// 0.052 ms with this kernel (45 to 50 us alone), the sum (10 us) and Adam (4).
+// 0.050 ms with this kernel (36 us alone; 50 with the weights converted in it), the
+// sum (10 us) and Adam (4).
 //
 // Inputs are padded to 16 features and outputs to 16 (the MMA's N >= 16 for
 // M = 128); the padding columns of W1 and rows of W4 are zero and stay zero
@@ -48,26 +50,40 @@ constexpr int kNetThreads = 256;
 constexpr int kRows = 128;                        // rows per tile
 constexpr uint32_t kTile = kRows * kHid * 2;      // a 128 x 128 BF16 tile
 constexpr uint32_t kThin = kRows * kIn * 2;       // a 128 x 16 (or 16 x 128) one
+// Transposed activations are written 2 bytes at a time, 32 rows (K values) of a
+// column by a warp: 16 bytes more between K blocks than their core matrices
+// take puts the four blocks on different banks (four-way conflicts without).
+constexpr uint32_t kTransLbo = (kHid / 8) * 128 + 16, kTrans = kTransLbo * (kRows / 8);
+constexpr uint32_t kThinLbo = (kIn / 8) * 128 + 16, kThinTrans = kThinLbo * (kRows / 8);
 constexpr uint32_t oSW1 = 0;                      // [128 x 16]
 constexpr uint32_t oSW2 = oSW1 + kThin;           // [128 x 128], in the backward pass transposed
 constexpr uint32_t oSW3 = oSW2 + kTile;
 constexpr uint32_t oSW4 = oSW3 + kTile;           // [16 x 128]
 constexpr uint32_t oSW4T = oSW4 + kThin;          // [128 x 16]
 constexpr uint32_t oSX = oSW4T + kThin;           // [rows x 16]
-constexpr uint32_t oSXT = oSX + kThin;            // [16 x rows]
-constexpr uint32_t oSH = oSXT + kThin;            // activations, then dpre: [rows x 128]
-constexpr uint32_t oST = oSH + kTile;             // three tiles [128 x rows]: h1, h2, h3 transposed, then dpre
-constexpr uint32_t oSDy = oST + 3 * kTile;        // [rows x 16]
-constexpr uint32_t oSDyT = oSDy + kThin;          // [16 x rows]
-constexpr uint32_t oSBias = oSDyT + kThin;        // b1, b2, b3, b4 (FP32)
+constexpr uint32_t oSXT = oSX + kThin;            // [16 x rows], padded
+constexpr uint32_t oSH = oSXT + kThinTrans;       // activations, then dpre: [rows x 128]
+constexpr uint32_t oST = oSH + kTile;             // three padded tiles [128 x rows]: h1, h2, h3 transposed, then dpre
+constexpr uint32_t oSDy = oST + 3 * kTrans;       // [rows x 16]
+constexpr uint32_t oSDyT = oSDy + kThin;          // [16 x rows], padded
+constexpr uint32_t oSBias = oSDyT + kThinTrans;   // b1, b2, b3, b4 (FP32)
 constexpr uint32_t oSLoss = oSBias + (3 * kHid + kOut) * 4;     // the warps' losses
-constexpr uint32_t oSBar = oSLoss + 32;
+constexpr uint32_t oSBar = oSLoss + 32;           // products, weights; the tensor-memory slot
 constexpr uint32_t kNetSmem = oSBar + 32;
 static_assert(kNetSmem <= 227 * 1024, "one CTA's shared memory");
+static_assert(oSH % 16 == 0 && oSBar % 8 == 0, "tile and barrier alignment");
+// The weights as the tiles the kernel stages: W1, W2, W3, W4, then W4, W3 and W2
+// transposed, K-major BF16 (written by Adam, or by pack_kernel for new weights).
+constexpr uint32_t kImg = 3 * kThin + 4 * kTile;
+constexpr uint32_t oIW1 = 0, oIW2 = oIW1 + kThin, oIW3 = oIW2 + kTile, oIW4 = oIW3 + kTile, oIW4T = oIW4 + kThin,
+                   oIW3T = oIW4T + kThin, oIW2T = oIW3T + kTile;
+static_assert(oIW2T + kTile == kImg && oIW1 == oSW1 && oIW4T == oSW4T, "weight image layout");
+constexpr uint32_t kLbo = (kRows / 8) * 128, kOutLbo = (kOut / 8) * 128;      // K blocks of 128 and 16 rows
 constexpr int kPart = kParams + 4;                // a partial gradient and its loss
 
 struct NetArgs {
     const float* P;
+    const unsigned char* img; // BF16 tiles of the weights
     const float* X;           // [n x 16]
     const float* T;           // [n x 3], null: forward only
     float* Y;                 // [n x 16], forward only
@@ -86,43 +102,40 @@ __device__ __forceinline__ uint32_t bf16x2(float lo, float hi)
     return *reinterpret_cast<const uint32_t*>(&v);
 }
 
-// W [rows x cols] (FP32, row-major) as a BF16 K-major tile; transposed: the
-// tile of W^T (cols x rows).
-__device__ __forceinline__ void stage_weights(unsigned char* tile, const float* W, int rows, int cols)
+// Parameter i's places in the weight image (biases have none).
+__device__ __forceinline__ void put_weight(unsigned char* img, int i, float v)
 {
-#pragma unroll 4
-    for (int e = threadIdx.x; e < rows * (cols / 8); e += kNetThreads) {
-        const int r = e % rows, k8 = (e / rows) * 8;
-        const float4* q = reinterpret_cast<const float4*>(W + r * cols + k8);
-        const float4 a = q[0], b = q[1];
-        *reinterpret_cast<uint4*>(tile + tc::kmajor_offset(r, k8, rows)) =
-            make_uint4(bf16x2(a.x, a.y), bf16x2(a.z, a.w), bf16x2(b.x, b.y), bf16x2(b.z, b.w));
-    }
-}
-__device__ __forceinline__ void stage_transposed(unsigned char* tile, const float* W, int rows, int cols)
-{
-    for (int e = threadIdx.x; e < (rows / 8) * (cols / 8); e += kNetThreads) {
-        const int r8 = (e % (cols / 8)) * 8, k8 = (e / (cols / 8)) * 8;      // tile row = W's column
-        float v[8][8];
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            const float4* q = reinterpret_cast<const float4*>(W + (k8 + k) * cols + r8);
-            const float4 a = q[0], b = q[1];
-            v[k][0] = a.x; v[k][1] = a.y; v[k][2] = a.z; v[k][3] = a.w;
-            v[k][4] = b.x; v[k][5] = b.y; v[k][6] = b.z; v[k][7] = b.w;
-        }
-#pragma unroll
-        for (int r = 0; r < 8; ++r)
-            *reinterpret_cast<uint4*>(tile + tc::kmajor_offset(r8 + r, k8, cols)) =
-                make_uint4(bf16x2(v[0][r], v[1][r]), bf16x2(v[2][r], v[3][r]), bf16x2(v[4][r], v[5][r]),
-                           bf16x2(v[6][r], v[7][r]));
+    const __nv_bfloat16 h = __float2bfloat16_rn(v);
+    auto put = [&](uint32_t tile, int r, int k, int rows) {
+        *reinterpret_cast<__nv_bfloat16*>(img + tile + tc::kmajor_offset(r, k, rows)) = h;
+    };
+    if (i < ob1) {
+        put(oIW1, (i - oW1) / kIn, (i - oW1) % kIn, kHid);
+    } else if (i >= oW2 && i < ob2) {
+        const int r = (i - oW2) / kHid, k = (i - oW2) % kHid;
+        put(oIW2, r, k, kHid);
+        put(oIW2T, k, r, kHid);
+    } else if (i >= oW3 && i < ob3) {
+        const int r = (i - oW3) / kHid, k = (i - oW3) % kHid;
+        put(oIW3, r, k, kHid);
+        put(oIW3T, k, r, kHid);
+    } else if (i >= oW4 && i < ob4) {
+        const int r = (i - oW4) / kHid, k = (i - oW4) % kHid;
+        put(oIW4, r, k, kOut);
+        put(oIW4T, k, r, kHid);
     }
 }
 
-// One product D (+)= A B^T over K = 16 nk, issued by the calling thread.
-__device__ __forceinline__ void product(uint32_t tmem, uint32_t a, int arows, uint32_t b, int brows, int nk, int N)
+__global__ void pack_kernel(const float* P, unsigned char* img)
 {
-    const uint32_t alb = (uint32_t)(arows / 8) * 128, blb = (uint32_t)(brows / 8) * 128;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < kParams) put_weight(img, i, P[i]);
+}
+
+// One product D (+)= A B^T over K = 16 nk, issued by the calling thread; alb,
+// blb: bytes between the operands' K blocks.
+__device__ __forceinline__ void product(uint32_t tmem, uint32_t a, uint32_t alb, uint32_t b, uint32_t blb, int nk, int N)
+{
     const uint32_t id = tc::idesc_bf16(kRows, N);
     for (int j = 0; j < nk; ++j)
         tc::mma_bf16(tmem, tc::smem_desc(a + j * 2 * alb, alb, 128), tc::smem_desc(b + j * 2 * blb, blb, 128), id, j > 0);
@@ -149,12 +162,18 @@ __device__ __forceinline__ bool products(uint64_t* bar, uint32_t& phase, Issue i
     return !bad;
 }
 
+// Element (r, k) of a transposed tile, K blocks lbo bytes apart.
+__device__ __forceinline__ uint32_t trans_offset(int r, int k, uint32_t lbo)
+{
+    return (uint32_t)(k >> 3) * lbo + (uint32_t)((r >> 3) * 128 + (r & 7) * 16 + (k & 7) * 2);
+}
+
 // 32 consecutive columns of one row into a transposed tile [columns x rows].
 __device__ __forceinline__ void put_transposed(unsigned char* tile, const float (&h)[32], int row, int c0)
 {
 #pragma unroll
     for (int i = 0; i < 32; ++i)
-        *reinterpret_cast<__nv_bfloat16*>(tile + tc::kmajor_offset(c0 + i, row, kHid)) = __float2bfloat16_rn(h[i]);
+        *reinterpret_cast<__nv_bfloat16*>(tile + trans_offset(c0 + i, row, kTransLbo)) = __float2bfloat16_rn(h[i]);
 }
 __device__ __forceinline__ void put_row(unsigned char* tile, const float (&h)[32], int row, int c0)
 {
@@ -177,15 +196,9 @@ __global__ void __launch_bounds__(kNetThreads, 1) net_kernel(const NetArgs a)
     const int row = t & 127, half = t >> 7;
     if (warp == 0) tc::alloc(slot, 512);
     if (t == 0) {
-        mbar_init(bar, 1);
+        mbar_init(&bar[0], 1);
+        mbar_init(&bar[1], 1);
         fence_mbar_init();
-    }
-    stage_weights(sm + oSW1, a.P + oW1, kHid, kIn);
-    stage_weights(sm + oSW4, a.P + oW4, kOut, kHid);
-    if (kTrain) stage_transposed(sm + oSW4T, a.P + oW4, kOut, kHid);
-    if (!kTrain) {
-        stage_weights(sm + oSW2, a.P + oW2, kHid, kHid);
-        stage_weights(sm + oSW3, a.P + oW3, kHid, kHid);
     }
     for (int e = t; e < 3 * kHid + kOut; e += kNetThreads)
         bias[e] = a.P[e < kHid ? ob1 + e : e < 2 * kHid ? ob2 + e - kHid : e < 3 * kHid ? ob3 + e - 2 * kHid
@@ -197,9 +210,19 @@ __global__ void __launch_bounds__(kNetThreads, 1) net_kernel(const NetArgs a)
     const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;             // this warp's tensor-memory lanes
     const uint32_t s0 = smem_addr(sm);
     const int c0 = half * (kHid / 2);
-    uint32_t phase = 0;
+    uint32_t phase = 0, wphase = 0;
     bool ok = true;
     float loss = 0.0f;
+    // weight tiles by bulk copy, `bytes` of the image at `from` to `to`; every
+    // copy in flight completes the phase of bar[1] that its wait names
+    auto fetch = [&](uint32_t to, uint32_t from, uint32_t bytes) { stage_load(sm + to, a.img + from, bytes, &bar[1]); };
+    auto fetched = [&]() {
+        const bool mine = mbar_wait_bounded(&bar[1], wphase);
+        wphase ^= 1;
+        return mine;
+    };
+    if (t == 0) fetch(oSW1, oIW1, oSX - oSW1);
+    bool staged = false;                          // the first copy has been waited for
     float* const part = kTrain ? a.part + (int64_t)blockIdx.x * kPart : nullptr;
 
     // a hidden layer's activations from its pre-activation in columns `col`
@@ -218,10 +241,7 @@ __global__ void __launch_bounds__(kNetThreads, 1) net_kernel(const NetArgs a)
         const int64_t r = (int64_t)tile * kRows + row;
         const bool valid = r < a.n;
         const bool first = tile == (int)blockIdx.x;
-        if (kTrain) {
-            stage_weights(sm + oSW2, a.P + oW2, kHid, kHid);
-            stage_weights(sm + oSW3, a.P + oW3, kHid, kHid);
-        }
+        if (kTrain && staged && t == 0) fetch(oSW2, oIW2, 2 * kTile);    // over the last tile's transposed ones
         {
             float x[kIn];
 #pragma unroll
@@ -248,20 +268,29 @@ __global__ void __launch_bounds__(kNetThreads, 1) net_kernel(const NetArgs a)
             } else if (kTrain) {
 #pragma unroll
                 for (int k = 0; k < kIn; ++k)
-                    *reinterpret_cast<__nv_bfloat16*>(sm + oSXT + tc::kmajor_offset(k, row, kIn)) = __float2bfloat16_rn(x[k]);
+                    *reinterpret_cast<__nv_bfloat16*>(sm + oSXT + trans_offset(k, row, kThinLbo)) = __float2bfloat16_rn(x[k]);
             }
         }
+        if (!staged || kTrain) ok = fetched();
+        staged = true;
+        if (__syncthreads_or(!ok)) { ok = false; break; }
         // forward
-        ok = products(bar, phase, [&] { product(tmem, s0 + oSX, kRows, s0 + oSW1, kHid, kIn / 16, kHid); });
+        ok = products(bar, phase, [&] { product(tmem, s0 + oSX, kLbo, s0 + oSW1, kLbo, kIn / 16, kHid); });
         if (!ok) break;
         activate(0, bias, sm + oST);
-        ok = products(bar, phase, [&] { product(tmem + 128, s0 + oSH, kRows, s0 + oSW2, kHid, kHid / 16, kHid); });
+        ok = products(bar, phase, [&] { product(tmem + 128, s0 + oSH, kLbo, s0 + oSW2, kLbo, kHid / 16, kHid); });
         if (!ok) break;
-        activate(128, bias + kHid, sm + oST + kTile);
-        ok = products(bar, phase, [&] { product(tmem + 256, s0 + oSH, kRows, s0 + oSW3, kHid, kHid / 16, kHid); });
+        activate(128, bias + kHid, sm + oST + kTrans);
+        ok = products(bar, phase, [&] { product(tmem + 256, s0 + oSH, kLbo, s0 + oSW3, kLbo, kHid / 16, kHid); });
         if (!ok) break;
-        activate(256, bias + 2 * kHid, sm + oST + 2 * kTile);
-        ok = products(bar, phase, [&] { product(tmem + 384, s0 + oSH, kRows, s0 + oSW4, kOut, kHid / 16, kOut); });
+        // the weights of dh2 and dh1 over those the forward pass is done with
+        if (kTrain && t == 0) {
+            mbar_arrive_expect_tx(&bar[1], 2 * kTile);
+            bulk_load(sm + oSW3, a.img + oIW3T, kTile, &bar[1]);
+            bulk_load(sm + oSW2, a.img + oIW2T, kTile, &bar[1]);
+        }
+        activate(256, bias + 2 * kHid, sm + oST + 2 * kTrans);
+        ok = products(bar, phase, [&] { product(tmem + 384, s0 + oSH, kLbo, s0 + oSW4, kOutLbo, kHid / 16, kOut); });
         if (!ok) break;
         if (!kTrain) {
             if (half == 0) {
@@ -301,13 +330,10 @@ __global__ void __launch_bounds__(kNetThreads, 1) net_kernel(const NetArgs a)
             *reinterpret_cast<uint4*>(sm + oSDy + tc::kmajor_offset(row, 8, kRows)) = make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
             for (int k = 0; k < kOut; ++k)
-                *reinterpret_cast<__nv_bfloat16*>(sm + oSDyT + tc::kmajor_offset(k, row, kOut)) =
+                *reinterpret_cast<__nv_bfloat16*>(sm + oSDyT + trans_offset(k, row, kThinLbo)) =
                     __float2bfloat16_rn(k < kOutReal ? g[k] : 0.0f);
             if (valid) reinterpret_cast<float4*>(a.dy)[r] = make_float4(g[0], g[1], g[2], 0.0f);
         }
-        // the weights of dh2 and dh1 over those the forward pass is done with
-        stage_transposed(sm + oSW3, a.P + oW3, kHid, kHid);
-        stage_transposed(sm + oSW2, a.P + oW2, kHid, kHid);
         auto put = [&](float* dst, float v) { *dst = first ? v : *dst + v; };
         auto put4 = [&](float* dst, float x, float y, float z, float w) {
             float4* d = reinterpret_cast<float4*>(dst);
@@ -349,7 +375,7 @@ __global__ void __launch_bounds__(kNetThreads, 1) net_kernel(const NetArgs a)
         };
         // dW4 = (h3^T dy)^T
         ok = products(bar, phase, [&] {
-            product(tmem + 384, s0 + oST + 2 * kTile, kHid, s0 + oSDyT, kOut, kRows / 16, kOut);
+            product(tmem + 384, s0 + oST + 2 * kTrans, kTransLbo, s0 + oSDyT, kThinLbo, kRows / 16, kOut);
         });
         if (!ok) break;
         if (half == 0) {
@@ -359,27 +385,29 @@ __global__ void __launch_bounds__(kNetThreads, 1) net_kernel(const NetArgs a)
             for (int k = 0; k < kOut; ++k) put(part + oW4 + k * kHid + row, k < kOutReal ? v[k] : 0.0f);
         }
         // dh3 = dy W4
-        ok = products(bar, phase, [&] { product(tmem + 384, s0 + oSDy, kRows, s0 + oSW4T, kHid, kOut / 16, kHid); });
+        ok = products(bar, phase, [&] { product(tmem + 384, s0 + oSDy, kLbo, s0 + oSW4T, kLbo, kOut / 16, kHid); });
         if (!ok) break;
-        dpre(256, bias + 2 * kHid, sm + oST + 2 * kTile, 2, true);
+        dpre(256, bias + 2 * kHid, sm + oST + 2 * kTrans, 2, true);
         // dh2 = dpre3 W3, dW3 = dpre3^T h2
+        ok = fetched();
+        if (__syncthreads_or(!ok)) { ok = false; break; }
         ok = products(bar, phase, [&] {
-            product(tmem + 384, s0 + oSH, kRows, s0 + oSW3, kHid, kHid / 16, kHid);
-            product(tmem + 256, s0 + oST + 2 * kTile, kHid, s0 + oST + kTile, kHid, kRows / 16, kHid);
+            product(tmem + 384, s0 + oSH, kLbo, s0 + oSW3, kLbo, kHid / 16, kHid);
+            product(tmem + 256, s0 + oST + 2 * kTrans, kTransLbo, s0 + oST + kTrans, kTransLbo, kRows / 16, kHid);
         });
         if (!ok) break;
-        dpre(128, bias + kHid, sm + oST + kTile, 1, true);
+        dpre(128, bias + kHid, sm + oST + kTrans, 1, true);
         put_gradient(256, oW3);
         // dh1 = dpre2 W2, dW2 = dpre2^T h1
         ok = products(bar, phase, [&] {
-            product(tmem + 384, s0 + oSH, kRows, s0 + oSW2, kHid, kHid / 16, kHid);
-            product(tmem + 128, s0 + oST + kTile, kHid, s0 + oST, kHid, kRows / 16, kHid);
+            product(tmem + 384, s0 + oSH, kLbo, s0 + oSW2, kLbo, kHid / 16, kHid);
+            product(tmem + 128, s0 + oST + kTrans, kTransLbo, s0 + oST, kTransLbo, kRows / 16, kHid);
         });
         if (!ok) break;
         dpre(0, bias, sm + oST, 0, false);
         put_gradient(128, oW2);
         // dW1 = dpre1^T x
-        ok = products(bar, phase, [&] { product(tmem, s0 + oST, kHid, s0 + oSXT, kIn, kRows / 16, kIn); });
+        ok = products(bar, phase, [&] { product(tmem, s0 + oST, kTransLbo, s0 + oSXT, kThinLbo, kRows / 16, kIn); });
         if (!ok) break;
         if (half == 0) {
             float v[16];
@@ -392,7 +420,8 @@ __global__ void __launch_bounds__(kNetThreads, 1) net_kernel(const NetArgs a)
     }
     if (!ok && t == 0) {
         report(a.status, DISCO_ETIMEOUT);
-        mbar_wait_bounded(bar, phase ^ 1);
+        mbar_wait_bounded(&bar[0], phase ^ 1);
+        mbar_wait_bounded(&bar[1], wphase);
     }
     if (kTrain) {
         for (int o = 16; o > 0; o >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, o);
@@ -464,7 +493,7 @@ __global__ void __launch_bounds__(256) sum_kernel(const float* part, const float
 }
 
 __global__ void adam_kernel(float* p, float* g, float* m, float* v, int n, float lr, float b1, float b2,
-                            float eps, float bc1, float bc2, float wd)
+                            float eps, float bc1, float bc2, float wd, unsigned char* img)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -474,7 +503,9 @@ __global__ void adam_kernel(float* p, float* g, float* m, float* v, int n, float
     m[i] = mi;
     v[i] = vi;
     const float upd = (mi / bc1) / (sqrtf(vi / bc2) + eps) + wd * p[i];
-    p[i] -= lr * upd;
+    const float pi = p[i] - lr * upd;
+    p[i] = pi;
+    put_weight(img, i, pi);
     g[i] = 0.0f;
 }
 
@@ -503,10 +534,9 @@ int mcuda(cudaError_t e, const char* what)
 void free_mlp(disco_mlp* p)
 {
     if (!p) return;
-    float* fs[] = { p->params, p->grads, p->m, p->v, p->loss, p->part };
-    for (float* f : fs) if (f) cudaFree(f);
-    if (p->status) cudaFree(p->status);
+    if (p->part) cudaFree(p->part);
     if (p->packed) cudaFree(p->packed);
+    if (p->img) cudaFree(p->img);
     delete p;
 }
 
@@ -525,7 +555,12 @@ int run_net(disco_mlp* p, const float* X, const float* T, int64_t n, float* Y, c
     }
     NetArgs a;
     std::memset(&a, 0, sizeof(a));
+    if (p->img_stale) {
+        pack_kernel<<<(kParams + 255) / 256, 256, 0, s>>>(p->params, p->img);
+        p->img_stale = false;
+    }
     a.P = p->params;
+    a.img = p->img;
     a.X = X; a.T = T; a.Y = Y;
     a.n = n;
     a.tiles = (int32_t)((n + kRows - 1) / kRows);
@@ -566,11 +601,14 @@ int disco_b200_mlp_create(uint64_t seed, disco_mlp** out)
     if (cudaGetDeviceCount(&count) != cudaSuccess || count == 0) return mfail(DISCO_ENODEV, "no CUDA device");
     disco_mlp* p = new disco_mlp();
     cudaError_t e = cudaSuccess;
+    // one block: weight image, weights, gradients, Adam's moments, loss, status
+    constexpr size_t kVec = ((size_t)kParams * sizeof(float) + 255) / 256 * 256;
+    e = cudaMalloc(&p->img, kImg + 4 * kVec + 512);
+    if (e != cudaSuccess) { p->img = nullptr; free_mlp(p); return mcuda(e, "MLP allocation"); }
     float** bufs[] = { &p->params, &p->grads, &p->m, &p->v };
-    for (float** b : bufs) if (e == cudaSuccess) e = cudaMalloc(b, kParams * sizeof(float));
-    if (e == cudaSuccess) e = cudaMalloc(&p->loss, sizeof(float));
-    if (e == cudaSuccess) e = cudaMalloc(&p->status, sizeof(int));
-    if (e != cudaSuccess) { free_mlp(p); return mcuda(e, "MLP allocation"); }
+    for (int k = 0; k < 4; ++k) *bufs[k] = reinterpret_cast<float*>(p->img + kImg + k * kVec);
+    p->loss = reinterpret_cast<float*>(p->img + kImg + 4 * kVec);
+    p->status = reinterpret_cast<int*>(p->img + kImg + 4 * kVec + 256);
     // Kaiming-uniform weights (a SplitMix64 stream), zero biases and padding
     std::vector<float> h(kParams, 0.0f);
     uint64_t st = seed * 0x9E3779B97F4A7C15ull + 1;
@@ -593,10 +631,7 @@ int disco_b200_mlp_create(uint64_t seed, disco_mlp** out)
     fill(oW3, kHid, kHid, kHid, kHid);
     fill(oW4, kOut, kHid, kOutReal, kHid);
     e = cudaMemcpy(p->params, h.data(), kParams * sizeof(float), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemset(p->grads, 0, kParams * sizeof(float));
-    if (e == cudaSuccess) e = cudaMemset(p->m, 0, kParams * sizeof(float));
-    if (e == cudaSuccess) e = cudaMemset(p->v, 0, kParams * sizeof(float));
-    if (e == cudaSuccess) e = cudaMemset(p->status, 0, sizeof(int));
+    if (e == cudaSuccess) e = cudaMemset(p->grads, 0, 3 * kVec + 512);
     if (e != cudaSuccess) { free_mlp(p); return mcuda(e, "MLP init"); }
     *out = p;
     return DISCO_OK;
@@ -621,6 +656,7 @@ int disco_b200_mlp_set_params(disco_mlp* p, const float* host)
 {
     if (!p || !host) return mfail(DISCO_EINVAL, "null argument");
     const cudaError_t e = cudaMemcpy(p->params, host, kParams * sizeof(float), cudaMemcpyHostToDevice);
+    p->img_stale = true;
     return e == cudaSuccess ? DISCO_OK : mcuda(e, "params upload");
 }
 
@@ -662,7 +698,8 @@ int disco_b200_mlp_adam(disco_mlp* p, float lr, float beta1, float beta2, float 
     p->step++;
     const float bc1 = 1.0f - std::pow(beta1, (float)p->step), bc2 = 1.0f - std::pow(beta2, (float)p->step);
     adam_kernel<<<(kParams + 255) / 256, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        p->params, p->grads, p->m, p->v, kParams, lr, beta1, beta2, eps, bc1, bc2, weight_decay);
+        p->params, p->grads, p->m, p->v, kParams, lr, beta1, beta2, eps, bc1, bc2, weight_decay, p->img);
+    p->img_stale = false;
     const cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? DISCO_OK : mcuda(e, "adam");
 }
