@@ -189,6 +189,7 @@ struct MatterArgs {
     int32_t G;                    // CTAs, all resident at once (cooperative launch)
     double idLx, idLy, idLz;      // 1 / box lengths, rounded (the exact test's fast path)
     int64_t S;                    // segments of kSegAtoms atoms
+    uint4* seg_mask;              // [S] which atoms those are (bit per atom), written where there are any
     int32_t* seg_removed;         // [S] atoms a vacancy slab removes
     int32_t* seg_members;         // [S] slab-member atoms
     int32_t* seg_off;             // [S] first member record of the segment
@@ -446,81 +447,13 @@ __device__ __forceinline__ void copy_plain(const MatterArgs& a, int64_t s, int64
     }
 }
 
-// Segment with slab members (its m records at `rec`): the records' masks and
-// sides go back into the warp's per-slot table (smask / ssides), then per
-// loop its slab entries and interstitial copies at the warp's running
-// positions wrun[l] / wrun[nl + l] (ascending atom order within the loop;
-// copies of removed atoms dropped, sources renumbered), then the survivors,
-// the removed atoms skipped.
-__device__ __forceinline__ void copy_members(const MatterArgs& a, const SlabHead* sh, uint64_t vac, int64_t s,
-                                             int64_t sb, const MemberRec* rec, int m, uint64_t* smask,
-                                             uint64_t* ssides, int64_t* wrun, uint64_t pol, int lane)
+// Segment with removed atoms: its survivors, in order, from `sb` on.
+__device__ __forceinline__ void copy_removed(const MatterArgs& a, int64_t s, int64_t sb, uint64_t pol, int lane)
 {
+    const uint4 bits = __ldcg(a.seg_mask + s);
+    const unsigned rb[kSegRounds] = { bits.x, bits.y, bits.z, bits.w };
     const int64_t i0 = s * kSegAtoms;
-    const int nl = a.nl;
     const unsigned ltm = (1u << lane) - 1u;
-#pragma unroll
-    for (int r = 0; r < kSegRounds; ++r) { smask[r * 32 + lane] = 0; ssides[r * 32 + lane] = 0; }
-    __syncwarp();
-    for (int e = lane; e < m; e += 32) {
-        const int slot = __ldcg(&rec[e].atom) - (int)i0;
-        if (slot >= 0 && slot < kSegAtoms) {
-            smask[slot] = __ldcg(reinterpret_cast<const unsigned long long*>(&rec[e].mask));
-            ssides[slot] = __ldcg(reinterpret_cast<const unsigned long long*>(&rec[e].sides));
-        }
-    }
-    __syncwarp();
-    unsigned rb[kSegRounds];
-    uint64_t un = 0;
-#pragma unroll
-    for (int r = 0; r < kSegRounds; ++r) {
-        const uint64_t mk = smask[r * 32 + lane];
-        rb[r] = __ballot_sync(0xffffffffu, (mk & vac) != 0);
-        un |= mk;
-    }
-    un = ((uint64_t)__reduce_or_sync(0xffffffffu, (unsigned)(un >> 32)) << 32) |
-         __reduce_or_sync(0xffffffffu, (unsigned)un);
-    for (uint64_t u = un; u; u &= u - 1) {
-        const int l = __ffsll((long long)u) - 1;
-        const bool inter = sh[l].type == DISCO_MATTER_INTERSTITIAL;
-        int64_t qs = wrun[l], qc = wrun[nl + l];
-        int rem_before = 0;
-#pragma unroll
-        for (int r = 0; r < kSegRounds; ++r) {
-            const uint64_t mk = smask[r * 32 + lane];
-            const bool in = (mk >> l) & 1ull;
-            const bool removed = (rb[r] >> lane) & 1u;
-            const bool kp = in && inter && !removed;
-            const bool pos = (ssides[r * 32 + lane] >> l) & 1ull;
-            const unsigned bi = __ballot_sync(0xffffffffu, in);
-            const unsigned bk = __ballot_sync(0xffffffffu, kp);
-            if (in) {
-                const int64_t q = qs + __popc(bi & ltm);
-                if (q >= 0 && q < a.slab_cap) {
-                    a.slab_atoms[q] = (int32_t)(i0 + r * 32 + lane);
-                    a.slab_side[q] = pos ? 1 : -1;
-                }
-            }
-            if (kp) {
-                const int64_t q = qc + __popc(bk & ltm);
-                if (q >= 0 && q < a.copy_cap) {
-                    const disco_slab_loop& g = a.loops[l].L;
-                    const double* shf = pos ? g.shift_pos : g.shift_neg;
-                    disco_copy cp;
-                    cp.atom = (int32_t)(sb + r * 32 + lane - (rem_before + __popc(rb[r] & ltm)));
-                    cp.reserved = 0;
-                    cp.shift[0] = shf[0]; cp.shift[1] = shf[1]; cp.shift[2] = shf[2];
-                    a.copies[q] = cp;
-                }
-            }
-            qs += __popc(bi);
-            qc += __popc(bk);
-            rem_before += __popc(rb[r]);
-        }
-        __syncwarp();
-        if (lane == 0) { wrun[l] = qs; wrun[nl + l] = qc; }
-        __syncwarp();
-    }
     double px[kSegRounds], py[kSegRounds], pz[kSegRounds];
 #pragma unroll
     for (int r = 0; r < kSegRounds; ++r) {
@@ -543,13 +476,12 @@ __device__ __forceinline__ void copy_members(const MatterArgs& a, const SlabHead
         }
         before += __popc(rb[r]);
     }
-    __syncwarp();                                               // the table is rewritten
 }
 
 // From the masks and sides of segment s in the warp's shared-memory buffer:
-// its removed and member counts, the per-loop slab and kept-copy counts
-// (added to wcnt), and its member records in atom order at `off` (taken here
-// from the global record counter when off < 0).
+// its removed bits, removed and member counts, the per-loop slab and kept-copy
+// counts (added to wcnt), and its member records in atom order at `off` (taken
+// from the global record counter).
 __device__ __forceinline__ void aggregate_segment(const MatterArgs& a, const SlabHead* sh, uint64_t vac, int64_t s,
                                                   const uint64_t* smask, const uint64_t* ssides, int* wcnt,
                                                   int& rc, int& mc, int& off, int lane)
@@ -557,7 +489,7 @@ __device__ __forceinline__ void aggregate_segment(const MatterArgs& a, const Sla
     const int64_t i0 = s * kSegAtoms;
     const int nl = a.nl;
     const unsigned ltm = (1u << lane) - 1u;
-    unsigned bm[kSegRounds];
+    unsigned bm[kSegRounds], rb[kSegRounds];
     rc = 0;
     mc = 0;
 #pragma unroll
@@ -565,7 +497,8 @@ __device__ __forceinline__ void aggregate_segment(const MatterArgs& a, const Sla
         const uint64_t mask = smask[r * 32 + lane];
         const bool removed = (mask & vac) != 0;
         bm[r] = __ballot_sync(0xffffffffu, mask != 0);
-        rc += __popc(__ballot_sync(0xffffffffu, removed));
+        rb[r] = __ballot_sync(0xffffffffu, removed);
+        rc += __popc(rb[r]);
         mc += __popc(bm[r]);
         for (uint64_t u = mask; u; u &= u - 1) {             // members are rare
             const int l = __ffsll((long long)u) - 1;
@@ -573,11 +506,10 @@ __device__ __forceinline__ void aggregate_segment(const MatterArgs& a, const Sla
             if (sh[l].type == DISCO_MATTER_INTERSTITIAL && !removed) atomicAdd(&wcnt[nl + l], 1);
         }
     }
-    if (off < 0) {
-        int o = 0;
-        if (lane == 0 && mc > 0) o = (int)atomicAdd(a.ctl + 2, (unsigned)mc);
-        off = __shfl_sync(0xffffffffu, o, 0);
-    }
+    if (lane == 0 && rc > 0) a.seg_mask[s] = make_uint4(rb[0], rb[1], rb[2], rb[3]);
+    off = 0;
+    if (lane == 0 && mc > 0) off = (int)atomicAdd(a.ctl + 2, (unsigned)mc);
+    off = __shfl_sync(0xffffffffu, off, 0);
     int e = off;
 #pragma unroll
     for (int r = 0; r < kSegRounds; ++r) {
@@ -624,7 +556,7 @@ __device__ __noinline__ int3 direct_segment(const MatterArgs& a, const SlabHead*
         }
     }
     __syncwarp();
-    int rc = 0, mc = 0, off = -1;
+    int rc = 0, mc = 0, off = 0;
     aggregate_segment(a, sh, vac, s, smask, ssides, wcnt, rc, mc, off, lane);
     __syncwarp();
     return make_int3(rc, mc, mc > 0 ? off : 0);
@@ -638,20 +570,28 @@ __device__ __noinline__ int3 direct_segment(const MatterArgs& a, const SlabHead*
 //     box and a per-loop cull; for the few segments a loop can reach, the
 //     FP32 pre-test per atom, its candidate (atom, loop) pairs queued per
 //     warp.  Once 32 tests are queued (or 32 segments listed) the warp runs
-//     the exact FP64 tests of its queue spread over its lanes, then per listed
-//     segment the masks, counts and member records (atom order, one block of
-//     records per flush).  Per segment: removed and member counts, first record; per
-//     call: the per-loop slab and kept-copy totals.
+//     the exact FP64 tests of its queue spread over its lanes, then with a
+//     lane per listed segment the counts and with a lane per atom the member
+//     records (atom order, one block of records per flush).  Per segment: the
+//     removed atoms' bits, removed and member counts, first record; per call:
+//     the per-loop slab and kept-copy totals.
 //   Barrier; per CTA, its counts from the per-segment results, per warp of
 //     its contiguous range; barrier; CTA c scans category c over the CTAs;
 //     barrier.
 //   Phase 2, ordered writes.  CTA k owns a contiguous range of segments, cut
 //     into eight contiguous warp ranges; each warp walks its range with the
-//     running survivor rank: a member-free segment is a shifted copy; a
-//     segment with members writes their slab entries and copies at the warp's
-//     running per-loop positions (loop base + CTA prefix + earlier warps'
-//     counts), in atom order (Code/prismatic.cpp:61-72,
-//     Code/main.cpp:651-654,676-679), then its survivors.
+//     running survivor rank: a segment without removed atoms is a shifted
+//     copy, one with some is compacted by its bits.  After each batch of 32
+//     segments come the slab entries and copies of its members, a lane per
+//     record, at the warp's running per-loop positions (loop base + CTA prefix
+//     + earlier warps' counts), in atom order (Code/prismatic.cpp:61-72,
+//     Code/main.cpp:651-654,676-679).
+// What bounds it (BCC 128^3, 16 loops, cold L2): phase 1 ends after 37 us, the
+// counts, scan and barriers after 49, phase 2 after 81 (42, 54 and 92 with one
+// listed segment after the other in a flush and one segment with members after
+// the other in phase 2): both phases wait on loads with 24 warps an SM, their
+// slowest warps 5 us behind the mean.  Four CTAs an SM (64 registers) spill:
+// 12 us slower.
 // No look-back and no second kernel: the only waits are the three barriers.
 // The outputs must not overlap the positions.
 __global__ void __launch_bounds__(kMatterThreads, 3) matter_kernel(const MatterArgs a)
@@ -660,8 +600,7 @@ __global__ void __launch_bounds__(kMatterThreads, 3) matter_kernel(const MatterA
     __shared__ SlabHead sh[kMaxSlabLoops];
     __shared__ __align__(16) unsigned char wq_raw[kMatterWarps * kWarpQueue * 4];   // phase 1 queues, phase 2 wrun
     __shared__ int wl_seg[kMatterWarps][kGroupSegs];           // listed segments of a group (index in the group)
-    __shared__ int wl_q[kMatterWarps][kGroupSegs];             // their first queue entry | count << 16
-    __shared__ int wl_mr[kMatterWarps][kGroupSegs];            // their member count | removed count << 16
+    __shared__ int wl_off[kMatterWarps][kGroupSegs];           // their first member record
     __shared__ int wcnt[kMatterWarps][kSegRow];                // per warp: slab / kept-copy counts per loop
     __shared__ int wrem[kMatterWarps], wmem[kMatterWarps];
     __shared__ int64_t run[kSegRow];                           // CTA's first slab entry / copy per loop
@@ -801,10 +740,7 @@ __global__ void __launch_bounds__(kMatterThreads, 3) matter_kernel(const MatterA
                             for (uint64_t c = cand[r]; c; c &= c - 1)
                                 wq[q++] = (uint32_t)(__ffsll((long long)c) - 1) | ((uint32_t)slot_of(r, lane) << 6) |
                                           ((uint32_t)nlst << 13);
-                        if (lane == 0) {
-                            wl_seg[warp][nlst] = (int)s;
-                            wl_q[warp][nlst] = nq | (T << 16);
-                        }
+                        if (lane == 0) wl_seg[warp][nlst] = (int)s;
                         nq += T;
                         ++nlst;
                         listed = true;
@@ -829,76 +765,80 @@ __global__ void __launch_bounds__(kMatterThreads, 3) matter_kernel(const MatterA
             }
             if (nq > 0) {
                 // flush: the exact tests of the queue spread over the lanes, the
-                // result in bits 29 (member) and 30 (positive side) of each entry
+                // members in bit 29 of their entries (bit 30: positive side) and
+                // in the listed segments' member and removed bits
+                uint32_t* bits = reinterpret_cast<uint32_t*>(smask);
+                for (int q = lane; q < nlst * 8; q += 32) bits[q] = 0u;
                 __syncwarp();
                 for (int q = lane; q < nq; q += 32) {
                     const uint32_t e = wq[q];
-                    const int l = e & 63, slot = (e >> 6) & 127;
-                    const int64_t i = (int64_t)wl_seg[warp][(e >> 13) & 31] * kSegAtoms + slot;
+                    const int l = e & 63, slot = (e >> 6) & 127, li = (e >> 13) & 31;
+                    const int64_t i = (int64_t)wl_seg[warp][li] * kSegAtoms + slot;
                     bool ps = false;
-                    const bool in = slab_member(a.loops[l], a.x[i], a.y[i], a.z[i], a.Lx, a.Ly, a.Lz, a.idLx,
-                                                a.idLy, a.idLz, ps);
-                    wq[q] = e | (in ? 1u << 29 : 0u) | (ps ? 1u << 30 : 0u);
+                    if (slab_member(a.loops[l], a.x[i], a.y[i], a.z[i], a.Lx, a.Ly, a.Lz, a.idLx, a.idLy, a.idLz, ps)) {
+                        wq[q] = e | 1u << 29 | (ps ? 1u << 30 : 0u);
+                        atomicOr(&bits[li * 8 + (slot >> 5)], 1u << (slot & 31));
+                        if ((vac >> l) & 1ull) atomicOr(&bits[li * 8 + 4 + (slot >> 5)], 1u << (slot & 31));
+                    }
                 }
                 __syncwarp();
-                // member and removed counts per listed segment, then one block of records
-                int tot = 0;
-                for (int jj = 0; jj < nlst; ++jj) {
-                    const int qo = wl_q[warp][jj] & 0xffff, qn = wl_q[warp][jj] >> 16;
-                    unsigned mb[kSegRounds], rbm[kSegRounds];
-#pragma unroll
-                    for (int r = 0; r < kSegRounds; ++r) { mb[r] = 0u; rbm[r] = 0u; }
-                    for (int q0 = 0; q0 < qn; q0 += 32) {
-                        unsigned slot = 0xffffffffu;
-                        bool rmv = false;
-                        if (q0 + lane < qn) {
-                            const uint32_t e = wq[qo + q0 + lane];
-                            if (e & (1u << 29)) {
-                                slot = (e >> 6) & 127;
-                                rmv = (vac >> (e & 63)) & 1ull;
-                            }
-                        }
-#pragma unroll
-                        for (int r = 0; r < kSegRounds; ++r) {
-                            const unsigned bit = (slot >> 5) == (unsigned)r ? 1u << (slot & 31u) : 0u;
-                            mb[r] |= __reduce_or_sync(0xffffffffu, bit);
-                            rbm[r] |= __reduce_or_sync(0xffffffffu, rmv ? bit : 0u);
-                        }
-                    }
-                    int m = 0, rm = 0;
-#pragma unroll
-                    for (int r = 0; r < kSegRounds; ++r) { m += __popc(mb[r]); rm += __popc(rbm[r]); }
-                    if (lane == 0) wl_mr[warp][jj] = m | (rm << 16);
-                    tot += m;
+                // a lane per listed segment: counts, removed bits, one block of records
+                uint4 mb = make_uint4(0u, 0u, 0u, 0u), rb = mb;
+                if (lane < nlst) {
+                    mb = *reinterpret_cast<const uint4*>(&bits[lane * 8]);
+                    rb = *reinterpret_cast<const uint4*>(&bits[lane * 8 + 4]);
                 }
+                const int m = __popc(mb.x) + __popc(mb.y) + __popc(mb.z) + __popc(mb.w);
+                const int rm = __popc(rb.x) + __popc(rb.y) + __popc(rb.z) + __popc(rb.w);
+                int incl = m;
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int y = __shfl_up_sync(0xffffffffu, incl, o);
+                    if (lane >= o) incl += y;
+                }
+                const int tot = __shfl_sync(0xffffffffu, incl, 31);
                 int base = 0;
                 if (lane == 0 && tot > 0) base = (int)atomicAdd(a.ctl + 2, (unsigned)tot);
-                base = __shfl_sync(0xffffffffu, base, 0);
+                base = __shfl_sync(0xffffffffu, base, 0) + incl - m;
+                if (lane < nlst) {
+                    const int64_t sj = wl_seg[warp][lane];
+                    a.seg_removed[sj] = rm;
+                    a.seg_members[sj] = m;
+                    a.seg_off[sj] = m > 0 ? base : 0;
+                    if (rm > 0) a.seg_mask[sj] = rb;
+                    wl_off[warp][lane] = base;
+                }
                 __syncwarp();
-                for (int jj = 0; jj < nlst; ++jj) {
-                    const int64_t sj = wl_seg[warp][jj];
-                    const int m = wl_mr[warp][jj] & 0xffff, rm = wl_mr[warp][jj] >> 16;
-                    if (m > 0) {
-                        const int qo = wl_q[warp][jj] & 0xffff, qn = wl_q[warp][jj] >> 16;
-#pragma unroll
-                        for (int r = 0; r < kSegRounds; ++r) { smask[r * 32 + lane] = 0; ssides[r * 32 + lane] = 0; }
-                        __syncwarp();
-                        for (int q = lane; q < qn; q += 32) {
-                            const uint32_t e = wq[qo + q];
-                            if (e & (1u << 29)) {
-                                const int slot = (e >> 6) & 127;
-                                atomicOr(reinterpret_cast<unsigned long long*>(&smask[slot]), 1ull << (e & 63));
-                                if (e & (1u << 30))
-                                    atomicOr(reinterpret_cast<unsigned long long*>(&ssides[slot]), 1ull << (e & 63));
-                            }
-                        }
-                        __syncwarp();
-                        int rc2 = 0, mc2 = 0, off2 = base;
-                        aggregate_segment(a, sh, vac, sj, smask, ssides, wcnt[warp], rc2, mc2, off2, lane);
-                        __syncwarp();
+                // a lane per atom with members among its entries (they are
+                // neighbours in the queue): its record, in atom order
+                for (int q = lane; q < nq && tot > 0; q += 32) {
+                    const uint32_t key = (wq[q] >> 6) & 0xfffu;
+                    if (q > 0 && ((wq[q - 1] >> 6) & 0xfffu) == key) continue;
+                    uint64_t mask = 0, sides = 0;
+                    for (int f = q; f < nq; ++f) {
+                        const uint32_t e = wq[f];
+                        if (((e >> 6) & 0xfffu) != key) break;
+                        if (e & (1u << 29)) mask |= 1ull << (e & 63);
+                        if (e & (1u << 30)) sides |= 1ull << (e & 63);
                     }
-                    if (lane == 0) { a.seg_removed[sj] = rm; a.seg_members[sj] = m; a.seg_off[sj] = m > 0 ? base : 0; }
-                    base += m;
+                    if (!mask) continue;
+                    const int slot = key & 127, li = key >> 7;
+                    int64_t at = wl_off[warp][li];
+                    for (int r = 0; r < (slot >> 5); ++r) at += __popc(bits[li * 8 + r]);
+                    at += __popc(bits[li * 8 + (slot >> 5)] & ((1u << (slot & 31)) - 1u));
+                    const bool removed = (mask & vac) != 0;
+                    for (uint64_t u = mask; u; u &= u - 1) {
+                        const int l = __ffsll((long long)u) - 1;
+                        atomicAdd(&wcnt[warp][l], 1);
+                        if (sh[l].type == DISCO_MATTER_INTERSTITIAL && !removed) atomicAdd(&wcnt[warp][nl + l], 1);
+                    }
+                    if (at < a.member_cap) {
+                        MemberRec rec;
+                        rec.atom = (int32_t)((int64_t)wl_seg[warp][li] * kSegAtoms + slot);
+                        rec.removed = removed;
+                        rec.mask = mask;
+                        rec.sides = sides;
+                        a.members[at] = rec;
+                    }
                 }
                 __syncwarp();                                   // the queue and the list are rewritten
             }
@@ -1039,8 +979,6 @@ __global__ void __launch_bounds__(kMatterThreads, 3) matter_kernel(const MatterA
     {
         const uint64_t last = l2_policy_last_use();
         int64_t* wrun = reinterpret_cast<int64_t*>(wq_raw) + warp * kSegRow;   // this warp's next entry per loop
-        uint64_t* smask = reinterpret_cast<uint64_t*>(dyn) + warp * (2 * kSegAtoms);
-        uint64_t* ssides = smask + kSegAtoms;
         for (int c = lane; c < 2 * nl; c += 32) {
             int64_t v = run[c];
             for (int w = 0; w < warp; ++w) v += wcnt[w][c];
@@ -1057,8 +995,6 @@ __global__ void __launch_bounds__(kMatterThreads, 3) matter_kernel(const MatterA
         for (int64_t c0 = wlo; c0 < whi; c0 += 32) {
             const int cn = (int)(whi - c0 < 32 ? whi - c0 : 32);
             const int v_rem = lane < cn ? __ldcg(a.seg_removed + c0 + lane) : 0;
-            const int v_mem = lane < cn ? __ldcg(a.seg_members + c0 + lane) : 0;
-            const int v_off = lane < cn ? __ldcg(a.seg_off + c0 + lane) : 0;
             int incl = v_rem;
             for (int o = 1; o < 32; o <<= 1) {
                 const int y = __shfl_up_sync(0xffffffffu, incl, o);
@@ -1069,11 +1005,82 @@ __global__ void __launch_bounds__(kMatterThreads, 3) matter_kernel(const MatterA
 #pragma unroll 1
             for (int j = 0; j < cn; ++j) {
                 const int64_t sbj = base + (int64_t)j * kSegAtoms - __shfl_sync(0xffffffffu, ex_rem, j);
-                const int m = __shfl_sync(0xffffffffu, v_mem, j), off = __shfl_sync(0xffffffffu, v_off, j);
-                if (m > 0 && (int64_t)off + m <= a.member_cap)
-                    copy_members(a, sh, vac, c0 + j, sbj, a.members + off, m, smask, ssides, wrun, last, lane);
-                else
-                    copy_plain(a, c0 + j, sbj, last, lane);
+                if (__shfl_sync(0xffffffffu, v_rem, j) > 0) copy_removed(a, c0 + j, sbj, last, lane);
+                else copy_plain(a, c0 + j, sbj, last, lane);
+            }
+            // the batch's slab entries and copies from its member records, a
+            // lane per record: per loop in atom order at the running positions
+            // (copies of removed atoms dropped, sources renumbered)
+            const int v_mem = lane < cn ? __ldcg(a.seg_members + c0 + lane) : 0;
+            const int v_off = lane < cn ? __ldcg(a.seg_off + c0 + lane) : 0;
+            const int mm = v_mem > 0 && (int64_t)v_off + v_mem <= a.member_cap ? v_mem : 0;
+            int mi = mm;
+            for (int o = 1; o < 32; o <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, mi, o);
+                if (lane >= o) mi += y;
+            }
+            const int ex = mi - mm, tot = __shfl_sync(0xffffffffu, mi, 31);
+            const unsigned ltm = (1u << lane) - 1u;
+#pragma unroll 1
+            for (int e0 = 0; e0 < tot; e0 += 32) {
+                const int e = e0 + lane;
+                int j = 0;                                      // the last segment whose records start at or before e
+#pragma unroll
+                for (int step = 16; step > 0; step >>= 1)
+                    if (__shfl_sync(0xffffffffu, ex, j + step) <= e) j += step;
+                const int oj = __shfl_sync(0xffffffffu, v_off, j), exj = __shfl_sync(0xffffffffu, ex, j);
+                const int remj = __shfl_sync(0xffffffffu, v_rem, j);
+                uint64_t mk = 0, sd = 0;
+                int atom = 0;
+                uint4 bits = make_uint4(0u, 0u, 0u, 0u);
+                if (e < tot) {
+                    if (remj > 0) bits = __ldcg(a.seg_mask + c0 + j);
+                    const MemberRec* rec = a.members + oj + (e - exj);
+                    mk = __ldcg(reinterpret_cast<const unsigned long long*>(&rec->mask));
+                    sd = __ldcg(reinterpret_cast<const unsigned long long*>(&rec->sides));
+                    atom = __ldcg(&rec->atom);
+                }
+                const int slot = (int)(atom - (c0 + j) * kSegAtoms) & (kSegAtoms - 1);
+                int before = __shfl_sync(0xffffffffu, ex_rem, j);              // removed atoms before this one
+                const unsigned rb[kSegRounds] = { bits.x, bits.y, bits.z, bits.w };
+#pragma unroll
+                for (int r = 0; r < kSegRounds; ++r)
+                    before += __popc(slot >= 32 * r + 32 ? rb[r] : slot > 32 * r ? rb[r] & ((1u << (slot & 31)) - 1u) : 0u);
+                const int32_t source = (int32_t)(base + (int64_t)j * kSegAtoms + slot - before);
+                const bool removed = (mk & vac) != 0;
+                uint64_t un = ((uint64_t)__reduce_or_sync(0xffffffffu, (unsigned)(mk >> 32)) << 32) |
+                              __reduce_or_sync(0xffffffffu, (unsigned)mk);
+                for (; un; un &= un - 1) {
+                    const int l = __ffsll((long long)un) - 1;
+                    const bool in = (mk >> l) & 1ull;
+                    const bool kp = in && !removed && sh[l].type == DISCO_MATTER_INTERSTITIAL;
+                    const bool pos = (sd >> l) & 1ull;
+                    const unsigned bi = __ballot_sync(0xffffffffu, in);
+                    const unsigned bk = __ballot_sync(0xffffffffu, kp);
+                    const int64_t qs = wrun[l], qc = wrun[nl + l];
+                    __syncwarp();
+                    if (lane == 0) { wrun[l] = qs + __popc(bi); wrun[nl + l] = qc + __popc(bk); }
+                    if (in) {
+                        const int64_t q = qs + __popc(bi & ltm);
+                        if (q >= 0 && q < a.slab_cap) {
+                            a.slab_atoms[q] = atom;
+                            a.slab_side[q] = pos ? 1 : -1;
+                        }
+                    }
+                    if (kp) {
+                        const int64_t q = qc + __popc(bk & ltm);
+                        if (q >= 0 && q < a.copy_cap) {
+                            const disco_slab_loop& g = a.loops[l].L;
+                            const double* shf = pos ? g.shift_pos : g.shift_neg;
+                            disco_copy cp;
+                            cp.atom = source;
+                            cp.reserved = 0;
+                            cp.shift[0] = shf[0]; cp.shift[1] = shf[1]; cp.shift[2] = shf[2];
+                            a.copies[q] = cp;
+                        }
+                    }
+                    __syncwarp();
+                }
             }
             rem_run += __shfl_sync(0xffffffffu, incl, 31);
         }
@@ -1312,6 +1319,7 @@ int stage_loops(const disco_slab_loop* loops, int nloops, const double box[3], d
 // Bytes of the control words (barrier arrivals, exits, member records taken,
 // error word, per-loop totals); the last CTA of every completed call leaves
 // them at zero.
+constexpr size_t kSegInts = 7;   // per segment: removed bits (4), removed, members, first record
 constexpr size_t kCtlBytes = (disco::kCtlWords + 2 * disco::kMaxSlabLoops) * sizeof(unsigned int);
 
 // CTAs of the cooperative launch on the current device: resident CTAs per SM
@@ -1360,7 +1368,7 @@ void matter_shape(int64_t n, int grid_max, int64_t& S, int& G)
 struct MatterScratch {
     unsigned char* loops;        // heads then records (sizeof(LoopStage))
     unsigned int* ctl;           // kCtlBytes
-    int32_t* seg;                // 3 S: removed, members, first record per segment
+    int32_t* seg;                // kSegInts S: removed bits, then removed, members, first record per segment
     int32_t* cta;                // 2 G C: counts and prefixes per CTA
     disco::MemberRec* members;
     int64_t member_cap;
@@ -1379,9 +1387,10 @@ int matter_queue(disco::MatterArgs& a, const MatterScratch& m, int nl, int64_t S
     a.C = 2 + 2 * nl;
     a.G = G;
     a.S = S;
-    a.seg_removed = m.seg;
-    a.seg_members = m.seg + S;
-    a.seg_off = m.seg + 2 * S;
+    a.seg_mask = reinterpret_cast<uint4*>(m.seg);
+    a.seg_removed = m.seg + 4 * S;
+    a.seg_members = m.seg + 5 * S;
+    a.seg_off = m.seg + 6 * S;
     a.cta_tot = m.cta;
     a.cta_pre = m.cta + (int64_t)G * a.C;
     a.ctl = m.ctl;
@@ -1497,7 +1506,7 @@ int disco_b200_prismatic(const double* x, const double* y, const double* z, int6
     }
     if (e == cudaSuccess) e = cudaMalloc(&dloops.p, sizeof(LoopStage));
     if (e == cudaSuccess) e = cudaMalloc(&dctl.p, kCtlBytes);
-    if (e == cudaSuccess) e = cudaMalloc(&dseg.p, 3 * std::max<int64_t>(1, S) * sizeof(int32_t));
+    if (e == cudaSuccess) e = cudaMalloc(&dseg.p, kSegInts * std::max<int64_t>(1, S) * sizeof(int32_t));
     if (e == cudaSuccess) e = cudaMalloc(&dcta.p, 2 * (size_t)G * C * sizeof(int32_t));
     if (e == cudaSuccess) e = cudaMalloc(&dmem.p, (size_t)member_cap * sizeof(MemberRec));
     if (e == cudaSuccess) e = cudaMalloc(&dtot.p, (size_t)(C + 1) * sizeof(int64_t));
@@ -1647,7 +1656,7 @@ constexpr size_t align256c(size_t v) { return (v + 255) & ~size_t(255); }
 constexpr size_t kNoAllocLoopOff = 0;
 constexpr size_t kNoAllocCtlOff = kNoAllocLoopOff + align256c(sizeof(LoopStage));
 constexpr size_t kNoAllocSegOff = kNoAllocCtlOff + align256c(kCtlBytes);
-constexpr size_t kNoAllocCtaOff = kNoAllocSegOff + align256c(3 * (size_t)kNoAllocMaxSegs * sizeof(int32_t));
+constexpr size_t kNoAllocCtaOff = kNoAllocSegOff + align256c(kSegInts * (size_t)kNoAllocMaxSegs * sizeof(int32_t));
 constexpr size_t kNoAllocMemberOff =
     kNoAllocCtaOff + align256c(2 * (size_t)disco::kMaxGrid * disco::kMaxCats * sizeof(int32_t));
 constexpr size_t kNoAllocTotalsOff =

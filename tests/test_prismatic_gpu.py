@@ -67,6 +67,18 @@ def test_overlapping_slabs_large_grid():
     _same(P.prismatic(x, y, z, w.slab_loops, w.box), O.prismatic(x, y, z, w.slab_loops, w.box))
 
 
+@pytest.mark.parametrize("keep", [1, 31, 127, 128, 129, 1023, 4095, 4097])
+def test_dense_members_at_segment_edges(keep):
+    """Atoms that nearly all lie in slabs, many in several at once, removed and
+    copied, with the count at the edges of the 128-atom segments and of the
+    record batches (the densest stretch of the box is kept)."""
+    w = W.bcc_prismatic(cells=14, rmin=12.0, rmax=14.0, n_inter=30, n_vac=30, seed=5)
+    q = O.prismatic(w.x, w.y, w.z, w.slab_loops, w.box)
+    order = np.argsort(-np.bincount(q["slab_atoms"], minlength=w.n), kind="stable")
+    x, y, z = (np.ascontiguousarray(v[order][:keep]) for v in (w.x, w.y, w.z))
+    _same(P.prismatic(x, y, z, w.slab_loops, w.box), O.prismatic(x, y, z, w.slab_loops, w.box))
+
+
 def test_unwrapped_coordinates():
     """Atoms moved by whole box lengths, up to 2000 L from the box, as an
     unwrapped trajectory gives them: the minimum image decides membership
