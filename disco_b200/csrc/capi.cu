@@ -145,7 +145,7 @@ double now_s()
 namespace {
 
 constexpr int kMaxDevices = 64;
-constexpr uint64_t kScratchKeep = 32ull << 20, kScratchKeepPlans = 256ull << 20;
+constexpr uint64_t kScratchKeep = 32ull << 20, kScratchKeepPlans = 1024ull << 20;
 std::mutex g_scratch_mutex;
 cudaMemPool_t g_scratch[kMaxDevices] = {};
 unsigned long long g_scratch_ctx[kMaxDevices] = {};     // the context each pool was made in

@@ -20,10 +20,11 @@ void set_last_error(const char* msg);
 unsigned long long current_context_id();
 
 // Stream-ordered scratch memory, one pool per device (null where none could be
-// made).  32 MB (one block of the driver's) stay reserved in it, and up to 256 MB
+// made).  32 MB (one block of the driver's) stay reserved in it, and up to 1 GB
 // while a plan that has used it lives (retain / release): the default pool gives
 // its memory back at every synchronisation, and a call after one then pays for
-// mapping it again (0.2 to 0.4 ms).
+// mapping it again (0.2 to 0.4 ms; 13.5 M atoms, 640 MB of scratch: 5.8 ms of an
+// execute of 79).
 cudaMemPool_t scratch_pool(int device);
 void scratch_retain(int device);
 void scratch_release(int device);
