@@ -11,8 +11,11 @@ GPU.  A step is one full displacement sum over all atoms.
           host arrays: table build, allocation, H2D of positions and
           displacements, kernel, D2H of the displacements, per step.
   roofline  W = 128 flop per segment-image evaluation (66 per loopon-image)
-          against the FP64 peak measured here with a DGEMM (the driver's peak
-          file has no FP64 figure); traffic from the committed ncu summary.
+          against the FMA pipe's peak at the sampled clock.  A plan that sums
+          by cells does a small part of those evaluations: its line carries
+          the rate that the term-by-term sum would need under
+          "term_by_term_equivalent", no fraction of a peak from it, and the
+          FP64 pipe's measured share of cycles from the committed ncu summary.
   cpu_baseline  the oracle (CPU restatement, the reference's flags) on a
           seeded atom sample, all host threads, rank 0 only.
 
@@ -122,6 +125,42 @@ def timed_steps(torch, step, steps, stream, flush):
         e1.synchronize()
         total += e0.elapsed_time(e1) * 1e-3
     return total
+
+
+def kernels_per_call(torch, fn, least):
+    """Kernels that one call of fn launches, counted by the profiler outside any
+    timed region; `least` where it cannot be used."""
+    try:
+        from torch.profiler import ProfilerActivity, profile
+        torch.cuda.synchronize()
+        with profile(activities=[ProfilerActivity.CUDA], acc_events=True) as p:
+            fn()
+            torch.cuda.synchronize()
+        count = sum(1 for e in p.events() if "CUDA" in str(e.device_type)
+                    and not e.name.lower().startswith(("memcpy", "memset")) and "at::native" not in e.name)
+        return max(least, count)
+    except Exception:
+        return least
+
+
+def field_roofline(torch, clk, fp64, evals, flop, seconds, by_cells, traffic=None):
+    """Roofline of a field launch of `evals` segment- or loopon-image terms."""
+    gemm = fp64_peak_tflops(torch) if fp64 else fp32_peak_tflops(torch)
+    peak, src = pipe_peak_tflops(torch, clk, fp64)
+    rate = evals * flop / seconds / 1e12
+    roof = {"bound": "fp64" if fp64 else "fp32", "achieved": rate, "peak": peak, "unit": "TFLOP/s",
+            "frac": rate / peak, "traffic": traffic,
+            "peak_source": src + "; MEASURED_PEAKS.json has no FP64 or FP32 CUDA-core figure",
+            "peak_gemm": gemm, "frac_of_gemm": rate / gemm if gemm else None,
+            "peak_gemm_source": ("torch DGEMM 8192^3, best of 5: it runs on the FP64 tensor-core path, "
+                                 "not on the DFMA pipe this kernel uses") if fp64 else
+                                "torch SGEMM 8192^3 without TF32, best of 5",
+            "flop_per_eval": flop, "evals_per_launch": evals}
+    if by_cells:
+        roof.update(achieved=None, frac=None, frac_of_gemm=None, term_by_term_equivalent=rate,
+                    form="far pairs by cells: most terms are never formed, so their rate is no share of a peak",
+                    fp64_pipe_active=profile_value("tree_fcc_large", "fp64_pipe_active"))
+    return roof
 
 
 def measured_peaks():
@@ -283,18 +322,23 @@ def pipe_peak_tflops(torch, clk, fp64=True):
                 f"{mhz:.0f} MHz ({src})")
 
 
-def traffic_from_profiles(kernel_key):
-    """DRAM bytes per launch from the committed ncu summary, if any."""
-    path = os.path.join(ROOT, "profiles", f"{kernel_key}.md")
+def profile_value(name, key):
+    """The number after `key:` in a committed ncu summary, if any."""
+    path = os.path.join(ROOT, "profiles", f"{name}.md")
     if not os.path.exists(path):
         return None
     for line in open(path):
-        if line.strip().startswith("traffic_per_launch_bytes:"):
+        if line.strip().startswith(key + ":"):
             try:
                 return float(line.split(":", 1)[1].strip().split()[0])
             except ValueError:
                 return None
     return None
+
+
+def traffic_from_profiles(kernel_key):
+    """DRAM bytes per launch from the committed ncu summary, if any."""
+    return profile_value(kernel_key, "traffic_per_launch_bytes")
 
 
 class quiet_stdout:
@@ -675,7 +719,6 @@ def run_ours(args):
     stream = torch.cuda.current_stream()
     pos = torch.tensor(np.stack([w.x, w.y, w.z]), dtype=torch.float64, device="cuda")
     u = torch.zeros_like(pos)
-    launches_per_step = int(st["n_line_loops"] > 0) + int(st["n_loopon_loops"] > 0)
 
     def barrier():
         if world > 1:
@@ -702,6 +745,8 @@ def run_ours(args):
     plan.execute(pos, u1d)
     plan.sync(stream.cuda_stream)
     u1 = u1d.cpu().numpy()
+    launches_per_step = kernels_per_call(torch, lambda: (plan.execute(pos, u), plan.sync(stream.cuda_stream)),
+                                         int(st["n_line_loops"] > 0) + int(st["n_loopon_loops"] > 0))
     output = write_output(w, pos, u1d, stream) if (rank == 0 and not args.no_output) else None
     del u1d
 
@@ -774,20 +819,10 @@ def run_ours(args):
 
     if rank == 0:
         fp64 = prec == C.DISCO_FP64
-        gemm = fp64_peak_tflops(torch) if fp64 else fp32_peak_tflops(torch)
-        peak, peak_src = pipe_peak_tflops(torch, clk, fp64)
-        flops = evals_atom * n * flop_per_eval(w)
-        achieved = flops / per_launch / 1e12
         key = f"{'line' if w.method == 'line' else 'loopon'}_{args.precision}_{args.config}"
-        traffic = traffic_from_profiles(key)
-        roof = {"bound": "fp64" if fp64 else "fp32", "achieved": achieved,
-                "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak, "traffic": traffic,
-                "peak_source": peak_src + "; MEASURED_PEAKS.json has no FP64 or FP32 CUDA-core figure",
-                "peak_gemm": gemm, "frac_of_gemm": achieved / gemm if gemm else None,
-                "peak_gemm_source": ("torch DGEMM 8192^3, best of 5: it runs on the FP64 tensor-core path, "
-                                     "not on the DFMA pipe this kernel uses") if fp64 else
-                                    "torch SGEMM 8192^3 without TF32, best of 5",
-                "flop_per_eval": flop_per_eval(w), "evals_per_launch": evals_atom * n}
+        by_cells = launches_per_step > 2
+        roof = field_roofline(torch, clk, fp64, evals_atom * n, flop_per_eval(w), per_launch, by_cells,
+                              None if by_cells else traffic_from_profiles(key))
         cpu = None
         parity = None
         if not args.no_cpu:
@@ -1255,6 +1290,7 @@ def run_prismatic(args, embedded=False):
     clk = clocks.stop()
     plan.sync(stream.cuda_stream)
     k, nc = kn
+    launches_per_step = kernels_per_call(torch, lambda: (step(), plan.sync(stream.cuda_stream)), 3)
     elapsed = max_over_ranks(elapsed, world)
     per = elapsed / args.steps
     evals = st_plan["evals_per_atom"] * k
@@ -1321,9 +1357,8 @@ def run_prismatic(args, embedded=False):
             refgpu["ours"] = {"kernel_s": f0.elapsed_time(f1) * 1e-3,
                               "note": "this library's loopon field over the same survivors, nu 0.35"}
             del u35
-        gemm = fp64_peak_tflops(torch) if prec == C.DISCO_FP64 else fp32_peak_tflops(torch)
-        peak, peak_src = pipe_peak_tflops(torch, clk, prec == C.DISCO_FP64)
-        achieved = evals * W_LOOPON / per / 1e12
+        roof = field_roofline(torch, clk, prec == C.DISCO_FP64, evals, W_LOOPON, per, launches_per_step > 4)
+        roof["kernel"] = "loopon field (the step also holds the matter step and epilogue)"
         line = {
             "metric": METRIC, "value": n * world / per, "unit": "atoms/s", "n_gpus": world,
             "steps": args.steps, "warmup": args.warmup, "ms_per_step": 1e3 * per,
@@ -1335,16 +1370,12 @@ def run_prismatic(args, embedded=False):
                        "step": "matter step + loopon field + copy/add-u/wrap epilogue, all on device",
                        "l2": flush.note(48 * n), "parallelism": f"replicas x{world}"},
             "evals_per_s": evals * world / per,
-            "roofline": {"bound": "fp64" if prec == C.DISCO_FP64 else "fp32", "kernel": "loopon field",
-                         "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
-                         "peak_source": peak_src + " (the step also holds the matter step and epilogue)",
-                         "peak_gemm": gemm, "frac_of_gemm": achieved / gemm,
-                         "traffic": None, "flop_per_eval": W_LOOPON, "evals_per_launch": evals},
+            "roofline": roof,
             "cpu_baseline": cpu,
             "e2e": {"value": n * world * e2e_steps / e2e_t, "unit": "atoms/s",
                     "h2d_bytes_per_step": 24 * n + 48 * k + 48 * k,
                     "d2h_bytes_per_step": 28 * n + 24 * k + 48 * (k + nc), "steps": e2e_steps},
-            "clocks": clk, "gpu_launches": args.steps * 3,     # matter kernel, field kernel, epilogue
+            "clocks": clk, "gpu_launches": args.steps * launches_per_step,     # matter kernel, field kernels, epilogue
             "parity": parity, "compaction": compaction, "compaction_13m": compaction_13m,
             **({"reference_gpu": refgpu} if refgpu else {}),
         }

@@ -995,6 +995,9 @@ __global__ void __launch_bounds__(kMatterThreads, 3) matter_kernel(const MatterA
         for (int64_t c0 = wlo; c0 < whi; c0 += 32) {
             const int cn = (int)(whi - c0 < 32 ? whi - c0 : 32);
             const int v_rem = lane < cn ? __ldcg(a.seg_removed + c0 + lane) : 0;
+            const int v_mem = lane < cn ? __ldcg(a.seg_members + c0 + lane) : 0;
+            const int v_off = lane < cn ? __ldcg(a.seg_off + c0 + lane) : 0;
+            const int mm = v_mem > 0 && (int64_t)v_off + v_mem <= a.member_cap ? v_mem : 0;
             int incl = v_rem;
             for (int o = 1; o < 32; o <<= 1) {
                 const int y = __shfl_up_sync(0xffffffffu, incl, o);
@@ -1011,9 +1014,6 @@ __global__ void __launch_bounds__(kMatterThreads, 3) matter_kernel(const MatterA
             // the batch's slab entries and copies from its member records, a
             // lane per record: per loop in atom order at the running positions
             // (copies of removed atoms dropped, sources renumbered)
-            const int v_mem = lane < cn ? __ldcg(a.seg_members + c0 + lane) : 0;
-            const int v_off = lane < cn ? __ldcg(a.seg_off + c0 + lane) : 0;
-            const int mm = v_mem > 0 && (int64_t)v_off + v_mem <= a.member_cap ? v_mem : 0;
             int mi = mm;
             for (int o = 1; o < 32; o <<= 1) {
                 const int y = __shfl_up_sync(0xffffffffu, mi, o);

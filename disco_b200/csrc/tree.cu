@@ -36,9 +36,9 @@
 // part of what it returns, and its far terms summed in FP64 would change it.
 //
 // Measured against the plain kernel on one B200 (ms a call): FCC 100^3 cells
-// (4.0 M atoms), 16 loops, +-2 images 986 -> 15.3; BCC 61 x 47 x 33 (184 k
-// atoms), 9 loops, +-3 86.9 -> 9.5; BCC 40^3 (128 k), 4 loops of 64 segments,
-// +-1 4.94 -> 3.33; loopons: BCC 40^3 (127 k), 8 prismatic loops of R 20 to 50
+// (4.0 M atoms), 16 loops, +-2 images 986 -> 14.7; BCC 61 x 47 x 33 (184 k
+// atoms), 9 loops, +-3 76 -> 8.3; BCC 40^3 (128 k), 4 loops of 64 segments,
+// +-1 4.93 -> 3.10; loopons: BCC 40^3 (127 k), 8 prismatic loops of R 20 to 50
 // (39 k loopons), +-1 255 -> 57.  A sum too small to gain (2 000 atoms, 2 loops: 0.02 ms of
 // terms) stays with the plain kernel: tree_shape compares operation counts of
 // both, launches included.

@@ -159,14 +159,19 @@ const char *disco_b200_strerror(int status);
 /* ---- displacement sum ---------------------------------------------------------- */
 
 /* Host buffers in, host buffers out: uploads the atoms, sums every loop over
- * every image in one launch, adds the result into atoms->ux/uy/uz.  Replaces
+ * every image, adds the result into atoms->ux/uy/uz.  Replaces
  * kroupaGPU (Code/backend.hpp:61-62, Code/backend_cuda.cu:568-722). */
 int disco_b200_displace(const disco_atoms *atoms, const disco_loop *loops, int32_t nloops,
                         const double box[3], const disco_options *opt, disco_timing *timing);
 
 /* Resident form: the loop tables are built and uploaded once by plan_create;
  * plan_execute adds the field of every loop into DEVICE arrays on `stream`
- * (a cudaStream_t, NULL = legacy default stream) without any host copy. */
+ * (a cudaStream_t, NULL = legacy default stream) without any host copy.  An
+ * FP64 plan large enough to gain sums its far pairs by cells (16 bytes of
+ * scratch per atom and the cells' values, stream-ordered, from a pool that
+ * keeps at most 32 MB, 1 GB while such a plan lives); without that scratch, or
+ * under stream capture, the call sums term by term.  The two differ by the
+ * rounding of the sum (3.6e-14 A at most where it was measured). */
 int disco_b200_plan_create(const disco_loop *loops, int32_t nloops, const double box[3],
                            const disco_options *opt, int64_t max_atoms, disco_plan **out);
 int disco_b200_plan_execute(disco_plan *plan, const disco_atoms *device_atoms, void *stream);
