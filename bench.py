@@ -207,7 +207,8 @@ def flop_per_eval(w):
 
 
 class Clocks:
-    """nvidia-smi samples during the timed region (every 200 ms)."""
+    """nvidia-smi samples during the timed region (every 20 ms; a region may last
+    a fifth of a second)."""
     Q = ("index,clocks.sm,clocks.max.sm,power.draw,clocks_event_reasons.active,"
          "clocks_event_reasons.hw_slowdown,clocks_event_reasons.hw_thermal_slowdown,"
          "clocks_event_reasons.sw_thermal_slowdown,clocks_event_reasons.sw_power_cap")
@@ -216,14 +217,24 @@ class Clocks:
         self.device = device
         self.f = tempfile.NamedTemporaryFile(mode="w+", suffix=".csv", delete=False)
         self.p = None
+        self.at = 0
 
-    def start(self):
+    def start(self, load=None):
+        """Starts sampling; with `load` (an untimed step that waits for itself),
+        runs it until the first sample is there, so that a short region has
+        samples of its own (mark() drops those before it)."""
         try:
             self.p = subprocess.Popen(["nvidia-smi", "-i", str(self.device), f"--query-gpu={self.Q}",
-                                       "--format=csv,noheader,nounits", "-lms", "200"],
+                                       "--format=csv,noheader,nounits", "-lms", "20"],
                                       stdout=self.f, stderr=subprocess.DEVNULL)
         except Exception:
             self.p = None
+        limit = time.perf_counter() + 5.0
+        while load and self.p and os.path.getsize(self.f.name) == 0 and time.perf_counter() < limit:
+            load()
+
+    def mark(self):
+        self.at = os.path.getsize(self.f.name)
 
     def stop(self):
         if self.p is None:
@@ -234,7 +245,10 @@ class Clocks:
         except Exception:
             self.p.kill()
         self.f.flush()
-        rows = [r.split(",") for r in open(self.f.name).read().strip().splitlines() if r.strip()]
+        text = open(self.f.name).read()
+        # the line being written at mark() belongs to before the region
+        at = text.find("\n", self.at - 1) + 1 if self.at else 0
+        rows = [r.split(",") for r in text[at:].strip().splitlines() if r.strip()]
         os.unlink(self.f.name)
         sm, mx, reasons = [], 0.0, set()
         names = ["hw_slowdown", "hw_thermal_slowdown", "sw_thermal_slowdown", "sw_power_cap"]
@@ -730,8 +744,9 @@ def run_ours(args):
     plan.sync(stream.cuda_stream)
     flush = L2Flush(torch, 48 * n)
     clocks = Clocks(local)
+    clocks.start(lambda: (plan.execute(pos, u), plan.sync(stream.cuda_stream)))
     barrier()
-    clocks.start()
+    clocks.mark()
     elapsed = timed_steps(torch, lambda: plan.execute(pos, u), args.steps, stream, flush)
     barrier()
     clk = clocks.stop()
@@ -1283,8 +1298,9 @@ def run_prismatic(args, embedded=False):
         kn[0], kn[1] = step()
 
     clocks = Clocks(local)
+    clocks.start(lambda: (step(), plan.sync(stream.cuda_stream)))
     barrier()
-    clocks.start()
+    clocks.mark()
     elapsed = timed_steps(torch, timed_step, args.steps, stream, flush)
     barrier()
     clk = clocks.stop()
