@@ -808,11 +808,15 @@ __global__ void __launch_bounds__(kMatterThreads, 3) matter_kernel(const MatterA
                     wl_off[warp][lane] = base;
                 }
                 __syncwarp();
-                // a lane per atom with members among its entries (they are
-                // neighbours in the queue): its record, in atom order
+                // a lane per member atom (its first member entry; an atom's
+                // entries are neighbours in the queue): its record, in atom order
                 for (int q = lane; q < nq && tot > 0; q += 32) {
+                    if (!(wq[q] & (1u << 29))) continue;
                     const uint32_t key = (wq[q] >> 6) & 0xfffu;
-                    if (q > 0 && ((wq[q - 1] >> 6) & 0xfffu) == key) continue;
+                    bool first = true;
+                    for (int f = q - 1; f >= 0 && ((wq[f] >> 6) & 0xfffu) == key && first; --f)
+                        first = !(wq[f] & (1u << 29));
+                    if (!first) continue;
                     uint64_t mask = 0, sides = 0;
                     for (int f = q; f < nq; ++f) {
                         const uint32_t e = wq[f];
@@ -820,7 +824,6 @@ __global__ void __launch_bounds__(kMatterThreads, 3) matter_kernel(const MatterA
                         if (e & (1u << 29)) mask |= 1ull << (e & 63);
                         if (e & (1u << 30)) sides |= 1ull << (e & 63);
                     }
-                    if (!mask) continue;
                     const int slot = key & 127, li = key >> 7;
                     int64_t at = wl_off[warp][li];
                     for (int r = 0; r < (slot >> 5); ++r) at += __popc(bits[li * 8 + r]);
@@ -909,18 +912,22 @@ __global__ void __launch_bounds__(kMatterThreads, 3) matter_kernel(const MatterA
     grid_sync(a.ctl, 2u * (unsigned)G, err);
 
     // ---- scan: exclusive prefixes over the CTAs per category.  A small grid
-    // (small boxes) is scanned by CTA 0 alone, one category per thread; a
+    // (small boxes) is scanned by CTA 0 alone, one category per warp; a
     // large one by CTA c for category c.
     if (G <= kSmallGrid) {
         if (blockIdx.x == 0)
-            for (int c = tid; c < C; c += kMatterThreads) {
-                int64_t runv = 0;
-                for (int q = 0; q < G; ++q) {
-                    const int32_t v = __ldcg(a.cta_tot + (int64_t)q * C + c);
-                    a.cta_pre[(int64_t)q * C + c] = (int32_t)runv;
-                    runv += v;
+            for (int c = warp; c < C; c += kMatterWarps) {
+                const int32_t v0 = lane < G ? __ldcg(a.cta_tot + (int64_t)lane * C + c) : 0;
+                const int32_t v1 = lane + 32 < G ? __ldcg(a.cta_tot + (int64_t)(lane + 32) * C + c) : 0;
+                int32_t i0 = v0, i1 = v1;
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int32_t y0 = __shfl_up_sync(0xffffffffu, i0, o), y1 = __shfl_up_sync(0xffffffffu, i1, o);
+                    if (lane >= o) { i0 += y0; i1 += y1; }
                 }
-                a.totals[c] = c < 2 ? runv : (int64_t)__ldcg(a.ctl + kCtlWords + (c - 2));
+                const int32_t t0 = __shfl_sync(0xffffffffu, i0, 31), t1 = __shfl_sync(0xffffffffu, i1, 31);
+                if (lane < G) a.cta_pre[(int64_t)lane * C + c] = i0 - v0;
+                if (lane + 32 < G) a.cta_pre[(int64_t)(lane + 32) * C + c] = t0 + i1 - v1;
+                if (lane == 0) a.totals[c] = c < 2 ? (int64_t)t0 + t1 : (int64_t)__ldcg(a.ctl + kCtlWords + (c - 2));
             }
     } else
     for (int c = blockIdx.x; c < C; c += G) {
