@@ -540,6 +540,15 @@ void free_mlp(disco_mlp* p)
     delete p;
 }
 
+// The tiles of new weights, complete when this returns: every later launch, and
+// every replay of a captured one, reads them whatever its stream.
+cudaError_t pack_weights(disco_mlp* p)
+{
+    pack_kernel<<<(kParams + 255) / 256, 256>>>(p->params, p->img);
+    const cudaError_t e = cudaGetLastError();
+    return e == cudaSuccess ? cudaStreamSynchronize(nullptr) : e;
+}
+
 // Queues the network over n rows of X: forward into Y (T null), or forward and
 // backward into the gradients and the loss.
 int run_net(disco_mlp* p, const float* X, const float* T, int64_t n, float* Y, cudaStream_t s)
@@ -555,10 +564,6 @@ int run_net(disco_mlp* p, const float* X, const float* T, int64_t n, float* Y, c
     }
     NetArgs a;
     std::memset(&a, 0, sizeof(a));
-    if (p->img_stale) {
-        pack_kernel<<<(kParams + 255) / 256, 256, 0, s>>>(p->params, p->img);
-        p->img_stale = false;
-    }
     a.P = p->params;
     a.img = p->img;
     a.X = X; a.T = T; a.Y = Y;
@@ -632,6 +637,7 @@ int disco_b200_mlp_create(uint64_t seed, disco_mlp** out)
     fill(oW4, kOut, kHid, kOutReal, kHid);
     e = cudaMemcpy(p->params, h.data(), kParams * sizeof(float), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemset(p->grads, 0, 3 * kVec + 512);
+    if (e == cudaSuccess) e = pack_weights(p);
     if (e != cudaSuccess) { free_mlp(p); return mcuda(e, "MLP init"); }
     *out = p;
     return DISCO_OK;
@@ -655,8 +661,8 @@ int disco_b200_mlp_get_params(const disco_mlp* p, float* host)
 int disco_b200_mlp_set_params(disco_mlp* p, const float* host)
 {
     if (!p || !host) return mfail(DISCO_EINVAL, "null argument");
-    const cudaError_t e = cudaMemcpy(p->params, host, kParams * sizeof(float), cudaMemcpyHostToDevice);
-    p->img_stale = true;
+    cudaError_t e = cudaMemcpy(p->params, host, kParams * sizeof(float), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = pack_weights(p);
     return e == cudaSuccess ? DISCO_OK : mcuda(e, "params upload");
 }
 
@@ -699,7 +705,6 @@ int disco_b200_mlp_adam(disco_mlp* p, float lr, float beta1, float beta2, float 
     const float bc1 = 1.0f - std::pow(beta1, (float)p->step), bc2 = 1.0f - std::pow(beta2, (float)p->step);
     adam_kernel<<<(kParams + 255) / 256, 256, 0, static_cast<cudaStream_t>(stream)>>>(
         p->params, p->grads, p->m, p->v, kParams, lr, beta1, beta2, eps, bc1, bc2, weight_decay, p->img);
-    p->img_stale = false;
     const cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? DISCO_OK : mcuda(e, "adam");
 }

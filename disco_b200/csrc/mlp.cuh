@@ -45,8 +45,7 @@ struct disco_mlp {
     float* loss = nullptr;     // device scalar
     float* part = nullptr;     // one call's partial gradients, dpre and dy
     int64_t cap = 0;           // rows that `part` holds
-    unsigned char* img = nullptr;      // BF16 tiles of the weights (mlp.cu)
-    bool img_stale = true;             // the weights are newer than those
+    unsigned char* img = nullptr;      // BF16 tiles of the weights (mlp.cu), always those of params
     int sms = 0;
     int64_t step = 0;
     int* status = nullptr;

@@ -91,3 +91,37 @@ def test_row_counts_and_unaligned_rows(n):
     m.grad(Xd, Td)
     assert np.array_equal(m.grads(), g + g)
     assert torch.equal(m.forward(Xd), m.forward(torch.from_numpy(X).cuda()))
+
+
+def test_captured_forward_and_new_weights():
+    """A captured forward replays with the weights of the moment, whoever set
+    them (set_params, Adam), and a capture that is not replayed leaves calls
+    outside it alone: each result equals, to the bit, an eager one of a model
+    that was given the same weights."""
+    torch = pytest.importorskip("torch")
+    X, T = (torch.from_numpy(a).cuda() for a in _data(300))
+    m, fresh = MLP(seed=7), MLP(seed=8)
+    m.forward(X)
+    m.grad(X, T)
+    half = (m.params() * 0.5).astype(np.float32)
+
+    def eager(p):
+        fresh.set_params(p)
+        return fresh.forward(X)
+    m.set_params(half)
+    stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, stream=stream):
+        Y = m.forward(X)
+    assert torch.equal(m.forward(X), eager(half))            # the capture has not run
+    for p in (half, half * 3.0):
+        m.set_params(p)
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(Y, eager(p))
+    m.grad(X, T)
+    m.adam(lr=1e-2)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(Y, eager(m.params()))
+    del graph
