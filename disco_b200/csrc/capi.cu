@@ -47,12 +47,12 @@ struct disco_plan {
     int32_t near_cap = 0;
     std::vector<double> loop_evals;          // per input loop: segments or loopons
     disco_plan_stats stats;
-    // the sum by cells: its shape for the last atom count, and whether this
-    // plan holds the device's scratch pool (both set by execute)
+    // the sum by cells: its shape for the last atom count, and the context
+    // whose scratch pool this plan holds (0: none); both set by execute
     std::mutex tree_mutex;
     int64_t tree_n[2] = { -1, -1 };
     disco::TreeShape tree[2];
-    bool tree_pool = false;
+    unsigned long long tree_pool = 0;
 };
 
 namespace {
@@ -106,7 +106,7 @@ void free_plan(disco_plan* p)
     if (!p) return;
     if (p->own && p->block && p->pooled) cudaFreeAsync(p->block, p->stream);
     else if (p->own && p->block) cudaFree(p->block);
-    if (p->tree_pool) disco::scratch_release(p->device);
+    if (p->tree_pool) disco::scratch_release(p->device, p->tree_pool);
     delete p;
 }
 
@@ -127,10 +127,7 @@ disco::TreeShape plan_tree(disco_plan* p, int k, int64_t n, cudaStream_t s)
         p->tree[k] = disco::tree_shape(p->tables[k], n, p->box, p->opt.images);
         p->tree_n[k] = n;
     }
-    if (p->tree[k].use && !p->tree_pool) {
-        disco::scratch_retain(p->device);
-        p->tree_pool = true;
-    }
+    if (p->tree[k].use && !p->tree_pool) p->tree_pool = disco::scratch_retain(p->device);
     return p->tree[k];
 }
 
@@ -144,12 +141,14 @@ double now_s()
 
 namespace {
 
-constexpr int kMaxDevices = 64;
 constexpr uint64_t kScratchKeep = 32ull << 20, kScratchKeepPlans = 1024ull << 20;
+
+// The scratch pools, one per device and context (two contexts of a device do
+// not share one; the memory of a context that is gone went with it, and its
+// entry stays).
+struct ScratchPool { int device; unsigned long long ctx; cudaMemPool_t pool; int plans; };
 std::mutex g_scratch_mutex;
-cudaMemPool_t g_scratch[kMaxDevices] = {};
-unsigned long long g_scratch_ctx[kMaxDevices] = {};     // the context each pool was made in
-int g_scratch_plans[kMaxDevices] = {};
+std::vector<ScratchPool> g_scratch;
 
 // Idle non-blocking streams of host calls, at most four: making and destroying
 // one costs 0.12 ms, more than such a call's copies.
@@ -161,11 +160,38 @@ std::vector<IdleStream> g_idle;
 using CtxGetCurrentFn = CUresult (*)(CUcontext*);
 using CtxGetIdFn = CUresult (*)(CUcontext, unsigned long long*);
 
-void scratch_keep(int device, uint64_t bytes)
+void scratch_keep(cudaMemPool_t pool, uint64_t bytes)
 {
-    if (!g_scratch[device]) return;
-    if (cudaMemPoolSetAttribute(g_scratch[device], cudaMemPoolAttrReleaseThreshold, &bytes) != cudaSuccess)
-        cudaGetLastError();
+    if (cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &bytes) != cudaSuccess) cudaGetLastError();
+}
+
+// Identifier of the calling thread's context; a thread that has none yet gets
+// the device's primary one.
+unsigned long long bound_context_id()
+{
+    unsigned long long id = disco::current_context_id();
+    if (id == 0 && cudaFree(nullptr) == cudaSuccess) id = disco::current_context_id();
+    return id;
+}
+
+// The entry of the calling thread's context, made if there is none (null when
+// that fails); the mutex is held.
+ScratchPool* scratch_entry(int device)
+{
+    const unsigned long long ctx = bound_context_id();
+    if (ctx == 0) return nullptr;
+    for (ScratchPool& p : g_scratch)
+        if (p.device == device && p.ctx == ctx) return &p;
+    cudaMemPoolProps props;
+    std::memset(&props, 0, sizeof(props));
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = device;
+    cudaMemPool_t pool = nullptr;
+    if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+    scratch_keep(pool, kScratchKeep);
+    g_scratch.push_back({ device, ctx, pool, 0 });
+    return &g_scratch.back();
 }
 
 cudaError_t take_stream(int device, IdleStream& out)
@@ -223,22 +249,9 @@ unsigned long long disco::current_context_id()
 
 cudaMemPool_t disco::scratch_pool(int device)
 {
-    if (device < 0 || device >= kMaxDevices) return nullptr;
-    const unsigned long long ctx = current_context_id();
     std::lock_guard<std::mutex> lock(g_scratch_mutex);
-    if (!g_scratch[device] || ctx == 0 || ctx != g_scratch_ctx[device]) {
-        cudaMemPoolProps props;
-        std::memset(&props, 0, sizeof(props));
-        props.allocType = cudaMemAllocationTypePinned;
-        props.location.type = cudaMemLocationTypeDevice;
-        props.location.id = device;
-        cudaMemPool_t p = nullptr;
-        if (cudaMemPoolCreate(&p, &props) != cudaSuccess) { cudaGetLastError(); return nullptr; }
-        g_scratch[device] = p;
-        g_scratch_ctx[device] = ctx;
-        scratch_keep(device, g_scratch_plans[device] > 0 ? kScratchKeepPlans : kScratchKeep);
-    }
-    return g_scratch[device];
+    const ScratchPool* p = scratch_entry(device);
+    return p ? p->pool : nullptr;
 }
 
 cudaError_t disco::scratch_alloc(void** p, size_t bytes, cudaStream_t s)
@@ -250,21 +263,31 @@ cudaError_t disco::scratch_alloc(void** p, size_t bytes, cudaStream_t s)
     return cudaMallocAsync(p, bytes, s);
 }
 
-void disco::scratch_retain(int device)
+unsigned long long disco::scratch_retain(int device)
 {
-    if (device < 0 || device >= kMaxDevices) return;
     std::lock_guard<std::mutex> lock(g_scratch_mutex);
-    if (++g_scratch_plans[device] == 1 && current_context_id() == g_scratch_ctx[device])
-        scratch_keep(device, kScratchKeepPlans);
+    ScratchPool* p = scratch_entry(device);
+    if (!p) return 0;
+    if (++p->plans == 1) scratch_keep(p->pool, kScratchKeepPlans);
+    return p->ctx;
 }
 
-void disco::scratch_release(int device)
+void disco::scratch_release(int device, unsigned long long ctx)
 {
-    if (device < 0 || device >= kMaxDevices) return;
     std::lock_guard<std::mutex> lock(g_scratch_mutex);
-    if (--g_scratch_plans[device] > 0 || !g_scratch[device] || current_context_id() != g_scratch_ctx[device]) return;
-    scratch_keep(device, kScratchKeep);
-    if (cudaMemPoolTrimTo(g_scratch[device], kScratchKeep) != cudaSuccess) cudaGetLastError();
+    for (ScratchPool& p : g_scratch) {
+        if (p.device != device || p.ctx != ctx || --p.plans > 0) continue;
+        // a pool of a context that is gone must not be touched; the plan's device
+        // need not be the current one
+        int current = device;
+        const bool other = cudaGetDevice(&current) == cudaSuccess && current != device;
+        if (other) cudaSetDevice(device);
+        if (bound_context_id() == ctx) {
+            scratch_keep(p.pool, kScratchKeep);
+            if (cudaMemPoolTrimTo(p.pool, kScratchKeep) != cudaSuccess) cudaGetLastError();
+        }
+        if (other) cudaSetDevice(current);
+    }
 }
 
 void disco::set_last_error(const std::string& msg) { store_error(msg.c_str()); }

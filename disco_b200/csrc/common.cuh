@@ -19,15 +19,16 @@ void set_last_error(const char* msg);
 // be read (a device reset gives the device a new one).
 unsigned long long current_context_id();
 
-// Stream-ordered scratch memory, one pool per device (null where none could be
-// made).  32 MB (one block of the driver's) stay reserved in it, and up to 1 GB
-// while a plan that has used it lives (retain / release): the default pool gives
+// Stream-ordered scratch memory, one pool per device and context (null where
+// none could be made).  32 MB (one block of the driver's) stay reserved in it, and up to 1 GB
+// while a plan that has used it lives (retain gives the context whose pool it
+// is, release takes it): the default pool gives
 // its memory back at every synchronisation, and a call after one then pays for
 // mapping it again (0.2 to 0.4 ms; 13.5 M atoms, 640 MB of scratch: 5.8 ms of an
 // execute of 79).
 cudaMemPool_t scratch_pool(int device);
-void scratch_retain(int device);
-void scratch_release(int device);
+unsigned long long scratch_retain(int device);
+void scratch_release(int device, unsigned long long ctx);
 int plan_create_on(const disco_loop* loops, int32_t nloops, const double box[3], const disco_options* opt,
                    int64_t max_atoms, cudaStream_t s, disco_plan** out);
 int batch_plan_create_on(const disco_sample* samples, int32_t nsamples, const disco_options* opt, cudaStream_t s,

@@ -5,12 +5,14 @@ formatting, fixed, 8 decimals): random positions, exact ties (odd multiples of
 magnitudes; the short-buffer error; and the chain finalize_resident ->
 format_atoms on a matter-step workload."""
 import ctypes
+import threading
 
 import numpy as np
 import pytest
 
 import oracle as O
 from disco_b200 import _capi as C
+from disco_b200 import backend as B
 from disco_b200 import prismatic as P
 from disco_b200 import workloads as W
 
@@ -127,3 +129,34 @@ def test_lengths_at_powers_of_ten_and_any_output_address():
         b = bytes(buf.cpu().numpy())
         assert b[off:off + len(want)] == want
         assert set(b[:off]) <= {7} and set(b[off + len(want):]) == {7}
+
+
+def test_fresh_threads_share_one_scratch_pool():
+    """Calls whose scratch is the first thing that a host thread asks the GPU
+    for use the pool of the threads before them: device memory does not shrink
+    from thread to thread (a pool of its own holds 32 MB or more), while a plan
+    that sums by cells keeps its scratch."""
+    w = W.quadrupole(cells=40)
+    pos = torch.tensor(np.stack([w.x, w.y, w.z]), dtype=torch.float64, device="cuda")
+    u = torch.zeros_like(pos)
+    plan = B.Plan(w.loops, w.box, images=w.images, nu=w.nu, max_atoms=w.n)
+    lib = C.cuda_lib()
+    text = torch.empty(64 * w.n, dtype=torch.uint8, device="cuda")
+    stream = torch.cuda.current_stream().cuda_stream
+    status, free = [], []
+
+    def call():
+        got = ctypes.c_int64()
+        status.append(lib.disco_b200_format_atoms(0, b"Fe", pos[0].data_ptr(), pos[1].data_ptr(), pos[2].data_ptr(),
+                                                  w.n, text.data_ptr(), text.numel(), ctypes.byref(got),
+                                                  ctypes.c_void_p(stream)))
+    for _ in range(6):
+        plan.execute(pos, u)
+        t = threading.Thread(target=call)
+        t.start()
+        t.join()
+        torch.cuda.synchronize()
+        free.append(torch.cuda.mem_get_info()[0])
+    plan.close()
+    assert status == [C.DISCO_OK] * 6
+    assert free[0] - free[-1] < 16 << 20
