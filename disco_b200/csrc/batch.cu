@@ -312,7 +312,7 @@ int launch_batch_policy(const disco::BatchArgs& a, int grid, int split, cudaStre
     case 4: kern = batch_kernel<Policy, 4>; break;
     default: kern = batch_kernel<Policy, 8>; break;
     }
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemLimit);
     if (e != cudaSuccess) { err = cudaGetErrorString(e); return DISCO_ECUDA; }
     kern<<<grid, kBatchThreads, smem, s>>>(a);
     e = cudaGetLastError();
@@ -333,7 +333,7 @@ int occupancy_of(int split, size_t smem)
     default: kern = batch_kernel<Policy, 8>; break;
     }
     int per_sm = 0;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemLimit) != cudaSuccess ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kBatchThreads, smem) != cudaSuccess)
         return 0;
     return per_sm;
@@ -423,7 +423,7 @@ int batch_create(const disco_sample* samples, int32_t nsamples, const disco_opti
     if (stage < 16 * 1024u || stage > 100 * 1024u) return bfail(DISCO_EINVAL, "stage_kb must be in 16..100");
     const int stages = o.stages > 0 ? o.stages : 2;
     if (stages < 2 || stages > kMaxStages) return bfail(DISCO_EINVAL, "stages must be in 2..4");
-    if (kSmemHeader + (size_t)stages * stage > 227u * 1024u)
+    if (kSmemHeader + (size_t)stages * stage > kSmemLimit)
         return bfail(DISCO_EINVAL, "stages x stage_kb exceeds the 227 KB of shared memory of a CTA");
     for (int s = 0; s < nsamples; ++s) {
         const disco_sample& sm = samples[s];

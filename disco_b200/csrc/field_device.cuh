@@ -17,6 +17,10 @@ constexpr int kMaxLinePiece = 256;         // segments per piece
 constexpr int kMaxLooponPiece = 960;       // loopons per piece (fits a 48 KB stage)
 constexpr uint32_t kResidentMax = 110u * 1024u;
 constexpr uint32_t kStageMax = 48u * 1024u;
+// Dynamic shared memory of a CTA.  The kernels' attribute is set to this, never
+// to one launch's size: it holds for the whole process, and another thread may
+// launch the same kernel with a larger table in between.
+constexpr uint32_t kSmemLimit = 227u * 1024u;
 constexpr uint32_t kSmemHeader = 128;      // mbarriers at the start of shared memory
 
 // Image img of the (2 images + 1)^3 cube, kk fastest (Code/backend_cpu.cpp:51-53).

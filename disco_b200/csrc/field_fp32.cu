@@ -165,7 +165,7 @@ template <class Policy, int S>
 int launch_one_f(const FieldArgs& a, int sm_count, size_t smem, cudaStream_t stream, std::string& err)
 {
     auto kern = field_kernel<Policy, S>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemLimit);
     if (e != cudaSuccess) { err = cudaGetErrorString(e); return DISCO_ECUDA; }
     int per_sm = 0;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads, smem);

@@ -66,6 +66,7 @@ namespace {
 constexpr int kOrders = 9;
 constexpr int kOrderQ[kOrders] = { 9, 10, 11, 12, 13, 15, 17, 19, 21 };
 constexpr double kOrderTheta[kOrders] = { 18.0, 13.2, 10.2, 8.2, 6.9, 5.1, 4.15, 3.55, 3.1 };
+constexpr int kMaxRefine = 8;                  // final cells per axis in a cell of the last level, at most
 constexpr int kMaxFinalQ = 13;                 // the atoms' cells hold three components in shared memory
 constexpr int kWarps = 4;                      // warps per CTA of the tile kernels
 constexpr int kMaxCells = 1 << 18;
@@ -1411,7 +1412,7 @@ TreeShape tree_shape(const HostTable& T, int64_t n, const double box[3], int ima
         int levels = 1, end = -1;
         for (int b = st[p].prev; b >= 0; b = st[b].prev) ++levels;
         if (levels + 6 > TreeShape::kMaxLevels) continue;
-        for (int r = 1; r <= 8; r *= 2) {
+        for (int r = 1; r <= kMaxRefine; r *= 2) {
             const double cells = st[p].cells * r * r * r;
             if (cells > (line ? kMaxCells : 32768)) break;
             const int o = order_for((theta - 1.0) * r + 1.0);
@@ -1485,30 +1486,45 @@ TreeShape tree_shape(const HostTable& T, int64_t n, const double box[3], int ima
 
 namespace {
 
+// Shared memory of one CTA for parent cells of qp nodes per axis (and rz final
+// cells along z).
+template <int QC>
+constexpr size_t down_smem(int qp)
+{
+    return ((size_t)(qp > QC ? QC * qp * qp : QC * QC * QC) + (size_t)QC * QC * qp + 3 * (size_t)qp * QC) * sizeof(double);
+}
+template <int QC>
+constexpr size_t leaf_smem(int qp, int rz)
+{
+    return ((size_t)QC * QC * padded(QC) + padded(QC * QC * qp) +
+            padded(QC * qp * qp > 8 * 64 ? QC * qp * qp : 8 * 64) + (size_t)(2 + rz) * qp * padded(QC)) * sizeof(double);
+}
+
+// A kernel's limit of dynamic shared memory holds for the whole process, so it
+// is set to the largest size of any shape, never to one call's: another thread
+// may launch a larger one in between.
 template <int QC>
 cudaError_t down(const TreeArgs& a, int t, int cells, cudaStream_t s)
 {
-    const int qp = a.lv[t - 1].q;
-    const size_t smem = ((size_t)std::max(QC * qp * qp, QC * QC * QC) + (size_t)QC * QC * qp + 3 * (size_t)qp * QC) *
-                        sizeof(double);
+    constexpr size_t most = down_smem<QC>(kMaxQ);
+    static_assert(most <= kSmemLimit, "one CTA's shared memory");
     const cudaError_t e = cudaFuncSetAttribute(tree_down_kernel<QC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               (int)smem);
+                                               (int)most);
     if (e != cudaSuccess) return e;
-    tree_down_kernel<QC><<<dim3((unsigned)cells, 3), 256, smem, s>>>(a, t);
+    tree_down_kernel<QC><<<dim3((unsigned)cells, 3), 256, down_smem<QC>(a.lv[t - 1].q), s>>>(a, t);
     return cudaGetLastError();
 }
 
 template <int QC>
 cudaError_t leaf(const TreeArgs& a, cudaStream_t s)
 {
-    const int qp = a.lv[a.levels - 1].q;
-    constexpr int QP = padded(QC);
-    const size_t smem = ((size_t)QC * QC * QP + padded(QC * QC * qp) + padded(std::max(QC * qp * qp, 8 * 64)) +
-                         (size_t)(2 + a.rf[2]) * qp * QP) * sizeof(double);
+    constexpr size_t most = leaf_smem<QC>(kMaxQ, kMaxRefine);
+    static_assert(most <= kSmemLimit, "one CTA's shared memory");
     const cudaError_t e = cudaFuncSetAttribute(tree_leaf_kernel<QC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               (int)smem);
+                                               (int)most);
     if (e != cudaSuccess) return e;
-    tree_leaf_kernel<QC><<<dim3((unsigned)(a.cells_f / a.rf[2]), 3), 256, smem, s>>>(a);
+    tree_leaf_kernel<QC><<<dim3((unsigned)(a.cells_f / a.rf[2]), 3), 256, leaf_smem<QC>(a.lv[a.levels - 1].q, a.rf[2]),
+                           s>>>(a);
     return cudaGetLastError();
 }
 

@@ -7,6 +7,8 @@ and the plain sum itself is within 1e-14 A of the oracle on these sizes: 2e-14
 A per loop, plus 2e-14 A.  Loopons: the plain sum over 1e4 to 1e6 terms is
 within about 1e-13 A of the reference's, and the squares' interpolation is of
 the line's size per loop: 2e-14 A per loop, plus 2e-13 A."""
+import threading
+
 import numpy as np
 import pytest
 
@@ -160,3 +162,38 @@ def test_loopons_off_one_plane():
     pos = _positions(torch, w)
     a, b = _sum(torch, w, pos, 1), _sum(torch, w, pos, 0)
     assert float((a - b).abs().max()) <= _tolerance(w)
+
+
+def test_threads_with_plans_of_different_shapes():
+    """Host threads, each with a plan, a stream and an atom count of its own, so
+    that kernels of one instance are launched with different shared memory at
+    the same time: every call succeeds and gives the thread's own sum."""
+    torch = pytest.importorskip("torch")
+    ws = [W.fcc_random(cells=c, n_circles=4, n_hex=2, n_rect=2, images=im) for c, im in ((24, 2), (36, 2), (30, 3), (20, 4))]
+    ws += [_prismatic(24, 2, 8.0, 20.0), _prismatic(30, 4, 12.0, 30.0)]
+    poss = [_positions(torch, w) for w in ws]
+    want = [_sum(torch, w, p, 0) for w, p in zip(ws, poss)]
+    failures = []
+
+    def go(w, pos, one):
+        try:
+            stream = torch.cuda.Stream()
+            plan = B.Plan(w.loops, w.box, images=w.images, nu=w.nu, max_atoms=w.n)
+            u = torch.zeros_like(pos)
+            torch.cuda.synchronize()
+            for _ in range(60):
+                with torch.cuda.stream(stream):
+                    u.zero_()
+                plan.execute(pos, u, stream)
+            stream.synchronize()
+            if not torch.equal(u, one):
+                failures.append("another sum")
+            plan.close()
+        except Exception as e:
+            failures.append(repr(e))
+    threads = [threading.Thread(target=go, args=a) for a in list(zip(ws, poss, want)) * 2]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert failures == []
