@@ -249,6 +249,7 @@ unsigned long long disco::current_context_id()
 
 cudaMemPool_t disco::scratch_pool(int device)
 {
+    OutsideCapture relaxed;
     std::lock_guard<std::mutex> lock(g_scratch_mutex);
     const ScratchPool* p = scratch_entry(device);
     return p ? p->pool : nullptr;
@@ -256,6 +257,7 @@ cudaMemPool_t disco::scratch_pool(int device)
 
 cudaError_t disco::scratch_alloc(void** p, size_t bytes, cudaStream_t s)
 {
+    OutsideCapture relaxed;
     int dev = 0;
     cudaMemPool_t pool = cudaGetDevice(&dev) == cudaSuccess ? scratch_pool(dev) : nullptr;
     if (pool && cudaMallocFromPoolAsync(p, bytes, pool, s) == cudaSuccess) return cudaSuccess;
@@ -265,6 +267,7 @@ cudaError_t disco::scratch_alloc(void** p, size_t bytes, cudaStream_t s)
 
 unsigned long long disco::scratch_retain(int device)
 {
+    OutsideCapture relaxed;
     std::lock_guard<std::mutex> lock(g_scratch_mutex);
     ScratchPool* p = scratch_entry(device);
     if (!p) return 0;
@@ -274,6 +277,7 @@ unsigned long long disco::scratch_retain(int device)
 
 void disco::scratch_release(int device, unsigned long long ctx)
 {
+    OutsideCapture relaxed;
     std::lock_guard<std::mutex> lock(g_scratch_mutex);
     for (ScratchPool& p : g_scratch) {
         if (p.device != device || p.ctx != ctx || --p.plans > 0) continue;

@@ -19,6 +19,17 @@ void set_last_error(const char* msg);
 // be read (a device reset gives the device a new one).
 unsigned long long current_context_id();
 
+// While this lives, the thread may allocate and make or trim pools for streams
+// that are not being captured although another stream is (by default such a
+// call fails and ends that capture).
+struct OutsideCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    OutsideCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~OutsideCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    OutsideCapture(const OutsideCapture&) = delete;
+    OutsideCapture& operator=(const OutsideCapture&) = delete;
+};
+
 // Stream-ordered scratch memory, one pool per device and context (null where
 // none could be made).  32 MB (one block of the driver's) stay reserved in it, and up to 1 GB
 // while a plan that has used it lives (retain gives the context whose pool it

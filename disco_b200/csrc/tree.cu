@@ -1560,6 +1560,7 @@ int launch_tree(const FieldArgs& f, const HostTable& T, const TreeShape& S, int 
                 cudaStream_t s, bool* ran, std::string& err)
 {
     *ran = false;
+    OutsideCapture relaxed;
     TreeArgs a;
     std::memset(&a, 0, sizeof(a));
     a.f = f;

@@ -7,6 +7,9 @@ and the plain sum itself is within 1e-14 A of the oracle on these sizes: 2e-14
 A per loop, plus 2e-14 A.  Loopons: the plain sum over 1e4 to 1e6 terms is
 within about 1e-13 A of the reference's, and the squares' interpolation is of
 the line's size per loop: 2e-14 A per loop, plus 2e-13 A."""
+import os
+import subprocess
+import sys
 import threading
 
 import numpy as np
@@ -197,3 +200,37 @@ def test_threads_with_plans_of_different_shapes():
     for t in threads:
         t.join()
     assert failures == []
+
+
+def test_beside_a_capture():
+    """A call on one stream while another stream is being captured: its first,
+    which makes the scratch pool, a repeated one, and the plan's end.  The
+    capture goes on, and both results are right."""
+    torch = pytest.importorskip("torch")
+    code = """
+import sys
+import numpy as np, torch
+from disco_b200 import backend as B, workloads as W
+w = W.quadrupole(cells=40)
+pos = torch.tensor(np.stack([w.x, w.y, w.z]), device="cuda")
+plan = B.Plan(w.loops, w.box, images=w.images, nu=w.nu, max_atoms=w.n)
+u, a = torch.zeros_like(pos), torch.zeros(4, device="cuda")
+side, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+torch.cuda.synchronize()
+with torch.cuda.graph(graph, stream=torch.cuda.Stream()):
+    a += 1
+    for _ in range(2):
+        plan.execute(pos, u, side)
+    a += 1
+graph.replay()
+torch.cuda.synchronize()
+assert a.tolist() == [2.0] * 4
+v = torch.zeros_like(pos)
+for _ in range(2):
+    plan.execute(pos, v)
+torch.cuda.synchronize()
+assert float(u.abs().max()) > 0 and torch.equal(u, v)
+"""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", code], cwd=root, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
