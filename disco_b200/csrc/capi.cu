@@ -617,9 +617,12 @@ int disco_b200_displace(const disco_atoms* atoms, const disco_loop* loops, int32
     IdleStream is = { nullptr, 0, 0 };
     cudaEvent_t ev[2] = { nullptr, nullptr };
     auto cleanup = [&]() {
-        disco_b200_plan_destroy(plan);
         if (block && pooled) cudaFreeAsync(block, is.stream);
         else if (block) cudaFree(block);
+        // the pool gives back what it holds above its 32 MB when it is waited for
+        // or trimmed (by the plan's end): a large call leaves neither to its caller
+        if (pooled && atoms_at + plan->bytes > (8ull << 20)) cudaStreamSynchronize(is.stream);
+        disco_b200_plan_destroy(plan);
         give_stream(is, healthy);
         for (auto& x : ev) if (x) cudaEventDestroy(x);
     };

@@ -512,18 +512,25 @@ uint64_t splitmix(uint64_t& st)
 
 // Device buffers of one learned call, released on every exit path, in the
 // order of its stream (cudaMalloc and cudaFree map and unmap memory, 0.3 ms
-// each, and wait for the device).
+// each, and wait for the device).  The pool gives back what it holds above its
+// 32 MB at a wait, so large buffers are waited for.
 struct Bufs {
     cudaStream_t s;
     std::vector<void*> ptrs;
+    size_t total = 0;
     explicit Bufs(cudaStream_t stream) : s(stream) {}
-    ~Bufs() { for (void* p : ptrs) cudaFreeAsync(p, s); }
+    ~Bufs()
+    {
+        for (void* p : ptrs) cudaFreeAsync(p, s);
+        if (total > (8ull << 20)) cudaStreamSynchronize(s);
+    }
     template <class T>
     cudaError_t get(T** out, size_t count)
     {
         void* p = nullptr;
-        const cudaError_t e = disco::scratch_alloc(&p, std::max<size_t>(count, 1) * sizeof(T), s);
-        if (e == cudaSuccess) ptrs.push_back(p);
+        const size_t bytes = std::max<size_t>(count, 1) * sizeof(T);
+        const cudaError_t e = disco::scratch_alloc(&p, bytes, s);
+        if (e == cudaSuccess) { ptrs.push_back(p); total += bytes; }
         *out = static_cast<T*>(p);
         return e;
     }

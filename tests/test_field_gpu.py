@@ -229,3 +229,17 @@ def test_atoms_on_loop_planes_fp32c_and_batched():
     us, _ = B.batch_gpu([w, w], C.DISCO_FP64)
     for u in us:
         assert np.abs(np.stack(u, 1) - ref).max() <= TOL
+
+
+def test_large_host_call_gives_its_memory_back():
+    """A host call returns with the device memory that it found free: what its
+    pool keeps is at most one block of the driver's (32 MB), held already by a
+    small call before."""
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(0)
+    w = W.quadrupole(cells=10, radius=8.0, eps=0.0365)
+    _gpu(w)
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    _gpu(w, atoms=[(rng.random(2000003) - 0.5) * w.box[0] for _ in range(3)])
+    assert free - torch.cuda.mem_get_info()[0] < 1 << 20

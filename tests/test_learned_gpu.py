@@ -211,3 +211,23 @@ def test_learned_displace_falls_back_and_matches_exact():
     net = torch.zeros_like(d)
     Ln.far_apply(m, norm, d, loops, w.box, u=net)
     assert (u2 - near - net).abs().max().item() <= 1e-9 + 1e-6 * net.abs().max().item()
+
+
+def test_large_check_gives_its_memory_back():
+    """A call whose check takes over 100 MB of scratch returns with the device
+    memory that it found free, but for one block of the pool's (32 MB, which a
+    small call before has taken)."""
+    loops, box, pos = _small(nloops=8, n=300007)
+    mlp = Ln.MLP(seed=1)
+    isd = np.ones(16, dtype=np.float32)
+    norm = Ln.FarNorm(np.zeros(16, dtype=np.float32), isd, 1.0, 2, 2)
+
+    def call(n):
+        d = torch.tensor(pos[:, :n].copy(), dtype=torch.float64, device="cuda")
+        u = torch.zeros_like(d)
+        torch.cuda.synchronize()
+        free = torch.cuda.mem_get_info()[0]
+        Ln.learned_displace(mlp, norm, d, u, loops, box, 0.34, check_fraction=1.0)
+        return free - torch.cuda.mem_get_info()[0]
+    call(1000)
+    assert call(pos.shape[1]) < 1 << 20
