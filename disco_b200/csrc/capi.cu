@@ -124,7 +124,7 @@ disco::TreeShape plan_tree(disco_plan* p, int k, int64_t n, cudaStream_t s)
     if (cap != cudaStreamCaptureStatusNone) return none;
     std::lock_guard<std::mutex> lock(p->tree_mutex);
     if (p->tree_n[k] != n) {
-        p->tree[k] = disco::tree_shape(p->tables[k], n, p->box, p->opt.images);
+        p->tree[k] = disco::tree_shape(p->tables[k], n, p->box, p->opt.images, p->sm_count);
         p->tree_n[k] = n;
     }
     if (p->tree[k].use && !p->tree_pool) p->tree_pool = disco::scratch_retain(p->device);

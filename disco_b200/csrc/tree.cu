@@ -59,6 +59,8 @@
 
 namespace disco {
 
+int choose_split(int64_t n, int nimg, int resident_ctas);
+
 namespace {
 
 // ---- orders ----------------------------------------------------------------------------
@@ -1229,6 +1231,43 @@ const Depth& depth_at(const Root& r, double cut)
     return r.depth[k];
 }
 
+// What the choice below settled on, in FP64 operations.
+struct Choice {
+    double cost, node, near, fill;      // all of it; the nodes; the near pass, and the lanes it starts for one it uses
+    double node_lanes, sources;         // lanes of the node kernel; sources that a warp of the near pass looks at
+    double node_scans;                  // (warp, source) pairs of the node kernel
+    int near_split, levels;
+};
+
+// Whether the chosen cells beat the plain sum.  The operation counts rank cells
+// against cells; against the plain sum, what they leave out decides, so both
+// sides are turned into times: the plain kernel's rounds of tiles; for the
+// cells the warps that are missing to fill the GPU (16 an SM), the sources
+// looked at, and the launches.  The weights are fitted to 414 random plans (500
+// to 2.6 M atoms, 1 to 256 loops, 0 to 4 shells) on both sides of the line.  Of
+// 190 that the operation counts alone sent to the cells 29 lost by it, up to 2.5
+// times (16 loopon loops of R 6, 2 000 atoms, +-4: 7.2 ms plain, 17.7 by cells);
+// by this rule 4 lose, by 1 to 4 and 12 %, and of the gains that it passes up one
+// is above 10 % (22 %: 32 loopon loops of R 7, 1.1 M atoms, no images).
+bool worth_cells(const Choice& c, bool line, int64_t n, double terms, double nimg, double e64, double us, int sm_count)
+{
+    const int S = choose_split(n, (int)nimg, sm_count * 2);
+    const double tiles = std::ceil((double)n * S / kThreads);
+    const double rounds = 0.5 * std::ceil(tiles / sm_count);          // two CTAs an SM; one alone has all of it
+    const double plain = rounds * 2.0 * sm_count * kThreads * std::ceil(nimg / S) * terms * e64;
+    const double full = 16.0 * sm_count;
+    const double near_warps = (double)n * c.near_split / 32.0 * c.fill;
+    const double node_part = c.node * (1.0 + (line ? 0.92 : 0.21) * full / (c.node_lanes / 32.0));
+    const double near_part = c.near * (1.0 + (line ? 0.22 : 0.47) * full / near_warps);
+    const double rest = std::max(0.0, c.cost - c.node - c.near * c.fill);
+    if (line)
+        return 30.0 * us + 0.573 * node_part + 1.05 * near_part + 1.06 * rest + 38.0 * us * c.levels <
+               0.97 * (18.0 * us + 1.054 * plain);
+    return 120.0 * us + 1.129 * node_part + 0.877 * near_part + 0.758 * rest +
+               (0.00118 * c.node_scans + 0.00116 * near_warps * c.sources) * us <
+           1.05 * (10.0 * us + 0.938 * plain);
+}
+
 } // namespace
 
 void append_tree_pieces(HostTable& T)
@@ -1266,7 +1305,7 @@ void append_tree_pieces(HostTable& T)
     T.bytes.insert(T.bytes.end(), s, s + T.tree.size() * sizeof(TreePiece));
 }
 
-TreeShape tree_shape(const HostTable& T, int64_t n, const double box[3], int images)
+TreeShape tree_shape(const HostTable& T, int64_t n, const double box[3], int images, int sm_count)
 {
     TreeShape S;
     if (!T.aux_tree || T.tree.empty() || n > 0x7FFFFFFF - 64) return S;
@@ -1405,6 +1444,7 @@ TreeShape tree_shape(const HostTable& T, int64_t n, const double box[3], int ima
     };
     double best = S.direct;
     int pick = -1, pick_r = 1, pick_q = 0, pick_end = -1;
+    Choice chosen = {};
     std::vector<Step> pick_steps;
     for (int p = 0; p < (int)st.size(); ++p) {
         const double theta = kOrderTheta[st[p].o];
@@ -1421,14 +1461,16 @@ TreeShape tree_shape(const HostTable& T, int64_t n, const double box[3], int ima
             const double atoms = std::max(1.0, (double)n / cells);
             const double fill = (std::floor(atoms / 64.0) + 1.0) * 64.0 / atoms;
             std::vector<Step> steps;
-            double near = near_steps(st[p], st[p].h / r, cells, steps, end);
-            if (!line) near *= (std::floor(atoms / 16.0) + 1.0) * 16.0 / atoms;     // partly filled warps
-            const double c = st[p].cost + near + (double)n * st[p].np * 0.5 +
+            const double near = near_steps(st[p], st[p].h / r, cells, steps, end);
+            const double part = line ? 1.0 : (std::floor(atoms / 16.0) + 1.0) * 16.0 / atoms;     // partly filled warps
+            const double c = st[p].cost + near * part + (double)n * st[p].np * 0.5 +
                              3.0 * cells * ((q * qp * qp * qp + q * q * qp * qp) / r + q3 * qp) * 2.5 +
                              (double)n * 3.0 * q3 * 2.0 * std::min(fill, 64.0) + 60.0 * us + (double)n * 60.0;
             if (c < best) {
                 best = c; pick = p; pick_r = r; pick_q = o; pick_end = end;
                 pick_steps = steps;
+                chosen.near = near;
+                chosen.fill = part;
             }
         }
     }
@@ -1437,8 +1479,20 @@ TreeShape tree_shape(const HostTable& T, int64_t n, const double box[3], int ima
     std::vector<int> chain;
     for (int p = pick; p >= 0; p = st[p].prev) chain.push_back(p);
     std::reverse(chain.begin(), chain.end());
-    S.use = true;
     S.levels = (int)chain.size();
+    // far images per source of a level, and those that each lane would sum if all
+    // lanes of the GPU (16 warps an SM) shared them evenly
+    auto pairs = [&](int k) {
+        double p = 0.0;
+        for (size_t l = 0; l < roots.size(); ++l) p += (k ? st[chain[k - 1]].v[l] : nimg) - st[chain[k]].v[l];
+        return p;
+    };
+    const double gpu_lanes = 16.0 * 32.0 * sm_count;
+    double fair = 0.0;
+    for (int k = 0; k < S.levels; ++k) {
+        const double q = kOrderQ[st[chain[k]].o];
+        fair += st[chain[k]].cells * q * q * q * pairs(k) / gpu_lanes;
+    }
     for (int k = 0; k < S.levels; ++k) {
         const State& s = st[chain[k]];
         for (int d = 0; d < 3; ++d) S.m[k][d] = m0[d] << s.a;
@@ -1449,13 +1503,20 @@ TreeShape tree_shape(const HostTable& T, int64_t n, const double box[3], int ima
         S.eq[k] = s.eq;
         // lanes per node: many images per source for each lane, or their uneven
         // shares idle lanes (BCC 61 x 47 x 33, 9 loops, +-3: 8.69 ms with 6 images
-        // a lane, 8.27 with 48, 8.81 with one lane everywhere)
-        double per = 0.0;
-        for (size_t l = 0; l < roots.size(); ++l)
-            per += ((k ? st[chain[k - 1]].v[l] : nimg) - s.v[l]) / (double)roots.size();
+        // a lane, 8.27 with 48, 8.81 with one lane everywhere); fewer where one
+        // lane's chain would be longer than an even share of all levels' (32
+        // loops of R 13, 11 206 atoms, +-2: 9.68 ms without, 5.81 with)
+        const double per = pairs(k) / (double)roots.size();
+        const int q3 = S.q[k] * S.q[k] * S.q[k];
         int split = 1;
-        if (line) while (split < 32 && per >= 48.0 * split) split *= 2;
-        else while (split < 8 && s.cells * S.q[k] * S.q[k] * S.q[k] * split < 300000.0) split *= 2;
+        if (line) {
+            while (split < 32 && per >= 48.0 * split) split *= 2;
+            while (split < 32 && per >= 4.0 * split && pairs(k) / split > 1.5 * fair) split *= 2;
+        } else {
+            while (split < 8 && s.cells * q3 * split < 300000.0) split *= 2;
+        }
+        chosen.node_lanes += s.cells * q3 * split;
+        chosen.node_scans += s.cells * q3 * split / 32.0 * s.np;
         S.split[k] = split;
     }
     S.total = S.levels;
@@ -1479,6 +1540,13 @@ TreeShape tree_shape(const HostTable& T, int64_t n, const double box[3], int ima
     const double per_atom = st[pick].near / terms;
     if (line) while (S.near_split < 32 && per_atom >= 4.0 * S.near_split && n * S.near_split < 600000) S.near_split *= 2;
     else while (S.near_split < 8 && n * S.near_split < 600000) S.near_split *= 2;
+    chosen.cost = best;
+    chosen.node = st[pick].cost;
+    chosen.levels = S.levels;
+    chosen.near_split = S.near_split;
+    chosen.sources = st[pick].np;
+    for (int k = S.levels; k < S.total; ++k) chosen.sources += S.np[k];
+    S.use = worth_cells(chosen, line, n, terms, nimg, e64, us, sm_count);
     return S;
 }
 

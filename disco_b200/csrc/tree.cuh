@@ -35,9 +35,9 @@ struct TreeShape {
     double cost = 0.0, direct = 0.0;
 };
 
-// Picks levels, orders and cells for n atoms by their operation counts;
-// `use` is false where the plain sum over every image is cheaper.
-TreeShape tree_shape(const HostTable& T, int64_t n, const double box[3], int images);
+// Picks levels, orders and cells for n atoms by their operation counts; `use`
+// is false where the plain sum over every image is estimated to be faster.
+TreeShape tree_shape(const HostTable& T, int64_t n, const double box[3], int images, int sm_count);
 
 // Queues the sum on `stream`.  *ran is false (and nothing was queued) when the
 // scratch memory could not be had: the caller then sums directly.
