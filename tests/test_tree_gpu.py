@@ -309,3 +309,36 @@ def test_these_sizes_go_by_cells(name):
     names = _kernels(torch, lambda: plan.execute(pos, u))
     plan.close()
     assert any("tree_near_sum" in k for k in names) and not any("field_kernel" in k for k in names), names
+
+
+def test_threads_launch_one_kernel_with_other_shared_memory():
+    """Two plans whose last kernel is the same instance with 58 and 92 KB of
+    shared memory, executed over and over by eight host threads."""
+    torch = pytest.importorskip("torch")
+    plans = []
+    for radius, atoms, images in ((7.1, 38682, 2), (12.1, 14140, 3)):
+        edge = (atoms / 0.08) ** (1.0 / 3.0)
+        g = torch.Generator(device="cuda")
+        g.manual_seed(atoms)
+        pos = (torch.rand((3, atoms), dtype=torch.float64, device="cuda", generator=g) - 0.5) * edge
+        plans.append((B.Plan(_random_loops("line", 1, radius, edge, 3), (edge,) * 3, images=images, max_atoms=atoms), pos))
+    failures = []
+
+    def go(plan, pos):
+        try:
+            stream = torch.cuda.Stream()
+            u = torch.zeros_like(pos)
+            torch.cuda.synchronize()
+            for _ in range(400):
+                plan.execute(pos, u, stream)
+            stream.synchronize()
+        except Exception as e:
+            failures.append(repr(e))
+    threads = [threading.Thread(target=go, args=plans[k % 2]) for k in range(8)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for plan, _ in plans:
+        plan.close()
+    assert failures == []
