@@ -155,7 +155,8 @@ struct FieldArgs {
     // FP32 line form: the atoms with at least one near-cut (piece, image).
     // near_mode 1: the FP32 pass appends them (warp-aggregated, *near_count
     // counts past near_cap); 2: the FP64 pass visits only the listed atoms, or
-    // every atom when the list overflowed; 0: no list (every atom).
+    // every atom when the list overflowed; 0: no list (every atom).  near_mode 3
+    // (behind the sum by cells): every atom if *near_count is 0, else none.
     int32_t* near_list;
     unsigned int* near_count;
     int32_t near_cap, near_mode;

@@ -376,6 +376,8 @@ __global__ void __launch_bounds__(kThreads, Policy::kMinBlocks) field_kernel(con
     if (a.near_mode == 2 && a.near_list) {
         const unsigned c = *a.near_count;
         if (c <= (unsigned)a.near_cap) { n = c; list = a.near_list; }
+    } else if (a.near_mode == 3 && *a.near_count != 0) {
+        return;
     }
     const int64_t ntiles = (n + kAtomsPerCta - 1) / kAtomsPerCta;
     if ((int64_t)blockIdx.x >= ntiles) return;

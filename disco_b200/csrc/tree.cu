@@ -109,7 +109,8 @@ struct TreeArgs {
     int32_t near_split;
     int32_t images;
     int64_t level_cells;      // cells over all levels
-    unsigned long long* box;  // 6: ordered bits of min x, y, z and max x, y, z
+    unsigned long long* box;  // 8: ordered bits of min x, y, z and max x, y, z; sorted atoms; 0: all to the plain kernel
+    int32_t from, least;      // that is for `from` sorted atoms up to 1 / least of all
     uint64_t* near;           // [level cell][source]: packed box of near images
     int64_t near_size;
     uint8_t* occ;             // [level cell]: holds atoms
@@ -145,6 +146,7 @@ __device__ __forceinline__ bool sorted_in(const FieldArgs& f, double x, double y
 
 struct Geo {
     double lo[3], ext[3];
+    bool few;               // too few atoms to sort: every atom is left to the plain kernel
 };
 
 // The cells' grid: the bounding box of the sorted atoms, no axis thinner than
@@ -152,6 +154,7 @@ struct Geo {
 __device__ __forceinline__ Geo load_geo(const TreeArgs& a)
 {
     Geo g;
+    g.few = a.box[6] >= (unsigned long long)a.from && a.box[6] * (unsigned long long)a.least < (unsigned long long)a.f.n;
     double hi[3];
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
@@ -209,7 +212,7 @@ __device__ __forceinline__ void final_cell(const TreeArgs& a, int index, int (&c
 }
 __device__ __forceinline__ int cell_of(const TreeArgs& a, const Geo& g, double x, double y, double z)
 {
-    if (!sorted_in(a.f, x, y, z)) return a.cells_f;
+    if (g.few || !sorted_in(a.f, x, y, z)) return a.cells_f;
     int c[3];
     final_coord(a, g, x, y, z, c);
     return final_index(a, c);
@@ -220,9 +223,11 @@ __device__ __forceinline__ int cell_of(const TreeArgs& a, const Geo& g, double x
 __global__ void __launch_bounds__(256) tree_box_kernel(const TreeArgs a)
 {
     unsigned long long k[6] = { ~0ull, ~0ull, ~0ull, 0ull, 0ull, 0ull };
+    unsigned in = 0;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < a.f.n; i += (int64_t)gridDim.x * blockDim.x) {
         const double p[3] = { a.f.x[i], a.f.y[i], a.f.z[i] };
         if (!sorted_in(a.f, p[0], p[1], p[2])) continue;
+        ++in;
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
             const unsigned long long b = ord_bits(p[d]);
@@ -236,22 +241,27 @@ __global__ void __launch_bounds__(256) tree_box_kernel(const TreeArgs a)
             const unsigned long long t = __shfl_xor_sync(0xffffffffu, k[d], o);
             k[d] = d < 3 ? min(k[d], t) : max(k[d], t);
         }
-    __shared__ unsigned long long part[8][6];
-    if ((threadIdx.x & 31) == 0)
+    in = __reduce_add_sync(0xffffffffu, in);
+    __shared__ unsigned long long part[8][7];
+    if ((threadIdx.x & 31) == 0) {
         for (int d = 0; d < 6; ++d) part[threadIdx.x >> 5][d] = k[d];
+        part[threadIdx.x >> 5][6] = in;
+    }
     __syncthreads();
-    if (threadIdx.x < 6) {
+    if (threadIdx.x < 7) {
         const int d = threadIdx.x;
         unsigned long long v = part[0][d];
-        for (int w = 1; w < 8; ++w) v = d < 3 ? min(v, part[w][d]) : max(v, part[w][d]);
-        if (d < 3) atomicMin(&a.box[d], v); else atomicMax(&a.box[d], v);
+        for (int w = 1; w < 8; ++w) v = d < 3 ? min(v, part[w][d]) : d < 6 ? max(v, part[w][d]) : v + part[w][d];
+        if (d < 3) atomicMin(&a.box[d], v);
+        else if (d < 6) atomicMax(&a.box[d], v);
+        else atomicAdd(&a.box[d], v);
     }
 }
 
 __global__ void tree_init_kernel(const TreeArgs a)
 {
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
-    if (t < 6) a.box[t] = t < 3 ? ~0ull : 0ull;
+    if (t < 7) a.box[t] = t < 3 ? ~0ull : 0ull;
     for (int64_t i = t; i < a.level_cells; i += step) a.occ[i] = 0;
 }
 
@@ -407,11 +417,14 @@ __global__ void __launch_bounds__(1024) tree_scan_kernel(const TreeArgs a)
             a.occ[L.cell0 + lc] = 1;
         }
     }
+    const bool few = load_geo(a).few;
+    if (threadIdx.x == 0) a.box[7] = few ? 0 : 1;
     const int ns = a.cells_n + 1, per = (ns + 1023) / 1024;
     const int s0 = min(ns, (int)threadIdx.x * per), s1 = min(ns, s0 + per);
     const uint32_t per_tile = 32u / (uint32_t)a.near_split;
     auto tiles_of = [&](int s) {
         const uint32_t k = a.start[s < a.cells_n ? (s + 1) * a.near_rr : a.cells_f + 1] - a.start[s * a.near_rr];
+        if (s == a.cells_n && few) return 0u;                                // the plain kernel's
         return (k + per_tile - 1) / per_tile;
     };
     uint32_t mine = 0, tot;
@@ -553,6 +566,7 @@ __device__ __forceinline__ bool uses_eq(const LevelArgs& v, const TreePiece& t, 
 __global__ void __launch_bounds__(256) tree_near_kernel(const TreeArgs a)
 {
     const Geo g = load_geo(a);
+    if (g.few) return;
     const double L[3] = { a.f.Lx, a.f.Ly, a.f.Lz };
     for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < a.near_size;
          t += (int64_t)gridDim.x * blockDim.x) {
@@ -612,7 +626,7 @@ constexpr int kEqThreads = 448;                    // 21 x 21 and whole warps
 __global__ void __launch_bounds__(kEqThreads) tree_equivalent_kernel(const TreeArgs a)
 {
     const LevelArgs& v = a.lv[blockIdx.y];
-    if (v.eq == nullptr || blockIdx.x >= (unsigned)v.np) return;
+    if (v.eq == nullptr || blockIdx.x >= (unsigned)v.np || a.box[7] == 0) return;
     const int self = a.list[v.list0 + blockIdx.x];
     const TreePiece& tp = a.pieces[self];
     if (!uses_eq(v, tp, self)) return;
@@ -1642,7 +1656,7 @@ int launch_tree(const FieldArgs& f, const HostTable& T, const TreeShape& S, int 
     // scratch layout
     size_t at = 0;
     auto take = [&](size_t bytes) { const size_t o = at; at += (bytes + 255) & ~size_t(255); return o; };
-    const size_t o_box = take(6 * sizeof(unsigned long long));
+    const size_t o_box = take(8 * sizeof(unsigned long long));
     int64_t lcells = 0, tiles = 0;
     size_t o_val[TreeShape::kMaxLevels], o_eq[TreeShape::kMaxLevels], mats = 0;
     int64_t sources = 0;
@@ -1738,6 +1752,14 @@ int launch_tree(const FieldArgs& f, const HostTable& T, const TreeShape& S, int 
     a.mat = reinterpret_cast<double*>(ws + o_mat);
 
     const bool line = T.kind == kLineKind;
+    // Atoms away from the box (unwrapped trajectories) take every image in the
+    // near pass, beside the others.  Where nearly all of them are away, the nodes
+    // still work for all atoms, on cells as large as the few inside spread, and
+    // the plain kernel is faster: 864 k atoms, 5 % inside, 8 line loops, +-2: 121 ms
+    // against 137; 53 k atoms, 4 loopon loops, 5 %: 16.3 against 18.3, none: 16.3
+    // against 18.7 (line loops, none: 115 ms in the near pass, 120 plain).
+    a.from = line ? 1 : 0;
+    a.least = line ? 8 : 4;
     auto queue = [&]() -> cudaError_t {
         const int64_t sweep = std::min<int64_t>((f.n + 255) / 256, (int64_t)sm_count * 8);
         cudaError_t e;
@@ -1780,10 +1802,17 @@ int launch_tree(const FieldArgs& f, const HostTable& T, const TreeShape& S, int 
         return cudaGetLastError();
     };
     const cudaError_t e = queue();
+    int plain = DISCO_OK;
+    if (e == cudaSuccess) {
+        FieldArgs out = a.f;
+        out.near_mode = 3;
+        out.near_count = reinterpret_cast<unsigned int*>(a.box + 7);
+        plain = launch_field(out, T.kind, false, sm_count, 0, 0, s, err);
+    }
     const cudaError_t ef = cudaFreeAsync(ws, s);
     if (e != cudaSuccess) { err = cudaGetErrorString(e); return DISCO_ECUDA; }
     if (ef != cudaSuccess) { err = cudaGetErrorString(ef); return DISCO_ECUDA; }
-    return DISCO_OK;
+    return plain;
 }
 
 } // namespace disco

@@ -295,7 +295,6 @@ def test_choice_between_cells_and_the_plain_sum(method, count, radius, atoms, im
     names = _kernels(torch, lambda: plan.execute(pos, u))
     plan.close()
     assert any("tree_node" in k for k in names) == cells, names
-    assert any("field_kernel" in k for k in names) != cells, names
 
 
 @pytest.mark.parametrize("name", list(CASES))
@@ -308,7 +307,7 @@ def test_these_sizes_go_by_cells(name):
     plan = B.Plan(w.loops, w.box, images=w.images, nu=w.nu, max_atoms=w.n)
     names = _kernels(torch, lambda: plan.execute(pos, u))
     plan.close()
-    assert any("tree_near_sum" in k for k in names) and not any("field_kernel" in k for k in names), names
+    assert any("tree_near_sum" in k for k in names), names
 
 
 def test_threads_launch_one_kernel_with_other_shared_memory():
@@ -342,3 +341,52 @@ def test_threads_launch_one_kernel_with_other_shared_memory():
     for plan, _ in plans:
         plan.close()
     assert failures == []
+
+
+@pytest.mark.parametrize("name", ["fcc", "loopons"])
+@pytest.mark.parametrize("left", [0.0, 1.0 / 9.0, 1.0 / 7.0, 1.0 / 5.0, 1.0 / 3.0])
+def test_most_atoms_outside_the_cells(name, left):
+    """Unwrapped atoms: all but a share on both sides of the eighth (lines) and
+    the quarter (loopons) below which the plain kernel takes every atom, several
+    box lengths away, every second one of those with a coordinate that is not a
+    number."""
+    torch = pytest.importorskip("torch")
+    w = CASES[name]()
+    pos = _positions(torch, w)
+    n = pos.shape[1]
+    g = torch.Generator(device="cuda")
+    g.manual_seed(5)
+    away = torch.randperm(n, generator=g, device="cuda")[int(left * n):]
+    box = torch.tensor(w.box, dtype=torch.float64, device="cuda")
+    pos[:, away] += box[:, None] * torch.randint(3, 6, (3, len(away)), generator=g, device="cuda").double()
+    nan = away[::2]
+    pos[1, nan] = float("nan")
+    a, b = _sum(torch, w, pos, 1), _sum(torch, w, pos, 0)
+    fine = torch.ones(n, dtype=torch.bool, device="cuda")
+    fine[nan] = False
+    assert torch.isnan(a[:, nan]).all() and torch.isnan(b[:, nan]).all()
+    assert float((a - b)[:, fine].abs().max()) <= _tolerance(w)
+
+
+def test_unwrapped_atoms_are_no_slower_than_in_the_plain_sum():
+    """All atoms several box lengths away: the cells have nothing to sum, and the
+    call takes the plain kernel's time (1.18 of it when the near pass summed
+    them)."""
+    torch = pytest.importorskip("torch")
+    w = CASES["loopons, two shells"]()
+    pos = _positions(torch, w) + 5.0 * w.box[0]
+    times = []
+    for split in (1, 0):
+        plan = B.Plan(w.loops, w.box, images=w.images, nu=w.nu, image_split=split, max_atoms=w.n)
+        u = torch.zeros_like(pos)
+        best = 1e300
+        for _ in range(6):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            plan.execute(pos, u)
+            b.record()
+            torch.cuda.synchronize()
+            best = min(best, a.elapsed_time(b))
+        plan.close()
+        times.append(best)
+    assert times[1] <= 1.1 * times[0], times
