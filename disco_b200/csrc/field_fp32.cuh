@@ -167,62 +167,90 @@ __device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c)
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
     return r;
 }
-__device__ __forceinline__ F2 dot2(F2 ax, F2 bx, F2 ay, F2 by, F2 az, F2 bz)
+// One value with the same operations.
+struct F1 {
+    float v;
+    __device__ __forceinline__ F1() {}
+    __device__ __forceinline__ F1(float a) : v(a) {}
+    __device__ __forceinline__ F1(float2 p) : v(p.x) {}
+};
+__device__ __forceinline__ F1 add2(F1 a, F1 b) { return __fadd_rn(a.v, b.v); }
+__device__ __forceinline__ F1 mul2(F1 a, F1 b) { return __fmul_rn(a.v, b.v); }
+__device__ __forceinline__ F1 fma2(F1 a, F1 b, F1 c) { return __fmaf_rn(a.v, b.v, c.v); }
+
+// A lane's values for N images: one, or two in a register pair.
+template <int N> struct Images;
+template <> struct Images<1> {
+    using V = F1;
+    static __device__ __forceinline__ V all(float a) { return F1(a); }
+    static __device__ __forceinline__ V of(const float (&a)[1]) { return F1(a[0]); }
+    static __device__ __forceinline__ void get(V p, float (&a)[1]) { a[0] = p.v; }
+};
+template <> struct Images<2> {
+    using V = F2;
+    static __device__ __forceinline__ V all(float a) { return F2(a, a); }
+    static __device__ __forceinline__ V of(const float (&a)[2]) { return F2(a[0], a[1]); }
+    static __device__ __forceinline__ void get(V p, float (&a)[2]) { p.get(a[0], a[1]); }
+};
+
+template <class V>
+__device__ __forceinline__ V dot2(V ax, V bx, V ay, V by, V az, V bz)
 {
     return fma2(az, bz, fma2(ax, bx, mul2(ay, by)));
 }
 
-// An atom's position relative to a piece's centre, for two of its images.
-struct TwoImages {
-    float x[2], y[2], z[2];
-};
-
-// Code/kroupa.hpp:52-73 in FP32 on centre-relative coordinates, two images at a
-// time in packed instructions: 28 FP32 instructions for a loopon of two images
-// instead of 28 for one.  Every operation is written out, in the order and with
-// the fused products that the scalar form was compiled to, so the sums are the
-// same to the bit.  27.6 k atoms, 6 loops (4.9 k loopons), +-1 images: 4.69 ms
-// scalar, 4.00 ms packed (unrolled by 8; 4.13 by 2).
-__device__ __forceinline__ void loopon_piece_fp32(const LooponPieceF& pc, const LooponRecF* rec, const TwoImages& P,
-                                                  float c2, float (&fx)[2], float (&fy)[2], float (&fz)[2])
+// Code/kroupa.hpp:52-73 in FP32 on centre-relative coordinates, for N images at
+// a time: two in packed instructions (28 FP32 instructions for a loopon of two
+// images instead of 28 for one), or one.  Every operation is written out, in the
+// order and with the fused products that the scalar form was first compiled to,
+// so both give the same bits.  27.6 k atoms, 6 loops (4.9 k loopons), +-1
+// images: 4.69 ms one by one, 4.00 ms packed (unrolled by 8; 4.13 by 2).
+template <int N>
+__device__ __forceinline__ void loopon_piece_fp32(const LooponPieceF& pc, const LooponRecF* rec, const float (&px)[N],
+                                                  const float (&py)[N], const float (&pz)[N], float c2, float (&fx)[N],
+                                                  float (&fy)[N], float (&fz)[N])
 {
+    using I = Images<N>;
+    using V = typename I::V;
     // regrouped as loopon_piece_fp64: fb (alpha n + beta m + gamma rho) fac
-    const F2 Px(P.x[0], P.x[1]), Py(P.y[0], P.y[1]), Pz(P.z[0], P.z[1]);
-    const F2 mx(pc.mx, pc.mx), my(pc.my, pc.my), mz(pc.mz, pc.mz), nx(pc.nx, pc.nx), ny(pc.ny, pc.ny), nz(pc.nz, pc.nz);
-    const F2 mP = dot2(mx, Px, my, Py, mz, Pz), nP = dot2(nx, Px, ny, Py, nz, Pz);
+    const V Px = I::of(px), Py = I::of(py), Pz = I::of(pz);
+    const V mx = I::all(pc.mx), my = I::all(pc.my), mz = I::all(pc.mz), nx = I::all(pc.nx), ny = I::all(pc.ny),
+            nz = I::all(pc.nz);
+    const V mP = dot2(mx, Px, my, Py, mz, Pz), nP = dot2(nx, Px, ny, Py, nz, Pz);
     const float c2bn = __fmul_rn(c2, pc.b_n);
-    const F2 c(c2, c2), nc2bn(-c2bn, -c2bn), three(3.0f, 3.0f), zero(0.0f, 0.0f);
-    F2 dx = zero, dy = zero, dz = zero;
+    const V c = I::all(c2), nc2bn = I::all(-c2bn), three = I::all(3.0f), zero = I::all(0.0f);
+    V dx = zero, dy = zero, dz = zero;
     const int n = pc.n;
 #pragma unroll 8
     for (int k = 0; k < n; ++k) {
         const LooponRecF& l = rec[k];
-        const F2 rx = add2(Px, F2(l.x)), ry = add2(Py, F2(l.y)), rz = add2(Pz, F2(l.z));
-        float ra, rb;
-        dot2(rx, rx, ry, ry, rz, rz).get(ra, rb);
-        const bool ka = ra >= 1e-20f, kb = rb >= 1e-20f;
-        const F2 ir(rsqrt_ftz(ka ? ra : 1.0f), rsqrt_ftz(kb ? rb : 1.0f));
-        const F2 ir2 = mul2(ir, ir);
-        const F2 mr = add2(mP, F2(l.ml)), nr = add2(nP, F2(l.nl));
-        const F2 cir = mul2(c, ir);
-        const F2 al = mul2(cir, mr), be = mul2(cir, nr);
-        const F2 ga = mul2(ir, fma2(mul2(mul2(three, mr), nr), ir2, nc2bn));
-        float fa, fb;
-        ir2.get(fa, fb);
-        const F2 fac(ka ? fa : 0.0f, kb ? fb : 0.0f);
+        const V rx = add2(Px, V(l.x)), ry = add2(Py, V(l.y)), rz = add2(Pz, V(l.z));
+        float r2[N], q[N];
+        I::get(dot2(rx, rx, ry, ry, rz, rz), r2);
+#pragma unroll
+        for (int h = 0; h < N; ++h) q[h] = rsqrt_ftz(r2[h] >= 1e-20f ? r2[h] : 1.0f);
+        const V ir = I::of(q);
+        const V ir2 = mul2(ir, ir);
+        const V mr = add2(mP, V(l.ml)), nr = add2(nP, V(l.nl));
+        const V cir = mul2(c, ir);
+        const V al = mul2(cir, mr), be = mul2(cir, nr);
+        const V ga = mul2(ir, fma2(mul2(mul2(three, mr), nr), ir2, nc2bn));
+        I::get(ir2, q);
+#pragma unroll
+        for (int h = 0; h < N; ++h) q[h] = r2[h] >= 1e-20f ? q[h] : 0.0f;
+        const V fac = I::of(q);
         dx = fma2(fac, fma2(al, nx, fma2(be, mx, mul2(ga, rx))), dx);
         dy = fma2(fac, fma2(al, ny, fma2(be, my, mul2(ga, ry))), dy);
         dz = fma2(fac, fma2(al, nz, fma2(be, mz, mul2(ga, rz))), dz);
     }
-    float x[2], y[2], z[2];
-    dx.get(x[0], x[1]);
-    dy.get(y[0], y[1]);
-    dz.get(z[0], z[1]);
+    I::get(dx, fx);
+    I::get(dy, fy);
+    I::get(dz, fz);
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        fx[h] = __fmul_rn(pc.fbx, x[h]);
-        fy[h] = __fmul_rn(pc.fby, y[h]);
-        fz[h] = __fmul_rn(pc.fbz, z[h]);
+    for (int h = 0; h < N; ++h) {
+        fx[h] = __fmul_rn(pc.fbx, fx[h]);
+        fy[h] = __fmul_rn(pc.fby, fy[h]);
+        fz[h] = __fmul_rn(pc.fbz, fz[h]);
     }
 }
 
@@ -321,23 +349,30 @@ struct LooponFp32 {
         for (int p = 0; p < npieces; ++p) {
             const LooponPieceF& pc = pieces[p];
             const double qx = px - pc.cx, qy = py - pc.cy, qz = pz - pc.cz;
-            // the lane's next two images, in their order
-            for (int img = split; img < a.nimg;) {
-                TwoImages P;
+            // the lane's next two images, in their order, or one where no lane of
+            // the warp has a second (no images, 27 over 32 lanes, a last odd one)
+            for (int img = split;;) {
+                float x[2] = {}, y[2] = {}, z[2] = {}, fx[2], fy[2], fz[2];
                 int have = 0;
                 for (; have < 2 && img < a.nimg; img += S) {
                     double sx, sy, sz;
                     if (!image_shift(img, a.images, a.image_min, a.Lx, a.Ly, a.Lz, sx, sy, sz)) continue;
                     const float Px = (float)(qx - sx), Py = (float)(qy - sy), Pz = (float)(qz - sz);
-                    if (have == 0) { P.x[0] = Px; P.y[0] = Py; P.z[0] = Pz; }
-                    P.x[1] = Px; P.y[1] = Py; P.z[1] = Pz;
+                    if (have == 0) { x[0] = Px; y[0] = Py; z[0] = Pz; }
+                    x[1] = Px; y[1] = Py; z[1] = Pz;
                     ++have;
                 }
-                if (have == 0) break;
-                float fx[2], fy[2], fz[2];
-                loopon_piece_fp32(pc, recs + pc.rec, P, c2, fx, fy, fz);
-                acc.add(fx[0], fy[0], fz[0]);
-                if (have == 2) acc.add(fx[1], fy[1], fz[1]);
+                if (!__any_sync(0xffffffffu, have > 0)) break;
+                if (__any_sync(0xffffffffu, have == 2)) {
+                    loopon_piece_fp32<2>(pc, recs + pc.rec, x, y, z, c2, fx, fy, fz);
+                    if (have > 0) acc.add(fx[0], fy[0], fz[0]);
+                    if (have == 2) acc.add(fx[1], fy[1], fz[1]);
+                } else {
+                    const float x1[1] = { x[0] }, y1[1] = { y[0] }, z1[1] = { z[0] };
+                    float gx[1], gy[1], gz[1];
+                    loopon_piece_fp32<1>(pc, recs + pc.rec, x1, y1, z1, c2, gx, gy, gz);
+                    if (have > 0) acc.add(gx[0], gy[0], gz[0]);
+                }
             }
         }
     }

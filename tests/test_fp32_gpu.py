@@ -108,3 +108,49 @@ def test_loopons_over_odd_and_even_image_counts_per_lane(images, split):
         p.close()
         out.append(u)
     assert float((out[0] - out[1]).abs().max()) <= 5e-6
+
+
+def _plan_sum(torch, w, pos, repeat=0, **kw):
+    """The sum, and the best time of `repeat` more calls (ms)."""
+    p = B.Plan(w.loops, kw.pop("box", w.box), precision=C.DISCO_FP32C, nu=w.nu, **kw)
+    u = torch.zeros_like(pos)
+    p.execute(pos, u)
+    out, best = u.clone(), 1e300
+    for _ in range(repeat):
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        a.record()
+        p.execute(pos, u)
+        b.record()
+        torch.cuda.synchronize()
+        best = min(best, a.elapsed_time(b))
+    p.close()
+    return out, best
+
+
+def test_one_loopon_image_alone_or_in_a_pair():
+    """One loop that is one piece, so that an atom's compensated sum takes a
+    single term of size: its image at the origin alone (images = 0), as the
+    second of a pair and as the first, the other images so far away that they add
+    below 1e-20 A.  The same value to that, where another rounding anywhere in the
+    term would show at 1e-9."""
+    torch = pytest.importorskip("torch")
+    w = W.bcc_prismatic(cells=12, n_inter=2, n_vac=1, rmin=5.0, rmax=9.0)
+    w.loops = w.loops[:1]
+    assert len(w.loops[0].x) <= 960
+    pos = torch.tensor(np.stack([w.x, w.y, w.z]), dtype=torch.float64, device="cuda")
+    pos[:, 0] = torch.tensor([w.loops[0].x[0], w.loops[0].y[0], w.loops[0].z[0]])       # on a loopon
+    alone, _ = _plan_sum(torch, w, pos, images=0)
+    assert float(alone.abs().max()) > 0.1
+    for split in (1, 2):
+        pair, _ = _plan_sum(torch, w, pos, images=1, image_split=split, box=(1e12,) * 3)
+        assert float((pair - alone).abs().max()) <= 1e-20
+
+
+def test_one_loopon_image_per_lane_does_not_pay_for_two():
+    """27 images over 32 lanes are one each: as fast as 14 pairs on one lane, or
+    nearly (1.1 times; 1.7 with every image evaluated in a pair)."""
+    torch = pytest.importorskip("torch")
+    w = W.bcc_prismatic(cells=24, n_inter=2, n_vac=2, rmin=12.0, rmax=20.0)
+    pos = torch.tensor(np.stack([w.x, w.y, w.z]), dtype=torch.float64, device="cuda")
+    t = {s: _plan_sum(torch, w, pos, 8, images=1, image_split=s)[1] for s in (1, 32)}
+    assert t[32] <= 1.35 * t[1], t
