@@ -308,6 +308,7 @@ struct LineFp64 {
     using Acc = AccF64;
     static constexpr int kMinBlocks = 2;
     static constexpr bool kAppendsNear = false;
+    static constexpr bool kAfterCells = true;       // may follow the sum by cells (near_mode 3)
     template <int S>
     static __device__ __forceinline__ void chunk(const FieldArgs& a, const unsigned char* st, int npieces,
                                                  int split, double px, double py, double pz, Acc& acc)
@@ -341,6 +342,7 @@ struct LooponFp64 {
     using Acc = AccF64;
     static constexpr int kMinBlocks = 2;
     static constexpr bool kAppendsNear = false;
+    static constexpr bool kAfterCells = true;       // may follow the sum by cells (near_mode 3)
     template <int S>
     static __device__ __forceinline__ void chunk(const FieldArgs& a, const unsigned char* st, int npieces,
                                                  int split, double px, double py, double pz, Acc& acc)
@@ -376,9 +378,9 @@ __global__ void __launch_bounds__(kThreads, Policy::kMinBlocks) field_kernel(con
     if (a.near_mode == 2 && a.near_list) {
         const unsigned c = *a.near_count;
         if (c <= (unsigned)a.near_cap) { n = c; list = a.near_list; }
-    } else if (a.near_mode == 3 && *a.near_count != 0) {
-        return;
     }
+    if constexpr (Policy::kAfterCells)
+        if (a.near_mode == 3 && *a.near_count != 0) return;
     const int64_t ntiles = (n + kAtomsPerCta - 1) / kAtomsPerCta;
     if ((int64_t)blockIdx.x >= ntiles) return;
     const int nch = a.nchunks;

@@ -270,6 +270,7 @@ struct LineFp32 {
     using Acc = AccF32K;
     static constexpr int kMinBlocks = 2;
     static constexpr bool kAppendsNear = true;
+    static constexpr bool kAfterCells = false;
     template <int S>
     static __device__ __forceinline__ void chunk(const FieldArgs& a, const unsigned char* st, int npieces,
                                                  int split, double px, double py, double pz, Acc& acc)
@@ -298,6 +299,7 @@ struct LineNearFp64 {
     using Acc = AccF64;
     static constexpr int kMinBlocks = 2;
     static constexpr bool kAppendsNear = false;
+    static constexpr bool kAfterCells = false;
     template <int S>
     static __device__ __forceinline__ void chunk(const FieldArgs& a, const unsigned char* st, int npieces,
                                                  int split, double px, double py, double pz, Acc& acc)
@@ -339,6 +341,7 @@ struct LooponFp32 {
     using Acc = AccF32K;
     static constexpr int kMinBlocks = 2;
     static constexpr bool kAppendsNear = false;
+    static constexpr bool kAfterCells = false;
     template <int S>
     static __device__ __forceinline__ void chunk(const FieldArgs& a, const unsigned char* st, int npieces,
                                                  int split, double px, double py, double pz, Acc& acc)
