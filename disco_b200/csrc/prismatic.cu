@@ -562,6 +562,38 @@ __device__ __noinline__ int3 direct_segment(const MatterArgs& a, const SlabHead*
     return make_int3(rc, mc, mc > 0 ? off : 0);
 }
 
+// A flush of one listed segment with more candidates than atoms (small boxes full
+// of overlapping slabs: an atom has many entries, and a lane per member's first
+// entry would leave most lanes idle and search its neighbours): the exact tests
+// spread over the lanes, each atom's members and sides by shared-memory ORs, then
+// its counts and records with a lane per atom.  BCC 8^3 cells, 24 loops: 157 us a
+// call without, 125 with it; 12^3, 24 loops: 114 and 101; 10 x 17 x 14, 15 loops:
+// 94 and 91; BCC 128^3, whose segments have fewer: 125 both.  Out of line as
+// direct_segment.
+__device__ __noinline__ int3 queued_segment(const MatterArgs& a, const SlabHead* sh, uint64_t vac, int64_t s,
+                                            const uint32_t* wq, int nq, uint64_t* smask, uint64_t* ssides, int* wcnt,
+                                            int lane)
+{
+#pragma unroll
+    for (int r = 0; r < kSegRounds; ++r) { smask[r * 32 + lane] = 0; ssides[r * 32 + lane] = 0; }
+    __syncwarp();
+    for (int q = lane; q < nq; q += 32) {
+        const uint32_t e = wq[q];
+        const int l = e & 63, slot = (e >> 6) & 127;
+        const int64_t i = s * kSegAtoms + slot;
+        bool ps = false;
+        if (slab_member(a.loops[l], a.x[i], a.y[i], a.z[i], a.Lx, a.Ly, a.Lz, a.idLx, a.idLy, a.idLz, ps)) {
+            atomicOr(reinterpret_cast<unsigned*>(smask + slot) + (l >> 5), 1u << (l & 31));
+            if (ps) atomicOr(reinterpret_cast<unsigned*>(ssides + slot) + (l >> 5), 1u << (l & 31));
+        }
+    }
+    __syncwarp();
+    int rc = 0, mc = 0, off = 0;
+    aggregate_segment(a, sh, vac, s, smask, ssides, wcnt, rc, mc, off, lane);
+    __syncwarp();
+    return make_int3(rc, mc, mc > 0 ? off : 0);
+}
+
 // The matter step in one cooperative launch.
 //   Phase 1, masks.  The grid's warps take the 128-atom segments in chunks
 //     of two from a ticket, so that the warps whose chunks cross slabs take
@@ -763,7 +795,13 @@ __global__ void __launch_bounds__(kMatterThreads, 3) matter_kernel(const MatterA
                     }
                 }
             }
-            if (nq > 0) {
+            if (nlst == 1 && nq > kSegAtoms) {
+                __syncwarp();
+                const int64_t sj = wl_seg[warp][0];
+                const int3 res = queued_segment(sa, sh, vac, sj, wq, nq, smask, ssides, wcnt[warp], lane);
+                if (lane == 0) { a.seg_removed[sj] = res.x; a.seg_members[sj] = res.y; a.seg_off[sj] = res.z; }
+                __syncwarp();                                   // the queue and the list are rewritten
+            } else if (nq > 0) {
                 // flush: the exact tests of the queue spread over the lanes, the
                 // members in bit 29 of their entries (bit 30: positive side) and
                 // in the listed segments' member and removed bits

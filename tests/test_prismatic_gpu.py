@@ -185,3 +185,17 @@ def test_finalize_matches_oracle():
     ref = O.finalize(xs, ys, zs, *u, r["copy_atom"], r["copy_shift"], w.box)
     for a, b in zip(got, ref):
         assert np.array_equal(a, b)
+
+
+
+@pytest.mark.parametrize("loops", [1, 2, 3, 4, 5, 6, 8, 12, 24])
+@pytest.mark.parametrize("keep", [100, 128, 300])
+def test_overlapping_slabs_over_one_segment(loops, keep):
+    """The densest stretch of a box, one segment of 128 atoms or about, in more
+    and more overlapping slabs: a queue of fewer candidates than atoms, of more
+    (the flush of a single segment), and one that is full."""
+    w = W.bcc_prismatic(cells=14, rmin=12.0, rmax=14.0, n_inter=12, n_vac=12, seed=9)
+    q = O.prismatic(w.x, w.y, w.z, w.slab_loops, w.box)
+    order = np.argsort(-np.bincount(q["slab_atoms"], minlength=w.n), kind="stable")
+    x, y, z = (np.ascontiguousarray(v[order][:keep]) for v in (w.x, w.y, w.z))
+    _same(P.prismatic(x, y, z, w.slab_loops[:loops], w.box), O.prismatic(x, y, z, w.slab_loops[:loops], w.box))
