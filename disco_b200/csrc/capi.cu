@@ -32,10 +32,10 @@ struct disco_plan {
     int nimg = 1;
     int nloops = 0;
     disco::HostTable tables[2];              // line, loopon
-    // one block of device memory: the image (status word, tables, chunk lists)
-    // and behind it the FP32 line form's list of atoms with near-cut pairs
-    std::vector<unsigned char> image;        // host copy until the upload
-    size_t table_at[2] = { 0, 0 }, chunks_at[2] = { 0, 0 }, near_at = 0, bytes = 0;
+    // one block of device memory: the image (status word, tables, chunk lists;
+    // plan_image) and behind it the FP32 line form's list of atoms with near-cut
+    // pairs
+    size_t table_at[2] = { 0, 0 }, chunks_at[2] = { 0, 0 }, image_bytes = 0, near_at = 0, bytes = 0;
     unsigned char* block = nullptr;          // owned where `own`: cudaMalloc'd, or from the
     bool own = false, pooled = false;        // scratch pool in the order of `stream`
     cudaStream_t stream = nullptr;
@@ -414,14 +414,7 @@ int plan_build(const disco_loop* loops, int32_t nloops, const double box[3], con
         p->table_at[k] = take(p->tables[k].bytes.size());
         p->chunks_at[k] = take(p->tables[k].chunks.size() * sizeof(disco::Chunk));
     }
-    p->image.assign(at, 0);
-    for (int k = 0; k < 2; ++k) {
-        disco::HostTable& T = p->tables[k];
-        if (T.chunks.empty()) continue;
-        std::memcpy(p->image.data() + p->table_at[k], T.bytes.data(), T.bytes.size());
-        std::memcpy(p->image.data() + p->chunks_at[k], T.chunks.data(), T.chunks.size() * sizeof(disco::Chunk));
-        std::vector<unsigned char>().swap(T.bytes);
-    }
+    p->image_bytes = at;
     if (o.precision == DISCO_FP32C && !p->tables[0].chunks.empty()) {
         // the list of atoms with near-cut pairs: up to 2^21 (a longer list
         // overflows and the FP64 pass visits every atom)
@@ -431,6 +424,46 @@ int plan_build(const disco_loop* loops, int32_t nloops, const double box[3], con
     p->bytes = at;
     *out = p;
     return DISCO_OK;
+}
+
+// Copies the parts of a plan's image by copy(offset in the image, source, bytes)
+// until one fails.
+template <class Copy>
+cudaError_t plan_image(const disco_plan* p, Copy copy)
+{
+    static const unsigned char zero[256] = {};
+    cudaError_t e = copy((size_t)0, static_cast<const void*>(zero), sizeof(zero));       // the status word
+    for (int k = 0; k < 2; ++k) {
+        const disco::HostTable& T = p->tables[k];
+        if (T.chunks.empty()) continue;
+        if (e == cudaSuccess) e = copy(p->table_at[k], static_cast<const void*>(T.bytes.data()), T.bytes.size());
+        if (e == cudaSuccess)
+            e = copy(p->chunks_at[k], static_cast<const void*>(T.chunks.data()), T.chunks.size() * sizeof(disco::Chunk));
+    }
+    return e;
+}
+
+// The image on the host, behind `at` bytes of other data.
+std::vector<unsigned char> plan_packed(const disco_plan* p, size_t at)
+{
+    std::vector<unsigned char> pack(at + p->image_bytes, 0);
+    plan_image(p, [&](size_t o, const void* src, size_t bytes) {
+        std::memcpy(pack.data() + at + o, src, bytes);
+        return cudaSuccess;
+    });
+    return pack;
+}
+
+// The image of a plan that has its block, on `s`: small ones in one copy.
+cudaError_t plan_upload(const disco_plan* p, cudaStream_t s)
+{
+    if (p->image_bytes <= (size_t)64 << 10) {
+        const std::vector<unsigned char> pack = plan_packed(p, 0);
+        return cudaMemcpyAsync(p->block, pack.data(), pack.size(), cudaMemcpyHostToDevice, s);
+    }
+    return plan_image(p, [&](size_t o, const void* src, size_t bytes) {
+        return cudaMemcpyAsync(p->block + o, src, bytes, cudaMemcpyHostToDevice, s);
+    });
 }
 
 // Gives a plan its block (p->bytes, 256-byte aligned; the image still has to be
@@ -475,7 +508,7 @@ int disco::plan_create_on(const disco_loop* loops, int32_t nloops, const double 
     plan_place(p, block);
     p->own = true;
     p->stream = s;
-    e = cudaMemcpyAsync(block, p->image.data(), p->image.size(), cudaMemcpyHostToDevice, s);
+    e = plan_upload(p, s);
     if (e != cudaSuccess) { free_plan(p); return cuda_fail(e, "loop table upload"); }
     *out = p;
     return DISCO_OK;
@@ -495,9 +528,10 @@ int disco_b200_plan_create(const disco_loop* loops, int32_t nloops, const double
     if (e != cudaSuccess) { free_plan(p); return cuda_fail(e, "plan memory"); }
     plan_place(p, block);
     p->own = true;
-    e = cudaMemcpy(block, p->image.data(), p->image.size(), cudaMemcpyHostToDevice);
+    e = plan_upload(p, nullptr);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
     if (e != cudaSuccess) { free_plan(p); return cuda_fail(e, "loop table upload"); }
-    std::vector<unsigned char>().swap(p->image);
+    for (disco::HostTable& T : p->tables) std::vector<unsigned char>().swap(T.bytes);
     *out = p;
     return DISCO_OK;
 }
@@ -645,18 +679,17 @@ int disco_b200_displace(const disco_atoms* atoms, const disco_loop* loops, int32
     plan_place(plan, block + atoms_at);
     // small calls: one copy each way through a packed host buffer
     std::vector<unsigned char> pack;
-    const bool small = atoms_at + plan->image.size() <= (size_t)128 << 10;
+    const bool small = atoms_at + plan->image_bytes <= (size_t)128 << 10;
     const double* src[6] = { atoms->x, atoms->y, atoms->z, atoms->ux, atoms->uy, atoms->uz };
     if (small) {
-        pack.resize(atoms_at + plan->image.size());
+        pack = plan_packed(plan, atoms_at);
         for (int k = 0; k < 6 && n > 0; ++k) std::memcpy(pack.data() + k * bytes, src[k], bytes);
-        std::memcpy(pack.data() + atoms_at, plan->image.data(), plan->image.size());
         e = cudaMemcpyAsync(block, pack.data(), pack.size(), cudaMemcpyHostToDevice, s);
     } else {
         for (int k = 0; k < 6 && e == cudaSuccess && n > 0; ++k)
             e = cudaMemcpyAsync(block + k * bytes, src[k], bytes, cudaMemcpyHostToDevice, s);
         if (e == cudaSuccess)
-            e = cudaMemcpyAsync(block + atoms_at, plan->image.data(), plan->image.size(), cudaMemcpyHostToDevice, s);
+            e = plan_upload(plan, s);
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) { cleanup(); return cuda_fail(e, "atom upload"); }

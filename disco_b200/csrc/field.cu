@@ -84,15 +84,28 @@ bool quadtree(const disco_loop& lp, std::vector<int32_t>& order, std::vector<Tre
     int depth = 0;
     while (depth < 8 && (double)np / std::ldexp(1.0, 2 * depth) > 256.0) ++depth;
     const int side = 1 << depth;
+    // extents of the squares of every depth, the finest from the loopons
+    struct Extent { double l[2], h[2]; };
+    std::vector<std::vector<Extent>> ext((size_t)depth + 1);
+    for (int t = 0; t <= depth; ++t) ext[t].assign((size_t)1 << (2 * t), { { 1e300, 1e300 }, { -1e300, -1e300 } });
+    auto widen = [](Extent& e, const double (&l)[2], const double (&h)[2]) {
+        for (int d = 0; d < 2; ++d) { e.l[d] = std::min(e.l[d], l[d]); e.h[d] = std::max(e.h[d], h[d]); }
+    };
+    std::vector<int32_t> spread((size_t)side, 0);                // bit t of a number at bit 2 t
+    for (int i = 0; i < side; ++i)
+        for (int t = 0; t < depth; ++t) spread[i] |= (i >> t & 1) << (2 * t);
     std::vector<int32_t> code((size_t)np), first((size_t)side * side + 1, 0);
     for (int k = 0; k < np; ++k) {
         const int i = std::min(side - 1, std::max(0, (int)((a[k] - mid[0] + half) / (2.0 * half) * side)));
         const int j = std::min(side - 1, std::max(0, (int)((b[k] - mid[1] + half) / (2.0 * half) * side)));
-        int c = 0;
-        for (int t = 0; t < depth; ++t) c |= ((i >> t & 1) << (2 * t + 1)) | ((j >> t & 1) << (2 * t));
+        const int c = spread[i] << 1 | spread[j];
         code[k] = c;
         ++first[c + 1];
+        const double p[2] = { a[k], b[k] };
+        widen(ext[depth][c], p, p);
     }
+    for (int t = depth; t > 0; --t)
+        for (size_t c = 0; c < ext[t].size(); ++c) widen(ext[t - 1][c >> 2], ext[t][c].l, ext[t][c].h);
     for (int c = 0; c < side * side; ++c) {
         if (first[c + 1] > kMaxLooponPiece) return false;
         first[c + 1] += first[c];
@@ -108,11 +121,7 @@ bool quadtree(const disco_loop& lp, std::vector<int32_t>& order, std::vector<Tre
         for (int c = 0; c < cells; ++c) {
             const int k0 = first[c * span], k1 = first[(c + 1) * span];
             if (k0 == k1) continue;
-            double l[2] = { 1e300, 1e300 }, h[2] = { -1e300, -1e300 };
-            for (int k = k0; k < k1; ++k) {
-                l[0] = std::min(l[0], a[order[k]]); h[0] = std::max(h[0], a[order[k]]);
-                l[1] = std::min(l[1], b[order[k]]); h[1] = std::max(h[1], b[order[k]]);
-            }
+            const double (&l)[2] = ext[t][c].l, (&h)[2] = ext[t][c].h;
             TreePiece q;
             std::memset(&q, 0, sizeof(q));
             const double ca = 0.5 * (l[0] + h[0]), cb = 0.5 * (l[1] + h[1]);
@@ -228,6 +237,7 @@ int build_table(const disco_loop* loops, int nloops, int kind, int precision, do
                 p.b_n = ph.mx * ph.nx + ph.my * ph.ny + ph.mz * ph.nz;
                 p.n = k1e - k0;
                 std::vector<LooponRec> recs;
+                recs.reserve((size_t)(k1e - k0));
                 for (int k = k0; k < k1e; ++k) {
                     const int i = order.empty() ? k : order[k];
                     LooponRec r;

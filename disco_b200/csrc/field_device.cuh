@@ -583,6 +583,7 @@ void pack_chunks(PieceList<Piece, Rec>& L, HostTable& T, uint32_t stage_cap = 0)
     const uint32_t cap = resident ? kResidentMax : (stage_cap ? stage_cap : kStageMax);
     T.resident = resident;
     T.bytes.clear();
+    T.bytes.reserve(total + total / 16 + 4096);
     T.chunks.clear();
     size_t i = 0;
     uint32_t max_bytes = 16;
@@ -599,20 +600,20 @@ void pack_chunks(PieceList<Piece, Rec>& L, HostTable& T, uint32_t stage_cap = 0)
         c.offset = T.bytes.size();
         c.bytes = (uint32_t)((bytes + 15) & ~size_t(15));
         c.npieces = (int32_t)(j - i);
-        std::vector<unsigned char> blob(c.bytes, 0);
+        T.bytes.resize(T.bytes.size() + c.bytes, 0);
+        unsigned char* blob = T.bytes.data() + c.offset;
         int32_t rec = 0;
         for (size_t k = i; k < j; ++k) {
             Piece p = L.pieces[k];
             p.rec = rec;
-            std::memcpy(blob.data() + (k - i) * sizeof(Piece), &p, sizeof(Piece));
+            std::memcpy(blob + (k - i) * sizeof(Piece), &p, sizeof(Piece));
             rec += (int32_t)L.recs[k].size();
         }
         size_t off = (j - i) * sizeof(Piece);
         for (size_t k = i; k < j; ++k) {
-            std::memcpy(blob.data() + off, L.recs[k].data(), L.recs[k].size() * sizeof(Rec));
+            std::memcpy(blob + off, L.recs[k].data(), L.recs[k].size() * sizeof(Rec));
             off += L.recs[k].size() * sizeof(Rec);
         }
-        T.bytes.insert(T.bytes.end(), blob.begin(), blob.end());
         T.chunks.push_back(c);
         max_bytes = std::max(max_bytes, c.bytes);
         i = j;

@@ -140,6 +140,7 @@ int build_table_fp32(const disco_loop* loops, int nloops, int kind, double nu, H
                 p.b_n = (float)(ph.mx * ph.nx + ph.my * ph.ny + ph.mz * ph.nz);
                 p.n = k1e - k0;
                 std::vector<LooponRecF> recs;
+                recs.reserve((size_t)(k1e - k0));
                 for (int k = k0; k < k1e; ++k) {
                     const double x = lp.x[k] - cx, y = lp.y[k] - cy, z = lp.z[k] - cz;
                     LooponRecF r;
