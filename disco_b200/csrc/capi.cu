@@ -514,35 +514,13 @@ int disco::plan_create_on(const disco_loop* loops, int32_t nloops, const double 
     return DISCO_OK;
 }
 
-extern "C" {
-
-int disco_b200_plan_create(const disco_loop* loops, int32_t nloops, const double box[3],
-                           const disco_options* opt, int64_t max_atoms, disco_plan** out)
+int disco::plan_execute_counted(disco_plan* p, const disco_atoms* a, cudaStream_t s, int* launches)
 {
-    int st = plan_build(loops, nloops, box, opt, max_atoms, out);
-    if (st) return st;
-    disco_plan* p = *out;
-    *out = nullptr;
-    unsigned char* block = nullptr;
-    cudaError_t e = cudaMalloc(&block, p->bytes);
-    if (e != cudaSuccess) { free_plan(p); return cuda_fail(e, "plan memory"); }
-    plan_place(p, block);
-    p->own = true;
-    e = plan_upload(p, nullptr);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
-    if (e != cudaSuccess) { free_plan(p); return cuda_fail(e, "loop table upload"); }
-    for (disco::HostTable& T : p->tables) std::vector<unsigned char>().swap(T.bytes);
-    *out = p;
-    return DISCO_OK;
-}
-
-int disco_b200_plan_execute(disco_plan* p, const disco_atoms* a, void* stream)
-{
+    *launches = 0;
     if (!p || !a) return fail(DISCO_EINVAL, "null plan or atoms");
     if (a->n < 0) return fail(DISCO_EINVAL, "negative atom count");
     if (a->n == 0) return DISCO_OK;
     if (!a->x || !a->y || !a->z || !a->ux || !a->uy || !a->uz) return fail(DISCO_EINVAL, "null atom array");
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
     for (int k = 0; k < 2; ++k) {
         const disco::HostTable& T = p->tables[k];
         if (T.chunks.empty()) continue;
@@ -581,18 +559,48 @@ int disco_b200_plan_execute(disco_plan* p, const disco_atoms* a, void* stream)
         const int kind = k == 0 ? disco::kLineKind : disco::kLooponKind;
         const disco::TreeShape shape = plan_tree(p, k, a->n, s);
         if (shape.use) {
-            bool ran = false;
-            const int st = disco::launch_tree(fa, T, shape, p->sm_count, s, &ran, err);
+            int queued = 0;
+            const int st = disco::launch_tree(fa, T, shape, p->sm_count, s, &queued, err);
             if (st) return fail(st, err);
-            if (ran) continue;
+            *launches += queued;
+            if (queued) continue;
         }
         const int st = T.fp32
             ? disco::launch_field_fp32(fa, kind, p->sm_count, p->opt.image_split, s, err)
             : disco::launch_field(fa, kind, false, p->sm_count, p->opt.threads_per_block,
                                   p->opt.image_split, s, err);
         if (st) return fail(st, err);
+        *launches += T.fp32 && k == 0 ? 2 : 1;               // FP32 lines: the near-cut pairs' pass
     }
     return DISCO_OK;
+}
+
+extern "C" {
+
+int disco_b200_plan_create(const disco_loop* loops, int32_t nloops, const double box[3],
+                           const disco_options* opt, int64_t max_atoms, disco_plan** out)
+{
+    int st = plan_build(loops, nloops, box, opt, max_atoms, out);
+    if (st) return st;
+    disco_plan* p = *out;
+    *out = nullptr;
+    unsigned char* block = nullptr;
+    cudaError_t e = cudaMalloc(&block, p->bytes);
+    if (e != cudaSuccess) { free_plan(p); return cuda_fail(e, "plan memory"); }
+    plan_place(p, block);
+    p->own = true;
+    e = plan_upload(p, nullptr);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
+    if (e != cudaSuccess) { free_plan(p); return cuda_fail(e, "loop table upload"); }
+    for (disco::HostTable& T : p->tables) std::vector<unsigned char>().swap(T.bytes);
+    *out = p;
+    return DISCO_OK;
+}
+
+int disco_b200_plan_execute(disco_plan* p, const disco_atoms* a, void* stream)
+{
+    int launches;
+    return disco::plan_execute_counted(p, a, static_cast<cudaStream_t>(stream), &launches);
 }
 
 int disco_b200_plan_sync(disco_plan* p, void* stream)

@@ -42,6 +42,8 @@ unsigned long long scratch_retain(int device);
 void scratch_release(int device, unsigned long long ctx);
 int plan_create_on(const disco_loop* loops, int32_t nloops, const double box[3], const disco_options* opt,
                    int64_t max_atoms, cudaStream_t s, disco_plan** out);
+// disco_b200_plan_execute, and the kernels it launched.
+int plan_execute_counted(disco_plan* p, const disco_atoms* a, cudaStream_t s, int* launches);
 int batch_plan_create_on(const disco_sample* samples, int32_t nsamples, const disco_options* opt, cudaStream_t s,
                          disco_batch_plan** out);
 // Stream-ordered scratch of a call: from the pool, or the device's default one.

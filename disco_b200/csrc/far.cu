@@ -594,8 +594,6 @@ int disco_b200_learned_displace(disco_mlp* m, const disco_far_norm* norm, const 
     std::vector<int32_t> fb((size_t)nloops, 0);
     std::vector<float> lerr((size_t)nloops, 0.0f);
     const int64_t n = a->n;
-    // kernels of one exact sum of line loops: FP32C adds the near-cut FP64 pass
-    auto sum_launches = [](int precision) { return precision == DISCO_FP32C ? 2 : 1; };
     int launches = 0;
     int dev = 0, sms = 0;
     FAR_TRY(cudaGetDevice(&dev), "device query");
@@ -672,7 +670,7 @@ int disco_b200_learned_displace(disco_mlp* m, const disco_far_norm* norm, const 
         if (!st2) st2 = disco_b200_batch_plan_sync(bp, s);
         disco_b200_batch_plan_destroy(bp);
         if (st2) return st2;
-        launches += sum_launches(opt->check_precision);
+        launches += opt->check_precision == DISCO_FP32C ? 3 : 1;     // a batch of lines: with both near-cut passes
         disco_atoms ga = { gx, gy, gz, nullptr, nullptr, nullptr, nc };
         st2 = apply_impl(m, norm, &ga, loops, nloops, box, nullptr, nloops, net, s);
         if (st2) return st2;
@@ -726,11 +724,12 @@ int disco_b200_learned_displace(disco_mlp* m, const disco_far_norm* norm, const 
         disco_plan* p = nullptr;
         int st2 = disco::plan_create_on(loops, nloops, box, &no, n, s, &p);
         if (st2) return st2;
-        st2 = disco_b200_plan_execute(p, a, s);
+        int queued = 0;
+        st2 = disco::plan_execute_counted(p, a, s, &queued);
         if (!st2) st2 = disco_b200_plan_sync(p, s);
         disco_b200_plan_destroy(p);
         if (st2) return st2;
-        launches += sum_launches(opt->precision);
+        launches += queued;
     }
     cudaEventRecord(en.b, s);
 
@@ -759,11 +758,12 @@ int disco_b200_learned_displace(disco_mlp* m, const disco_far_norm* norm, const 
         disco_plan* p = nullptr;
         int st2 = disco::plan_create_on(sub.data(), (int32_t)sub.size(), box, &fo, n, s, &p);
         if (st2) return st2;
-        st2 = disco_b200_plan_execute(p, a, s);
+        int queued = 0;
+        st2 = disco::plan_execute_counted(p, a, s, &queued);
         if (!st2) st2 = disco_b200_plan_sync(p, s);
         disco_b200_plan_destroy(p);
         if (st2) return st2;
-        launches += sum_launches(opt->precision);
+        launches += queued;
     }
     cudaEventRecord(eb.b, s);
     FAR_TRY(cudaStreamSynchronize(s), "learned displacement");

@@ -1639,9 +1639,9 @@ cudaError_t leaf_any(const TreeArgs& a, cudaStream_t s)
 } // namespace
 
 int launch_tree(const FieldArgs& f, const HostTable& T, const TreeShape& S, int sm_count,
-                cudaStream_t s, bool* ran, std::string& err)
+                cudaStream_t s, int* launches, std::string& err)
 {
-    *ran = false;
+    *launches = 0;
     OutsideCapture relaxed;
     TreeArgs a;
     std::memset(&a, 0, sizeof(a));
@@ -1728,7 +1728,6 @@ int launch_tree(const FieldArgs& f, const HostTable& T, const TreeShape& S, int 
         cudaGetLastError();
         return DISCO_OK;
     }
-    *ran = true;
     a.box = reinterpret_cast<unsigned long long*>(ws + o_box);
     int most = 0;
     for (int k = 0; k < S.total; ++k) {
@@ -1763,6 +1762,7 @@ int launch_tree(const FieldArgs& f, const HostTable& T, const TreeShape& S, int 
     auto queue = [&]() -> cudaError_t {
         const int64_t sweep = std::min<int64_t>((f.n + 255) / 256, (int64_t)sm_count * 8);
         cudaError_t e;
+        int passes = 0;
         tree_init_kernel<<<(unsigned)std::min<int64_t>((lcells + 255) / 256, sm_count * 4), 256, 0, s>>>(a);
         tree_box_kernel<<<(unsigned)sweep, 256, 0, s>>>(a);
         const unsigned nt = (unsigned)a.sort_tiles;
@@ -1779,6 +1779,7 @@ int launch_tree(const FieldArgs& f, const HostTable& T, const TreeShape& S, int 
                                                                        a.idx[in ^ 1], shift);
             }
             in ^= 1;
+            ++passes;
         }
         a.perm = a.idx[in];
         tree_starts_kernel<<<(unsigned)((f.n + 256) / 256), 256, 0, s>>>(a, a.key[in]);
@@ -1799,6 +1800,9 @@ int launch_tree(const FieldArgs& f, const HostTable& T, const TreeShape& S, int 
         const unsigned ngrid = (unsigned)((ntiles + kWarps - 1) / kWarps);
         if (line) tree_near_sum_kernel<kLineKind><<<ngrid, 32 * kWarps, 0, s>>>(a);
         else tree_near_sum_kernel<kLooponKind><<<ngrid, 32 * kWarps, 0, s>>>(a);
+        // init, box, three per sorting pass, starts, scan, list, near, (equivalent),
+        // matrix, node, one down per further level, leaf, near_sum
+        *launches = 2 + 3 * passes + 4 + (line ? 0 : 1) + 2 + (S.levels - 1) + 2;
         return cudaGetLastError();
     };
     const cudaError_t e = queue();
@@ -1808,6 +1812,7 @@ int launch_tree(const FieldArgs& f, const HostTable& T, const TreeShape& S, int 
         out.near_mode = 3;
         out.near_count = reinterpret_cast<unsigned int*>(a.box + 7);
         plain = launch_field(out, T.kind, false, sm_count, 0, 0, s, err);
+        ++*launches;
     }
     const cudaError_t ef = cudaFreeAsync(ws, s);
     if (e != cudaSuccess) { err = cudaGetErrorString(e); return DISCO_ECUDA; }

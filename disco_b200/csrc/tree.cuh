@@ -39,9 +39,9 @@ struct TreeShape {
 // is false where the plain sum over every image is estimated to be faster.
 TreeShape tree_shape(const HostTable& T, int64_t n, const double box[3], int images, int sm_count);
 
-// Queues the sum on `stream`.  *ran is false (and nothing was queued) when the
-// scratch memory could not be had: the caller then sums directly.
+// Queues the sum on `stream`, *launches kernels.  None (nothing was queued) when
+// the scratch memory could not be had: the caller then sums directly.
 int launch_tree(const FieldArgs& a, const HostTable& T, const TreeShape& S, int sm_count,
-                cudaStream_t stream, bool* ran, std::string& err);
+                cudaStream_t stream, int* launches, std::string& err);
 
 } // namespace disco

@@ -21,6 +21,7 @@ import pytest
 import oracle as O
 from disco_b200 import _capi as C
 from disco_b200 import backend as B
+from disco_b200 import geometry as G
 from disco_b200 import learned as Ln
 from disco_b200 import workloads as W
 
@@ -231,3 +232,34 @@ def test_large_check_gives_its_memory_back():
         return free - torch.cuda.mem_get_info()[0]
     call(1000)
     assert call(pos.shape[1]) < 1 << 20
+
+
+@pytest.mark.parametrize("precision", [C.DISCO_FP64, C.DISCO_FP32C])
+@pytest.mark.parametrize("check_precision", [C.DISCO_FP64, C.DISCO_FP32C])
+@pytest.mark.parametrize("cells,check,fail", [(12, 0.0, False), (12, 0.05, True), (48, 0.0, False), (48, 0.01, False)])
+def test_report_counts_the_kernels(precision, check_precision, cells, check, fail):
+    """report.launches is the number of kernels that the profiler sees, with the
+    near images by cells (the larger FP64 boxes) or term by term, with and without
+    a check, with every loop falling back."""
+    from torch.profiler import ProfilerActivity, profile
+    loops, box, _ = _small(cells=cells, nloops=6)
+    x, y, z = G.lattice(G.FCC, cells, cells, cells, 3.615)
+    d = torch.tensor(np.stack([x, y, z]), dtype=torch.float64, device="cuda")
+    u = torch.zeros_like(d)
+    m = Ln.MLP(seed=1)
+    norm = Ln.FarNorm(np.zeros(16, dtype=np.float32), np.ones(16, dtype=np.float32), 1.0, 2, 2)
+    tol = 0.0 if fail else 1e9
+
+    def call():
+        return Ln.learned_displace(m, norm, d, u, loops, box, 0.34, precision=precision,
+                                   check_precision=check_precision, check_fraction=check, tol_loop=tol, tol_total=tol)
+    rep = call()
+    torch.cuda.synchronize()
+    with profile(activities=[ProfilerActivity.CUDA], acc_events=True) as p:
+        rep = call()
+        torch.cuda.synchronize()
+    names = [e.name for e in p.events() if "CUDA" in str(e.device_type)
+             and not e.name.lower().startswith(("memcpy", "memset")) and "at::native" not in e.name]
+    assert rep["launches"] == len(names), names
+    by_cells = any("tree_node" in k for k in names)
+    assert by_cells == (precision == C.DISCO_FP64 and cells == 48), names
