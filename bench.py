@@ -127,24 +127,30 @@ def timed_steps(torch, step, steps, stream, flush):
     return total
 
 
-def kernels_per_call(torch, fn, least):
-    """Kernels that one call of fn launches, counted by the profiler outside any
-    timed region; `least` where it cannot be used."""
+def kernels_per_call(torch, fn):
+    """Names of the kernels that one call of fn launches, by the profiler outside
+    any timed region; None where it cannot be used."""
     try:
         from torch.profiler import ProfilerActivity, profile
         torch.cuda.synchronize()
         with profile(activities=[ProfilerActivity.CUDA], acc_events=True) as p:
             fn()
             torch.cuda.synchronize()
-        count = sum(1 for e in p.events() if "CUDA" in str(e.device_type)
-                    and not e.name.lower().startswith(("memcpy", "memset")) and "at::native" not in e.name)
-        return max(least, count)
+        names = [e.name for e in p.events() if "CUDA" in str(e.device_type)
+                 and not e.name.lower().startswith(("memcpy", "memset")) and "at::native" not in e.name]
+        return names or None
     except Exception:
-        return least
+        return None
 
 
-def field_roofline(torch, clk, fp64, evals, flop, seconds, by_cells, traffic=None):
-    """Roofline of a field launch of `evals` segment- or loopon-image terms."""
+# The committed profile whose kernels (not sizes) a workload's sum by cells runs.
+CELLS_PROFILE = {"fcc_random": "tree_fcc_large", "bcc_prismatic": "tree_bcc_loopons"}
+
+
+def field_roofline(torch, clk, fp64, evals, flop, seconds, kernels, workload, traffic=None):
+    """Roofline of a field launch of `evals` segment- or loopon-image terms, by the
+    names of the kernels that ran (None: not known, and no share of a peak is
+    claimed for an FP64 sum, which may have gone by cells)."""
     gemm = fp64_peak_tflops(torch) if fp64 else fp32_peak_tflops(torch)
     peak, src = pipe_peak_tflops(torch, clk, fp64)
     rate = evals * flop / seconds / 1e12
@@ -156,10 +162,16 @@ def field_roofline(torch, clk, fp64, evals, flop, seconds, by_cells, traffic=Non
                                  "not on the DFMA pipe this kernel uses") if fp64 else
                                 "torch SGEMM 8192^3 without TF32, best of 5",
             "flop_per_eval": flop, "evals_per_launch": evals}
-    if by_cells:
-        roof.update(achieved=None, frac=None, frac_of_gemm=None, term_by_term_equivalent=rate,
-                    form="far pairs by cells: most terms are never formed, so their rate is no share of a peak",
-                    fp64_pipe_active=profile_value("tree_fcc_large", "fp64_pipe_active"))
+    cells = None if kernels is None else any("tree_node" in k for k in kernels)
+    if cells or (cells is None and fp64):
+        roof.update(achieved=None, frac=None, frac_of_gemm=None, term_by_term_equivalent=rate, traffic=None)
+    if cells:
+        name = CELLS_PROFILE.get(workload)
+        roof.update(form="far pairs by cells: most terms are never formed, so their rate is no share of a peak",
+                    fp64_pipe_active=profile_value(name, "fp64_pipe_active") if name else None,
+                    fp64_pipe_source=f"profiles/{name}.md: these kernels on a smaller box" if name else None)
+    elif cells is None and fp64:
+        roof.update(form="the profiler could not name the kernels: no share of a peak is claimed")
     return roof
 
 
@@ -760,8 +772,8 @@ def run_ours(args):
     plan.execute(pos, u1d)
     plan.sync(stream.cuda_stream)
     u1 = u1d.cpu().numpy()
-    launches_per_step = kernels_per_call(torch, lambda: (plan.execute(pos, u), plan.sync(stream.cuda_stream)),
-                                         int(st["n_line_loops"] > 0) + int(st["n_loopon_loops"] > 0))
+    kernels = kernels_per_call(torch, lambda: (plan.execute(pos, u), plan.sync(stream.cuda_stream)))
+    launches_per_step = len(kernels) if kernels else int(st["n_line_loops"] > 0) + int(st["n_loopon_loops"] > 0)
     output = write_output(w, pos, u1d, stream) if (rank == 0 and not args.no_output) else None
     del u1d
 
@@ -835,9 +847,8 @@ def run_ours(args):
     if rank == 0:
         fp64 = prec == C.DISCO_FP64
         key = f"{'line' if w.method == 'line' else 'loopon'}_{args.precision}_{args.config}"
-        by_cells = launches_per_step > 2
-        roof = field_roofline(torch, clk, fp64, evals_atom * n, flop_per_eval(w), per_launch, by_cells,
-                              None if by_cells else traffic_from_profiles(key))
+        roof = field_roofline(torch, clk, fp64, evals_atom * n, flop_per_eval(w), per_launch, kernels, args.config,
+                              traffic_from_profiles(key))
         cpu = None
         parity = None
         if not args.no_cpu:
@@ -1306,7 +1317,8 @@ def run_prismatic(args, embedded=False):
     clk = clocks.stop()
     plan.sync(stream.cuda_stream)
     k, nc = kn
-    launches_per_step = kernels_per_call(torch, lambda: (step(), plan.sync(stream.cuda_stream)), 3)
+    kernels = kernels_per_call(torch, lambda: (step(), plan.sync(stream.cuda_stream)))
+    launches_per_step = len(kernels) if kernels else 3
     elapsed = max_over_ranks(elapsed, world)
     per = elapsed / args.steps
     evals = st_plan["evals_per_atom"] * k
@@ -1373,7 +1385,7 @@ def run_prismatic(args, embedded=False):
             refgpu["ours"] = {"kernel_s": f0.elapsed_time(f1) * 1e-3,
                               "note": "this library's loopon field over the same survivors, nu 0.35"}
             del u35
-        roof = field_roofline(torch, clk, prec == C.DISCO_FP64, evals, W_LOOPON, per, launches_per_step > 4)
+        roof = field_roofline(torch, clk, prec == C.DISCO_FP64, evals, W_LOOPON, per, kernels, "bcc_prismatic")
         roof["kernel"] = "loopon field (the step also holds the matter step and epilogue)"
         line = {
             "metric": METRIC, "value": n * world / per, "unit": "atoms/s", "n_gpus": world,
