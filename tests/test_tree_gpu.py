@@ -390,3 +390,59 @@ def test_unwrapped_atoms_are_no_slower_than_in_the_plain_sum():
         plan.close()
         times.append(best)
     assert times[1] <= 1.1 * times[0], times
+
+
+def _circle(radius, chords, center, normal, seed):
+    rng = np.random.default_rng(seed)
+    n = np.asarray(normal, dtype=float) / np.linalg.norm(normal)
+    a = np.cross(n, rng.normal(size=3))
+    a /= np.linalg.norm(a)
+    b, t = np.cross(n, a), 2 * np.pi * np.arange(chords) / chords
+    p = np.asarray(center) + radius * (np.cos(t)[:, None] * a + np.sin(t)[:, None] * b)
+    return B.LoopData(phys=B.LoopPhys(2.5, 2.5, 2.5, *a, *n, 1.0), line=True, vx=p[:, 0].copy(), vy=p[:, 1].copy(),
+                      vz=p[:, 2].copy(), cx=center[0], cy=center[1], cz=center[2])
+
+
+def _forms():
+    """(loops, atoms, edge, shells, loops of each method): what the cases above
+    leave out."""
+    edge = (200000 / 0.08) ** (1.0 / 3.0)
+    rng = np.random.default_rng(4)
+    long = [_circle(30.0, c, rng.uniform(-40, 40, size=3), rng.normal(size=3), c) for c in (257, 600, 1100)]
+    mixed = _random_loops("line", 3, 20.0, edge, 1) + _random_loops("loopons", 2, 15.0, edge, 2)
+    e0 = (1000000 / 0.08) ** (1.0 / 3.0)
+    return {"open pieces": (long, 200000, edge, 2), "both methods": (mixed, 200000, edge, 1),
+            "no images": (_random_loops("line", 64, 6.0, e0, 3), 1000000, e0, 0),
+            "four shells": (_random_loops("line", 2, 15.0, edge, 5), 200000, edge, 4),
+            "eight shells": (_random_loops("line", 2, 10.0, 0.5 * edge, 6), 25000, 0.5 * edge, 8),
+            "eight shells, loopons": (_random_loops("loopons", 1, 6.0, 0.5 * edge, 7), 25000, 0.5 * edge, 8)}
+
+
+@pytest.mark.parametrize("name", ["open pieces", "both methods", "no images", "four shells", "eight shells",
+                                  "eight shells, loopons"])
+def test_other_forms_match_plain_sum(name):
+    """Lines of more than one piece (open ones), a plan with both methods, and the
+    ends of the range of shells.  Tolerance as above, its part for the plain sum's
+    own rounding with the square root of the terms it adds to an atom per loop,
+    from 48 segments and 125 images on."""
+    torch = pytest.importorskip("torch")
+    loops, atoms, edge, images = _forms()[name]
+    g = torch.Generator(device="cuda")
+    g.manual_seed(7)
+    pos = (torch.rand((3, atoms), dtype=torch.float64, device="cuda", generator=g) - 0.5) * edge
+    sums = []
+    for split in (1, 0):
+        plan = B.Plan(loops, (edge,) * 3, images=images, nu=0.3, image_split=split, max_atoms=atoms)
+        u = torch.zeros_like(pos)
+        plan.execute(pos, u)
+        if split == 0:
+            v = torch.zeros_like(pos)
+            names = _kernels(torch, lambda: plan.execute(pos, v))
+        plan.close()
+        sums.append(u)
+    kinds = len({lp.line for lp in loops})
+    assert sum("tree_node" in k for k in names) == kinds, names
+    terms = max(len(lp.vx) if lp.line else len(lp.x) for lp in loops)
+    growth = max(1.0, np.sqrt(terms / 48.0 * (2 * images + 1) ** 3 / 125.0))
+    base = 2e-14 if all(lp.line for lp in loops) else 2e-13
+    assert float((sums[0] - sums[1]).abs().max()) <= 2e-14 * len(loops) + base * growth
