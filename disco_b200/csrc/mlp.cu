@@ -22,9 +22,9 @@
 // Each CTA keeps its own partial gradient in global memory;
 // sum_kernel adds the partials in order, so a gradient is the same in every run.
 // The latency of one tile's chain of layers bounds a step (4096 rows are 32
-// tiles; the kernel issues on 15 % of the cycles, waiting for L2 and for
+// tiles; their SMs issue on 19 % of the cycles, waiting for L2 and for
 // barriers): 0.40 ms with one launch per product and reduction (18 launches),
-// 0.050 ms with this kernel (36 us alone; 50 with the weights converted in it), the
+// 0.050 ms with this kernel (37 us alone; 50 with the weights converted in it), the
 // sum (10 us) and Adam (4).
 //
 // Inputs are padded to 16 features and outputs to 16 (the MMA's N >= 16 for

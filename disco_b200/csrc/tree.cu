@@ -28,24 +28,27 @@
 //
 // theta(q): interpolation at q Chebyshev points converges like the Bernstein
 // ellipse's parameter to the power -q, and theta is where the measured worst
-// error over loops of 25 and 40 A radius, directions and cells of 12 to 30 A
-// half width falls below 4e-15 A for |b| = 2.5 A (plus 3 to 10 %), under the
-// rounding of the direct sum (1e-14 A).
+// truncation over loops of 25 and 40 A radius, directions and cells of 12 to 30 A
+// half width falls below 4e-15 A for |b| = 2.5 A (plus 3 to 10 %).  With the
+// rounding of the node values, which the weights of many nodes add up, q = 21
+// reaches 6e-15 A for loops as large as the cell and 1.2e-14 A for loops 60 times
+// as large; the direct sum's own rounding is 1e-14 A.
 //
-// FP64 tables only: the FP32 compensated form's own rounding (1e-6 A) is
-// part of what it returns, and its far terms summed in FP64 would change it.
+// FP64 tables only.  The FP32 compensated form would gain as well (FCC 40^3
+// cells, 12 loops, +-2: 25.1 -> 5.3 ms) and come closer to the exact sum (1.9e-6
+// -> 6e-7 A), but its results would move by up to 1.8e-6 A.
 //
 // Measured against the plain kernel on one B200 (ms a call): FCC 100^3 cells
 // (4.0 M atoms), 16 loops, +-2 images 986 -> 14.7; BCC 61 x 47 x 33 (184 k
 // atoms), 9 loops, +-3 76 -> 8.3; BCC 40^3 (128 k), 4 loops of 64 segments,
 // +-1 4.93 -> 3.10; loopons: BCC 40^3 (127 k), 8 prismatic loops of R 20 to 50
-// (39 k loopons), +-1 255 -> 57.  A sum too small to gain (2 000 atoms, 2 loops: 0.02 ms of
-// terms) stays with the plain kernel: tree_shape compares operation counts of
-// both, launches included.
+// (39 k loopons), +-1 255 -> 57.  A sum too small to gain stays with the plain
+// kernel (worth_cells).
 //
-// Every result is a fixed sequence of operations per atom (its cell's nodes,
-// then its near pairs in piece order), so it does not depend on the order of
-// the atoms or of the blocks.
+// The same atoms in the same order give the same bits, whatever the order of the
+// blocks.  In another order an atom can have other warp mates, which choose the
+// series of their near terms together, and the cells follow the bounding box and
+// the number of all atoms: then results agree to rounding.
 #include <algorithm>
 #include <cmath>
 #include <cstring>

@@ -16,7 +16,7 @@
 // time into shared memory, at the alignment of their place in the text, and
 // copies them out 16 bytes a thread: the text is written once, in whole
 // sectors (single bytes per thread to global memory: 352 us for 1.0 M atoms,
-// 45 MB; 49 us staged).
+// 45 MB; 50 us staged, bound by integer work).
 #include <algorithm>
 #include <cmath>
 #include <cstring>

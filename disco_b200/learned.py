@@ -189,8 +189,10 @@ def learned_displace(mlp, norm, pos, u, loops, box, nu, precision=C.DISCO_FP32C,
     (exact for the loops that miss the check).  The check's exact far shells
     are FP32 compensated by default: within about 1e-5 A of FP64 on a whole
     sum, two orders below the tolerances, at twice the FP64 rate (pass
-    check_precision=C.DISCO_FP64 for the plain FP64 sum).  Returns the report
-    as a dict."""
+    check_precision=C.DISCO_FP64 for the plain FP64 sum).  On large boxes
+    precision=C.DISCO_FP64 is the faster near shell, since it goes by cells (16
+    loops: 500 k atoms 7.8 ms against 14.9, 4.0 M atoms 17 against 111; 6 loops,
+    55 k atoms 1.6 against 0.9).  Returns the report as a dict."""
     lib = C.cuda_lib()
     arr, keep = B.loop_array(loops)
     b = (ctypes.c_double * 3)(*[float(v) for v in box])

@@ -42,7 +42,11 @@ extern "C" {
 /* ---- precision of the displacement sum ------------------------------------- */
 #define DISCO_FP64      0   /* plain drop-in: FP64 throughout                      */
 #define DISCO_FP32C     1   /* FP32 bulk on loop-centred coordinates, compensated
-                               sums over images and loops, FP64 image offsets     */
+                               sums over images and loops, FP64 image offsets;
+                               every term at every atom: twice the rate of the FP64
+                               sum term by term, but slower than FP64 wherever that
+                               goes by cells (disco_b200_plan_execute): 13.5 M atoms,
+                               64 loops, +-2 images 6.9 s against 73 ms            */
 
 /* ---- loop shapes (Code/loop.hpp:13) ----------------------------------------- */
 #define DISCO_SHAPE_CIRCLE         0
@@ -168,10 +172,14 @@ int disco_b200_displace(const disco_atoms *atoms, const disco_loop *loops, int32
  * plan_execute adds the field of every loop into DEVICE arrays on `stream`
  * (a cudaStream_t, NULL = legacy default stream) without any host copy.  An
  * FP64 plan large enough to gain sums its far pairs by cells (16 bytes of
- * scratch per atom and the cells' values, stream-ordered, from a pool that
- * keeps at most 32 MB, 1 GB while such a plan lives); without that scratch, or
- * under stream capture, the call sums term by term.  The two differ by the
- * rounding of the sum (3.6e-14 A at most where it was measured). */
+ * scratch per atom and the cells' values, stream-ordered, from a pool of the
+ * context that keeps at most 32 MB, 1 GB while such a plan lives); without that
+ * scratch the call sums term by term, and so does a call whose stream is being
+ * captured: a graph of 4 million atoms then replays some 70 times slower than
+ * the same call outside one.  The two sums differ by rounding (3.6e-14 A at most
+ * where it was measured).  The same atoms in the same order give the same bits
+ * in every call; in another order, or a part of them alone (a box split over
+ * ranks), they give the same sum to that rounding. */
 int disco_b200_plan_create(const disco_loop *loops, int32_t nloops, const double box[3],
                            const disco_options *opt, int64_t max_atoms, disco_plan **out);
 int disco_b200_plan_execute(disco_plan *plan, const disco_atoms *device_atoms, void *stream);
@@ -311,7 +319,8 @@ typedef struct {
  * max|n| < norm->image_min (opt->precision) plus the network's far shells
  * image_min <= max|n| <= norm->images, with the exact far-shell sum
  * (opt->check_precision: DISCO_FP64, or DISCO_FP32C, within about 1e-5 A of
- * FP64 on a whole sum and twice as fast) recomputed per loop on a random atom
+ * FP64 on a whole sum and, both being summed term by term there, twice as fast)
+ * recomputed per loop on a random atom
  * subsample every call and replacing the network for the loops that miss the
  * tolerances.
  * DEVICE atoms; the call returns when the work is done. */
