@@ -7,6 +7,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <exception>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -124,7 +125,11 @@ disco::TreeShape plan_tree(disco_plan* p, int k, int64_t n, cudaStream_t s)
     if (cap != cudaStreamCaptureStatusNone) return none;
     std::lock_guard<std::mutex> lock(p->tree_mutex);
     if (p->tree_n[k] != n) {
-        p->tree[k] = disco::tree_shape(p->tables[k], n, p->box, p->opt.images, p->sm_count);
+        try {
+            p->tree[k] = disco::tree_shape(p->tables[k], n, p->box, p->opt.images, p->sm_count);
+        } catch (const std::exception&) {        // no host memory for the choice: the plain kernel needs none
+            return none;
+        }
         p->tree_n[k] = n;
     }
     if (p->tree[k].use && !p->tree_pool) p->tree_pool = disco::scratch_retain(p->device);
@@ -190,7 +195,12 @@ ScratchPool* scratch_entry(int device)
     cudaMemPool_t pool = nullptr;
     if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) { cudaGetLastError(); return nullptr; }
     scratch_keep(pool, kScratchKeep);
-    g_scratch.push_back({ device, ctx, pool, 0 });
+    try {
+        g_scratch.push_back({ device, ctx, pool, 0 });
+    } catch (const std::exception&) {
+        cudaMemPoolDestroy(pool);
+        return nullptr;
+    }
     return &g_scratch.back();
 }
 
@@ -217,7 +227,12 @@ void give_stream(const IdleStream& s, bool healthy)
         // streams of a context that is gone are gone with it
         for (size_t k = g_idle.size(); k-- > 0;)
             if (g_idle[k].device == s.device && g_idle[k].ctx != s.ctx) g_idle.erase(g_idle.begin() + k);
-        if (g_idle.size() < kIdleStreams) { g_idle.push_back(s); return; }
+        if (g_idle.size() < kIdleStreams) {
+            try {
+                g_idle.push_back(s);
+                return;
+            } catch (const std::exception&) {}
+        }
     }
     cudaStreamDestroy(s.stream);
 }
