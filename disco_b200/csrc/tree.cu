@@ -1510,6 +1510,30 @@ TreeShape tree_shape(const HostTable& T, int64_t n, const double box[3], int ima
         const double q = kOrderQ[st[chain[k]].o];
         fair += st[chain[k]].cells * q * q * q * pairs(k) / gpu_lanes;
     }
+    // lanes per node of a line level: many images per source for each lane, or their
+    // uneven shares idle lanes (BCC 61 x 47 x 33, 9 loops, +-3: 8.69 ms with 6 images
+    // a lane, 8.27 with 48, 8.81 with one lane everywhere).  Where some lane's chain
+    // is over twice an even share, a small sum waits for it: then the level with the
+    // longest chain gets more lanes until none is over 1.8 shares (32 loops of R 13,
+    // 11 206 atoms, +-2: 9.7 ms without, 5.8 with; every level to 1.5 shares: sums of
+    // 30 000 atoms lose 4 to 9 %; only levels over two shares: 10 % of a sum whose
+    // next level is just below)
+    std::vector<int> lanes((size_t)S.levels, 1);
+    auto longest = [&] {
+        int worst = 0;
+        for (int k = 1; k < S.levels; ++k)
+            if (pairs(k) / lanes[k] > pairs(worst) / lanes[worst]) worst = k;
+        return worst;
+    };
+    if (line) {
+        const double loops = (double)roots.size();
+        for (int k = 0; k < S.levels; ++k)
+            while (lanes[k] < 32 && pairs(k) / loops >= 48.0 * lanes[k]) lanes[k] *= 2;
+        int k = longest();
+        if (pairs(k) / lanes[k] > 2.0 * fair)
+            for (; pairs(k) / lanes[k] > 1.8 * fair && lanes[k] < 32 && pairs(k) / loops >= 4.0 * lanes[k]; k = longest())
+                lanes[k] *= 2;
+    }
     for (int k = 0; k < S.levels; ++k) {
         const State& s = st[chain[k]];
         for (int d = 0; d < 3; ++d) S.m[k][d] = m0[d] << s.a;
@@ -1518,20 +1542,10 @@ TreeShape tree_shape(const HostTable& T, int64_t n, const double box[3], int ima
         S.cut[k] = s.cut;
         S.np[k] = s.np;
         S.eq[k] = s.eq;
-        // lanes per node: many images per source for each lane, or their uneven
-        // shares idle lanes (BCC 61 x 47 x 33, 9 loops, +-3: 8.69 ms with 6 images
-        // a lane, 8.27 with 48, 8.81 with one lane everywhere); fewer where one
-        // lane's chain would be longer than an even share of all levels' (32
-        // loops of R 13, 11 206 atoms, +-2: 9.68 ms without, 5.81 with)
-        const double per = pairs(k) / (double)roots.size();
         const int q3 = S.q[k] * S.q[k] * S.q[k];
-        int split = 1;
-        if (line) {
-            while (split < 32 && per >= 48.0 * split) split *= 2;
-            while (split < 32 && per >= 4.0 * split && pairs(k) / split > 1.5 * fair) split *= 2;
-        } else {
+        int split = lanes[k];
+        if (!line)
             while (split < 8 && s.cells * q3 * split < 300000.0) split *= 2;
-        }
         chosen.node_lanes += s.cells * q3 * split;
         chosen.node_scans += s.cells * q3 * split / 32.0 * s.np;
         S.split[k] = split;
