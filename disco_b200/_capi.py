@@ -156,6 +156,7 @@ def cuda_lib():
         _sig(lib, "disco_b200_plan_execute", c_int, [c_void_p, POINTER(DiscoAtoms), c_void_p])
         _sig(lib, "disco_b200_plan_sync", c_int, [c_void_p, c_void_p])
         _sig(lib, "disco_b200_plan_stats", c_int, [c_void_p, POINTER(DiscoPlanStats)])
+        _sig(lib, "disco_b200_plan_cells", c_int, [c_void_p, c_int64])
         _sig(lib, "disco_b200_plan_destroy", c_int, [c_void_p])
         _sig(lib, "disco_b200_batch", c_int,
              [POINTER(DiscoSample), c_int32, POINTER(DiscoOptions), POINTER(DiscoTiming)])

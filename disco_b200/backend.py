@@ -207,6 +207,10 @@ class Plan:
         C.check(self._lib.disco_b200_plan_stats(self._h, ctypes.byref(s)), self._lib)
         return {k: getattr(s, k) for k, _ in C.DiscoPlanStats._fields_}
 
+    def cells(self, n):
+        """Levels of cells by which n atoms are summed; 0: term by term."""
+        return int(self._lib.disco_b200_plan_cells(self._h, n))
+
     def execute_ptrs(self, x, y, z, ux, uy, uz, n, stream=0):
         a = C.DiscoAtoms(x, y, z, ux, uy, uz, n)
         C.check(self._lib.disco_b200_plan_execute(self._h, ctypes.byref(a), ctypes.c_void_p(stream)),

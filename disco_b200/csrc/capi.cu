@@ -116,13 +116,10 @@ void free_plan(disco_plan* p)
 // keeps to it (its launches allocate nothing), and so does a sum over far
 // shells alone (image_min > 0): that is the term-by-term sum the learned form
 // is measured and tested against, in error and in time.
-disco::TreeShape plan_tree(disco_plan* p, int k, int64_t n, cudaStream_t s)
+disco::TreeShape plan_shape(disco_plan* p, int k, int64_t n)
 {
     disco::TreeShape none;
     if (!p->tables[k].aux_tree || p->opt.image_split != 0 || p->opt.image_min > 0) return none;
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(s, &cap) != cudaSuccess) { cudaGetLastError(); return none; }
-    if (cap != cudaStreamCaptureStatusNone) return none;
     std::lock_guard<std::mutex> lock(p->tree_mutex);
     if (p->tree_n[k] != n) {
         try {
@@ -132,8 +129,22 @@ disco::TreeShape plan_tree(disco_plan* p, int k, int64_t n, cudaStream_t s)
         }
         p->tree_n[k] = n;
     }
-    if (p->tree[k].use && !p->tree_pool) p->tree_pool = disco::scratch_retain(p->device);
     return p->tree[k];
+}
+
+disco::TreeShape plan_tree(disco_plan* p, int k, int64_t n, cudaStream_t s)
+{
+    disco::TreeShape none;
+    if (!p->tables[k].aux_tree) return none;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &cap) != cudaSuccess) { cudaGetLastError(); return none; }
+    if (cap != cudaStreamCaptureStatusNone) return none;
+    const disco::TreeShape shape = plan_shape(p, k, n);
+    if (shape.use) {
+        std::lock_guard<std::mutex> lock(p->tree_mutex);
+        if (!p->tree_pool) p->tree_pool = disco::scratch_retain(p->device);
+    }
+    return shape;
 }
 
 double now_s()
@@ -636,6 +647,17 @@ int disco_b200_plan_stats(const disco_plan* p, disco_plan_stats* s)
     if (!p || !s) return fail(DISCO_EINVAL, "null argument");
     *s = p->stats;
     return DISCO_OK;
+}
+
+int disco_b200_plan_cells(disco_plan* p, int64_t n)
+{
+    if (!p || n <= 0) return 0;
+    int levels = 0;
+    for (int k = 0; k < 2; ++k) {
+        const disco::TreeShape shape = plan_shape(p, k, n);
+        if (shape.use) levels += shape.levels;
+    }
+    return levels;
 }
 
 int disco_b200_plan_destroy(disco_plan* p)

