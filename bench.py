@@ -147,10 +147,9 @@ def kernels_per_call(torch, fn):
 CELLS_PROFILE = {"fcc_random": "tree_fcc_large", "bcc_prismatic": "tree_bcc_loopons"}
 
 
-def field_roofline(torch, clk, fp64, evals, flop, seconds, kernels, workload, traffic=None):
-    """Roofline of a field launch of `evals` segment- or loopon-image terms, by the
-    names of the kernels that ran (None: not known, and no share of a peak is
-    claimed for an FP64 sum, which may have gone by cells)."""
+def field_roofline(torch, clk, fp64, evals, flop, seconds, cells, workload, traffic=None):
+    """Roofline of a field launch of `evals` segment- or loopon-image terms; cells:
+    the plan sums them by cells."""
     gemm = fp64_peak_tflops(torch) if fp64 else fp32_peak_tflops(torch)
     peak, src = pipe_peak_tflops(torch, clk, fp64)
     rate = evals * flop / seconds / 1e12
@@ -162,16 +161,12 @@ def field_roofline(torch, clk, fp64, evals, flop, seconds, kernels, workload, tr
                                  "not on the DFMA pipe this kernel uses") if fp64 else
                                 "torch SGEMM 8192^3 without TF32, best of 5",
             "flop_per_eval": flop, "evals_per_launch": evals}
-    cells = None if kernels is None else any("tree_node" in k for k in kernels)
-    if cells or (cells is None and fp64):
-        roof.update(achieved=None, frac=None, frac_of_gemm=None, term_by_term_equivalent=rate, traffic=None)
     if cells:
         name = CELLS_PROFILE.get(workload)
-        roof.update(form="far pairs by cells: most terms are never formed, so their rate is no share of a peak",
+        roof.update(achieved=None, frac=None, frac_of_gemm=None, term_by_term_equivalent=rate, traffic=None,
+                    form="far pairs by cells: most terms are never formed, so their rate is no share of a peak",
                     fp64_pipe_active=profile_value(name, "fp64_pipe_active") if name else None,
                     fp64_pipe_source=f"profiles/{name}.md: these kernels on a smaller box" if name else None)
-    elif cells is None and fp64:
-        roof.update(form="the profiler could not name the kernels: no share of a peak is claimed")
     return roof
 
 
@@ -847,7 +842,7 @@ def run_ours(args):
     if rank == 0:
         fp64 = prec == C.DISCO_FP64
         key = f"{'line' if w.method == 'line' else 'loopon'}_{args.precision}_{args.config}"
-        roof = field_roofline(torch, clk, fp64, evals_atom * n, flop_per_eval(w), per_launch, kernels, args.config,
+        roof = field_roofline(torch, clk, fp64, evals_atom * n, flop_per_eval(w), per_launch, plan.cells(n) > 0, args.config,
                               traffic_from_profiles(key))
         cpu = None
         parity = None
@@ -1385,7 +1380,7 @@ def run_prismatic(args, embedded=False):
             refgpu["ours"] = {"kernel_s": f0.elapsed_time(f1) * 1e-3,
                               "note": "this library's loopon field over the same survivors, nu 0.35"}
             del u35
-        roof = field_roofline(torch, clk, prec == C.DISCO_FP64, evals, W_LOOPON, per, kernels, "bcc_prismatic")
+        roof = field_roofline(torch, clk, prec == C.DISCO_FP64, evals, W_LOOPON, per, plan.cells(k) > 0, "bcc_prismatic")
         roof["kernel"] = "loopon field (the step also holds the matter step and epilogue)"
         line = {
             "metric": METRIC, "value": n * world / per, "unit": "atoms/s", "n_gpus": world,
